@@ -37,6 +37,7 @@ struct plato_graph {
   plato_graph_info info{};
   uint64_t stored_edges = 0;  // directed edges held in CSC/CSR
   bool relabeled = false;
+  bool own_sources = true;  // the columns' sources are this graph's vertices (not so for a partition)
 
   plato_b200::dbuf<uint64_t> in_off, out_off;
   plato_b200::dbuf<uint32_t> in_adj, out_adj;

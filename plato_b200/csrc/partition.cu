@@ -300,6 +300,7 @@ int build_partition(const plato_graph_info* info, const plato_vid_t* src, const 
   g->info.edges = off[n];
   g->info.max_v_i = n - 1;
   g->stored_edges = off[n];
+  g->own_sources = false;
   g->relabeled = true;  // rows sorted by descending in-degree: the binned pull plan applies
   PLATO_TRY(g->in_off.alloc(static_cast<size_t>(n) + 1));
   PLATO_TRY(g->in_adj.alloc(std::max<size_t>(adj.size(), 1)));

@@ -362,33 +362,20 @@ __global__ void __launch_bounds__(256) k_pull_short(pull_plan_view pv, const uin
   if (threadIdx.x == 0) partials[blockIdx.x] = dl;
 }
 
-// Device-side epoch control (the eps early exit of pagerank.hpp:137-139
-// without a host round trip).  ctrl[0] = mode of the next epoch (0 normal,
-// 1 final, 2 done), ctrl[1] = epochs run; delta[0] = last non-final delta
-// (scaled to the reference's units by `scale`).
+// Device-side epoch control without a host round trip (epoch_decide); `scale`
+// brings the delta to the reference's units.
 static __global__ void __launch_bounds__(1024) k_epoch_control(const double* __restrict__ partials,
                                                                uint32_t n, int* ctrl, double* delta,
                                                                double scale, double eps,
                                                                uint32_t iteration) {
   __shared__ double s_red[32];
-  const int mode = ctrl[0];
-  if (mode == 2) return;  // block-uniform
+  if (ctrl[0] == 2) return;  // block-uniform
   const uint32_t per = (n + 1023) / 1024;
   const uint32_t b = threadIdx.x * per, e = min(n, b + per);
   double s = 0.0;
   for (uint32_t i = b; i < e; ++i) s += partials[i];
   s = block_sum<1024>(s, s_red);
-  if (threadIdx.x == 0) {
-    const int ran = ctrl[1] + 1;
-    ctrl[1] = ran;
-    if (mode == 1) {
-      ctrl[0] = 2;
-    } else {
-      const double dlt = s * scale;
-      delta[0] = dlt;
-      if ((eps > 0.0 && dlt < eps) || static_cast<uint32_t>(ran) >= iteration - 1) ctrl[0] = 1;
-    }
-  }
+  if (threadIdx.x == 0) epoch_decide(ctrl, delta, s * scale, eps, iteration);
 }
 
 }  // namespace plato_b200

@@ -1,0 +1,501 @@
+// Builds the edge streams of the flat pull (pull_flat.cuh) on the device.
+#include <algorithm>
+#include <vector>
+
+#include <cub/device/device_scan.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
+
+#include "graph.cuh"
+#include "pull_flat.cuh"
+
+namespace plato_b200 {
+namespace {
+
+// Which edges are hot.  Rows above kFlatRowDeg0 in-edges take part in block 0,
+// rows above kFlatRowDeg1 in the further blocks: a segment costs a store and a
+// load of its sum, so it has to hold a few edges (RMAT s24, epoch: further
+// blocks above 32 / 48 / 64 / 96 / 128 in-edges 562 / 539 / 532 / 537 / 577 us;
+// block 0 above 4 / 8 / 16 / 32: 580 / 577 / 583 / 589).  Block 0 is used where
+// it holds kFlatFirst edges: below, one more launch and the copies of the
+// block cost what its gathers save (epoch without / with it: RMAT s18 20.6 /
+// 24.4 us, s19 32.4 / 33.4, s20 55.8 / 48.5).  A further block is used where it
+// holds kFlatMore edges, and one per row that takes part (RMAT s22 with 4 / 6 /
+// 10 / 16 blocks 153 / 144 / 138 / 144 us; s24 with 1 / 3 / 6 / 10 / 16 / 24:
+// 743 / 674 / 633 / 595 / 577 / 568).
+constexpr uint32_t kFlatRowDeg0 = 8;
+constexpr uint32_t kFlatRowDeg1 = 64;
+constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 600000;
+
+// out[0..1]: rows above the two in-degree limits; out[2 + k]: out-edges of block k.
+__global__ void __launch_bounds__(256) k_flat_survey(const uint32_t* __restrict__ in_deg,
+                                                     const uint32_t* __restrict__ out_deg, uint32_t V,
+                                                     uint32_t nblocks, unsigned long long* out) {
+  __shared__ unsigned long long s_red[32];
+  if (blockIdx.x == 0 && threadIdx.x < 2) {
+    const uint32_t limit = threadIdx.x == 0 ? kFlatRowDeg0 : kFlatRowDeg1;
+    uint32_t lo = 0, hi = V;
+    while (lo < hi) {
+      const uint32_t mid = lo + (hi - lo) / 2;
+      if (in_deg[mid] > limit) lo = mid + 1; else hi = mid;
+    }
+    out[threadIdx.x] = lo;
+  }
+  // 8 CTAs a block of sources
+  const uint32_t k = blockIdx.x / 8, q = blockIdx.x % 8;
+  if (k >= nblocks) return;
+  const uint32_t b = k * kFlatBlock, e = min(V, b + kFlatBlock);
+  unsigned long long n = 0;
+  for (uint32_t v = b + q * 256 + threadIdx.x; v < e; v += 8 * 256) n += out_deg[v];
+  n = block_sum_u64<256>(n, s_red);
+  if (threadIdx.x == 0) atomicAdd(out + 2 + k, n);
+}
+
+// Whether the columns are in order of descending in-degree.
+__global__ void k_flat_unsorted(const uint32_t* __restrict__ deg, uint32_t V, uint32_t* bad) {
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x + 1; v < V;
+       v += (uint64_t)gridDim.x * blockDim.x)
+    if (deg[v] > deg[v - 1]) *bad = 1;
+}
+
+struct flat_rows {
+  const uint64_t* off;
+  const uint32_t* adj;
+  uint32_t V, nb, r0, r1, rows1;  // rows1: r1 rounded up to whole 32-row words
+  // hot streams that row v takes part in
+  __device__ __forceinline__ uint32_t streams(uint32_t v) const {
+    return v < r1 ? nb : v < r0 ? min(nb, 1u) : 0u;
+  }
+  __device__ __forceinline__ uint64_t cell(uint32_t k, uint32_t v) const { return flat_place(k, V, rows1) + v; }
+};
+
+// cnt[cell(k, v)] = edges of row v in stream k.
+__global__ void k_flat_split(flat_rows f, uint32_t* cnt) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < f.V;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t v = static_cast<uint32_t>(i);
+    uint64_t pos = f.off[v];
+    const uint64_t end = f.off[v + 1];
+    const uint32_t ns = f.streams(v);
+    for (uint32_t k = 0; k < f.nb; ++k) {
+      if (k > 0 && v >= f.rows1) break;
+      uint64_t lo = pos;
+      if (k < ns) {
+        const uint32_t bound = (k + 1) * kFlatBlock;
+        uint64_t hi = end;
+        while (lo < hi) {
+          const uint64_t mid = (lo + hi) >> 1;
+          if (f.adj[mid] < bound) lo = mid + 1; else hi = mid;
+        }
+      }
+      cnt[f.cell(k, v)] = static_cast<uint32_t>(lo - pos);
+      pos = lo;
+    }
+    cnt[f.cell(f.nb, v)] = static_cast<uint32_t>(end - pos);
+  }
+}
+
+struct flat_starts {
+  uint32_t edge[kFlatMaxBlocks + 1];  // first edge of each stream (padded numbering)
+  uint32_t sum[kFlatMaxBlocks + 1];   // edges of the streams before it (unpadded)
+};
+
+// Copies every edge (and its weight) to its stream and flags segment ends.  A
+// warp takes a merge tile of the CSC; a lane finds its edge's row in the tile.
+__global__ void __launch_bounds__(256) k_flat_fill(flat_rows f, const uint32_t* __restrict__ trow,
+                                                   const uint64_t* __restrict__ tedge, uint32_t tiles,
+                                                   const uint32_t* __restrict__ cnt,
+                                                   const uint32_t* __restrict__ pos, flat_starts st,
+                                                   const float* __restrict__ w, uint16_t* hid, uint32_t* cid,
+                                                   float* hw, float* cw, uint32_t* hflags, uint32_t* cflags) {
+  const unsigned lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t cold0 = st.edge[f.nb];
+  for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tiles; t += nwarps) {
+    const uint32_t ra = trow[t], rb = min(trow[t + 1], f.V - 1);
+    const uint64_t je = tedge[t + 1];
+    for (uint64_t e = tedge[t] + lane; e < je; e += 32) {
+      uint32_t lo = ra, hi = rb;  // the last row of the tile that starts at or before e
+      while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo + 1) / 2;
+        if (f.off[mid] <= e) lo = mid; else hi = mid - 1;
+      }
+      const uint32_t v = lo;
+      const uint32_t id = f.adj[e];
+      const uint32_t ns = f.streams(v);
+      uint32_t k = id / kFlatBlock;
+      if (k >= ns) k = f.nb;
+      uint32_t before = 0;
+      for (uint32_t j = 0; j < min(k, ns); ++j) before += cnt[f.cell(j, v)];
+      const size_t at = f.cell(k, v);
+      const uint32_t i = static_cast<uint32_t>(e - f.off[v]) - before;
+      uint32_t to = st.edge[k] + (pos[at] - st.sum[k]) + i;
+      uint32_t* flags = hflags;
+      if (k < f.nb) {
+        hid[to] = static_cast<uint16_t>(id - k * kFlatBlock);
+        if (w) hw[to] = w[e];
+      } else {
+        to -= cold0;
+        flags = cflags;
+        cid[to] = id;
+        if (w) cw[to] = w[e];
+      }
+      if (i + 1 == cnt[at]) atomicOr(flags + (to >> 5), 1u << (to & 31));
+    }
+  }
+}
+
+// Rows with a segment, 32 at a time, and the ordinal of the first.
+__global__ void k_flat_meta(flat_rows f, const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ ord,
+                            uint32_t words, uint64_t total, uint4* meta) {
+  const unsigned lane = threadIdx.x & 31;
+  const uint32_t words1 = (f.rows1 + 31) / 32;
+  const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < total; i += nwarps) {
+    uint32_t k = 0, w = static_cast<uint32_t>(i);
+    if (i >= words) {
+      k = words1 ? static_cast<uint32_t>(min(static_cast<uint64_t>(f.nb), 1 + (i - words) / words1)) : f.nb;
+      w = static_cast<uint32_t>(i - flat_place(k, words, words1));
+    }
+    const uint32_t v = w * 32 + lane;
+    const bool has = v < f.V && cnt[f.cell(k, v)] != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, has);
+    if (lane == 0) meta[i] = make_uint4(m, ord[f.cell(k, w * 32)], 0u, 0u);
+  }
+}
+
+struct flat_has {
+  __host__ __device__ uint32_t operator()(uint32_t c) const { return c != 0 ? 1u : 0u; }
+};
+
+// The marks of each step from its flag bits, and the number of segments that
+// end in it; a warp per step, N edges a lane.
+template <int N, typename T>
+__global__ void k_flat_marks(const uint32_t* __restrict__ flags, uint32_t steps, T* marks, uint32_t* ends) {
+  const unsigned lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < steps; s += nwarps) {
+    const uint64_t e = static_cast<uint64_t>(s) * 32 * N + lane * N;
+    const uint32_t fl = (flags[e / 32] >> (e % 32)) & ((1u << N) - 1u);
+    const uint32_t n = __popc(fl);
+    uint32_t c = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xffffffffu, c, d);
+      if (static_cast<int>(lane) >= d) c += o;
+    }
+    marks[static_cast<size_t>(s) * 32 + lane] = static_cast<T>((c - n) << N | fl);
+    if (lane == 31) ends[s] = c;
+  }
+}
+
+struct flat_crossing {
+  const uint4* meta;
+  __device__ uint32_t operator()(uint32_t i) const { return __popc(meta[i].z); }
+};
+
+// Piece p continues a segment of an earlier piece; *j is its ordinal.
+__device__ __forceinline__ bool flat_continues(const flat_view& f, uint32_t p, uint32_t* j) {
+  const uint2 pc = f.pieces[p];
+  if ((pc.x & kPieceFirst) || pc.x >= pc.y) return false;
+  const size_t before = static_cast<size_t>(pc.x) * 32 - 1;
+  if (p < f.cold_piece0) {
+    if (f.hmark[before] >> (kFlatHotLane - 1) & 1u) return false;
+    *j = f.hseg[pc.x];
+  } else {
+    if (f.cmark[before] >> (kFlatColdLane - 1) & 1u) return false;
+    *j = f.cseg[pc.x];
+  }
+  return true;
+}
+
+// Segments cut by piece boundaries, one thread per piece; the first piece
+// that continues a segment records it.  fill = false marks the rows in
+// meta.z, fill = true writes the spans (meta.w scanned in between).
+template <bool kFill>
+__global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans) {
+  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t j = 0;
+  if (p >= npieces || !flat_continues(f, p, &j) || j >= segments) return;
+  uint32_t q = p - 1;  // the piece before that is not empty
+  while (f.pieces[q].x >= f.pieces[q].y && !(f.pieces[q].x & kPieceFirst)) --q;
+  uint32_t jq = 0;
+  if (flat_continues(f, q, &jq) && jq == j) return;
+  uint32_t last = p;
+  for (uint32_t r = p + 1; r < npieces; ++r) {
+    const uint2 pc = f.pieces[r];
+    if (pc.x & kPieceFirst) break;
+    if (pc.x >= pc.y) continue;
+    uint32_t jr = 0;
+    if (!flat_continues(f, r, &jr) || jr != j) break;
+    last = r;
+  }
+  // the row: the last word whose first ordinal is at most j
+  const uint64_t total = flat_place(f.nb, f.words, f.words1) + f.words;
+  uint64_t lo = 0, hi = total - 1;
+  while (lo < hi) {
+    const uint64_t mid = lo + (hi - lo + 1) / 2;
+    if (f.meta[mid].y <= j) lo = mid; else hi = mid - 1;
+  }
+  // the bit of the (j - first)-th segment of the word
+  uint32_t bits = f.meta[lo].x;
+  for (uint32_t n = j - f.meta[lo].y; n > 0; --n) bits &= bits - 1;
+  const uint32_t bit = bits & (0u - bits);
+  if (!kFill)
+    atomicOr(&meta[lo].z, bit);
+  else
+    spans[meta[lo].w + __popc(meta[lo].z & (bit - 1u))] = make_uint2(q, last);
+}
+
+__global__ void k_flat_span_base(const uint32_t* __restrict__ scan, uint64_t n, uint4* meta) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    meta[i].w = scan[i];
+}
+
+template <class It>
+int scan_u32(It in, uint32_t* out, uint64_t n, dbuf<uint8_t>& tmp, cudaStream_t st) {
+  size_t bytes = 0;
+  PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, static_cast<int64_t>(n), st));
+  PLATO_TRY(tmp.alloc(std::max<size_t>(bytes, 1)));
+  PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, in, out, static_cast<int64_t>(n), st));
+  count_launch();
+  return PLATO_OK;
+}
+
+template <typename T>
+int put(dbuf<T>& d, const std::vector<T>& h, cudaStream_t st) {
+  PLATO_TRY(d.alloc(std::max<size_t>(h.size(), 1)));
+  if (!h.empty())
+    PLATO_CUDA_TRY(cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+  return PLATO_OK;
+}
+
+}  // namespace
+
+int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
+  const uint32_t V = g->info.vertices;
+  const uint64_t E = g->stored_edges;
+  pl.valid = false;
+  if (!g->relabeled || !g->own_sources || E == 0 || E > 0xF0000000ull) return PLATO_OK;
+  const uint32_t nblocks = std::min<uint32_t>((V + kFlatBlock - 1) / kFlatBlock, kFlatMaxBlocks);
+  dbuf<unsigned long long> d_survey;
+  PLATO_TRY(d_survey.alloc(2 + kFlatMaxBlocks + 1));
+  PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, d_survey.bytes(), st));
+  k_flat_survey<<<nblocks * 8, 256, 0, st>>>(g->in_deg.p, g->out_deg.p, V, nblocks, d_survey.p);
+  PLATO_LAUNCHED("k_flat_survey");
+  k_flat_unsorted<<<grid_for(V, 256), 256, 0, st>>>(
+      g->in_deg.p, V, reinterpret_cast<uint32_t*>(d_survey.p + 2 + kFlatMaxBlocks));
+  PLATO_LAUNCHED("k_flat_unsorted");
+  unsigned long long h[2 + kFlatMaxBlocks + 1];
+  PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h[2 + kFlatMaxBlocks]) return PLATO_OK;  // another vertex order
+  flat_rows rows{g->in_off.p, g->in_adj.p, V, 0, static_cast<uint32_t>(h[0]), static_cast<uint32_t>(h[1]), 0};
+  uint32_t nb = 0;
+  if (h[2] >= kFlatFirst)
+    for (nb = 1; nb < nblocks && h[2 + nb] >= std::max(kFlatMore, h[1]) && h[1] > 0;) ++nb;
+  rows.nb = nb;
+  rows.rows1 = std::min((rows.r1 + 31) / 32 * 32, V);  // V: the last word may be short
+  const uint32_t streams = nb + 1, words = (V + 31) / 32, words1 = (rows.rows1 + 31) / 32;
+  const uint64_t cells = flat_place(nb, V, rows.rows1) + V;
+
+  dbuf<uint32_t> cnt, pos, ord;
+  dbuf<uint8_t> tmp;
+  PLATO_TRY(cnt.alloc(cells));
+  PLATO_TRY(pos.alloc(cells));
+  PLATO_TRY(ord.alloc(cells));
+  k_flat_split<<<grid_for(V, 256), 256, 0, st>>>(rows, cnt.p);
+  PLATO_LAUNCHED("k_flat_split");
+  PLATO_TRY(scan_u32(cnt.p, pos.p, cells, tmp, st));
+  PLATO_TRY(scan_u32(thrust::make_transform_iterator(cnt.p, flat_has()), ord.p, cells, tmp, st));
+  // edges before each stream, and the last cells for the number of segments
+  std::vector<uint32_t> sum(streams + 1, 0);
+  uint32_t last_cnt = 0, segments = 0;
+  for (uint32_t k = 0; k < streams; ++k)
+    PLATO_CUDA_TRY(cudaMemcpyAsync(&sum[k], pos.p + flat_place(k, V, rows.rows1), 4, cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaMemcpyAsync(&last_cnt, cnt.p + cells - 1, 4, cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaMemcpyAsync(&segments, ord.p + cells - 1, 4, cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  segments += last_cnt != 0;
+  sum[streams] = static_cast<uint32_t>(E);
+  flat_starts fs{};
+  uint32_t edges = 0;
+  for (uint32_t k = 0; k < streams; ++k) {
+    const uint32_t step = k < nb ? kFlatHotStep : kFlatColdStep;
+    fs.edge[k] = edges;
+    fs.sum[k] = sum[k];
+    edges += (sum[k + 1] - sum[k] + step - 1) / step * step;
+  }
+  const uint32_t hot_edges = fs.edge[nb], cold_edges = edges - hot_edges;
+  const uint32_t hot_steps = hot_edges / kFlatHotStep, cold_steps = cold_edges / kFlatColdStep;
+  const bool weighted = g->weighted;
+  PLATO_TRY(pl.hid.alloc(std::max<uint32_t>(hot_edges, 8)));
+  PLATO_TRY(pl.cid.alloc(std::max<uint32_t>(cold_edges, 8)));
+  if (weighted) {
+    PLATO_TRY(pl.hw.alloc(std::max<uint32_t>(hot_edges, 8)));
+    PLATO_TRY(pl.cw.alloc(std::max<uint32_t>(cold_edges, 8)));
+  }
+  dbuf<uint32_t> hflags, cflags;
+  PLATO_TRY(hflags.alloc(std::max<uint32_t>(hot_edges / 32, 1)));
+  PLATO_TRY(cflags.alloc(std::max<uint32_t>(cold_edges / 32, 1)));
+  PLATO_CUDA_TRY(cudaMemsetAsync(hflags.p, 0, hot_edges / 8, st));
+  PLATO_CUDA_TRY(cudaMemsetAsync(cflags.p, 0, cold_edges / 8, st));
+  // the padding of a stream's last step: source 0, weight 0, no flag
+  for (uint32_t k = 0; k < streams; ++k) {
+    const uint32_t end = k + 1 < streams ? fs.edge[k + 1] : edges;
+    if (end == fs.edge[k]) continue;
+    if (k < nb) {
+      PLATO_CUDA_TRY(cudaMemsetAsync(pl.hid.p + (end - kFlatHotStep), 0, kFlatHotStep * 2, st));
+      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(pl.hw.p + (end - kFlatHotStep), 0, kFlatHotStep * 4, st));
+    } else {
+      const uint32_t b = cold_edges - kFlatColdStep;
+      PLATO_CUDA_TRY(cudaMemsetAsync(pl.cid.p + b, 0, kFlatColdStep * 4, st));
+      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(pl.cw.p + b, 0, kFlatColdStep * 4, st));
+    }
+  }
+  const merge_tiles* mt = nullptr;
+  PLATO_TRY(ensure_pull_tiles(g, 224, st, &mt));
+  k_flat_fill<<<grid_for(static_cast<uint64_t>(mt->count) * 32, 256), 256, 0, st>>>(
+      rows, mt->row.p, mt->edge.p, mt->count, cnt.p, pos.p, fs, weighted ? g->in_w.p : nullptr, pl.hid.p,
+      pl.cid.p, pl.hw.p, pl.cw.p, hflags.p, cflags.p);
+  PLATO_LAUNCHED("k_flat_fill");
+  // marks, and segments that end before each step (numbered through all streams)
+  PLATO_TRY(pl.hmark.alloc(std::max<uint32_t>(hot_steps * 32, 1)));
+  PLATO_TRY(pl.cmark.alloc(std::max<uint32_t>(cold_steps * 32, 1)));
+  PLATO_TRY(pl.hseg.alloc(std::max<uint32_t>(hot_steps + cold_steps, 1)));
+  dbuf<uint32_t> ends;
+  PLATO_TRY(ends.alloc(std::max<uint32_t>(hot_steps + cold_steps, 1)));
+  if (hot_steps) {
+    k_flat_marks<kFlatHotLane, uint32_t><<<grid_for(hot_steps * 32ull, 256), 256, 0, st>>>(hflags.p, hot_steps,
+                                                                                           pl.hmark.p, ends.p);
+    PLATO_LAUNCHED("k_flat_marks");
+  }
+  if (cold_steps) {
+    k_flat_marks<kFlatColdLane, uint16_t><<<grid_for(cold_steps * 32ull, 256), 256, 0, st>>>(
+        cflags.p, cold_steps, pl.cmark.p, ends.p + hot_steps);
+    PLATO_LAUNCHED("k_flat_marks");
+  }
+  PLATO_TRY(scan_u32(ends.p, pl.hseg.p, hot_steps + cold_steps, tmp, st));
+  const uint64_t nmeta = flat_place(nb, words, words1) + words;
+  PLATO_TRY(pl.meta.alloc(nmeta));
+  k_flat_meta<<<grid_for(nmeta * 32, 256), 256, 0, st>>>(rows, cnt.p, ord.p, words, nmeta, pl.meta.p);
+  PLATO_LAUNCHED("k_flat_meta");
+
+  // Pieces: the hot steps split evenly over one CTA per SM, cut at block
+  // ends, each part split over the CTA's warps; the cold steps over all warps
+  // of the cold grid.
+  int sms = 0;
+  PLATO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
+  // Cost of the hot steps before each one: a step with segment ends costs
+  // about half as much again, and every end is a store.  (RMAT s24, k_flat_hot
+  // with the steps split evenly 291 us, by this cost 182.)
+  const uint32_t all_steps = hot_steps + cold_steps;
+  std::vector<uint32_t> seg(all_steps);
+  PLATO_CUDA_TRY(cudaMemcpyAsync(seg.data(), pl.hseg.p, all_steps * 4ull, cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  std::vector<float> cost(hot_steps + 1);
+  {
+    double c = 0.0;
+    for (uint32_t s = 0; s < hot_steps; ++s) {
+      cost[s] = static_cast<float>(c);
+      const uint32_t n = (s + 1 < all_steps ? seg[s + 1] : segments) - seg[s];
+      c += 1.0 + (n ? 0.5 : 0.0) + 0.01 * n;
+    }
+    cost[hot_steps] = static_cast<float>(c);
+  }
+  std::vector<uint2> pieces;
+  std::vector<flat_sub> subs;
+  std::vector<uint32_t> cta_sub;
+  auto add = [&pieces](uint32_t first, uint32_t a, uint32_t b) {
+    pieces.push_back(make_uint2(a == first ? a | kPieceFirst : a, b));
+  };
+  // first step in [lo, hi] whose cost is at least c
+  auto at_cost = [&cost](uint32_t lo, uint32_t hi, double c) {
+    return static_cast<uint32_t>(std::lower_bound(cost.begin() + lo, cost.begin() + hi, static_cast<float>(c)) -
+                                 cost.begin());
+  };
+  pl.hot_ctas = std::min<uint32_t>(sms, (hot_steps + kFlatHotWarps - 1) / kFlatHotWarps);
+  uint32_t a = 0;
+  for (uint32_t c = 0; c < pl.hot_ctas; ++c) {
+    cta_sub.push_back(static_cast<uint32_t>(subs.size()));
+    const uint32_t b = c + 1 == pl.hot_ctas ? hot_steps : at_cost(a, hot_steps, static_cast<double>(cost[hot_steps]) * (c + 1) / pl.hot_ctas);
+    for (uint32_t k = 0; k < nb; ++k) {
+      const uint32_t k0 = fs.edge[k] / kFlatHotStep, k1 = fs.edge[k + 1] / kFlatHotStep;
+      const uint32_t lo = std::max(a, k0), hi = std::min(b, k1);
+      if (lo >= hi) continue;
+      subs.push_back(flat_sub{k, static_cast<uint32_t>(pieces.size())});
+      uint32_t p0 = lo;
+      for (uint32_t w = 0; w < kFlatHotWarps; ++w) {
+        const uint32_t p1 = w + 1 == kFlatHotWarps ? hi : at_cost(p0, hi, cost[lo] + (static_cast<double>(cost[hi]) - cost[lo]) * (w + 1) / kFlatHotWarps);
+        add(k0, p0, p1);
+        p0 = p1;
+      }
+    }
+    a = b;
+  }
+  cta_sub.push_back(static_cast<uint32_t>(subs.size()));
+  const uint32_t cold_piece0 = static_cast<uint32_t>(pieces.size());
+  auto cut = [&](uint32_t n) {
+    for (uint32_t w = 0; w < n; ++w)
+      add(0, static_cast<uint32_t>(static_cast<uint64_t>(cold_steps) * w / n),
+          static_cast<uint32_t>(static_cast<uint64_t>(cold_steps) * (w + 1) / n));
+  };
+  const uint32_t per_block = kFlatColdThreads / 32;
+  pl.cold_blocks = 0;
+  if (cold_steps) {
+    // a wave of resident CTAs, and more (up to about five waves, so that the
+    // last one is short) while a warp keeps 8 steps
+    const uint32_t wave = sms * 5u, fill = cold_steps / (8 * per_block);
+    pl.cold_blocks = std::min<uint32_t>((cold_steps + per_block - 1) / per_block, std::min<uint32_t>(sms * 24u, std::max(wave, fill)));
+    cut(pl.cold_blocks * per_block);
+  }
+  const uint32_t npieces = static_cast<uint32_t>(pieces.size());
+  PLATO_TRY(put(pl.pieces, pieces, st));
+  PLATO_TRY(put(pl.subs, subs, st));
+  PLATO_TRY(put(pl.cta_sub, cta_sub, st));
+  PLATO_TRY(pl.part.alloc(std::max<uint32_t>(segments, 1)));
+  PLATO_TRY(pl.head.alloc(npieces));
+  PLATO_TRY(pl.carry.alloc(npieces));
+  PLATO_TRY(pl.spans.alloc(npieces));
+  flat_view& f = pl.v;
+  f = flat_view{};
+  f.V = f.nsrc = V;
+  f.nb = nb;
+  f.words = words;
+  f.words1 = words1;
+  f.cold_piece0 = cold_piece0;
+  f.cold_pieces = npieces - cold_piece0;
+  f.hid = pl.hid.p;
+  f.cid = pl.cid.p;
+  f.hw = pl.hw.p;
+  f.cw = pl.cw.p;
+  f.hmark = pl.hmark.p;
+  f.cmark = pl.cmark.p;
+  f.hseg = pl.hseg.p;
+  f.cseg = pl.hseg.p + hot_steps;
+  f.pieces = pl.pieces.p;
+  f.cta_sub = pl.cta_sub.p;
+  f.subs = pl.subs.p;
+  f.meta = pl.meta.p;
+  f.spans = pl.spans.p;
+  f.part = pl.part.p;
+  f.head = pl.head.p;
+  f.carry = pl.carry.p;
+  const unsigned span_grid = (npieces + 127) / 128;
+  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, pl.meta.p, nullptr);
+  PLATO_LAUNCHED("k_flat_spans");
+  dbuf<uint32_t> base;
+  PLATO_TRY(base.alloc(nmeta));
+  PLATO_TRY(scan_u32(thrust::make_transform_iterator(thrust::counting_iterator<uint32_t>(0), flat_crossing{pl.meta.p}),
+                     base.p, nmeta, tmp, st));
+  k_flat_span_base<<<grid_for(nmeta, 256), 256, 0, st>>>(base.p, nmeta, pl.meta.p);
+  PLATO_LAUNCHED("k_flat_span_base");
+  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, pl.meta.p, pl.spans.p);
+  PLATO_LAUNCHED("k_flat_spans");
+  pl.update_blocks = std::min<uint32_t>(sms * 4, (words + 15) / 16);
+  PLATO_CUDA_TRY(cudaStreamSynchronize(st));  // the temporaries and the host vectors go
+  pl.valid = true;
+  return PLATO_OK;
+}
+
+}  // namespace plato_b200

@@ -1,0 +1,454 @@
+// Flat pull: the pull gather as segmented sums over blocked edge streams.
+//
+// The sources [0, nb * kFlatBlock) of a relabelled graph are the most
+// gathered ones (descending in-degree; out-degree goes with it).  The in-edges
+// of a plan are split by source into nb hot streams, stream k holding the
+// edges whose source lies in block k = [k * kFlatBlock, (k+1) * kFlatBlock),
+// and one cold stream with the rest.  A stream is in row order; a row's edges
+// of one stream are a segment.  k_flat_hot copies a block's ranks to shared
+// memory (224 KB, one CTA of 32 warps per SM) and gathers there, with 16-bit
+// ids; k_flat_cold gathers from global memory with 32-bit ids;
+// k_flat_update adds each row's segment sums in stream order and applies the
+// rank update.
+//
+// A stream is cut into steps of 512 (hot) or 256 (cold) edges, 16 or 8 per
+// lane, and a warp walks a contiguous run of steps (a piece), so the work per
+// warp does not depend on the row lengths.  One flag bit per edge marks the last edge of a segment.
+// A step without a flag only adds to the lane's running sum; a step with
+// flags joins the lanes with a segmented scan and stores each finished
+// segment's sum at its ordinal in part[] (segments are numbered in stream
+// order, so the stores of a warp are consecutive).  A segment cut by a piece
+// boundary leaves its sums in carry[] and head[] of the pieces it crosses; the
+// update adds those in piece order.  Every sum has a fixed order: results are
+// the same from run to run.
+//
+// Why.  A gather of 4 random bytes costs an L2 request, and the chip answers
+// 276 G of them a second whatever the array's size (64 warps per SM, 4 to 16 in
+// flight a lane); L1 hits go at 560-790 G/s, shared memory at 1700 G/s.  RMAT
+// s24's 263M gathers are 0.95 ms of L2 requests; its hottest 57344 sources are
+// 46% of them, 24 blocks 90%.  RMAT s24, one PageRank epoch on one B200: 826 us
+// with the degree bins (pull_binned.cuh), 532 us here: k_flat_hot 210 us (210M
+// edges), k_flat_cold 229 (53M), k_flat_update 96.  RMAT s22 220 -> 138 us, s20
+// 98 -> 49, 16M uniform edges over 1M vertices 107 -> 82, 64M over 1M 303 -> 144.
+#pragma once
+
+#include "common.cuh"
+#include "pull_merge.cuh"
+
+struct plato_graph;
+
+namespace plato_b200 {
+
+constexpr int kFlatHotLane = 16;          // edges of a lane in a hot step
+constexpr int kFlatColdLane = 8;          // and in a cold step
+constexpr uint32_t kFlatHotStep = 32 * kFlatHotLane;
+constexpr uint32_t kFlatColdStep = 32 * kFlatColdLane;
+constexpr uint32_t kFlatBlock = 57344;    // sources of a hot block
+constexpr uint32_t kFlatMaxBlocks = 24;
+constexpr uint32_t kFlatHotWarps = 32;
+constexpr uint32_t kFlatColdThreads = 256;
+constexpr uint32_t kPieceFirst = 0x80000000u;  // a piece at the start of its stream
+
+// A part of one hot block that a CTA walks, its steps shared by its 32 warps.
+struct flat_sub {
+  uint32_t block, piece0;
+};
+
+struct flat_view {
+  uint32_t V, nsrc, nb, words;      // words = ceil(V / 32)
+  uint32_t words1;                  // 32-row words that take part in the hot streams after the first
+  uint32_t cold_piece0, cold_pieces;
+  const uint16_t* hid;              // hot ids, relative to their block
+  const uint32_t* cid;              // cold ids
+  const float* hw;                  // weights of the same edges, or null
+  const float* cw;
+  // a mark per lane and step: a bit per edge, set on the last of a segment,
+  // and above it the number of such bits in the step's lanes before
+  const uint32_t* hmark;            // 16 + 16 bits
+  const uint16_t* cmark;            // 8 + 8 bits
+  const uint32_t* hseg;             // segments that end before each step
+  const uint32_t* cseg;
+  const uint2* pieces;              // [pieces] first step | kPieceFirst, end step
+  const uint32_t* cta_sub;          // [hot CTAs + 1]
+  const flat_sub* subs;
+  // per stream and 32 rows (flat_place): rows with a segment, ordinal of the
+  // first, rows whose segment crosses pieces, index of the first of those in spans
+  const uint4* meta;
+  const uint2* spans;               // first and last piece of a crossing segment
+  float* part;                      // [segments]
+  float* head;                      // [pieces]
+  float* carry;                     // [pieces]
+};
+
+// Place of stream k in arrays by stream and row (or 32-row word): every row
+// for the first and the last stream, `rows1` for those between.
+__host__ __device__ inline uint64_t flat_place(uint32_t k, uint64_t rows, uint64_t rows1) {
+  return k == 0 ? 0 : rows + (k - 1) * rows1;
+}
+
+struct flat_plan {
+  bool valid = false;
+  uint32_t hot_ctas = 0, cold_blocks = 0, update_blocks = 0;
+  flat_view v{};
+  dbuf<uint16_t> hid, cmark;
+  dbuf<uint32_t> cid, hmark, hseg, cseg, cta_sub;
+  dbuf<float> hw, cw, part, head, carry;
+  dbuf<uint2> pieces, spans;
+  dbuf<flat_sub> subs;
+  dbuf<uint4> meta;
+};
+
+// Builds the plan of g's pull on `st` (pull_flat.cu); plan.valid stays false
+// where the degree bins are the better kernels.
+int build_flat_plan(plato_graph* g, flat_plan& plan, cudaStream_t st);
+
+__device__ __forceinline__ void flat_prefetch(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// 32 consecutive bytes in one load, so that a warp's ids are read once.  The
+// streams are read once an epoch and pass L1 and L2 by.
+struct flat_words {
+  uint32_t w[8];
+};
+template <bool kOnce>
+__device__ __forceinline__ void flat_load(const void* p, flat_words& r) {
+  if constexpr (kOnce)
+    asm volatile("ld.global.nc.L1::no_allocate.L2::evict_first.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]),
+                   "=r"(r.w[7])
+                 : "l"(p));
+  else
+    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]),
+                   "=r"(r.w[7])
+                 : "l"(p));
+}
+
+// A lane's weights of one step, multiplied into its values.
+template <bool kOnce, int N>
+__device__ __forceinline__ void flat_weigh(const float* w, float (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 8) {
+    flat_words t;
+    flat_load<kOnce>(w + i, t);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[i + k] *= __uint_as_float(t.w[k]);
+  }
+}
+
+// The edges of a lane in one step, hot: 16-bit ids into shared memory.
+template <bool kW>
+struct flat_hot_gather {
+  static constexpr int kLane = kFlatHotLane;
+  static constexpr uint32_t kAhead = 6;  // steps whose ids are on their way to L2
+  const uint16_t* ids;
+  const float* w;
+  const uint32_t* marks;
+  const uint32_t* seg;
+  const float* xs;
+  using regs = flat_words;
+  __device__ __forceinline__ void ahead(uint32_t step, unsigned lane) const {
+    const size_t e = static_cast<size_t>(step) * kFlatHotStep;
+    if (lane < 8) flat_prefetch(ids + e + lane * 64);
+    if (lane == 8) flat_prefetch(marks + static_cast<size_t>(step) * 32);
+    if (kW && lane >= 16) flat_prefetch(w + e + (lane - 16) * 32);
+  }
+  __device__ __forceinline__ void load(uint32_t step, unsigned lane, regs& r) const {
+    flat_load<true>(ids + static_cast<size_t>(step) * kFlatHotStep + lane * kLane, r);
+  }
+  __device__ __forceinline__ uint32_t mark(uint32_t step, unsigned lane) const {
+    return __ldcs(marks + static_cast<size_t>(step) * 32 + lane);
+  }
+  __device__ __forceinline__ void values(uint32_t step, unsigned lane, const regs& r, float (&v)[kLane]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[2 * i] = xs[r.w[i] & 0xFFFFu];
+      v[2 * i + 1] = xs[r.w[i] >> 16];
+    }
+    if constexpr (kW) flat_weigh<true>(w + static_cast<size_t>(step) * kFlatHotStep + lane * kLane, v);
+  }
+};
+
+// Cold: 32-bit ids into global memory.
+template <bool kW>
+struct flat_cold_gather {
+  static constexpr int kLane = kFlatColdLane;
+  static constexpr uint32_t kAhead = 4;
+  const uint32_t* ids;
+  const float* w;
+  const uint16_t* marks;
+  const uint32_t* seg;
+  const float* x;
+  using regs = flat_words;
+  __device__ __forceinline__ void ahead(uint32_t step, unsigned lane) const {
+    const size_t e = static_cast<size_t>(step) * kFlatColdStep;
+    if (lane < 8) flat_prefetch(ids + e + lane * 32);
+    if (lane == 8) flat_prefetch(marks + static_cast<size_t>(step) * 32);
+    if (kW && lane >= 16 && lane < 24) flat_prefetch(w + e + (lane - 16) * 32);
+  }
+  __device__ __forceinline__ void load(uint32_t step, unsigned lane, regs& r) const {
+    flat_load<true>(ids + static_cast<size_t>(step) * kFlatColdStep + lane * kLane, r);
+  }
+  __device__ __forceinline__ uint32_t mark(uint32_t step, unsigned lane) const {
+    const uint16_t* p = marks + static_cast<size_t>(step) * 32 + lane;
+    return __ldcs(p);
+  }
+  __device__ __forceinline__ void values(uint32_t step, unsigned lane, const regs& r, float (&v)[kLane]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __ldg(x + r.w[i]);
+    if constexpr (kW) flat_weigh<true>(w + static_cast<size_t>(step) * kFlatColdStep + lane * kLane, v);
+  }
+};
+
+// A store that a lane skips without leaving its warp.
+__device__ __forceinline__ void flat_store_if(uint32_t on, float* p, float v) {
+  asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.global.f32 [%1], %2; }" ::"r"(on), "l"(p), "f"(v)
+               : "memory");
+}
+
+// One warp's walk over the steps of piece p.
+template <class Gather>
+__device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const Gather& g) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int N = Gather::kLane;
+  constexpr uint32_t kEnds = (1u << N) - 1u;
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const uint2 pc = f.pieces[p];
+  const uint32_t s0 = pc.x & ~kPieceFirst, s1 = pc.y;
+  if (s0 >= s1) {
+    if (lane == 0) f.carry[p] = 0.f;
+    return;
+  }
+  typename Gather::regs cur;
+  g.load(s0, lane, cur);
+  uint32_t mark = g.mark(s0, lane);
+  uint32_t base = __ldg(g.seg + s0);
+  if constexpr (Gather::kAhead > 0)
+    for (uint32_t s = s0 + 1; s < min(s1, s0 + Gather::kAhead); ++s) g.ahead(s, lane);
+  const bool open =
+      !(pc.x & kPieceFirst) && !(__ldg(g.marks + static_cast<size_t>(s0) * 32 - 1) & (1u << (N - 1)));
+  const uint32_t j0 = open ? base : 0xffffffffu;  // the segment that began in an earlier piece
+  float acc = 0.f;       // this lane's part of the open segment, from steps without an end
+  float carry = 0.f;     // the open segment's sum before those, the same in every lane
+  for (uint32_t s = s0; s < s1; ++s) {
+    float v[N];
+    g.values(s, lane, cur, v);
+    uint32_t mark_n = 0, base_n = 0;
+    if (s + 1 < s1) {
+      g.load(s + 1, lane, cur);
+      mark_n = g.mark(s + 1, lane);
+      base_n = __ldg(g.seg + s + 1);
+    }
+    if constexpr (Gather::kAhead > 0)
+      if (s + Gather::kAhead < s1) g.ahead(s + Gather::kAhead, lane);
+    const uint32_t fl = mark & kEnds;
+    const unsigned ends = __ballot_sync(kAll, fl != 0);
+    if (ends == 0) {
+#pragma unroll
+      for (int i = 0; i < N; i += 8)
+        acc += ((v[i] + v[i + 1]) + (v[i + 2] + v[i + 3])) + ((v[i + 4] + v[i + 5]) + (v[i + 6] + v[i + 7]));
+    } else {
+      // this lane's sum after its last segment end, joined over the lanes
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        t += v[i];
+        t = (fl >> i) & 1u ? 0.f : t;
+      }
+      const unsigned le = ends & (kAll >> (31 - lane));
+      const int lo = le ? 31 - __clz(le) : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const float o = __shfl_up_sync(kAll, t, d);
+        if (static_cast<int>(lane) - d >= lo) t += o;
+      }
+      carry += warp_sum(acc);
+      acc = 0.f;
+      float run = __shfl_up_sync(kAll, t, 1);
+      if (lane == 0) run = 0.f;
+      if (!(ends & below)) run += carry;
+      carry = __shfl_sync(kAll, t, 31);
+      // the segments that end here; a step of several pieces' segment goes to head
+      const uint32_t ord = base + (mark >> N);
+      float* to = f.part + ord;
+      if (ord == j0 && fl) {
+        // its first end closes a segment of an earlier piece
+        const int e = __ffs(fl) - 1;
+        float h = run;
+#pragma unroll
+        for (int i = 0; i < N; ++i) h += i <= e ? v[i] : 0.f;
+        f.head[p] = h;
+      }
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        run += v[i];
+        const uint32_t on = fl & (1u << i);
+        flat_store_if(on, to, run);
+        to += on ? 1 : 0;
+        run = on ? 0.f : run;
+      }
+    }
+    mark = mark_n;
+    base = base_n;
+  }
+  acc = warp_sum(acc);
+  if (lane == 0) f.carry[p] = carry + acc;
+}
+
+// Hot streams (bound by issue: about 300 instructions a step of 512 edges, and
+// 3.4-way bank conflicts): CTA c walks its parts [cta_sub[c], cta_sub[c+1]), each within
+// one block whose ranks it first copies to shared memory.
+template <bool kW>
+__global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_hot(flat_view f, const float* __restrict__ x,
+                                                                   const int* mode) {
+  extern __shared__ float4 s_x4[];
+  if (mode && *mode == 2) return;
+  const uint32_t sub1 = f.cta_sub[blockIdx.x + 1];
+  for (uint32_t sub = f.cta_sub[blockIdx.x]; sub < sub1; ++sub) {
+    const flat_sub sb = f.subs[sub];
+    const uint32_t src0 = sb.block * kFlatBlock;
+    const uint32_t n = min(kFlatBlock, f.nsrc - src0);
+    __syncthreads();
+    const float4* x4 = reinterpret_cast<const float4*>(x + src0);
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < n / 4; i += kFlatHotWarps * 32) s_x4[i] = __ldg(x4 + i);
+    if (threadIdx.x < n % 4)
+      reinterpret_cast<float*>(s_x4)[n / 4 * 4 + threadIdx.x] = __ldg(x + src0 + n / 4 * 4 + threadIdx.x);
+    __syncthreads();
+    const flat_hot_gather<kW> g{f.hid, f.hw, f.hmark, f.hseg, reinterpret_cast<const float*>(s_x4)};
+    flat_piece(f, sb.piece0 + (threadIdx.x >> 5), g);
+  }
+}
+
+// The cold stream, bound by L2 requests.
+template <bool kW>
+__global__ void __launch_bounds__(kFlatColdThreads, 5) k_flat_cold(flat_view f, const float* __restrict__ x,
+                                                                   const int* mode) {
+  if (mode && *mode == 2) return;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w >= f.cold_pieces) return;
+  const flat_cold_gather<kW> g{f.cid, f.cw, f.cmark, f.cseg, x};
+  flat_piece(f, f.cold_piece0 + w, g);
+}
+
+// The sums of one 32-row word's segments of a stream: lane l gets row l's.
+__device__ __forceinline__ float flat_segment(const flat_view& f, const uint4& m, unsigned lane) {
+  const unsigned below = (1u << lane) - 1u;
+  if (!((m.x >> lane) & 1u)) return 0.f;
+  if (!((m.z >> lane) & 1u)) return __ldcg(f.part + m.y + __popc(m.x & below));
+  const uint2 sp = __ldg(f.spans + m.w + __popc(m.z & below));
+  float y = 0.f;
+  for (uint32_t p = sp.x; p < sp.y; p += 4) {  // 4 loads in flight
+    float t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = p + i < sp.y ? __ldcg(f.carry + p + i) : 0.f;
+    y += (t[0] + t[1]) + (t[2] + t[3]);
+  }
+  return y + __ldcg(f.head + sp.y);
+}
+
+__device__ __forceinline__ uint4 flat_shfl(const uint4& m, int l) {
+  return make_uint4(__shfl_sync(0xffffffffu, m.x, l), __shfl_sync(0xffffffffu, m.y, l),
+                    __shfl_sync(0xffffffffu, m.z, l), __shfl_sync(0xffffffffu, m.w, l));
+}
+
+// The sums of the hot streams between the first and the cold one, for the 32
+// rows of word w.
+__device__ __forceinline__ float flat_middle(const flat_view& f, uint32_t w, unsigned lane) {
+  float y = 0.f;
+  uint4 mk = make_uint4(0, 0, 0, 0);  // lane k holds the meta of stream k + 1
+  if (lane + 1 < f.nb) mk = __ldg(f.meta + f.words + static_cast<size_t>(lane) * f.words1 + w);
+  for (uint32_t k = 0; k + 1 < f.nb; k += 4) {
+    float t[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = flat_segment(f, flat_shfl(mk, k + i), lane);  // streams past nb: empty
+    y += (t[0] + t[1]) + (t[2] + t[3]);
+  }
+  return y;
+}
+
+// Adds each row's segment sums, in stream order, and applies the update.  A
+// warp takes two words of 32 rows at a time, nwarps apart, and loads the metas
+// of its next two one round ahead: the sums' loads wait for the metas, and
+// what bounds the kernel is how many of them are in flight.
+// With c.ctrl the last CTA to finish sums the partials in a fixed order and
+// takes the epoch decision (epoch_decide).
+struct flat_control {
+  int* ctrl;       // [0] mode of the next epoch, [1] epochs run, [2] CTAs that finished
+  double* delta;
+  double scale, eps;
+  uint32_t iteration;
+};
+
+template <class Update>
+__global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd, double* partials, flat_control c) {
+  constexpr int R = 2;
+  __shared__ double s_red[32];
+  __shared__ bool s_last;
+  if (upd.skip()) return;
+  const unsigned lane = threadIdx.x & 31;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint4* cold = f.meta + flat_place(f.nb, f.words, f.words1);
+  double dl = 0.0;
+  uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  uint4 m0[R], m1[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint32_t wr = w + r * nwarps;
+    m0[r] = f.nb && wr < f.words ? __ldg(f.meta + wr) : make_uint4(0, 0, 0, 0);
+    m1[r] = wr < f.words ? __ldg(cold + wr) : make_uint4(0, 0, 0, 0);
+  }
+  for (; w < f.words; w += R * nwarps) {
+    typename Update::operands ops[R];
+    float y[R], z[R];
+    uint4 n0[R], n1[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t v = (w + r * nwarps) * 32 + lane;
+      ops[r] = upd.load(v < f.V ? v : 0u);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t wr = w + (R + r) * nwarps;
+      n0[r] = f.nb && wr < f.words ? __ldg(f.meta + wr) : make_uint4(0, 0, 0, 0);
+      n1[r] = wr < f.words ? __ldg(cold + wr) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      y[r] = flat_segment(f, m0[r], lane);
+      z[r] = flat_segment(f, m1[r], lane);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t wr = w + r * nwarps, v = wr * 32 + lane;
+      if (wr < f.words1) y[r] += flat_middle(f, wr, lane);
+      y[r] += z[r];
+      if (wr < f.words && v < f.V) dl += upd.apply(v, y[r], ops[r]);
+      m0[r] = n0[r];
+      m1[r] = n1[r];
+    }
+  }
+  dl = block_sum<256>(dl, s_red);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = dl;
+    if (c.ctrl) {
+      __threadfence();
+      s_last = atomicAdd(c.ctrl + 2, 1) == static_cast<int>(gridDim.x) - 1;
+    }
+  }
+  if (!c.ctrl) return;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double t = 0.0;
+  for (uint32_t i = threadIdx.x; i < gridDim.x; i += 256) t += __ldcg(partials + i);
+  t = block_sum<256>(t, s_red);
+  if (threadIdx.x == 0) {
+    c.ctrl[2] = 0;
+    epoch_decide(c.ctrl, c.delta, t * c.scale, c.eps, c.iteration);
+  }
+}
+
+}  // namespace plato_b200

@@ -40,10 +40,25 @@ struct teleport_seeds {  // trustrank.hpp:226-245: (seed ? (1-d)/|S| : 0)
   }
 };
 
+// The eps early exit of pagerank.hpp:137-139 after an epoch whose delta is
+// `delta`: ctrl[0] = mode of the next epoch (0 normal, 1 final, 2 done),
+// ctrl[1] = epochs run, *last_delta = delta of the last non-final epoch.
+__device__ __forceinline__ void epoch_decide(int* ctrl, double* last_delta, double delta, double eps,
+                                             uint32_t iteration) {
+  const int mode = ctrl[0], ran = ctrl[1] + 1;
+  ctrl[1] = ran;
+  if (mode == 1) {
+    ctrl[0] = 2;
+    return;
+  }
+  *last_delta = delta;
+  if ((eps > 0.0 && delta < eps) || static_cast<uint32_t>(ran) >= iteration - 1) ctrl[0] = 1;
+}
+
 template <class Teleport>
 struct rank_update {
-  const float* __restrict__ x;    // current state
-  float* __restrict__ xn;         // next state
+  const float* x;                 // current state
+  float* xn;                      // next state
   const uint32_t* __restrict__ deg;
   Teleport tele;
   float d;

@@ -17,6 +17,7 @@
 #include "profile.cuh"
 #include "pull_merge.cuh"
 #include "pull_binned.cuh"
+#include "pull_flat.cuh"
 #include "pull_warp.cuh"
 #include "push.cuh"
 
@@ -47,15 +48,19 @@ struct rank_workspace {
   uint32_t hub_cap = 0;       // ranks the pull kernel can stage in shared memory
   bool plan_built = false;
   pull_plan plan;
+  flat_plan flat;
   dbuf<uint32_t> seed_bits, seed_list;  // seed-set PPR
   dbuf<float> out_stage;                // caller-id ranks before the copy to the host
   dbuf<int> ctrl;                       // device epoch control (k_epoch_control)
   double* h_delta = nullptr;  // pinned
-  int* h_ctrl = nullptr;      // pinned [2]
+  int* h_ctrl = nullptr;      // pinned [8]: two control words
+  cudaEvent_t polled[2] = {nullptr, nullptr};  // control words copied to h_ctrl
   push_frontier frontier;
   ~rank_workspace() {
     if (h_delta) cudaFreeHost(h_delta);
     if (h_ctrl) cudaFreeHost(h_ctrl);
+    for (cudaEvent_t e : polled)
+      if (e) cudaEventDestroy(e);
   }
 };
 
@@ -75,31 +80,32 @@ using cfg = pull_warp_cfg<kIPT>;
 // A vertex whose out-weights sum to 0 gets x' = inf, so its edges give
 // inf * 0 = NaN, as the reference's 0 / 0 does.
 struct wrank_update {
-  const float* __restrict__ r;     // current ranks
-  float* __restrict__ rn;          // next ranks
-  float* __restrict__ xn;          // next gathered state
+  const float* r;                  // current ranks
+  float* rn;                       // next ranks
+  float* xn;                       // next gathered state
   const float* __restrict__ wsum;  // v_weight_sum
   float base;                      // 1 - d
   float d;
   int final_epoch;
+  const int* mode = nullptr;  // epoch kind on the device, as in rank_update
 
-  __device__ __forceinline__ bool skip() const { return false; }
+  __device__ __forceinline__ bool skip() const { return mode && *mode == 2; }
+  __device__ __forceinline__ bool storing_rank() const { return mode ? (*mode == 1) : (final_epoch != 0); }
 
   struct operands {
     float ro;
     float ws;
   };
   __device__ __forceinline__ operands load(uint32_t v) const {
-    if (final_epoch) return {0.f, 1.f};
+    if (storing_rank()) return {0.f, 1.f};
     return {__ldcs(r + v), __ldcs(wsum + v)};
   }
-
   __device__ __forceinline__ double apply(uint32_t v, float y) const { return apply(v, y, load(v)); }
 
   __device__ __forceinline__ double apply(uint32_t v, float y, operands o) const {
     const float rv = fmaf(d, y, base);
     rn[v] = rv;
-    if (final_epoch) return 0.0;
+    if (storing_rank()) return 0.0;
     xn[v] = rv / o.ws;
     return static_cast<double>(fabsf(rv - o.ro));
   }
@@ -245,7 +251,8 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
   rank_workspace* ws = g->rank_ws;
   const uint32_t V = g->info.vertices;
   if (!ws->plan_built) {
-    PLATO_TRY(build_plan(g, ws->plan, st));
+    PLATO_TRY(build_flat_plan(g, ws->flat, st));
+    if (!ws->flat.valid) PLATO_TRY(build_plan(g, ws->plan, st));
     ws->plan_built = true;
   }
   PLATO_TRY(ensure_pull_tiles(g, cfg::kItems, st));
@@ -262,11 +269,16 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
   // pull epochs: one partial per CTA + one per fixup block (merge path) or one
   // per block of each bin kernel; dense epochs up to 148 * 8
   PLATO_TRY(ws->partials.alloc(std::max<size_t>(
-      {ws->sms + (W + 255) / 256 + 1, static_cast<size_t>(ws->plan.partials()) + 1, 148 * 8})));
+      {ws->sms + (W + 255) / 256 + 1, static_cast<size_t>(ws->plan.partials()) + 1,
+       static_cast<size_t>(ws->flat.update_blocks) + 1, 148 * 8})));
   PLATO_TRY(ws->delta.alloc(1));
-  PLATO_TRY(ws->ctrl.alloc(2));
+  PLATO_TRY(ws->ctrl.alloc(4));
   if (!ws->h_delta) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_delta), sizeof(double)));
-  if (!ws->h_ctrl) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_ctrl), 2 * sizeof(int)));
+  if (!ws->h_ctrl) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_ctrl), 8 * sizeof(int)));
+  for (cudaEvent_t& e : ws->polled)
+    if (!e) PLATO_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlatBlock * 4));
+  PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlatBlock * 4));
   uint32_t cap_a = 0, cap_b = 0;
   PLATO_TRY(set_pull_smem_attr<rank_update<teleport_uniform>>(g->device, &cap_a));
   PLATO_TRY(set_pull_smem_attr<rank_update<teleport_single>>(g->device, &cap_b));
@@ -303,13 +315,35 @@ __global__ void k_init_single(const uint32_t* __restrict__ deg, uint32_t V, uint
   }
 }
 
-// One pull epoch gathering x (times the edge weights w when kW) with the
-// fused update `upd`: the degree bins on a relabelled graph, else the
-// persistent warp-tile merge path + cross-range fixup.  Partial deltas go to
-// ws->partials (one per CTA of each kernel).
+int partial_count(const plato_graph* g) {
+  if (g->rank_ws->flat.valid) return static_cast<int>(g->rank_ws->flat.update_blocks);
+  if (g->rank_ws->plan.valid) return static_cast<int>(g->rank_ws->plan.partials());
+  const uint32_t W = g->rank_ws->sms * cfg::kWarps;
+  return static_cast<int>(g->rank_ws->sms + (W + 255) / 256);
+}
+
+// The kernels of one pull epoch (pull_epoch_with).
 template <class Upd, bool kW>
-int pull_epoch_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st) {
+int pull_sums_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st,
+                   const flat_control& c) {
   rank_workspace* ws = g->rank_ws;
+  if (ws->flat.valid) {
+    const flat_plan& fp = ws->flat;
+    if (fp.hot_ctas) {
+      prof_scope ps("k_flat_hot", st);
+      k_flat_hot<kW><<<fp.hot_ctas, kFlatHotWarps * 32, kFlatBlock * 4, st>>>(fp.v, x, c.ctrl);
+      PLATO_LAUNCHED("k_flat_hot");
+    }
+    if (fp.cold_blocks) {
+      prof_scope ps("k_flat_cold", st);
+      k_flat_cold<kW><<<fp.cold_blocks, kFlatColdThreads, 0, st>>>(fp.v, x, c.ctrl);
+      PLATO_LAUNCHED("k_flat_cold");
+    }
+    prof_scope ps("k_flat_update", st);
+    k_flat_update<Upd><<<fp.update_blocks, 256, 0, st>>>(fp.v, upd, ws->partials.p, c);
+    PLATO_LAUNCHED("k_flat_update");
+    return PLATO_OK;
+  }
   const pull_plan& pl = ws->plan;
   if (pl.valid) {
     const pull_plan_view pv{pl.n_long, pl.rows_begin[3], g->info.vertices, pl.n_items, pl.items.p,
@@ -375,19 +409,22 @@ int pull_epoch_with(plato_graph* g, const float* x, const Upd& upd, const float*
   return PLATO_OK;
 }
 
-template <class Tele>
-int pull_epoch(plato_graph* g, const float* x, float* xn, Tele tele, float d, bool final_epoch,
-               cudaStream_t st, const int* mode = nullptr) {
-  const rank_update<Tele> upd{x, xn, g->out_deg.p, tele, d, final_epoch ? 1 : 0, mode};
-  return pull_epoch_with<rank_update<Tele>, false>(g, x, upd, nullptr, st);
+// One pull epoch gathering x (times the edge weights w when kW) with the
+// fused update `upd`: the degree bins on a relabelled graph, else the
+// persistent warp-tile merge path + cross-range fixup.  Partial deltas go to
+// ws->partials (one per CTA of each kernel).  With c.ctrl the epoch also ends
+// in its decision (epoch_decide), which upd.mode reads.
+template <class Upd, bool kW>
+int pull_epoch_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st,
+                    const flat_control& c = flat_control{}) {
+  PLATO_TRY((pull_sums_with<Upd, kW>(g, x, upd, w, st, c)));
+  if (c.ctrl && !g->rank_ws->flat.valid) {
+    k_epoch_control<<<1, 1024, 0, st>>>(g->rank_ws->partials.p, static_cast<uint32_t>(partial_count(g)), c.ctrl,
+                                        c.delta, c.scale, c.eps, c.iteration);
+    PLATO_LAUNCHED("k_epoch_control");
+  }
+  return PLATO_OK;
 }
-
-int partial_count(const plato_graph* g) {
-  if (g->rank_ws->plan.valid) return static_cast<int>(g->rank_ws->plan.partials());
-  const uint32_t W = g->rank_ws->sms * cfg::kWarps;
-  return static_cast<int>(g->rank_ws->sms + (W + 255) / 256);
-}
-
 // Reads back the epoch's delta (sum of the partials).  Synchronises `st`.
 int read_delta(plato_graph* g, uint32_t nparts, cudaStream_t st, double* out) {
   rank_workspace* ws = g->rank_ws;
@@ -405,52 +442,69 @@ int check_rank_opts(uint32_t iteration, double damping) {
   return PLATO_OK;
 }
 
-// Pull-only epochs [start, iteration) from state x[*cur].  With eps == 0 the
-// schedule is known and nothing is read back.  With eps > 0 each epoch is
-// followed by k_epoch_control, which sums the delta on the device and sets
-// the next epoch's kind (pagerank.hpp:137-139); the host enqueues epochs in
-// batches and polls the control word between batches, so there is no host
-// round trip per epoch.  `scale` converts the delta to the reference's units.
-template <class Tele>
-int run_pull_epochs(plato_graph* g, Tele tele, float d, uint32_t iteration, uint32_t start,
-                    double eps, double scale, cudaStream_t st, int* cur, uint32_t* ran,
-                    double* delta) {
+// Pull epochs [start, iteration); make(c, last, mode) is the update that reads
+// state c and writes state c ^ 1 (epochs alternate, *cur holds the state).  With
+// eps == 0 the schedule is known and nothing is read back.  With eps > 0 each
+// epoch ends in its decision on the device (pagerank.hpp:137-139) and the host
+// enqueues a few epochs at a time, one batch ahead of the control word it
+// reads, so the device does not wait for the host; the epochs past the final
+// one return at once.  `scale` converts the delta to the reference's units.
+template <bool kW, class Make>
+int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteration, uint32_t start, double eps,
+                    double scale, cudaStream_t st, int* cur, uint32_t* ran, double* delta) {
   rank_workspace* ws = g->rank_ws;
+  using Upd = decltype(make(0, false, nullptr));
   *ran = 0;
   if (start >= iteration) return PLATO_OK;
   if (eps <= 0.0) {
     for (uint32_t epoch = start; epoch < iteration; ++epoch) {
-      PLATO_TRY(pull_epoch(g, ws->x[*cur].p, ws->x[*cur ^ 1].p, tele, d, epoch == iteration - 1, st));
+      PLATO_TRY((pull_epoch_with<Upd, kW>(g, ws->x[*cur].p, make(*cur, epoch == iteration - 1, nullptr), w, st)));
       *cur ^= 1;
       ++*ran;
     }
     return PLATO_OK;
   }
-  const int init[2] = {start == iteration - 1 ? 1 : 0, static_cast<int>(start)};
+  const int init[4] = {start == iteration - 1 ? 1 : 0, static_cast<int>(start), 0, 0};
   PLATO_CUDA_TRY(cudaMemcpyAsync(ws->ctrl.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
+  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration};
   const int cur0 = *cur;
-  constexpr uint32_t kBatch = 8;
-  uint32_t launched = 0;
-  const uint32_t nparts = static_cast<uint32_t>(partial_count(g));
+  constexpr uint32_t kBatch = 6;
+  uint32_t launched = 0, batches = 0;
+  const int* seen = ws->h_ctrl;  // the last control word read
   while (start + launched < iteration) {
     const uint32_t n = std::min(kBatch, iteration - start - launched);
-    for (uint32_t k = 0; k < n; ++k) {
-      const int c = (cur0 + static_cast<int>(launched + k)) & 1;
-      PLATO_TRY(pull_epoch(g, ws->x[c].p, ws->x[c ^ 1].p, tele, d, false, st, ws->ctrl.p));
-      k_epoch_control<<<1, 1024, 0, st>>>(ws->partials.p, nparts, ws->ctrl.p, ws->delta.p, scale,
-                                          eps, iteration);
-      PLATO_LAUNCHED("k_epoch_control");
+    for (uint32_t k = 0; k < n; ++k, ++launched) {
+      const int p = (cur0 + static_cast<int>(launched)) & 1;
+      PLATO_TRY((pull_epoch_with<Upd, kW>(g, ws->x[p].p, make(p, false, ws->ctrl.p), w, st, c)));
     }
-    launched += n;
-    PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl, ws->ctrl.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_delta, ws->delta.p, sizeof(double), cudaMemcpyDeviceToHost, st));
-    PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-    if (ws->h_ctrl[0] == 2) break;
+    const uint32_t slot = batches++ & 1u;
+    PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl + 4 * slot, ws->ctrl.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    PLATO_CUDA_TRY(cudaEventRecord(ws->polled[slot], st));
+    if (batches == 1) continue;
+    PLATO_CUDA_TRY(cudaEventSynchronize(ws->polled[slot ^ 1]));
+    seen = ws->h_ctrl + 4 * (slot ^ 1);
+    if (seen[0] == 2) break;
   }
-  *ran = static_cast<uint32_t>(ws->h_ctrl[1]) - start;
+  PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_delta, ws->delta.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  seen = ws->h_ctrl + 4 * ((batches - 1) & 1u);
+  *ran = static_cast<uint32_t>(seen[1]) - start;
   *cur = (cur0 + static_cast<int>(*ran)) & 1;
   *delta = *ws->h_delta;
   return PLATO_OK;
+}
+
+// The pull epochs of the PageRank family.
+template <class Tele>
+int run_rank_epochs(plato_graph* g, Tele tele, float d, uint32_t iteration, uint32_t start, double eps, double scale,
+                    cudaStream_t st, int* cur, uint32_t* ran, double* delta) {
+  rank_workspace* ws = g->rank_ws;
+  return run_pull_epochs<false>(
+      g,
+      [=](int c, bool last, const int* mode) {
+        return rank_update<Tele>{ws->x[c].p, ws->x[c ^ 1].p, g->out_deg.p, tele, d, last ? 1 : 0, mode};
+      },
+      nullptr, iteration, start, eps, scale, st, cur, ran, delta);
 }
 
 // PageRank into d_out (caller ids).  Internal buffers stay on the graph.
@@ -468,7 +522,7 @@ int pagerank_impl(plato_graph* g, const plato_pagerank_opts* o, float* d_out, cu
   uint32_t epochs = 0;
   double delta = 0.0;
   // reference units: the reference's ranks sum to ~V
-  PLATO_TRY(run_pull_epochs(g, tele, d, o->iteration, 0, o->eps, static_cast<double>(V), st, &cur,
+  PLATO_TRY(run_rank_epochs(g, tele, d, o->iteration, 0, o->eps, static_cast<double>(V), st, &cur,
                             &epochs, &delta));
   PLATO_TRY(scatter_to_external_f32(g, ws->x[cur].p, d_out, st));
   if (stats) {
@@ -552,7 +606,7 @@ int ppr_impl(plato_graph* g, const plato_ppr_opts* o, int mode, float* d_out, cu
   }
   // pull phase (sticky): device-controlled epochs
   uint32_t pulled = 0;
-  PLATO_TRY(run_pull_epochs(g, tele, d, o->iteration, epoch, o->eps, 1.0, st, &cur, &pulled, &delta));
+  PLATO_TRY(run_rank_epochs(g, tele, d, o->iteration, epoch, o->eps, 1.0, st, &cur, &pulled, &delta));
   epochs += pulled;
   PLATO_TRY(scatter_to_external_f32(g, ws->x[cur].p, d_out, st));
   if (stats) {
@@ -620,7 +674,7 @@ int seedset_impl(plato_graph* g, const uint32_t* seeds_ext, uint32_t n, const pl
   int cur = 0;
   uint32_t epochs = 0;
   double delta = 0.0;
-  PLATO_TRY(run_pull_epochs(g, tele, d, o->iteration, 0, o->eps, 1.0, st, &cur, &epochs, &delta));
+  PLATO_TRY(run_rank_epochs(g, tele, d, o->iteration, 0, o->eps, 1.0, st, &cur, &epochs, &delta));
   PLATO_TRY(scatter_to_external_f32(g, ws->x[cur].p, d_out, st));
   if (stats) {
     *stats = plato_run_stats{};
@@ -642,9 +696,8 @@ __global__ void k_init_weighted(const float* __restrict__ wsum, uint32_t V, floa
 
 // algo::weighted_pagerank (weighted_pagerank.hpp:60-149) into d_out (caller
 // ids, the reference's units).  Epochs are the pull epochs of PageRank with
-// the edge weights multiplied into the gathers; with eps > 0 the delta is read
-// back after each non-final epoch and a small one jumps to the last epoch
-// (:131-137).
+// the edge weights multiplied into the gathers; with eps > 0 a small delta
+// makes the next epoch the last (:131-137), decided on the device.
 int wpagerank_impl(plato_graph* g, const plato_pagerank_opts* o, float* d_out, cudaStream_t st,
                    plato_run_stats* stats) {
   if (!g->weighted)
@@ -658,23 +711,15 @@ int wpagerank_impl(plato_graph* g, const plato_pagerank_opts* o, float* d_out, c
   k_init_weighted<<<grid_for(V, 256), 256, 0, st>>>(g->out_wsum.p, V, ws->r[0].p, ws->x[0].p);
   PLATO_LAUNCHED("k_init_weighted");
   const float base = static_cast<float>(1.0 - o->damping), d = static_cast<float>(o->damping);
-  const uint32_t nparts = static_cast<uint32_t>(partial_count(g));
   int cur = 0;
   uint32_t epochs = 0;
   double delta = 0.0;
-  for (uint32_t epoch = 0; epoch < o->iteration; ++epoch) {
-    const bool last = epoch + 1 == o->iteration;
-    const wrank_update upd{ws->r[cur].p, ws->r[cur ^ 1].p, ws->x[cur ^ 1].p, g->out_wsum.p, base, d,
-                           last ? 1 : 0};
-    PLATO_TRY((pull_epoch_with<wrank_update, true>(g, ws->x[cur].p, upd, g->in_w.p, st)));
-    cur ^= 1;
-    ++epochs;
-    if (last) break;
-    if (o->eps > 0.0) {
-      PLATO_TRY(read_delta(g, nparts, st, &delta));
-      if (delta < o->eps) epoch = o->iteration - 2;  // the next epoch is the last
-    }
-  }
+  PLATO_TRY(run_pull_epochs<true>(
+      g,
+      [=](int c, bool last, const int* mode) {
+        return wrank_update{ws->r[c].p, ws->r[c ^ 1].p, ws->x[c ^ 1].p, g->out_wsum.p, base, d, last ? 1 : 0, mode};
+      },
+      g->in_w.p, o->iteration, 0, o->eps, 1.0, st, &cur, &epochs, &delta));
   PLATO_TRY(scatter_to_external_f32(g, ws->r[cur].p, d_out, st));
   if (stats) {
     *stats = plato_run_stats{};
