@@ -7,6 +7,7 @@
 #include <thrust/iterator/transform_iterator.h>
 
 #include "graph.cuh"
+#include "plato_b200/dualmode.cuh"
 #include "pull_flat.cuh"
 
 namespace plato_b200 {
@@ -25,6 +26,10 @@ namespace {
 // 743 / 674 / 633 / 595 / 577 / 568).
 constexpr uint32_t kFlatRowDeg0 = 8;
 constexpr uint32_t kFlatRowDeg1 = 64;
+// Up to this many edges all epochs run in one launch (k_flat_run; epoch with
+// one / three launches: RMAT s16 9.3 / 14.2 us, s17 12.8 / 15.6, s18 21.1 /
+// 19.4; 3.2M uniform edges 19.2 / 25.6).
+constexpr uint64_t kFlatRunEdges = 3500000;
 constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 600000;
 
 // out[0..1]: rows above the two in-degree limits; out[2 + k]: out-edges of block k.
@@ -252,21 +257,57 @@ __global__ void k_flat_span_base(const uint32_t* __restrict__ scan, uint64_t n, 
     meta[i].w = scan[i];
 }
 
+// Scratch of a plan's construction, from the engine's stream-ordered pool: no
+// cudaMalloc, and no cudaFree that waits for the device.
+template <typename T>
+struct scratch {
+  T* p = nullptr;
+  cudaStream_t st;
+  explicit scratch(cudaStream_t s) : st(s) {}
+  scratch(const scratch&) = delete;
+  scratch& operator=(const scratch&) = delete;
+  ~scratch() { release(); }
+  void release() {
+    if (p) cudaFreeAsync(p, st);
+    p = nullptr;
+  }
+  int alloc(cudaMemPool_t pool, size_t n) {
+    release();
+    const cudaError_t e =
+        cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), std::max<size_t>(n, 1) * sizeof(T), pool, st);
+    if (e == cudaSuccess) return PLATO_OK;
+    p = nullptr;
+    cudaGetLastError();
+    return set_error(e == cudaErrorMemoryAllocation ? PLATO_ENOMEM : PLATO_ECUDA,
+                     std::string("flat plan: scratch allocation failed: ") + cudaGetErrorString(e));
+  }
+};
+
 template <class It>
-int scan_u32(It in, uint32_t* out, uint64_t n, dbuf<uint8_t>& tmp, cudaStream_t st) {
+int scan_u32(It in, uint32_t* out, uint64_t n, cudaMemPool_t pool, cudaStream_t st) {
   size_t bytes = 0;
   PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, static_cast<int64_t>(n), st));
-  PLATO_TRY(tmp.alloc(std::max<size_t>(bytes, 1)));
+  scratch<uint8_t> tmp(st);
+  PLATO_TRY(tmp.alloc(pool, bytes));
   PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, in, out, static_cast<int64_t>(n), st));
   count_launch();
   return PLATO_OK;
 }
 
+// Lays arrays out one after another, each on a 256-byte boundary.
+struct layout {
+  size_t bytes = 0;
+  size_t add(size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  }
+};
+
 template <typename T>
-int put(dbuf<T>& d, const std::vector<T>& h, cudaStream_t st) {
-  PLATO_TRY(d.alloc(std::max<size_t>(h.size(), 1)));
+int put(T* d, const std::vector<T>& h, cudaStream_t st) {
   if (!h.empty())
-    PLATO_CUDA_TRY(cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+    PLATO_CUDA_TRY(cudaMemcpyAsync(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
   return PLATO_OK;
 }
 
@@ -278,9 +319,15 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   pl.valid = false;
   if (!g->relabeled || !g->own_sources || E == 0 || E > 0xF0000000ull) return PLATO_OK;
   const uint32_t nblocks = std::min<uint32_t>((V + kFlatBlock - 1) / kFlatBlock, kFlatMaxBlocks);
-  dbuf<unsigned long long> d_survey;
-  PLATO_TRY(d_survey.alloc(2 + kFlatMaxBlocks + 1));
-  PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, d_survey.bytes(), st));
+  cudaMemPool_t pool{};
+  try {
+    pool = engine_pool();
+  } catch (const std::exception& e) {
+    return set_error(PLATO_ECUDA, e.what());
+  }
+  scratch<unsigned long long> d_survey(st);
+  PLATO_TRY(d_survey.alloc(pool, 2 + kFlatMaxBlocks + 1));
+  PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, (2 + kFlatMaxBlocks + 1) * sizeof(unsigned long long), st));
   k_flat_survey<<<nblocks * 8, 256, 0, st>>>(g->in_deg.p, g->out_deg.p, V, nblocks, d_survey.p);
   PLATO_LAUNCHED("k_flat_survey");
   k_flat_unsorted<<<grid_for(V, 256), 256, 0, st>>>(
@@ -292,22 +339,22 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   if (h[2 + kFlatMaxBlocks]) return PLATO_OK;  // another vertex order
   flat_rows rows{g->in_off.p, g->in_adj.p, V, 0, static_cast<uint32_t>(h[0]), static_cast<uint32_t>(h[1]), 0};
   uint32_t nb = 0;
-  if (h[2] >= kFlatFirst)
+  const bool run = E <= kFlatRunEdges;
+  if (!run && h[2] >= kFlatFirst)
     for (nb = 1; nb < nblocks && h[2 + nb] >= std::max(kFlatMore, h[1]) && h[1] > 0;) ++nb;
   rows.nb = nb;
   rows.rows1 = std::min((rows.r1 + 31) / 32 * 32, V);  // V: the last word may be short
   const uint32_t streams = nb + 1, words = (V + 31) / 32, words1 = (rows.rows1 + 31) / 32;
   const uint64_t cells = flat_place(nb, V, rows.rows1) + V;
 
-  dbuf<uint32_t> cnt, pos, ord;
-  dbuf<uint8_t> tmp;
-  PLATO_TRY(cnt.alloc(cells));
-  PLATO_TRY(pos.alloc(cells));
-  PLATO_TRY(ord.alloc(cells));
+  scratch<uint32_t> cnt(st), pos(st), ord(st);
+  PLATO_TRY(cnt.alloc(pool, cells));
+  PLATO_TRY(pos.alloc(pool, cells));
+  PLATO_TRY(ord.alloc(pool, cells));
   k_flat_split<<<grid_for(V, 256), 256, 0, st>>>(rows, cnt.p);
   PLATO_LAUNCHED("k_flat_split");
-  PLATO_TRY(scan_u32(cnt.p, pos.p, cells, tmp, st));
-  PLATO_TRY(scan_u32(thrust::make_transform_iterator(cnt.p, flat_has()), ord.p, cells, tmp, st));
+  PLATO_TRY(scan_u32(cnt.p, pos.p, cells, pool, st));
+  PLATO_TRY(scan_u32(thrust::make_transform_iterator(cnt.p, flat_has()), ord.p, cells, pool, st));
   // edges before each stream, and the last cells for the number of segments
   std::vector<uint32_t> sum(streams + 1, 0);
   uint32_t last_cnt = 0, segments = 0;
@@ -329,15 +376,56 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   const uint32_t hot_edges = fs.edge[nb], cold_edges = edges - hot_edges;
   const uint32_t hot_steps = hot_edges / kFlatHotStep, cold_steps = cold_edges / kFlatColdStep;
   const bool weighted = g->weighted;
-  PLATO_TRY(pl.hid.alloc(std::max<uint32_t>(hot_edges, 8)));
-  PLATO_TRY(pl.cid.alloc(std::max<uint32_t>(cold_edges, 8)));
-  if (weighted) {
-    PLATO_TRY(pl.hw.alloc(std::max<uint32_t>(hot_edges, 8)));
-    PLATO_TRY(pl.cw.alloc(std::max<uint32_t>(cold_edges, 8)));
+  // grids, and bounds on the pieces
+  int sms = 0;
+  PLATO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
+  const uint32_t per_block = kFlatColdThreads / 32;
+  pl.hot_ctas = std::min<uint32_t>(sms, (hot_steps + kFlatHotWarps - 1) / kFlatHotWarps);
+  pl.run_ctas = pl.run_warps = pl.cold_blocks = 0;
+  if (run) {
+    if (cold_steps <= 64) {
+      pl.run_ctas = 1;
+      pl.run_warps = std::min<uint32_t>(32, std::max<uint32_t>(cold_steps, 4));
+    } else {
+      pl.run_ctas = std::min<uint32_t>(sms, (cold_steps + 7) / 8);
+      pl.run_warps = std::min<uint32_t>(32, (cold_steps + pl.run_ctas - 1) / pl.run_ctas);
+    }
+  } else if (cold_steps) {
+    // a wave of resident CTAs, and more (up to about five waves, so that the
+    // last one is short) while a warp keeps 8 steps
+    const uint32_t wave = sms * 5u, fill = cold_steps / (8 * per_block);
+    pl.cold_blocks = std::min<uint32_t>((cold_steps + per_block - 1) / per_block,
+                                        std::min<uint32_t>(sms * 24u, std::max(wave, fill)));
   }
-  dbuf<uint32_t> hflags, cflags;
-  PLATO_TRY(hflags.alloc(std::max<uint32_t>(hot_edges / 32, 1)));
-  PLATO_TRY(cflags.alloc(std::max<uint32_t>(cold_edges / 32, 1)));
+  const uint32_t cold_pieces = run ? pl.run_ctas * pl.run_warps : pl.cold_blocks * per_block;
+  const uint32_t max_subs = pl.hot_ctas + nb, max_pieces = max_subs * kFlatHotWarps + cold_pieces;
+  const uint64_t nmeta = flat_place(nb, words, words1) + words;
+  layout lay;
+  const size_t o_hid = lay.add(hot_edges * 2ull), o_cid = lay.add(cold_edges * 4ull);
+  const size_t o_hw = lay.add(weighted ? hot_edges * 4ull : 0), o_cw = lay.add(weighted ? cold_edges * 4ull : 0);
+  const size_t o_hmark = lay.add(hot_steps * 128ull), o_cmark = lay.add(cold_steps * 64ull);
+  const size_t o_seg = lay.add((hot_steps + cold_steps) * 4ull), o_meta = lay.add(nmeta * sizeof(uint4));
+  const size_t o_spans = lay.add(max_pieces * sizeof(uint2)), o_pieces = lay.add(max_pieces * sizeof(uint2));
+  const size_t o_subs = lay.add(max_subs * sizeof(flat_sub)), o_cta = lay.add((pl.hot_ctas + 1) * 4ull);
+  const size_t o_part = lay.add(segments * 4ull), o_head = lay.add(max_pieces * 4ull);
+  const size_t o_carry = lay.add(max_pieces * 4ull);
+  PLATO_TRY(pl.mem.alloc(lay.bytes));
+  unsigned char* mem = pl.mem.p;
+  uint16_t* hid = reinterpret_cast<uint16_t*>(mem + o_hid);
+  uint32_t* cid = reinterpret_cast<uint32_t*>(mem + o_cid);
+  float* hw = weighted ? reinterpret_cast<float*>(mem + o_hw) : nullptr;
+  float* cw = weighted ? reinterpret_cast<float*>(mem + o_cw) : nullptr;
+  uint32_t* hmark = reinterpret_cast<uint32_t*>(mem + o_hmark);
+  uint16_t* cmark = reinterpret_cast<uint16_t*>(mem + o_cmark);
+  uint32_t* seg = reinterpret_cast<uint32_t*>(mem + o_seg);
+  uint4* meta = reinterpret_cast<uint4*>(mem + o_meta);
+  uint2* spans = reinterpret_cast<uint2*>(mem + o_spans);
+  uint2* d_pieces = reinterpret_cast<uint2*>(mem + o_pieces);
+  flat_sub* d_subs = reinterpret_cast<flat_sub*>(mem + o_subs);
+  uint32_t* d_cta = reinterpret_cast<uint32_t*>(mem + o_cta);
+  scratch<uint32_t> hflags(st), cflags(st);
+  PLATO_TRY(hflags.alloc(pool, hot_edges / 32));
+  PLATO_TRY(cflags.alloc(pool, cold_edges / 32));
   PLATO_CUDA_TRY(cudaMemsetAsync(hflags.p, 0, hot_edges / 8, st));
   PLATO_CUDA_TRY(cudaMemsetAsync(cflags.p, 0, cold_edges / 8, st));
   // the padding of a stream's last step: source 0, weight 0, no flag
@@ -345,60 +433,56 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
     const uint32_t end = k + 1 < streams ? fs.edge[k + 1] : edges;
     if (end == fs.edge[k]) continue;
     if (k < nb) {
-      PLATO_CUDA_TRY(cudaMemsetAsync(pl.hid.p + (end - kFlatHotStep), 0, kFlatHotStep * 2, st));
-      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(pl.hw.p + (end - kFlatHotStep), 0, kFlatHotStep * 4, st));
+      PLATO_CUDA_TRY(cudaMemsetAsync(hid + (end - kFlatHotStep), 0, kFlatHotStep * 2, st));
+      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(hw + (end - kFlatHotStep), 0, kFlatHotStep * 4, st));
     } else {
       const uint32_t b = cold_edges - kFlatColdStep;
-      PLATO_CUDA_TRY(cudaMemsetAsync(pl.cid.p + b, 0, kFlatColdStep * 4, st));
-      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(pl.cw.p + b, 0, kFlatColdStep * 4, st));
+      PLATO_CUDA_TRY(cudaMemsetAsync(cid + b, 0, kFlatColdStep * 4, st));
+      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(cw + b, 0, kFlatColdStep * 4, st));
     }
   }
   const merge_tiles* mt = nullptr;
   PLATO_TRY(ensure_pull_tiles(g, 224, st, &mt));
   k_flat_fill<<<grid_for(static_cast<uint64_t>(mt->count) * 32, 256), 256, 0, st>>>(
-      rows, mt->row.p, mt->edge.p, mt->count, cnt.p, pos.p, fs, weighted ? g->in_w.p : nullptr, pl.hid.p,
-      pl.cid.p, pl.hw.p, pl.cw.p, hflags.p, cflags.p);
+      rows, mt->row.p, mt->edge.p, mt->count, cnt.p, pos.p, fs, weighted ? g->in_w.p : nullptr, hid, cid, hw,
+      cw, hflags.p, cflags.p);
   PLATO_LAUNCHED("k_flat_fill");
   // marks, and segments that end before each step (numbered through all streams)
-  PLATO_TRY(pl.hmark.alloc(std::max<uint32_t>(hot_steps * 32, 1)));
-  PLATO_TRY(pl.cmark.alloc(std::max<uint32_t>(cold_steps * 32, 1)));
-  PLATO_TRY(pl.hseg.alloc(std::max<uint32_t>(hot_steps + cold_steps, 1)));
-  dbuf<uint32_t> ends;
-  PLATO_TRY(ends.alloc(std::max<uint32_t>(hot_steps + cold_steps, 1)));
+  scratch<uint32_t> ends(st);
+  PLATO_TRY(ends.alloc(pool, hot_steps + cold_steps));
   if (hot_steps) {
     k_flat_marks<kFlatHotLane, uint32_t><<<grid_for(hot_steps * 32ull, 256), 256, 0, st>>>(hflags.p, hot_steps,
-                                                                                           pl.hmark.p, ends.p);
+                                                                                           hmark, ends.p);
     PLATO_LAUNCHED("k_flat_marks");
   }
   if (cold_steps) {
     k_flat_marks<kFlatColdLane, uint16_t><<<grid_for(cold_steps * 32ull, 256), 256, 0, st>>>(
-        cflags.p, cold_steps, pl.cmark.p, ends.p + hot_steps);
+        cflags.p, cold_steps, cmark, ends.p + hot_steps);
     PLATO_LAUNCHED("k_flat_marks");
   }
-  PLATO_TRY(scan_u32(ends.p, pl.hseg.p, hot_steps + cold_steps, tmp, st));
-  const uint64_t nmeta = flat_place(nb, words, words1) + words;
-  PLATO_TRY(pl.meta.alloc(nmeta));
-  k_flat_meta<<<grid_for(nmeta * 32, 256), 256, 0, st>>>(rows, cnt.p, ord.p, words, nmeta, pl.meta.p);
+  PLATO_TRY(scan_u32(ends.p, seg, hot_steps + cold_steps, pool, st));
+  k_flat_meta<<<grid_for(nmeta * 32, 256), 256, 0, st>>>(rows, cnt.p, ord.p, words, nmeta, meta);
   PLATO_LAUNCHED("k_flat_meta");
 
   // Pieces: the hot steps split evenly over one CTA per SM, cut at block
   // ends, each part split over the CTA's warps; the cold steps over all warps
   // of the cold grid.
-  int sms = 0;
-  PLATO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
   // Cost of the hot steps before each one: a step with segment ends costs
   // about half as much again, and every end is a store.  (RMAT s24, k_flat_hot
   // with the steps split evenly 291 us, by this cost 182.)
   const uint32_t all_steps = hot_steps + cold_steps;
-  std::vector<uint32_t> seg(all_steps);
-  PLATO_CUDA_TRY(cudaMemcpyAsync(seg.data(), pl.hseg.p, all_steps * 4ull, cudaMemcpyDeviceToHost, st));
-  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  std::vector<uint32_t> h_seg(hot_steps + 1, segments);
+  if (hot_steps) {
+    PLATO_CUDA_TRY(cudaMemcpyAsync(h_seg.data(), seg, std::min(hot_steps + 1, all_steps) * 4ull,
+                                   cudaMemcpyDeviceToHost, st));
+    PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  }
   std::vector<float> cost(hot_steps + 1);
   {
     double c = 0.0;
     for (uint32_t s = 0; s < hot_steps; ++s) {
       cost[s] = static_cast<float>(c);
-      const uint32_t n = (s + 1 < all_steps ? seg[s + 1] : segments) - seg[s];
+      const uint32_t n = h_seg[s + 1] - h_seg[s];
       c += 1.0 + (n ? 0.5 : 0.0) + 0.01 * n;
     }
     cost[hot_steps] = static_cast<float>(c);
@@ -414,7 +498,6 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
     return static_cast<uint32_t>(std::lower_bound(cost.begin() + lo, cost.begin() + hi, static_cast<float>(c)) -
                                  cost.begin());
   };
-  pl.hot_ctas = std::min<uint32_t>(sms, (hot_steps + kFlatHotWarps - 1) / kFlatHotWarps);
   uint32_t a = 0;
   for (uint32_t c = 0; c < pl.hot_ctas; ++c) {
     cta_sub.push_back(static_cast<uint32_t>(subs.size()));
@@ -435,28 +518,13 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   }
   cta_sub.push_back(static_cast<uint32_t>(subs.size()));
   const uint32_t cold_piece0 = static_cast<uint32_t>(pieces.size());
-  auto cut = [&](uint32_t n) {
-    for (uint32_t w = 0; w < n; ++w)
-      add(0, static_cast<uint32_t>(static_cast<uint64_t>(cold_steps) * w / n),
-          static_cast<uint32_t>(static_cast<uint64_t>(cold_steps) * (w + 1) / n));
-  };
-  const uint32_t per_block = kFlatColdThreads / 32;
-  pl.cold_blocks = 0;
-  if (cold_steps) {
-    // a wave of resident CTAs, and more (up to about five waves, so that the
-    // last one is short) while a warp keeps 8 steps
-    const uint32_t wave = sms * 5u, fill = cold_steps / (8 * per_block);
-    pl.cold_blocks = std::min<uint32_t>((cold_steps + per_block - 1) / per_block, std::min<uint32_t>(sms * 24u, std::max(wave, fill)));
-    cut(pl.cold_blocks * per_block);
-  }
+  for (uint32_t w = 0; w < cold_pieces; ++w)
+    add(0, static_cast<uint32_t>(static_cast<uint64_t>(cold_steps) * w / cold_pieces),
+        static_cast<uint32_t>(static_cast<uint64_t>(cold_steps) * (w + 1) / cold_pieces));
   const uint32_t npieces = static_cast<uint32_t>(pieces.size());
-  PLATO_TRY(put(pl.pieces, pieces, st));
-  PLATO_TRY(put(pl.subs, subs, st));
-  PLATO_TRY(put(pl.cta_sub, cta_sub, st));
-  PLATO_TRY(pl.part.alloc(std::max<uint32_t>(segments, 1)));
-  PLATO_TRY(pl.head.alloc(npieces));
-  PLATO_TRY(pl.carry.alloc(npieces));
-  PLATO_TRY(pl.spans.alloc(npieces));
+  PLATO_TRY(put(d_pieces, pieces, st));
+  PLATO_TRY(put(d_subs, subs, st));
+  PLATO_TRY(put(d_cta, cta_sub, st));
   flat_view& f = pl.v;
   f = flat_view{};
   f.V = f.nsrc = V;
@@ -465,32 +533,32 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   f.words1 = words1;
   f.cold_piece0 = cold_piece0;
   f.cold_pieces = npieces - cold_piece0;
-  f.hid = pl.hid.p;
-  f.cid = pl.cid.p;
-  f.hw = pl.hw.p;
-  f.cw = pl.cw.p;
-  f.hmark = pl.hmark.p;
-  f.cmark = pl.cmark.p;
-  f.hseg = pl.hseg.p;
-  f.cseg = pl.hseg.p + hot_steps;
-  f.pieces = pl.pieces.p;
-  f.cta_sub = pl.cta_sub.p;
-  f.subs = pl.subs.p;
-  f.meta = pl.meta.p;
-  f.spans = pl.spans.p;
-  f.part = pl.part.p;
-  f.head = pl.head.p;
-  f.carry = pl.carry.p;
+  f.hid = hid;
+  f.cid = cid;
+  f.hw = hw;
+  f.cw = cw;
+  f.hmark = hmark;
+  f.cmark = cmark;
+  f.hseg = seg;
+  f.cseg = seg + hot_steps;
+  f.pieces = d_pieces;
+  f.cta_sub = d_cta;
+  f.subs = d_subs;
+  f.meta = meta;
+  f.spans = spans;
+  f.part = reinterpret_cast<float*>(mem + o_part);
+  f.head = reinterpret_cast<float*>(mem + o_head);
+  f.carry = reinterpret_cast<float*>(mem + o_carry);
   const unsigned span_grid = (npieces + 127) / 128;
-  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, pl.meta.p, nullptr);
+  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr);
   PLATO_LAUNCHED("k_flat_spans");
-  dbuf<uint32_t> base;
-  PLATO_TRY(base.alloc(nmeta));
-  PLATO_TRY(scan_u32(thrust::make_transform_iterator(thrust::counting_iterator<uint32_t>(0), flat_crossing{pl.meta.p}),
-                     base.p, nmeta, tmp, st));
-  k_flat_span_base<<<grid_for(nmeta, 256), 256, 0, st>>>(base.p, nmeta, pl.meta.p);
+  scratch<uint32_t> base(st);
+  PLATO_TRY(base.alloc(pool, nmeta));
+  PLATO_TRY(scan_u32(thrust::make_transform_iterator(thrust::counting_iterator<uint32_t>(0), flat_crossing{meta}),
+                     base.p, nmeta, pool, st));
+  k_flat_span_base<<<grid_for(nmeta, 256), 256, 0, st>>>(base.p, nmeta, meta);
   PLATO_LAUNCHED("k_flat_span_base");
-  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, pl.meta.p, pl.spans.p);
+  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans);
   PLATO_LAUNCHED("k_flat_spans");
   pl.update_blocks = std::min<uint32_t>(sms * 4, (words + 15) / 16);
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));  // the temporaries and the host vectors go

@@ -89,13 +89,9 @@ __host__ __device__ inline uint64_t flat_place(uint32_t k, uint64_t rows, uint64
 struct flat_plan {
   bool valid = false;
   uint32_t hot_ctas = 0, cold_blocks = 0, update_blocks = 0;
+  uint32_t run_ctas = 0, run_warps = 0;  // not 0: k_flat_run's grid, the plan's only kernel
   flat_view v{};
-  dbuf<uint16_t> hid, cmark;
-  dbuf<uint32_t> cid, hmark, hseg, cseg, cta_sub;
-  dbuf<float> hw, cw, part, head, carry;
-  dbuf<uint2> pieces, spans;
-  dbuf<flat_sub> subs;
-  dbuf<uint4> meta;
+  dbuf<unsigned char> mem;  // every array of v
 };
 
 // Builds the plan of g's pull on `st` (pull_flat.cu); plan.valid stays false
@@ -170,11 +166,13 @@ struct flat_hot_gather {
   }
 };
 
-// Cold: 32-bit ids into global memory.
-template <bool kW>
+// Cold: 32-bit ids into global memory.  kRun: in a kernel that runs many
+// epochs the state is written by other SMs between epochs: plain loads, which
+// the barrier's acquire orders.
+template <bool kW, bool kRun>
 struct flat_cold_gather {
   static constexpr int kLane = kFlatColdLane;
-  static constexpr uint32_t kAhead = 4;
+  static constexpr uint32_t kAhead = kRun ? 0 : 4;
   const uint32_t* ids;
   const float* w;
   const uint16_t* marks;
@@ -188,16 +186,16 @@ struct flat_cold_gather {
     if (kW && lane >= 16 && lane < 24) flat_prefetch(w + e + (lane - 16) * 32);
   }
   __device__ __forceinline__ void load(uint32_t step, unsigned lane, regs& r) const {
-    flat_load<true>(ids + static_cast<size_t>(step) * kFlatColdStep + lane * kLane, r);
+    flat_load<!kRun>(ids + static_cast<size_t>(step) * kFlatColdStep + lane * kLane, r);
   }
   __device__ __forceinline__ uint32_t mark(uint32_t step, unsigned lane) const {
     const uint16_t* p = marks + static_cast<size_t>(step) * 32 + lane;
-    return __ldcs(p);
+    return kRun ? __ldg(p) : __ldcs(p);
   }
   __device__ __forceinline__ void values(uint32_t step, unsigned lane, const regs& r, float (&v)[kLane]) const {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __ldg(x + r.w[i]);
-    if constexpr (kW) flat_weigh<true>(w + static_cast<size_t>(step) * kFlatColdStep + lane * kLane, v);
+    for (int i = 0; i < 8; ++i) v[i] = kRun ? x[r.w[i]] : __ldg(x + r.w[i]);
+    if constexpr (kW) flat_weigh<!kRun>(w + static_cast<size_t>(step) * kFlatColdStep + lane * kLane, v);
   }
 };
 
@@ -329,11 +327,12 @@ __global__ void __launch_bounds__(kFlatColdThreads, 5) k_flat_cold(flat_view f, 
   if (mode && *mode == 2) return;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= f.cold_pieces) return;
-  const flat_cold_gather<kW> g{f.cid, f.cw, f.cmark, f.cseg, x};
+  const flat_cold_gather<kW, false> g{f.cid, f.cw, f.cmark, f.cseg, x};
   flat_piece(f, f.cold_piece0 + w, g);
 }
 
 // The sums of one 32-row word's segments of a stream: lane l gets row l's.
+// They were written by other SMs, in the same kernel when it runs many epochs.
 __device__ __forceinline__ float flat_segment(const flat_view& f, const uint4& m, unsigned lane) {
   const unsigned below = (1u << lane) - 1u;
   if (!((m.x >> lane) & 1u)) return 0.f;
@@ -448,6 +447,103 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
   if (threadIdx.x == 0) {
     c.ctrl[2] = 0;
     epoch_decide(c.ctrl, c.delta, t * c.scale, c.eps, c.iteration);
+  }
+}
+
+// Barrier over the CTAs of a cooperative launch: sync[0] counts arrivals over
+// the whole launch (`target` of them release this barrier), sync[1] is set
+// when a CTA gives up waiting, and then every CTA returns.
+constexpr uint32_t kFlatSpins = 1u << 24;
+__device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (gridDim.x == 1) return true;
+  if (threadIdx.x == 0) {
+    int ok = 0;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sync) : "memory");
+    for (uint32_t n = 0; n < kFlatSpins; ++n) {
+      uint32_t seen, failed;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync) : "memory");
+      if (seen >= target) {
+        ok = 1;
+        break;
+      }
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(failed) : "l"(sync + 1) : "memory");
+      if (failed) break;
+    }
+    if (!ok) asm volatile("st.relaxed.gpu.global.u32 [%0], 1;" ::"l"(sync + 1) : "memory");
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+template <class Update>
+__device__ __noinline__ void flat_poison(const flat_view& f, const Update& upd, uint32_t w0, uint32_t nwarps) {
+  for (uint32_t w = w0; w < f.words; w += nwarps) {
+    const uint32_t v = w * 32 + (threadIdx.x & 31);
+    if (v < f.V) upd.poison(v);
+  }
+}
+
+// Every epoch of a small graph in one cooperative launch of gridDim.x <= SMs
+// CTAs: gather, barrier, update, barrier.  The epoch kinds and the eps exit
+// follow epoch_decide; ctrl[1] = epochs run, counted from `start`.  Launches
+// bound these graphs: one epoch with a launch per degree bin / here, RMAT s10
+// 52 / 5.3 us, s12 54 / 6.4, s16 70 / 9.4, 48K uniform edges 28 / 6.5.  A CTA
+// that gives up waiting leaves NaN in its rows.
+template <class Update, bool kW>
+__global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f, Update upd, uint32_t start,
+                                                                   uint32_t iteration, double scale, double eps,
+                                                                   int* ctrl, double* delta, double* partials,
+                                                                   uint32_t* sync) {
+  __shared__ double s_red[32];
+  __shared__ double s_delta;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t cta_warps = blockDim.x >> 5;
+  const uint32_t w0 = blockIdx.x * cta_warps + warp, nwarps = gridDim.x * cta_warps;
+  uint32_t barriers = 0, ran = start;
+  bool last = start + 1 >= iteration;
+  for (;;) {
+    upd.final_epoch = last ? 1 : 0;
+    flat_piece(f, w0, flat_cold_gather<kW, true>{f.cid, f.cw, f.cmark, f.cseg, upd.gathered()});
+    if (!flat_barrier(sync, ++barriers * gridDim.x)) return flat_poison(f, upd, w0, nwarps);
+    double dl = 0.0;
+    for (uint32_t w = w0; w < f.words; w += nwarps) {
+      const uint32_t v = w * 32 + lane;
+      const bool mine = v < f.V;
+      const typename Update::operands ops = upd.load_l2(mine ? v : w * 32);
+      const float y = flat_segment(f, __ldg(f.meta + w), lane);
+      if (mine) dl += upd.apply(v, y, ops);
+    }
+    ++ran;
+    if (last) break;
+    double* sums = partials + (ran & 1u) * gridDim.x;
+    if (eps > 0.0) {
+      dl = warp_sum(dl);
+      if (lane == 0) s_red[warp] = dl;
+      __syncthreads();
+      dl = warp_sum(lane < cta_warps ? s_red[lane] : 0.0);
+      if (threadIdx.x == 0) __stcg(sums + blockIdx.x, dl);
+    }
+    if (!flat_barrier(sync, ++barriers * gridDim.x)) return flat_poison(f, upd, w0, nwarps);
+    last = ran + 1 >= iteration;
+    if (eps > 0.0) {  // every CTA sums the partials in the same order
+      if (warp == 0) {
+        double t = 0.0;
+        for (uint32_t i = lane; i < gridDim.x; i += 32) t += __ldcg(sums + i);
+        t = warp_sum(t) * scale;
+        if (lane == 0) s_delta = t;
+      }
+      __syncthreads();
+      if (s_delta < eps) last = true;
+    }
+    upd.flip();
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctrl[0] = 2;
+    ctrl[1] = static_cast<int>(ran);
+    if (eps > 0.0) *delta = ran > start + 1 ? s_delta : 0.0;
   }
 }
 

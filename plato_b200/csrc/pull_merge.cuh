@@ -82,6 +82,21 @@ struct rank_update {
     return {__ldcs(deg + v), __ldcs(x + v)};
   }
 
+  // load() inside a kernel that runs many epochs (the state is other SMs' work)
+  __device__ __forceinline__ operands load_l2(uint32_t v) const {
+    if (storing_rank()) return {0u, 0.f};
+    return {__ldg(deg + v), __ldcg(x + v)};
+  }
+  __device__ __forceinline__ const float* gathered() const { return x; }
+  __device__ __forceinline__ void flip() {
+    const float* t = x;
+    x = xn;
+    xn = const_cast<float*>(t);
+  }
+  __device__ __forceinline__ void poison(uint32_t v) const {
+    xn[v] = const_cast<float*>(x)[v] = __int_as_float(0x7fffffff);
+  }
+
   __device__ __forceinline__ double apply(uint32_t v, float y) const { return apply(v, y, load(v)); }
 
   __device__ __forceinline__ double apply(uint32_t v, float y, operands o) const {

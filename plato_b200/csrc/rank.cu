@@ -51,7 +51,7 @@ struct rank_workspace {
   flat_plan flat;
   dbuf<uint32_t> seed_bits, seed_list;  // seed-set PPR
   dbuf<float> out_stage;                // caller-id ranks before the copy to the host
-  dbuf<int> ctrl;                       // device epoch control (k_epoch_control)
+  dbuf<int> ctrl;                       // device epoch control (k_epoch_control); [2], [3] k_flat_run's barrier
   double* h_delta = nullptr;  // pinned
   int* h_ctrl = nullptr;      // pinned [8]: two control words
   cudaEvent_t polled[2] = {nullptr, nullptr};  // control words copied to h_ctrl
@@ -88,6 +88,7 @@ struct wrank_update {
   float d;
   int final_epoch;
   const int* mode = nullptr;  // epoch kind on the device, as in rank_update
+  const float* x = nullptr;   // current gathered state
 
   __device__ __forceinline__ bool skip() const { return mode && *mode == 2; }
   __device__ __forceinline__ bool storing_rank() const { return mode ? (*mode == 1) : (final_epoch != 0); }
@@ -100,6 +101,24 @@ struct wrank_update {
     if (storing_rank()) return {0.f, 1.f};
     return {__ldcs(r + v), __ldcs(wsum + v)};
   }
+  // load() inside a kernel that runs many epochs (the state is other SMs' work)
+  __device__ __forceinline__ operands load_l2(uint32_t v) const {
+    if (storing_rank()) return {0.f, 1.f};
+    return {__ldcg(r + v), __ldg(wsum + v)};
+  }
+  __device__ __forceinline__ const float* gathered() const { return x; }
+  __device__ __forceinline__ void flip() {
+    float* t = const_cast<float*>(r);
+    r = rn;
+    rn = t;
+    t = const_cast<float*>(x);
+    x = xn;
+    xn = t;
+  }
+  __device__ __forceinline__ void poison(uint32_t v) const {
+    rn[v] = const_cast<float*>(r)[v] = __int_as_float(0x7fffffff);
+  }
+
   __device__ __forceinline__ double apply(uint32_t v, float y) const { return apply(v, y, load(v)); }
 
   __device__ __forceinline__ double apply(uint32_t v, float y, operands o) const {
@@ -442,6 +461,36 @@ int check_rank_opts(uint32_t iteration, double damping) {
   return PLATO_OK;
 }
 
+// Every pull epoch of a small graph in one launch (k_flat_run); `upd` starts
+// at the current state.  With eps > 0 the host waits for the epoch count.
+template <class Upd, bool kW>
+int run_flat_epochs(plato_graph* g, const Upd& upd, uint32_t iteration, uint32_t start, double eps, double scale,
+                    cudaStream_t st, uint32_t* ran, double* delta) {
+  rank_workspace* ws = g->rank_ws;
+  PLATO_CUDA_TRY(cudaMemsetAsync(ws->ctrl.p, 0, 4 * sizeof(int), st));
+  {
+    prof_scope ps("k_flat_run", st);
+    Upd u = upd;
+    flat_view f = ws->flat.v;
+    int* ctrl = ws->ctrl.p;
+    uint32_t* sync = reinterpret_cast<uint32_t*>(ws->ctrl.p + 2);
+    double *d_delta = ws->delta.p, *partials = ws->partials.p;
+    void* args[] = {&f, &u, &start, &iteration, &scale, &eps, &ctrl, &d_delta, &partials, &sync};
+    PLATO_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_flat_run<Upd, kW>),
+                                               dim3(ws->flat.run_ctas), dim3(ws->flat.run_warps * 32), args, 0, st));
+    PLATO_LAUNCHED("k_flat_run");
+  }
+  *ran = iteration - start;
+  if (eps <= 0.0) return PLATO_OK;
+  PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl, ws->ctrl.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_delta, ws->delta.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  if (ws->h_ctrl[3]) return set_error(PLATO_ETIMEDOUT, "k_flat_run: a grid barrier ran out");
+  *ran = static_cast<uint32_t>(ws->h_ctrl[1]) - start;
+  *delta = *ws->h_delta;
+  return PLATO_OK;
+}
+
 // Pull epochs [start, iteration); make(c, last, mode) is the update that reads
 // state c and writes state c ^ 1 (epochs alternate, *cur holds the state).  With
 // eps == 0 the schedule is known and nothing is read back.  With eps > 0 each
@@ -456,6 +505,11 @@ int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteratio
   using Upd = decltype(make(0, false, nullptr));
   *ran = 0;
   if (start >= iteration) return PLATO_OK;
+  if (ws->flat.run_ctas) {
+    PLATO_TRY((run_flat_epochs<Upd, kW>(g, make(*cur, false, nullptr), iteration, start, eps, scale, st, ran, delta)));
+    *cur = (*cur + static_cast<int>(*ran)) & 1;
+    return PLATO_OK;
+  }
   if (eps <= 0.0) {
     for (uint32_t epoch = start; epoch < iteration; ++epoch) {
       PLATO_TRY((pull_epoch_with<Upd, kW>(g, ws->x[*cur].p, make(*cur, epoch == iteration - 1, nullptr), w, st)));
@@ -717,7 +771,8 @@ int wpagerank_impl(plato_graph* g, const plato_pagerank_opts* o, float* d_out, c
   PLATO_TRY(run_pull_epochs<true>(
       g,
       [=](int c, bool last, const int* mode) {
-        return wrank_update{ws->r[c].p, ws->r[c ^ 1].p, ws->x[c ^ 1].p, g->out_wsum.p, base, d, last ? 1 : 0, mode};
+        return wrank_update{ws->r[c].p, ws->r[c ^ 1].p, ws->x[c ^ 1].p, g->out_wsum.p, base,
+                            d,          last ? 1 : 0,   mode,           ws->x[c].p};
       },
       g->in_w.p, o->iteration, 0, o->eps, 1.0, st, &cur, &epochs, &delta));
   PLATO_TRY(scatter_to_external_f32(g, ws->r[cur].p, d_out, st));
