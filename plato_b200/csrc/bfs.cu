@@ -41,6 +41,7 @@ struct bfs_workspace {
   push_frontier fr[3];  // current, next, and the one cleared for the level after
   dbuf<uint32_t> visited;
   dbuf<uint32_t> level, parent;
+  dbuf<uint32_t> ext;             // a result in caller ids, before its copy to the host
   dbuf<bfs_control> ctrl;
   bfs_control* h_ctrl = nullptr;  // pinned
   unsigned level_blocks = 0;      // one full wave of resident k_bfs_level CTAs
@@ -524,12 +525,11 @@ extern "C" int plato_bfs(plato_graph* g, const plato_bfs_opts* opts,
   const uint32_t V = g->info.vertices;
   bfs_workspace* ws = g->bfs_ws;
   if (levels || parents) {
-    dbuf<uint32_t> ext;
+    dbuf<uint32_t>& ext = ws->ext;
     PLATO_TRY(ext.alloc(V));
     if (levels) {
       PLATO_TRY(scatter_to_external_u32(g, ws->level.p, ext.p, st));
-      PLATO_CUDA_TRY(cudaMemcpyAsync(levels, ext.p, V * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-      PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+      PLATO_TRY(copy_to_host(levels, ext.p, V * sizeof(uint32_t), st));
     }
     if (parents) {
       if (g->relabeled) {
@@ -540,8 +540,7 @@ extern "C" int plato_bfs(plato_graph* g, const plato_bfs_opts* opts,
         PLATO_CUDA_TRY(cudaMemcpyAsync(ext.p, ws->parent.p, V * sizeof(uint32_t),
                                        cudaMemcpyDeviceToDevice, st));
       }
-      PLATO_CUDA_TRY(cudaMemcpyAsync(parents, ext.p, V * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-      PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+      PLATO_TRY(copy_to_host(parents, ext.p, V * sizeof(uint32_t), st));
     }
   }
   return PLATO_OK;

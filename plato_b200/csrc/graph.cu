@@ -526,10 +526,7 @@ extern "C" int plato_graph_out_degrees(plato_graph* g, uint32_t* degrees_out) {
   dbuf<uint32_t> ext;
   PLATO_TRY(ext.alloc(g->info.vertices));
   PLATO_TRY(scatter_to_external_u32(g, g->out_deg.p, ext.p, g->stream));
-  PLATO_CUDA_TRY(cudaMemcpyAsync(degrees_out, ext.p, g->info.vertices * sizeof(uint32_t),
-                                 cudaMemcpyDeviceToHost, g->stream));
-  PLATO_CUDA_TRY(cudaStreamSynchronize(g->stream));
-  return PLATO_OK;
+  return copy_to_host(degrees_out, ext.p, g->info.vertices * sizeof(uint32_t), g->stream);
 }
 
 extern "C" int plato_graph_device_bytes(const plato_graph* g, uint64_t* bytes) {

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_copy.hpp"
 
 namespace plato_b200 {
 
@@ -49,6 +50,7 @@ struct plato_graph {
 
   cudaStream_t stream = nullptr;  // stream of the host-buffer entry points
   std::mutex mu;                  // one algorithm call at a time per graph
+  plato_b200::host_copy_user host_copies;
 
   std::map<uint32_t, plato_b200::merge_tiles> tiles;  // merge-path tiles by items per tile
   plato_b200::rank_workspace* rank_ws = nullptr;

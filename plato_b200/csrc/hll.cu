@@ -1007,9 +1007,7 @@ class hll_engine {
     const uint32_t* to_ext = g_->relabeled ? g_->to_ext.p : nullptr;
     k_rows_to_ext<<<grid_for(rows / 16, kHllThreads), kHllThreads, 0, st_>>>(latest, spare, to_ext, V_, m_);
     PLATO_LAUNCHED("k_rows_to_ext");
-    PLATO_CUDA_TRY(cudaMemcpyAsync(out, spare, rows, cudaMemcpyDeviceToHost, st_));
-    PLATO_CUDA_TRY(cudaStreamSynchronize(st_));
-    return PLATO_OK;
+    return copy_to_host(out, spare, rows, st_);
   }
 
   int degrees_out(const uint32_t* target, uint32_t* d_out) {
@@ -1271,10 +1269,8 @@ int nstep_impl(plato_graph* g, const plato_nstep_opts* o, const plato_dualmode_o
       PLATO_CUDA_TRY(cudaMemcpyAsync(d_out, d_in, 4ull * (V ? V : 1), cudaMemcpyDeviceToDevice, s));
     }
   }
-  if (in_degrees && V)
-    PLATO_CUDA_TRY(cudaMemcpyAsync(in_degrees, d_in, 4ull * V, cudaMemcpyDeviceToHost, s));
-  if (out_degrees && V)
-    PLATO_CUDA_TRY(cudaMemcpyAsync(out_degrees, d_out, 4ull * V, cudaMemcpyDeviceToHost, s));
+  if (in_degrees && V) PLATO_TRY(copy_to_host(in_degrees, d_in, 4ull * V, s));
+  if (out_degrees && V) PLATO_TRY(copy_to_host(out_degrees, d_out, 4ull * V, s));
   PLATO_CUDA_TRY(cudaStreamSynchronize(s));
   h.trim();
   if (stats) *stats = st;

@@ -1,0 +1,143 @@
+// Device to host copies of result vectors.
+//
+// A caller's result buffer is usually pageable (a numpy array, a vector); the
+// driver stages such a copy through its own pinned memory with one thread,
+// about 9 GB/s, and a V-sized result then costs more than many of the
+// algorithms.  copy_to_host stages it itself: the device writes pinned chunks
+// at the link's rate, and several host threads move finished chunks to the
+// caller while later ones arrive.  The staging memory is one block per process
+// (kHalves * kHalfBytes), used by one call at a time; a call that finds it
+// busy, a small result and a caller's pinned buffer take the plain copy.  The
+// block is freed with the last graph.
+#include <omp.h>
+
+#include <algorithm>
+#include <cstring>
+#include <mutex>
+
+#include "common.cuh"
+#include "host_copy.hpp"
+
+namespace plato_b200 {
+namespace {
+
+constexpr size_t kChunk = 256u << 10, kHalfBytes = 4u << 20, kHalves = 2;
+constexpr size_t kChunks = kHalfBytes / kChunk;
+constexpr size_t kSmall = 1u << 20;  // below, waking the threads costs more than they save
+constexpr int kThreads = 8;
+
+struct staging {
+  std::mutex mu;  // held by the copy that uses the block
+  unsigned char* p = nullptr;
+  int device = -1;  // of the events
+  cudaEvent_t done[kHalves * kChunks] = {};
+  void release() {
+    for (cudaEvent_t& e : done) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    device = -1;
+  }
+  bool ready(int dev) {
+    if (p && device == dev) return true;
+    release();
+    if (cudaHostAlloc(reinterpret_cast<void**>(&p), kHalves * kHalfBytes, cudaHostAllocPortable) != cudaSuccess)
+      p = nullptr;
+    for (cudaEvent_t& e : done)
+      if (p && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        e = nullptr;
+        release();
+      }
+    if (!p) cudaGetLastError();
+    device = p ? dev : -1;
+    return p != nullptr;
+  }
+};
+
+staging g_stage;
+std::mutex g_users_mu;
+int g_users = 0;
+
+int plain_copy(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  PLATO_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  return PLATO_OK;
+}
+
+bool pageable(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
+
+}  // namespace
+
+host_copy_user::host_copy_user() {
+  std::lock_guard<std::mutex> lock(g_users_mu);
+  ++g_users;
+}
+
+host_copy_user::~host_copy_user() {
+  std::lock_guard<std::mutex> lock(g_users_mu);
+  if (--g_users == 0) {
+    std::lock_guard<std::mutex> stage(g_stage.mu);
+    g_stage.release();
+  }
+}
+
+int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  if (bytes == 0) {
+    PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+    return PLATO_OK;
+  }
+  if (bytes < kSmall || !pageable(dst)) return plain_copy(dst, src, bytes, st);
+  std::unique_lock<std::mutex> lock(g_stage.mu, std::try_to_lock);
+  int dev = 0;
+  PLATO_CUDA_TRY(cudaGetDevice(&dev));
+  if (!lock.owns_lock() || !g_stage.ready(dev)) return plain_copy(dst, src, bytes, st);
+  unsigned char* out = static_cast<unsigned char*>(dst);
+  const unsigned char* in = static_cast<const unsigned char*>(src);
+  // part `k` of the result goes through half k % 2, a chunk at a time
+  const size_t parts = (bytes + kHalfBytes - 1) / kHalfBytes;
+  auto enqueue = [&](size_t k) -> cudaError_t {
+    const size_t lo = k * kHalfBytes, hi = std::min(bytes, lo + kHalfBytes);
+    for (size_t c = lo, i = (k % kHalves) * kChunks; c < hi; c += kChunk, ++i) {
+      cudaError_t e = cudaMemcpyAsync(g_stage.p + (k % kHalves) * kHalfBytes + (c - lo), in + c,
+                                      std::min(kChunk, hi - c), cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaEventRecord(g_stage.done[i], st);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  };
+  cudaError_t err = cudaSuccess;
+  for (size_t k = 0; k < std::min(kHalves, parts) && err == cudaSuccess; ++k) err = enqueue(k);
+  const int threads = std::max(1, std::min(kThreads, omp_get_max_threads()));
+  for (size_t k = 0; k < parts && err == cudaSuccess; ++k) {
+    const size_t lo = k * kHalfBytes, hi = std::min(bytes, lo + kHalfBytes);
+    const int n = static_cast<int>((hi - lo + kChunk - 1) / kChunk);
+    int failed = 0;
+#pragma omp parallel for schedule(dynamic, 1) num_threads(threads) reduction(| : failed)
+    for (int i = 0; i < n; ++i) {
+      if (cudaEventSynchronize(g_stage.done[(k % kHalves) * kChunks + i]) != cudaSuccess) {
+        failed = 1;
+        continue;
+      }
+      const size_t at = lo + static_cast<size_t>(i) * kChunk;
+      std::memcpy(out + at, g_stage.p + (k % kHalves) * kHalfBytes + (at - lo), std::min(kChunk, hi - at));
+    }
+    if (failed) err = cudaErrorUnknown;
+    if (err == cudaSuccess && k + kHalves < parts) err = enqueue(k + kHalves);
+  }
+  const cudaError_t sync = cudaStreamSynchronize(st);  // also before the block is given back after an error
+  if (err == cudaSuccess) err = sync;
+  if (err != cudaSuccess)
+    return set_error(PLATO_ECUDA, std::string("copy of a result to the host failed: ") + cudaGetErrorString(err));
+  return PLATO_OK;
+}
+
+}  // namespace plato_b200

@@ -417,9 +417,7 @@ int batch_engine::ranks(const std::vector<uint32_t>& cols, float* out) {
         X_[0].p, X_[1].p, parity_.p, V, kt_, d_cols.p, n, g_->relabeled ? g_->to_ext.p : nullptr,
         d_out.p);
     PLATO_LAUNCHED("k_gather_columns");
-    PLATO_CUDA_TRY(cudaMemcpyAsync(out + c0 * V, d_out.p, static_cast<size_t>(n) * V * sizeof(float),
-                                   cudaMemcpyDeviceToHost, st_));
-    PLATO_CUDA_TRY(cudaStreamSynchronize(st_));
+    PLATO_TRY(copy_to_host(out + c0 * V, d_out.p, static_cast<size_t>(n) * V * sizeof(float), st_));
   }
   return PLATO_OK;
 }

@@ -793,10 +793,7 @@ int with_host_output(plato_graph* g, float* host, F&& run) {
   dbuf<float>& out = g->rank_ws->out_stage;  // kept on the graph: no allocation per call
   PLATO_TRY(out.alloc(g->info.vertices));
   PLATO_TRY(run(out.p, st));
-  PLATO_CUDA_TRY(cudaMemcpyAsync(host, out.p, g->info.vertices * sizeof(float),
-                                 cudaMemcpyDeviceToHost, st));
-  PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  return PLATO_OK;
+  return copy_to_host(host, out.p, g->info.vertices * sizeof(float), st);
 }
 
 }  // namespace
