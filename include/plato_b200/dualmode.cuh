@@ -520,6 +520,8 @@ class dualmode_engine_t {
     dev_free(result_);
   }
 
+  void set_options(dualmode_engine_opts_t opts) { opts_ = opts; }
+
   const plato_graph_info& graph_info() const { return info_; }
   uint32_t vertices() const { return view_.vertices; }
 
