@@ -693,7 +693,7 @@ def _profiled(pb, names, fn):
     return out
 
 
-HLL_KERNELS = ("k_hll_rows", "k_hll_hubs", "k_hll_spread")
+HLL_KERNELS = ("k_hll_rows", "k_hll_spread")
 
 
 def suite_hll(pb, bits=6):
@@ -711,10 +711,10 @@ def suite_hll(pb, bits=6):
     out = {"workload": "hll_rmat_s22_ef16_seed2_sym", "vertices": V, "stored_edges": E, "bits": bits}
     g.hyperanf(1, bits)
     kt = _profiled(pb, HLL_KERNELS, lambda: g.hyperanf(1, bits))
-    dev_ms = kt["k_hll_rows"][0] + kt["k_hll_hubs"][0]
+    dev_ms = kt["k_hll_rows"][0]
     alg = E * m + 4 * E + 2 * V * m + 16 * V
     peak, peak_kind = measured_peak()
-    out["full_epoch"] = {"kernel_ms": dev_ms, "rows_ms": kt["k_hll_rows"][0], "hubs_ms": kt["k_hll_hubs"][0],
+    out["full_epoch"] = {"kernel_ms": dev_ms,
                          "algorithmic_bytes": alg, "achieved_gbs": alg / (dev_ms / 1e3) / 1e9,
                          "frac": alg / (dev_ms / 1e3) / 1e9 / peak, "peak_source": f"{peak_kind} hbm_gbs"}
     times = []
@@ -725,7 +725,7 @@ def suite_hll(pb, bits=6):
     kt = _profiled(pb, HLL_KERNELS, lambda: g.hyperanf(20, bits))
     out["hyperanf"] = {"ms_median": float(np.median(times)) * 1e3, "epochs": st.iterations,
                        "push_epochs": st.push_iterations, "avg_distance": avg, "anfs": len(anfs),
-                       "gather_kernel_ms": kt["k_hll_rows"][0] + kt["k_hll_hubs"][0],
+                       "gather_kernel_ms": kt["k_hll_rows"][0],
                        "timing": "host clock around plato_hyperanf (iteration 20), median of 3"}
     rng = np.random.default_rng(2)
     for label, tg in (("all_targets", None),

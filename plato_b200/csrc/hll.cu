@@ -64,11 +64,17 @@ constexpr int kHllThreads = 256;
 constexpr uint32_t kSumBlocks = 148u * 4u;
 constexpr uint32_t kNoVertex = 0xFFFFFFFFu;
 // Rows with more sources than hub_deg = clamp(kHubBytes / m, kHubMinDeg,
-// kHubMaxDeg) go to the block-per-row kernel (measured on RMAT s22: 2048 at
+// kHubMaxDeg) have a CTA each (measured on RMAT s22: 2048 at
 // 64-byte rows, 512 from 256-byte rows up).
 constexpr uint32_t kHubBytes = 131072u;
 constexpr uint32_t kHubMinDeg = 512u;
 constexpr uint32_t kHubMaxDeg = 2048u;
+// Rows with more sources than this are split over a warp's teams.  A row split
+// in 8 ends sooner but wastes the last round of each part, which pays where
+// few rows keep the warps busy (hyperanf at P = 6 with 64 / 128 / 256, one B200:
+// RMAT s16 symmetrised 0.73 / 0.72 / 0.80 ms, s20 3.28 / 3.19 / 3.03, s22 11.0 /
+// 9.78 / 9.77).
+constexpr uint32_t kTeamDeg = 64u, kTeamDegWide = 256u, kTeamWideV = 1u << 18;
 
 __device__ __forceinline__ uint32_t rotl32(uint32_t x, int r) { return (x << r) | (x >> (32 - r)); }
 
@@ -176,14 +182,16 @@ struct gather_args {
   uint32_t* changed;          // out: bitmap of rows changed this epoch (zeroed before)
   double* est;                // per-row estimate, rewritten for changed rows
   const uint32_t* fwd_outdeg; // forward out-degree (the engine's switch weight)
-  unsigned long long* counters;  // [0] changed rows, [1] their forward out-degrees, [2] hub cursor
+  unsigned long long* counters;  // [0] changed rows, [1] their forward out-degrees, [2], [3], [4] cursors of hubs, mids and chunks
   const uint32_t* hubs;       // rows with more than hub_deg sources
-  uint32_t n_hubs;
+  const uint32_t* mids;       // rows with more than team_deg, at most hub_deg
+  uint32_t n_hubs, n_mids;
   uint32_t V;
   uint32_t P;
   uint32_t m;                 // bytes per row (1 << P)
   uint32_t passes;            // m / slice bytes
-  uint32_t hub_deg;
+  uint32_t grab;              // chunks of 32 / T rows a warp takes at a time
+  uint32_t team_deg;          // a team takes the rows with at most this many sources
   double alpha_mm;
 };
 
@@ -316,94 +324,53 @@ __device__ __forceinline__ bool team_apply(const gather_args& a, uint32_t v, siz
   return ch;
 }
 
-// One epoch over the rows with at most hub_deg sources: a team of T lanes per
-// row (grid-strided over rows).
-template <int T, int VEC>
-__global__ void __launch_bounds__(kHllThreads, 4) k_hll_rows(gather_args a) {
-  constexpr int SLICE = T * VEC * 16;
-  const int lane = threadIdx.x & 31;
-  const int tl = lane & (T - 1);
-  const int tb = lane - tl;
-  const unsigned tmask = T == 32 ? 0xFFFFFFFFu : (((1u << T) - 1u) << tb);
-  const uint64_t team = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) / T;
-  const uint64_t nteams = static_cast<uint64_t>(gridDim.x) * blockDim.x / T;
-  __shared__ uint32_t s_stage[kHllThreads / T][kChunk];
-  uint32_t* s_ids = s_stage[threadIdx.x / T];
-  unsigned long long n_chg = 0, deg_chg = 0;
-  uint64_t nb = 0, ne = 0;
-  if (team < a.V) {
-    nb = __ldg(a.off + team);
-    ne = __ldg(a.off + team + 1);
-  }
-  for (uint64_t vv = team; vv < a.V; vv += nteams) {
-    const uint32_t v = static_cast<uint32_t>(vv);
-    const uint64_t b = nb, e = ne;
-    if (vv + nteams < a.V) {  // the next row's offsets, one latency early
-      nb = __ldg(a.off + vv + nteams);
-      ne = __ldg(a.off + vv + nteams + 1);
-    }
-    if (a.covered && !test_bit(a.covered, v)) continue;
-    if (e - b > a.hub_deg) continue;
-    const bool stale = a.stale && test_bit(a.stale, v);
-    bool row_changed = false;
-    unsigned long long sfx = 0;
-    uint32_t zeros = 0;
-    for (uint32_t pass = 0; pass < a.passes; ++pass) {
-      const size_t col = static_cast<size_t>(pass) * SLICE + static_cast<size_t>(tl) * 16;
-      uint4 agg[VEC], own[VEC];
+// Bookkeeping of a changed row by the first lane of its team: the estimate,
+// the changed bit, the switch weight.
+template <int T>
+__device__ __forceinline__ void row_done(const gather_args& a, uint32_t v, int tl, unsigned tmask,
+                                         unsigned long long sfx, uint32_t zeros, unsigned long long& n_chg,
+                                         unsigned long long& deg_chg) {
 #pragma unroll
-      for (int q = 0; q < VEC; ++q) {
-        agg[q] = make_uint4(0u, 0u, 0u, 0u);
-        own[q] = agg[q];
-      }
-      if (e > b || stale) load_own<T, VEC>(a, v, col, own);  // in flight during the merge
-      const bool any = team_merge<T, VEC>(a, b, e, kChunk, col, tl, tb, tmask, s_ids, agg);
-      if (!any && !stale) break;  // same scan every pass: nothing to merge, nxt is current
-      row_changed |= team_apply<T, VEC>(a, v, col, stale, tmask, own, agg, sfx, zeros);
-    }
-    if (row_changed) {
-#pragma unroll
-      for (int o = T / 2; o > 0; o >>= 1) {
-        sfx += __shfl_xor_sync(tmask, sfx, o);
-        zeros += __shfl_xor_sync(tmask, zeros, o);
-      }
-      if (tl == 0) {
-        a.est[v] = hll_estimate(a.P, a.alpha_mm, sfx, zeros);
-        atomicOr(a.changed + (v >> 5), 1u << (v & 31));
-        ++n_chg;
-        deg_chg += __ldg(a.fwd_outdeg + v);
-      }
-    }
+  for (int o = T / 2; o > 0; o >>= 1) {
+    sfx += __shfl_xor_sync(tmask, sfx, o);
+    zeros += __shfl_xor_sync(tmask, zeros, o);
   }
-  n_chg = warp_sum(n_chg);
-  deg_chg = warp_sum(deg_chg);
-  if (lane == 0 && n_chg) {
-    atomicAdd(a.counters, n_chg);
-    atomicAdd(a.counters + 1, deg_chg);
+  if (tl == 0) {
+    a.est[v] = hll_estimate(a.P, a.alpha_mm, sfx, zeros);
+    atomicOr(a.changed + (v >> 5), 1u << (v & 31));
+    ++n_chg;
+    deg_chg += __ldg(a.fwd_outdeg + v);
   }
 }
 
-// One epoch over the rows with more than hub_deg sources: a block per row,
-// its kHllThreads / T teams splitting the sources, then a max-reduction over
-// the teams (shuffles inside a warp, shared memory across warps).
+// One epoch.  Rows by their number of sources:
+//   > hub_deg   a CTA per row, its kHllThreads / T teams splitting the sources
+//               (heaviest first, taken dynamically), then a max over the teams;
+//   > team_deg  a warp per row, its 32 / T teams splitting them the same way;
+//   the rest    a team of T lanes per row, neighbouring rows in a warp;
+// in this order, so the long rows start first and no team walks one alone.  What
+// bounds an epoch of a small graph is the longest chain of source rows behind
+// one lane; with rows handed to fixed teams and hubs in a kernel of their own it
+// was a 2048-source row.  Hyperanf, one B200, before / now: P = 4 / 6 / 8 / 12 on
+// RMAT s16 symmetrised 14.3 / 2.6 / 0.91 / 8.6 -> 1.1 / 0.73 / 0.77 / 6.3 ms, on
+// s20 15.1 / 4.4 / 7.1 / 102 -> 4.7 / 3.0 / 5.9 / 76, P = 6 on s22 10.0 -> 9.8.
 template <int T, int VEC>
-__global__ void __launch_bounds__(kHllThreads, 3) k_hll_hubs(gather_args a) {
+__global__ void __launch_bounds__(kHllThreads, VEC <= 2 ? 4 : 3) k_hll_rows(gather_args a) {
   constexpr int SLICE = T * VEC * 16;
   constexpr int kWarps = kHllThreads / 32;
   constexpr int kTeams = kHllThreads / T;
+  constexpr int kTPW = 32 / T;
+  constexpr unsigned kAll = 0xFFFFFFFFu;
   __shared__ uint4 part[kWarps][T * VEC];
   __shared__ uint32_t s_stage[kTeams][kChunk];
+  __shared__ uint32_t s_next;
   uint32_t* s_ids = s_stage[threadIdx.x / T];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tl = lane & (T - 1);
   const int tb = lane - tl;
-  const unsigned tmask = T == 32 ? 0xFFFFFFFFu : (((1u << T) - 1u) << tb);
-  const uint64_t team_first = static_cast<uint64_t>(threadIdx.x / T) * kChunk;
-  __shared__ uint32_t s_next;
+  const unsigned tmask = T == 32 ? kAll : (((1u << T) - 1u) << tb);
   unsigned long long n_chg = 0, deg_chg = 0;
-  for (;;) {
-    // hubs are listed heaviest first (ascending internal ids); blocks take the
-    // next one as they finish
+  for (;;) {  // hubs
     if (threadIdx.x == 0) s_next = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 2), 1u);
     __syncthreads();
     const uint32_t h = s_next;
@@ -421,12 +388,12 @@ __global__ void __launch_bounds__(kHllThreads, 3) k_hll_hubs(gather_args a) {
       uint4 agg[VEC];
 #pragma unroll
       for (int q = 0; q < VEC; ++q) agg[q] = make_uint4(0u, 0u, 0u, 0u);
-      bool any = team_merge<T, VEC>(a, b + team_first, e, static_cast<uint64_t>(kTeams) * kChunk, col,
-                                    tl, tb, tmask, s_ids, agg);
+      bool any = team_merge<T, VEC>(a, b + static_cast<uint64_t>(threadIdx.x / T) * kChunk, e,
+                                    static_cast<uint64_t>(kTeams) * kChunk, col, tl, tb, tmask, s_ids, agg);
 #pragma unroll
       for (int o = T; o < 32; o <<= 1)
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) agg[q] = vmax4(agg[q], shfl_xor4(0xFFFFFFFFu, agg[q], o));
+        for (int q = 0; q < VEC; ++q) agg[q] = vmax4(agg[q], shfl_xor4(kAll, agg[q], o));
       if (lane < T) {
 #pragma unroll
         for (int q = 0; q < VEC; ++q) part[warp][q * T + tl] = agg[q];
@@ -447,21 +414,89 @@ __global__ void __launch_bounds__(kHllThreads, 3) k_hll_hubs(gather_args a) {
       }
       __syncthreads();  // part is rewritten by the next pass or row
     }
-    if (warp == 0 && lane < T && row_changed) {
+    if (warp == 0 && lane < T && row_changed) row_done<T>(a, v, tl, tmask, sfx, zeros, n_chg, deg_chg);
+  }
+  if constexpr (T < 32) {
+    for (;;) {  // rows split over a warp's teams
+      uint32_t i = 0;
+      if (lane == 0) i = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 3), 1u);
+      i = __shfl_sync(kAll, i, 0);
+      if (i >= a.n_mids) break;
+      const uint32_t v = __ldg(a.mids + i);
+      if (a.covered && !test_bit(a.covered, v)) continue;
+      const uint64_t b = __ldg(a.off + v), e = __ldg(a.off + v + 1);
+      const bool stale = a.stale && test_bit(a.stale, v);
+      bool row_changed = false;
+      unsigned long long sfx = 0;
+      uint32_t zeros = 0;
+      for (uint32_t pass = 0; pass < a.passes; ++pass) {
+        const size_t col = static_cast<size_t>(pass) * SLICE + static_cast<size_t>(tl) * 16;
+        uint4 agg[VEC];
 #pragma unroll
-      for (int o = T / 2; o > 0; o >>= 1) {
-        sfx += __shfl_xor_sync(tmask, sfx, o);
-        zeros += __shfl_xor_sync(tmask, zeros, o);
+        for (int q = 0; q < VEC; ++q) agg[q] = make_uint4(0u, 0u, 0u, 0u);
+        bool any = team_merge<T, VEC>(a, b + static_cast<uint64_t>(lane / T) * kChunk, e,
+                                      static_cast<uint64_t>(kTPW) * kChunk, col, tl, tb, tmask, s_ids, agg);
+        any = __any_sync(kAll, any);
+        if (!any && !stale) break;  // warp-uniform
+#pragma unroll
+        for (int o = T; o < 32; o <<= 1)
+#pragma unroll
+          for (int q = 0; q < VEC; ++q) agg[q] = vmax4(agg[q], shfl_xor4(kAll, agg[q], o));
+        if (lane < T) {
+          uint4 own[VEC];
+          load_own<T, VEC>(a, v, col, own);
+          row_changed |= team_apply<T, VEC>(a, v, col, stale, tmask, own, agg, sfx, zeros);
+        }
       }
-      if (lane == 0) {
-        a.est[v] = hll_estimate(a.P, a.alpha_mm, sfx, zeros);
-        atomicOr(a.changed + (v >> 5), 1u << (v & 31));
-        ++n_chg;
-        deg_chg += __ldg(a.fwd_outdeg + v);
-      }
+      if (lane < T && row_changed) row_done<T>(a, v, tl, tmask, sfx, zeros, n_chg, deg_chg);
+      __syncwarp();
     }
   }
-  if (threadIdx.x == 0 && n_chg) {
+  const uint32_t nchunks = (a.V + kTPW - 1) / kTPW;
+  for (;;) {
+    uint32_t c0 = 0;
+    if (lane == 0) c0 = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 4), a.grab);
+    c0 = __shfl_sync(kAll, c0, 0);
+    if (c0 >= nchunks) break;
+    const uint32_t c1 = min(nchunks, c0 + a.grab);
+    uint64_t nb = 0, ne = 0;
+    uint64_t vv = static_cast<uint64_t>(c0) * kTPW + lane / T;
+    if (vv < a.V) {
+      nb = __ldg(a.off + vv);
+      ne = __ldg(a.off + vv + 1);
+    }
+    for (uint32_t c = c0; c < c1; ++c, vv += kTPW) {  // teams of a warp may drift apart
+      const uint32_t v = static_cast<uint32_t>(vv);
+      const uint64_t b = nb, e = ne;
+      if (c + 1 < c1 && vv + kTPW < a.V) {  // the next row's offsets, one latency early
+        nb = __ldg(a.off + vv + kTPW);
+        ne = __ldg(a.off + vv + kTPW + 1);
+      }
+      if (vv >= a.V || e - b > a.team_deg || (a.covered && !test_bit(a.covered, v))) continue;
+      const bool stale = a.stale && test_bit(a.stale, v);
+      bool row_changed = false;
+      unsigned long long sfx = 0;
+      uint32_t zeros = 0;
+      for (uint32_t pass = 0; pass < a.passes; ++pass) {
+        const size_t col = static_cast<size_t>(pass) * SLICE + static_cast<size_t>(tl) * 16;
+        uint4 agg[VEC], own[VEC];
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) {
+          agg[q] = make_uint4(0u, 0u, 0u, 0u);
+          own[q] = agg[q];
+        }
+        if (e > b || stale) load_own<T, VEC>(a, v, col, own);  // in flight during the merge
+        const bool any = team_merge<T, VEC>(a, b, e, kChunk, col, tl, tb, tmask, s_ids, agg);
+        if (!any && !stale) break;  // same scan every pass: nothing to merge, nxt is current
+        row_changed |= team_apply<T, VEC>(a, v, col, stale, tmask, own, agg, sfx, zeros);
+      }
+      if (row_changed) row_done<T>(a, v, tl, tmask, sfx, zeros, n_chg, deg_chg);
+    }
+    __syncwarp();
+  }
+  n_chg = warp_sum(n_chg);
+  deg_chg = warp_sum(deg_chg);
+  if (lane == 0 && n_chg) {
     atomicAdd(a.counters, n_chg);
     atomicAdd(a.counters + 1, deg_chg);
   }
@@ -711,12 +746,15 @@ __global__ void k_bits_weight(const uint32_t* __restrict__ bits, const uint32_t*
   }
 }
 
-// Rows with more than hub_deg sources, selected in ascending id order (on a
+// Rows by their number of sources, selected in ascending id order (on a
 // graph relabelled by descending in-degree: heaviest first).
 struct heavy_row {
   const uint64_t* off;
-  uint32_t hub_deg;
-  __device__ bool operator()(uint32_t v) const { return off[v + 1] - off[v] > hub_deg; }
+  uint32_t lo, hi;
+  __device__ bool operator()(uint32_t v) const {
+    const uint64_t d = off[v + 1] - off[v];
+    return d > lo && d <= hi;
+  }
 };
 
 // Deterministic sum of the estimates: fixed contiguous ranges per block, a
@@ -773,7 +811,8 @@ struct hll_direction {
   const uint64_t* off;
   const uint32_t* adj;
   const uint32_t* hubs;
-  uint32_t n_hubs;
+  const uint32_t* mids;
+  uint32_t n_hubs, n_mids;
 };
 
 // Per-graph HLL state, kept between calls: register buffers (released after
@@ -792,12 +831,14 @@ class hll_engine {
     const uint32_t slice = P >= 12 ? 4096u : m_;
     passes_ = m_ / slice;
     hub_deg_ = std::min(kHubMaxDeg, std::max(kHubMinDeg, kHubBytes / m_));
+    // rows of 512 bytes and more have a whole warp as their team
+    team_deg_ = P >= 9 ? hub_deg_ : V_ >= kTeamWideV ? kTeamDegWide : kTeamDeg;
     const size_t rows = static_cast<size_t>(V_ ? V_ : 1) * m_;
     PLATO_TRY(A_.alloc(rows));
     PLATO_TRY(B_.alloc(rows));
     PLATO_TRY(est_.alloc(V_ ? V_ : 1));
     PLATO_TRY(partial_.alloc(kSumBlocks + 1));
-    PLATO_TRY(ctr_.alloc(3));
+    PLATO_TRY(ctr_.alloc(5));
     words_ = (V_ + 31) / 32;
     for (auto& b : bits_) PLATO_TRY(b.alloc(words_ ? words_ : 1));
     for (auto& d : deg_) PLATO_TRY(d.alloc(V_ ? V_ : 1));
@@ -809,12 +850,15 @@ class hll_engine {
   // true); the hub rows of each direction are listed once per width class.
   int direction(bool csr, hll_direction* d) {
     const int k = csr ? 1 : 0;
-    if (hub_deg_of_[k] != hub_deg_) {
-      PLATO_TRY(list_hubs(csr ? g_->out_off.p : g_->in_off.p, hub_list_[k], &hub_n_[k]));
+    const uint64_t* off = csr ? g_->out_off.p : g_->in_off.p;
+    if (hub_deg_of_[k] != hub_deg_ || team_deg_of_[k] != team_deg_) {
+      PLATO_TRY(list_rows(off, hub_deg_, 0xFFFFFFFFu, hub_list_[k], &hub_n_[k]));
+      mid_n_[k] = 0;
+      if (team_deg_ < hub_deg_) PLATO_TRY(list_rows(off, team_deg_, hub_deg_, mid_list_[k], &mid_n_[k]));
       hub_deg_of_[k] = hub_deg_;
+      team_deg_of_[k] = team_deg_;
     }
-    *d = hll_direction{csr ? g_->out_off.p : g_->in_off.p, csr ? g_->out_adj.p : g_->in_adj.p,
-                       hub_list_[k].p, hub_n_[k]};
+    *d = hll_direction{off, csr ? g_->out_adj.p : g_->in_adj.p, hub_list_[k].p, mid_list_[k].p, hub_n_[k], mid_n_[k]};
     return PLATO_OK;
   }
 
@@ -829,13 +873,14 @@ class hll_engine {
   uint32_t* degrees(int i) { return deg_[i].p; }
 
  private:
-  int list_hubs(const uint64_t* off, dbuf<uint32_t>& list, uint32_t* n) {
+  // Rows with more than `lo` and at most `hi` sources.
+  int list_rows(const uint64_t* off, uint32_t lo, uint32_t hi, dbuf<uint32_t>& list, uint32_t* n) {
     PLATO_TRY(list.alloc(V_ ? V_ : 1));
     *n = 0;
     if (!V_) return PLATO_OK;
     uint32_t* cnt = reinterpret_cast<uint32_t*>(ctr_.p);
     const thrust::counting_iterator<uint32_t> ids(0);
-    const heavy_row pred{off, hub_deg_};
+    const heavy_row pred{off, lo, hi};
     size_t bytes = 0;
     PLATO_CUDA_TRY(cub::DeviceSelect::If(nullptr, bytes, ids, list.p, cnt, V_, pred, st_));
     PLATO_TRY(select_tmp_.alloc(bytes ? bytes : 1));
@@ -856,7 +901,7 @@ class hll_engine {
     return PLATO_OK;
   }
   int zero_counters() {
-    PLATO_CUDA_TRY(cudaMemsetAsync(ctr_.p, 0, 3 * sizeof(unsigned long long), st_));
+    PLATO_CUDA_TRY(cudaMemsetAsync(ctr_.p, 0, 5 * sizeof(unsigned long long), st_));
     return PLATO_OK;
   }
   int read_counters(unsigned long long* n, unsigned long long* deg) {
@@ -910,12 +955,14 @@ class hll_engine {
       a.fwd_outdeg = g_->out_deg.p;
       a.counters = ctr_.p;
       a.hubs = dir.hubs;
+      a.mids = dir.mids;
       a.n_hubs = dir.n_hubs;
+      a.n_mids = dir.n_mids;
       a.V = V_;
       a.P = P_;
       a.m = m_;
       a.passes = passes_;
-      a.hub_deg = hub_deg_;
+      a.team_deg = team_deg_;
       a.alpha_mm = alpha_;
       PLATO_TRY(launch_gather(a));
     }
@@ -1037,26 +1084,25 @@ class hll_engine {
   }
 
   template <int T, int VEC>
-  int launch(const gather_args& a) {
-    {
-      prof_scope ps("k_hll_rows", st_);
-      const unsigned grid = grid_for(static_cast<uint64_t>(V_) * T, kHllThreads, 148u * 8u);
-      k_hll_rows<T, VEC><<<grid, kHllThreads, 0, st_>>>(a);
-      PLATO_LAUNCHED("k_hll_rows");
+  int launch(gather_args a) {
+    static int per_sm = 0;  // resident CTAs: the rows are taken dynamically
+    if (per_sm == 0) {
+      int n = 0;
+      PLATO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_hll_rows<T, VEC>, kHllThreads, 0));
+      per_sm = std::max(n, 1);
     }
-    if (a.n_hubs) {
-      prof_scope ps("k_hll_hubs", st_);
-      const unsigned grid = a.n_hubs < 148u * 8u ? a.n_hubs : 148u * 8u;
-      k_hll_hubs<T, VEC><<<grid, kHllThreads, 0, st_>>>(a);
-      PLATO_LAUNCHED("k_hll_hubs");
-    }
+    const uint32_t warps = 148u * per_sm * (kHllThreads / 32);
+    a.grab = std::min(8u, std::max(1u, V_ / (32 / T) / (8 * warps)));
+    prof_scope ps("k_hll_rows", st_);
+    k_hll_rows<T, VEC><<<148u * per_sm, kHllThreads, 0, st_>>>(a);
+    PLATO_LAUNCHED("k_hll_rows");
     return PLATO_OK;
   }
 
   plato_graph* g_;
   cudaStream_t st_;
   uint32_t V_;
-  uint32_t P_ = 0, m_ = 0, passes_ = 1, hub_deg_ = 0, words_ = 0;
+  uint32_t P_ = 0, m_ = 0, passes_ = 1, hub_deg_ = 0, team_deg_ = 0, words_ = 0;
   double alpha_ = 0.0;
   dbuf<uint8_t> A_, B_;
   uint8_t* cur_ = nullptr;
@@ -1066,9 +1112,9 @@ class hll_engine {
   dbuf<uint8_t> select_tmp_;
   dbuf<uint32_t> bits_[5];
   dbuf<uint32_t> deg_[2];
-  dbuf<uint32_t> hub_list_[2];
-  uint32_t hub_n_[2] = {0, 0};
-  uint32_t hub_deg_of_[2] = {0, 0};
+  dbuf<uint32_t> hub_list_[2], mid_list_[2];
+  uint32_t hub_n_[2] = {0, 0}, mid_n_[2] = {0, 0};
+  uint32_t hub_deg_of_[2] = {0, 0}, team_deg_of_[2] = {0, 0};
   struct pinned {
     unsigned long long* p = nullptr;
     int alloc(size_t n) {
