@@ -361,6 +361,13 @@ int create_impl(const plato_graph_info* info, const uint32_t* src, const uint32_
 
 }  // namespace
 
+int merge_tile_starts(const uint64_t* off, uint32_t V, uint64_t E, uint32_t items, uint32_t T, uint32_t* trow,
+                      uint64_t* tedge, cudaStream_t st) {
+  k_merge_tiles<<<grid_for(T + 1ull, 256), 256, 0, st>>>(off, V, E, items, T, trow, tedge);
+  PLATO_LAUNCHED("k_merge_tiles");
+  return PLATO_OK;
+}
+
 int ensure_pull_tiles(plato_graph* g, uint32_t items, cudaStream_t st, const merge_tiles** out) {
   auto it = g->tiles.find(items);
   if (it != g->tiles.end()) {
@@ -375,10 +382,8 @@ int ensure_pull_tiles(plato_graph* g, uint32_t items, cudaStream_t st, const mer
   mt.count = static_cast<uint32_t>(T);
   PLATO_TRY(mt.row.alloc(T + 1));
   PLATO_TRY(mt.edge.alloc(T + 1));
-  k_merge_tiles<<<grid_for(T + 1, 256), 256, 0, st>>>(g->in_off.p, g->info.vertices,
-                                                      g->stored_edges, items, mt.count, mt.row.p,
-                                                      mt.edge.p);
-  PLATO_LAUNCHED("k_merge_tiles");
+  PLATO_TRY(merge_tile_starts(g->in_off.p, g->info.vertices, g->stored_edges, items, mt.count, mt.row.p, mt.edge.p,
+                              st));
   auto& slot = g->tiles[items];
   slot = std::move(mt);
   if (out) *out = &slot;
@@ -444,6 +449,7 @@ plato_graph::~plato_graph() {
   plato_b200::destroy_bfs_workspace(bfs_ws);
   plato_b200::destroy_hll_workspace(hll_ws);
   plato_b200::destroy_cc_workspace(cc_ws);
+  plato_b200::destroy_trust_workspace(trust_ws);
   if (stream) cudaStreamDestroy(stream);
 }
 

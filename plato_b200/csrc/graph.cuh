@@ -27,10 +27,12 @@ struct bfs_workspace;    // bfs.cu
 class batch_engine;      // ppr_batch.cu
 struct hll_workspace;    // hll.cu
 struct cc_workspace;     // cc.cu
+struct trust_workspace;  // trustrank.cu
 void destroy_rank_workspace(rank_workspace*);
 void destroy_bfs_workspace(bfs_workspace*);
 void destroy_hll_workspace(hll_workspace*);
 void destroy_cc_workspace(cc_workspace*);
+void destroy_trust_workspace(trust_workspace*);
 void destroy_batch_engine(batch_engine*);
 
 }  // namespace plato_b200
@@ -59,6 +61,7 @@ struct plato_graph {
   plato_b200::bfs_workspace* bfs_ws = nullptr;
   plato_b200::hll_workspace* hll_ws = nullptr;  // HyperLogLog buffers (hll.cu)
   plato_b200::cc_workspace* cc_ws = nullptr;    // the engine of connected components (cc.cu)
+  plato_b200::trust_workspace* trust_ws = nullptr;  // seed selection (trustrank.cu)
   plato_b200::batch_engine* batch_cache = nullptr;  // plato_ppr_batch state, kept between calls
   std::vector<uint32_t> h_to_int;             // host copy of to_int (lazily)
   std::map<uint32_t, uint32_t> batch_tuned;   // K bucket -> columns per tile (kt)
@@ -67,6 +70,10 @@ struct plato_graph {
 };
 
 namespace plato_b200 {
+
+// Merge-path coordinates of the T + 1 tile starts of any offsets.
+int merge_tile_starts(const uint64_t* off, uint32_t V, uint64_t E, uint32_t items, uint32_t T, uint32_t* trow,
+                      uint64_t* tedge, cudaStream_t st);
 
 // Builds (once) the merge-path tiles of the CSC for `items` per tile.
 int ensure_pull_tiles(plato_graph* g, uint32_t items, cudaStream_t st,

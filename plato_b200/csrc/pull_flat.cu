@@ -32,44 +32,41 @@ constexpr uint32_t kFlatRowDeg1 = 64;
 constexpr uint64_t kFlatRunEdges = 3500000;
 constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 600000;
 
-// out[0..1]: rows above the two in-degree limits; out[2 + k]: out-edges of block k.
-__global__ void __launch_bounds__(256) k_flat_survey(const uint32_t* __restrict__ in_deg,
-                                                     const uint32_t* __restrict__ out_deg, uint32_t V,
+// out[0]: one past the last row above kFlatRowDeg1 edges, out[1]: how many there
+// are, out[2 + k]: gathers of the sources of block k (`uses` by source).
+__global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict__ off,
+                                                     const uint32_t* __restrict__ uses, uint32_t V, uint32_t block,
                                                      uint32_t nblocks, unsigned long long* out) {
   __shared__ unsigned long long s_red[32];
-  if (blockIdx.x == 0 && threadIdx.x < 2) {
-    const uint32_t limit = threadIdx.x == 0 ? kFlatRowDeg0 : kFlatRowDeg1;
-    uint32_t lo = 0, hi = V;
-    while (lo < hi) {
-      const uint32_t mid = lo + (hi - lo) / 2;
-      if (in_deg[mid] > limit) lo = mid + 1; else hi = mid;
+  unsigned long long last = 0, n = 0;
+  for (uint64_t v = blockIdx.x * 256ull + threadIdx.x; v < V; v += gridDim.x * 256ull)
+    if (off[v + 1] - off[v] > kFlatRowDeg1) {
+      last = v + 1;
+      ++n;
     }
-    out[threadIdx.x] = lo;
-  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
+  if ((threadIdx.x & 31) == 0 && last) atomicMax(out, last);
+  n = block_sum_u64<256>(n, s_red);
+  if (threadIdx.x == 0 && n) atomicAdd(out + 1, n);
   // 8 CTAs a block of sources
   const uint32_t k = blockIdx.x / 8, q = blockIdx.x % 8;
   if (k >= nblocks) return;
-  const uint32_t b = k * kFlatBlock, e = min(V, b + kFlatBlock);
-  unsigned long long n = 0;
-  for (uint32_t v = b + q * 256 + threadIdx.x; v < e; v += 8 * 256) n += out_deg[v];
+  const uint32_t b = k * block, e = min(V, b + block);
+  n = 0;
+  for (uint32_t v = b + q * 256 + threadIdx.x; v < e; v += 8 * 256) n += uses[v];
   n = block_sum_u64<256>(n, s_red);
   if (threadIdx.x == 0) atomicAdd(out + 2 + k, n);
-}
-
-// Whether the columns are in order of descending in-degree.
-__global__ void k_flat_unsorted(const uint32_t* __restrict__ deg, uint32_t V, uint32_t* bad) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x + 1; v < V;
-       v += (uint64_t)gridDim.x * blockDim.x)
-    if (deg[v] > deg[v - 1]) *bad = 1;
 }
 
 struct flat_rows {
   const uint64_t* off;
   const uint32_t* adj;
-  uint32_t V, nb, r0, r1, rows1;  // rows1: r1 rounded up to whole 32-row words
+  uint32_t V, nb, block, rows1;  // rows1: the rows of the middle streams, in whole 32-row words
   // hot streams that row v takes part in
   __device__ __forceinline__ uint32_t streams(uint32_t v) const {
-    return v < r1 ? nb : v < r0 ? min(nb, 1u) : 0u;
+    const uint64_t d = off[v + 1] - off[v];
+    return d > kFlatRowDeg1 ? nb : d > kFlatRowDeg0 ? min(nb, 1u) : 0u;
   }
   __device__ __forceinline__ uint64_t cell(uint32_t k, uint32_t v) const { return flat_place(k, V, rows1) + v; }
 };
@@ -86,7 +83,7 @@ __global__ void k_flat_split(flat_rows f, uint32_t* cnt) {
       if (k > 0 && v >= f.rows1) break;
       uint64_t lo = pos;
       if (k < ns) {
-        const uint32_t bound = (k + 1) * kFlatBlock;
+        const uint32_t bound = (k + 1) * f.block;
         uint64_t hi = end;
         while (lo < hi) {
           const uint64_t mid = (lo + hi) >> 1;
@@ -101,8 +98,8 @@ __global__ void k_flat_split(flat_rows f, uint32_t* cnt) {
 }
 
 struct flat_starts {
-  uint32_t edge[kFlatMaxBlocks + 1];  // first edge of each stream (padded numbering)
-  uint32_t sum[kFlatMaxBlocks + 1];   // edges of the streams before it (unpadded)
+  uint64_t edge[kFlatMaxBlocks + 1];  // first edge of each stream (padded numbering)
+  uint64_t sum[kFlatMaxBlocks + 1];   // edges of the streams before it (unpadded)
 };
 
 // Copies every edge (and its weight) to its stream and flags segment ends.  A
@@ -110,12 +107,12 @@ struct flat_starts {
 __global__ void __launch_bounds__(256) k_flat_fill(flat_rows f, const uint32_t* __restrict__ trow,
                                                    const uint64_t* __restrict__ tedge, uint32_t tiles,
                                                    const uint32_t* __restrict__ cnt,
-                                                   const uint32_t* __restrict__ pos, flat_starts st,
+                                                   const uint64_t* __restrict__ pos, flat_starts st,
                                                    const float* __restrict__ w, uint16_t* hid, uint32_t* cid,
                                                    float* hw, float* cw, uint32_t* hflags, uint32_t* cflags) {
   const unsigned lane = threadIdx.x & 31;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t cold0 = st.edge[f.nb];
+  const uint64_t cold0 = st.edge[f.nb];
   for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tiles; t += nwarps) {
     const uint32_t ra = trow[t], rb = min(trow[t + 1], f.V - 1);
     const uint64_t je = tedge[t + 1];
@@ -128,16 +125,16 @@ __global__ void __launch_bounds__(256) k_flat_fill(flat_rows f, const uint32_t* 
       const uint32_t v = lo;
       const uint32_t id = f.adj[e];
       const uint32_t ns = f.streams(v);
-      uint32_t k = id / kFlatBlock;
+      uint32_t k = id / f.block;
       if (k >= ns) k = f.nb;
       uint32_t before = 0;
       for (uint32_t j = 0; j < min(k, ns); ++j) before += cnt[f.cell(j, v)];
       const size_t at = f.cell(k, v);
       const uint32_t i = static_cast<uint32_t>(e - f.off[v]) - before;
-      uint32_t to = st.edge[k] + (pos[at] - st.sum[k]) + i;
+      uint64_t to = st.edge[k] + (pos[at] - st.sum[k]) + i;
       uint32_t* flags = hflags;
       if (k < f.nb) {
-        hid[to] = static_cast<uint16_t>(id - k * kFlatBlock);
+        hid[to] = static_cast<uint16_t>(id - k * f.block);
         if (w) hw[to] = w[e];
       } else {
         to -= cold0;
@@ -200,12 +197,13 @@ struct flat_crossing {
 };
 
 // Piece p continues a segment of an earlier piece; *j is its ordinal.
-__device__ __forceinline__ bool flat_continues(const flat_view& f, uint32_t p, uint32_t* j) {
+template <class S>
+__device__ __forceinline__ bool flat_continues(const flat_view<S>& f, uint32_t p, uint32_t* j) {
   const uint2 pc = f.pieces[p];
   if ((pc.x & kPieceFirst) || pc.x >= pc.y) return false;
   const size_t before = static_cast<size_t>(pc.x) * 32 - 1;
   if (p < f.cold_piece0) {
-    if (f.hmark[before] >> (kFlatHotLane - 1) & 1u) return false;
+    if (f.hmark[before] >> (flat_hot_lane<S> - 1) & 1u) return false;
     *j = f.hseg[pc.x];
   } else {
     if (f.cmark[before] >> (kFlatColdLane - 1) & 1u) return false;
@@ -217,8 +215,8 @@ __device__ __forceinline__ bool flat_continues(const flat_view& f, uint32_t p, u
 // Segments cut by piece boundaries, one thread per piece; the first piece
 // that continues a segment records it.  fill = false marks the rows in
 // meta.z, fill = true writes the spans (meta.w scanned in between).
-template <bool kFill>
-__global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans) {
+template <bool kFill, class S>
+__global__ void k_flat_spans(flat_view<S> f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t j = 0;
   if (p >= npieces || !flat_continues(f, p, &j) || j >= segments) return;
@@ -283,13 +281,14 @@ struct scratch {
   }
 };
 
-template <class It>
-int scan_u32(It in, uint32_t* out, uint64_t n, cudaMemPool_t pool, cudaStream_t st) {
+template <class It, typename T>
+int scan(It in, T* out, uint64_t n, cudaMemPool_t pool, cudaStream_t st) {
   size_t bytes = 0;
-  PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, static_cast<int64_t>(n), st));
+  const auto plus = [] __device__(T a, T b) -> T { return a + b; };  // sums in T, whatever the input's type
+  PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveScan(nullptr, bytes, in, out, plus, T(0), static_cast<int64_t>(n), st));
   scratch<uint8_t> tmp(st);
   PLATO_TRY(tmp.alloc(pool, bytes));
-  PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, in, out, static_cast<int64_t>(n), st));
+  PLATO_CUDA_TRY(cub::DeviceScan::ExclusiveScan(tmp.p, bytes, in, out, plus, T(0), static_cast<int64_t>(n), st));
   count_launch();
   return PLATO_OK;
 }
@@ -313,12 +312,18 @@ int put(T* d, const std::vector<T>& h, cudaStream_t st) {
 
 }  // namespace
 
-int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
+template <class S>
+int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st) {
+  constexpr uint32_t kBlock = flat_block<S>, kHotStep = flat_hot_step<S>;
+  constexpr int kHotLane = flat_hot_lane<S>;
   const uint32_t V = g->info.vertices;
   const uint64_t E = g->stored_edges;
   pl.valid = false;
-  if (!g->relabeled || !g->own_sources || E == 0 || E > 0xF0000000ull) return PLATO_OK;
-  const uint32_t nblocks = std::min<uint32_t>((V + kFlatBlock - 1) / kFlatBlock, kFlatMaxBlocks);
+  if (!g->own_sources || E == 0) return PLATO_OK;
+  const uint64_t* off = out ? g->out_off.p : g->in_off.p;
+  const uint32_t* adj = out ? g->out_adj.p : g->in_adj.p;
+  const bool weighted = g->weighted && !out && sizeof(S) == 4;
+  const uint32_t nblocks = std::min<uint32_t>((V + kBlock - 1) / kBlock, kFlatMaxBlocks);
   cudaMemPool_t pool{};
   try {
     pool = engine_pool();
@@ -326,56 +331,55 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
     return set_error(PLATO_ECUDA, e.what());
   }
   scratch<unsigned long long> d_survey(st);
-  PLATO_TRY(d_survey.alloc(pool, 2 + kFlatMaxBlocks + 1));
-  PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, (2 + kFlatMaxBlocks + 1) * sizeof(unsigned long long), st));
-  k_flat_survey<<<nblocks * 8, 256, 0, st>>>(g->in_deg.p, g->out_deg.p, V, nblocks, d_survey.p);
+  PLATO_TRY(d_survey.alloc(pool, 2 + kFlatMaxBlocks));
+  PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, (2 + kFlatMaxBlocks) * sizeof(unsigned long long), st));
+  k_flat_survey<<<std::max(nblocks * 8, grid_for(V, 256, 148 * 4)), 256, 0, st>>>(
+      off, out ? g->in_deg.p : g->out_deg.p, V, kBlock, nblocks, d_survey.p);
   PLATO_LAUNCHED("k_flat_survey");
-  k_flat_unsorted<<<grid_for(V, 256), 256, 0, st>>>(
-      g->in_deg.p, V, reinterpret_cast<uint32_t*>(d_survey.p + 2 + kFlatMaxBlocks));
-  PLATO_LAUNCHED("k_flat_unsorted");
-  unsigned long long h[2 + kFlatMaxBlocks + 1];
+  unsigned long long h[2 + kFlatMaxBlocks];
   PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  if (h[2 + kFlatMaxBlocks]) return PLATO_OK;  // another vertex order
-  flat_rows rows{g->in_off.p, g->in_adj.p, V, 0, static_cast<uint32_t>(h[0]), static_cast<uint32_t>(h[1]), 0};
+  flat_rows rows{off, adj, V, 0, kBlock, 0};
   uint32_t nb = 0;
   const bool run = E <= kFlatRunEdges;
   if (!run && h[2] >= kFlatFirst)
     for (nb = 1; nb < nblocks && h[2 + nb] >= std::max(kFlatMore, h[1]) && h[1] > 0;) ++nb;
   rows.nb = nb;
-  rows.rows1 = std::min((rows.r1 + 31) / 32 * 32, V);  // V: the last word may be short
+  // whole words; the last may be short
+  rows.rows1 = nb > 1 ? std::min((static_cast<uint32_t>(h[0]) + 31) / 32 * 32, V) : 0;
   const uint32_t streams = nb + 1, words = (V + 31) / 32, words1 = (rows.rows1 + 31) / 32;
   const uint64_t cells = flat_place(nb, V, rows.rows1) + V;
 
-  scratch<uint32_t> cnt(st), pos(st), ord(st);
+  scratch<uint32_t> cnt(st), ord(st);
+  scratch<uint64_t> pos(st);
   PLATO_TRY(cnt.alloc(pool, cells));
   PLATO_TRY(pos.alloc(pool, cells));
   PLATO_TRY(ord.alloc(pool, cells));
   k_flat_split<<<grid_for(V, 256), 256, 0, st>>>(rows, cnt.p);
   PLATO_LAUNCHED("k_flat_split");
-  PLATO_TRY(scan_u32(cnt.p, pos.p, cells, pool, st));
-  PLATO_TRY(scan_u32(thrust::make_transform_iterator(cnt.p, flat_has()), ord.p, cells, pool, st));
+  PLATO_TRY(scan(cnt.p, pos.p, cells, pool, st));
+  PLATO_TRY(scan(thrust::make_transform_iterator(cnt.p, flat_has()), ord.p, cells, pool, st));
   // edges before each stream, and the last cells for the number of segments
-  std::vector<uint32_t> sum(streams + 1, 0);
+  std::vector<uint64_t> sum(streams + 1, 0);
   uint32_t last_cnt = 0, segments = 0;
   for (uint32_t k = 0; k < streams; ++k)
-    PLATO_CUDA_TRY(cudaMemcpyAsync(&sum[k], pos.p + flat_place(k, V, rows.rows1), 4, cudaMemcpyDeviceToHost, st));
+    PLATO_CUDA_TRY(cudaMemcpyAsync(&sum[k], pos.p + flat_place(k, V, rows.rows1), 8, cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaMemcpyAsync(&last_cnt, cnt.p + cells - 1, 4, cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaMemcpyAsync(&segments, ord.p + cells - 1, 4, cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
   segments += last_cnt != 0;
-  sum[streams] = static_cast<uint32_t>(E);
+  sum[streams] = E;
   flat_starts fs{};
-  uint32_t edges = 0;
+  uint64_t edges = 0;
   for (uint32_t k = 0; k < streams; ++k) {
-    const uint32_t step = k < nb ? kFlatHotStep : kFlatColdStep;
+    const uint32_t step = k < nb ? kHotStep : kFlatColdStep;
     fs.edge[k] = edges;
     fs.sum[k] = sum[k];
     edges += (sum[k + 1] - sum[k] + step - 1) / step * step;
   }
-  const uint32_t hot_edges = fs.edge[nb], cold_edges = edges - hot_edges;
-  const uint32_t hot_steps = hot_edges / kFlatHotStep, cold_steps = cold_edges / kFlatColdStep;
-  const bool weighted = g->weighted;
+  const uint64_t hot_edges = fs.edge[nb], cold_edges = edges - hot_edges;
+  const uint32_t hot_steps = static_cast<uint32_t>(hot_edges / kHotStep);
+  const uint32_t cold_steps = static_cast<uint32_t>(cold_edges / kFlatColdStep);
   // grids, and bounds on the pieces
   int sms = 0;
   PLATO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
@@ -404,11 +408,11 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   const size_t o_hid = lay.add(hot_edges * 2ull), o_cid = lay.add(cold_edges * 4ull);
   const size_t o_hw = lay.add(weighted ? hot_edges * 4ull : 0), o_cw = lay.add(weighted ? cold_edges * 4ull : 0);
   const size_t o_hmark = lay.add(hot_steps * 128ull), o_cmark = lay.add(cold_steps * 64ull);
-  const size_t o_seg = lay.add((hot_steps + cold_steps) * 4ull), o_meta = lay.add(nmeta * sizeof(uint4));
+  const size_t o_seg = lay.add((static_cast<uint64_t>(hot_steps) + cold_steps) * 4), o_meta = lay.add(nmeta * sizeof(uint4));
   const size_t o_spans = lay.add(max_pieces * sizeof(uint2)), o_pieces = lay.add(max_pieces * sizeof(uint2));
   const size_t o_subs = lay.add(max_subs * sizeof(flat_sub)), o_cta = lay.add((pl.hot_ctas + 1) * 4ull);
-  const size_t o_part = lay.add(segments * 4ull), o_head = lay.add(max_pieces * 4ull);
-  const size_t o_carry = lay.add(max_pieces * 4ull);
+  const size_t o_part = lay.add(segments * sizeof(S)), o_head = lay.add(max_pieces * sizeof(S));
+  const size_t o_carry = lay.add(max_pieces * sizeof(S));
   PLATO_TRY(pl.mem.alloc(lay.bytes));
   unsigned char* mem = pl.mem.p;
   uint16_t* hid = reinterpret_cast<uint16_t*>(mem + o_hid);
@@ -430,28 +434,33 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   PLATO_CUDA_TRY(cudaMemsetAsync(cflags.p, 0, cold_edges / 8, st));
   // the padding of a stream's last step: source 0, weight 0, no flag
   for (uint32_t k = 0; k < streams; ++k) {
-    const uint32_t end = k + 1 < streams ? fs.edge[k + 1] : edges;
+    const uint64_t end = k + 1 < streams ? fs.edge[k + 1] : edges;
     if (end == fs.edge[k]) continue;
     if (k < nb) {
-      PLATO_CUDA_TRY(cudaMemsetAsync(hid + (end - kFlatHotStep), 0, kFlatHotStep * 2, st));
-      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(hw + (end - kFlatHotStep), 0, kFlatHotStep * 4, st));
+      PLATO_CUDA_TRY(cudaMemsetAsync(hid + (end - kHotStep), 0, kHotStep * 2, st));
+      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(hw + (end - kHotStep), 0, kHotStep * 4, st));
     } else {
-      const uint32_t b = cold_edges - kFlatColdStep;
+      const uint64_t b = cold_edges - kFlatColdStep;
       PLATO_CUDA_TRY(cudaMemsetAsync(cid + b, 0, kFlatColdStep * 4, st));
       if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(cw + b, 0, kFlatColdStep * 4, st));
     }
   }
-  const merge_tiles* mt = nullptr;
-  PLATO_TRY(ensure_pull_tiles(g, 224, st, &mt));
-  k_flat_fill<<<grid_for(static_cast<uint64_t>(mt->count) * 32, 256), 256, 0, st>>>(
-      rows, mt->row.p, mt->edge.p, mt->count, cnt.p, pos.p, fs, weighted ? g->in_w.p : nullptr, hid, cid, hw,
+  // merge tiles of the direction's rows and edges, 224 of both a tile
+  const uint32_t tiles = static_cast<uint32_t>((V + E + 223) / 224);
+  scratch<uint32_t> trow(st);
+  scratch<uint64_t> tedge(st);
+  PLATO_TRY(trow.alloc(pool, tiles + 1));
+  PLATO_TRY(tedge.alloc(pool, tiles + 1));
+  PLATO_TRY(merge_tile_starts(off, V, E, 224, tiles, trow.p, tedge.p, st));
+  k_flat_fill<<<grid_for(static_cast<uint64_t>(tiles) * 32, 256), 256, 0, st>>>(
+      rows, trow.p, tedge.p, tiles, cnt.p, pos.p, fs, weighted ? g->in_w.p : nullptr, hid, cid, hw,
       cw, hflags.p, cflags.p);
   PLATO_LAUNCHED("k_flat_fill");
   // marks, and segments that end before each step (numbered through all streams)
   scratch<uint32_t> ends(st);
   PLATO_TRY(ends.alloc(pool, hot_steps + cold_steps));
   if (hot_steps) {
-    k_flat_marks<kFlatHotLane, uint32_t><<<grid_for(hot_steps * 32ull, 256), 256, 0, st>>>(hflags.p, hot_steps,
+    k_flat_marks<kHotLane, uint32_t><<<grid_for(hot_steps * 32ull, 256), 256, 0, st>>>(hflags.p, hot_steps,
                                                                                            hmark, ends.p);
     PLATO_LAUNCHED("k_flat_marks");
   }
@@ -460,7 +469,7 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
         cflags.p, cold_steps, cmark, ends.p + hot_steps);
     PLATO_LAUNCHED("k_flat_marks");
   }
-  PLATO_TRY(scan_u32(ends.p, seg, hot_steps + cold_steps, pool, st));
+  PLATO_TRY(scan(ends.p, seg, hot_steps + cold_steps, pool, st));
   k_flat_meta<<<grid_for(nmeta * 32, 256), 256, 0, st>>>(rows, cnt.p, ord.p, words, nmeta, meta);
   PLATO_LAUNCHED("k_flat_meta");
 
@@ -503,7 +512,8 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
     cta_sub.push_back(static_cast<uint32_t>(subs.size()));
     const uint32_t b = c + 1 == pl.hot_ctas ? hot_steps : at_cost(a, hot_steps, static_cast<double>(cost[hot_steps]) * (c + 1) / pl.hot_ctas);
     for (uint32_t k = 0; k < nb; ++k) {
-      const uint32_t k0 = fs.edge[k] / kFlatHotStep, k1 = fs.edge[k + 1] / kFlatHotStep;
+      const uint32_t k0 = static_cast<uint32_t>(fs.edge[k] / kHotStep);
+      const uint32_t k1 = static_cast<uint32_t>(fs.edge[k + 1] / kHotStep);
       const uint32_t lo = std::max(a, k0), hi = std::min(b, k1);
       if (lo >= hi) continue;
       subs.push_back(flat_sub{k, static_cast<uint32_t>(pieces.size())});
@@ -525,8 +535,8 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   PLATO_TRY(put(d_pieces, pieces, st));
   PLATO_TRY(put(d_subs, subs, st));
   PLATO_TRY(put(d_cta, cta_sub, st));
-  flat_view& f = pl.v;
-  f = flat_view{};
+  flat_view<S>& f = pl.v;
+  f = flat_view<S>{};
   f.V = f.nsrc = V;
   f.nb = nb;
   f.words = words;
@@ -546,24 +556,34 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   f.subs = d_subs;
   f.meta = meta;
   f.spans = spans;
-  f.part = reinterpret_cast<float*>(mem + o_part);
-  f.head = reinterpret_cast<float*>(mem + o_head);
-  f.carry = reinterpret_cast<float*>(mem + o_carry);
+  f.part = reinterpret_cast<S*>(mem + o_part);
+  f.head = reinterpret_cast<S*>(mem + o_head);
+  f.carry = reinterpret_cast<S*>(mem + o_carry);
   const unsigned span_grid = (npieces + 127) / 128;
-  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr);
+  k_flat_spans<false, S><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr);
   PLATO_LAUNCHED("k_flat_spans");
   scratch<uint32_t> base(st);
   PLATO_TRY(base.alloc(pool, nmeta));
-  PLATO_TRY(scan_u32(thrust::make_transform_iterator(thrust::counting_iterator<uint32_t>(0), flat_crossing{meta}),
+  PLATO_TRY(scan(thrust::make_transform_iterator(thrust::counting_iterator<uint32_t>(0), flat_crossing{meta}),
                      base.p, nmeta, pool, st));
   k_flat_span_base<<<grid_for(nmeta, 256), 256, 0, st>>>(base.p, nmeta, meta);
   PLATO_LAUNCHED("k_flat_span_base");
-  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans);
+  k_flat_spans<true, S><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans);
   PLATO_LAUNCHED("k_flat_spans");
   pl.update_blocks = std::min<uint32_t>(sms * 4, (words + 15) / 16);
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));  // the temporaries and the host vectors go
+  if (pl.hot_ctas) {
+    PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        kFlatBlockBytes));
+    if constexpr (sizeof(S) == 4)
+      PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          kFlatBlockBytes));
+  }
   pl.valid = true;
   return PLATO_OK;
 }
+
+template int build_flat_plan<float>(plato_graph*, bool, flat_plan<float>&, cudaStream_t);
+template int build_flat_plan<double>(plato_graph*, bool, flat_plan<double>&, cudaStream_t);
 
 }  // namespace plato_b200

@@ -48,7 +48,7 @@ struct rank_workspace {
   uint32_t hub_cap = 0;       // ranks the pull kernel can stage in shared memory
   bool plan_built = false;
   pull_plan plan;
-  flat_plan flat;
+  flat_plan<float> flat;
   dbuf<uint32_t> seed_bits, seed_list;  // seed-set PPR
   dbuf<float> out_stage;                // caller-id ranks before the copy to the host
   dbuf<int> ctrl;                       // device epoch control (k_epoch_control); [2], [3] k_flat_run's barrier
@@ -80,6 +80,7 @@ using cfg = pull_warp_cfg<kIPT>;
 // A vertex whose out-weights sum to 0 gets x' = inf, so its edges give
 // inf * 0 = NaN, as the reference's 0 / 0 does.
 struct wrank_update {
+  using value = float;
   const float* r;                  // current ranks
   float* rn;                       // next ranks
   float* xn;                       // next gathered state
@@ -136,6 +137,7 @@ struct wrank_update {
 // epoch itself carries the exchange that an all-gather would do after it.
 constexpr uint32_t kMaxPartitionPeers = 7;  // 8 partitions (one node) at most
 struct bcast_rank_update {
+  using value = float;
   rank_update<teleport_uniform> u;  // local replica: u.xn
   float* peers[kMaxPartitionPeers];  // this partition's slice of the next state in the other replicas
   uint32_t npeers;
@@ -270,7 +272,7 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
   rank_workspace* ws = g->rank_ws;
   const uint32_t V = g->info.vertices;
   if (!ws->plan_built) {
-    PLATO_TRY(build_flat_plan(g, ws->flat, st));
+    PLATO_TRY(build_flat_plan(g, false, ws->flat, st));
     if (!ws->flat.valid) PLATO_TRY(build_plan(g, ws->plan, st));
     ws->plan_built = true;
   }
@@ -296,8 +298,6 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
   if (!ws->h_ctrl) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_ctrl), 8 * sizeof(int)));
   for (cudaEvent_t& e : ws->polled)
     if (!e) PLATO_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlatBlock * 4));
-  PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlatBlock * 4));
   uint32_t cap_a = 0, cap_b = 0;
   PLATO_TRY(set_pull_smem_attr<rank_update<teleport_uniform>>(g->device, &cap_a));
   PLATO_TRY(set_pull_smem_attr<rank_update<teleport_single>>(g->device, &cap_b));
@@ -346,23 +346,7 @@ template <class Upd, bool kW>
 int pull_sums_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st,
                    const flat_control& c) {
   rank_workspace* ws = g->rank_ws;
-  if (ws->flat.valid) {
-    const flat_plan& fp = ws->flat;
-    if (fp.hot_ctas) {
-      prof_scope ps("k_flat_hot", st);
-      k_flat_hot<kW><<<fp.hot_ctas, kFlatHotWarps * 32, kFlatBlock * 4, st>>>(fp.v, x, c.ctrl);
-      PLATO_LAUNCHED("k_flat_hot");
-    }
-    if (fp.cold_blocks) {
-      prof_scope ps("k_flat_cold", st);
-      k_flat_cold<kW><<<fp.cold_blocks, kFlatColdThreads, 0, st>>>(fp.v, x, c.ctrl);
-      PLATO_LAUNCHED("k_flat_cold");
-    }
-    prof_scope ps("k_flat_update", st);
-    k_flat_update<Upd><<<fp.update_blocks, 256, 0, st>>>(fp.v, upd, ws->partials.p, c);
-    PLATO_LAUNCHED("k_flat_update");
-    return PLATO_OK;
-  }
+  if (ws->flat.valid) return launch_flat_epoch<Upd, kW>(ws->flat, x, upd, ws->partials.p, c, st);
   const pull_plan& pl = ws->plan;
   if (pl.valid) {
     const pull_plan_view pv{pl.n_long, pl.rows_begin[3], g->info.vertices, pl.n_items, pl.items.p,
@@ -467,19 +451,8 @@ template <class Upd, bool kW>
 int run_flat_epochs(plato_graph* g, const Upd& upd, uint32_t iteration, uint32_t start, double eps, double scale,
                     cudaStream_t st, uint32_t* ran, double* delta) {
   rank_workspace* ws = g->rank_ws;
-  PLATO_CUDA_TRY(cudaMemsetAsync(ws->ctrl.p, 0, 4 * sizeof(int), st));
-  {
-    prof_scope ps("k_flat_run", st);
-    Upd u = upd;
-    flat_view f = ws->flat.v;
-    int* ctrl = ws->ctrl.p;
-    uint32_t* sync = reinterpret_cast<uint32_t*>(ws->ctrl.p + 2);
-    double *d_delta = ws->delta.p, *partials = ws->partials.p;
-    void* args[] = {&f, &u, &start, &iteration, &scale, &eps, &ctrl, &d_delta, &partials, &sync};
-    PLATO_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_flat_run<Upd, kW>),
-                                               dim3(ws->flat.run_ctas), dim3(ws->flat.run_warps * 32), args, 0, st));
-    PLATO_LAUNCHED("k_flat_run");
-  }
+  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration};
+  PLATO_TRY((launch_flat_run<Upd, kW>(ws->flat, upd, start, ws->partials.p, c, st)));
   *ran = iteration - start;
   if (eps <= 0.0) return PLATO_OK;
   PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl, ws->ctrl.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
