@@ -182,7 +182,9 @@ struct gather_args {
   uint32_t* changed;          // out: bitmap of rows changed this epoch (zeroed before)
   double* est;                // per-row estimate, rewritten for changed rows
   const uint32_t* fwd_outdeg; // forward out-degree (the engine's switch weight)
-  unsigned long long* counters;  // [0] changed rows, [1] their forward out-degrees, [2], [3], [4] cursors of hubs, mids and chunks
+  // [0] changed rows, [1] their forward out-degrees, [2], [3], [4] cursors of
+  // hubs, mids and chunks
+  unsigned long long* counters;
   const uint32_t* hubs;       // rows with more than hub_deg sources
   const uint32_t* mids;       // rows with more than team_deg, at most hub_deg
   uint32_t n_hubs, n_mids;

@@ -17,10 +17,11 @@ namespace {
 // rows above kFlatRowDeg1 in the further blocks: a segment costs a store and a
 // load of its sum, so it has to hold a few edges (RMAT s24, epoch: further
 // blocks above 32 / 48 / 64 / 96 / 128 in-edges 562 / 539 / 532 / 537 / 577 us;
-// block 0 above 4 / 8 / 16 / 32: 580 / 577 / 583 / 589).  Block 0 is used where
-// it holds kFlatFirst edges: below, one more launch and the copies of the
-// block cost what its gathers save (epoch without / with it: RMAT s18 20.6 /
-// 24.4 us, s19 32.4 / 33.4, s20 55.8 / 48.5).  A further block is used where it
+// block 0 above 4 / 8 / 16 / 32: 580 / 577 / 583 / 589).  There are hot streams
+// where they hold kFlatFirst edges: below, one more launch and the copies of the
+// blocks cost what the gathers save (epoch without / with them: RMAT s18 20.6 /
+// 24.4 us, s19 32.4 / 33.4, s20 55.8 / 48.5; 64M uniform edges over 1M vertices
+// 262 / 144).  A further block is used where it
 // holds kFlatMore edges, and one per row that takes part (RMAT s22 with 4 / 6 /
 // 10 / 16 blocks 153 / 144 / 138 / 144 us; s24 with 1 / 3 / 6 / 10 / 16 / 24:
 // 743 / 674 / 633 / 595 / 577 / 568).
@@ -63,10 +64,11 @@ struct flat_rows {
   const uint64_t* off;
   const uint32_t* adj;
   uint32_t V, nb, block, rows1;  // rows1: the rows of the middle streams, in whole 32-row words
+  uint32_t deg0, deg1;           // kFlatRowDeg0, kFlatRowDeg1, or 0 where no source is cold
   // hot streams that row v takes part in
   __device__ __forceinline__ uint32_t streams(uint32_t v) const {
     const uint64_t d = off[v + 1] - off[v];
-    return d > kFlatRowDeg1 ? nb : d > kFlatRowDeg0 ? min(nb, 1u) : 0u;
+    return d > deg1 ? nb : d > deg0 ? min(nb, 1u) : 0u;
   }
   __device__ __forceinline__ uint64_t cell(uint32_t k, uint32_t v) const { return flat_place(k, V, rows1) + v; }
 };
@@ -339,14 +341,21 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   unsigned long long h[2 + kFlatMaxBlocks];
   PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  flat_rows rows{off, adj, V, 0, kBlock, 0};
+  flat_rows rows{off, adj, V, 0, kBlock, 0, kFlatRowDeg0, kFlatRowDeg1};
   uint32_t nb = 0;
   const bool run = E <= kFlatRunEdges;
-  if (!run && h[2] >= kFlatFirst)
-    for (nb = 1; nb < nblocks && h[2 + nb] >= std::max(kFlatMore, h[1]) && h[1] > 0;) ++nb;
+  if (!run) {
+    unsigned long long hot = h[2];
+    for (nb = 1; nb < nblocks && h[2 + nb] >= std::max(kFlatMore, h[1]) && h[1] > 0; ++nb) hot += h[2 + nb];
+    if (hot < kFlatFirst) nb = 0;
+  }
   rows.nb = nb;
   // whole words; the last may be short
   rows.rows1 = nb > 1 ? std::min((static_cast<uint32_t>(h[0]) + 31) / 32 * 32, V) : 0;
+  if (nb > 0 && static_cast<uint64_t>(nb) * kBlock >= V) {  // every source is hot: no cold pass
+    rows.deg0 = rows.deg1 = 0;
+    rows.rows1 = nb > 1 ? V : 0;
+  }
   const uint32_t streams = nb + 1, words = (V + 31) / 32, words1 = (rows.rows1 + 31) / 32;
   const uint64_t cells = flat_place(nb, V, rows.rows1) + V;
 
@@ -386,10 +395,15 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   const uint32_t per_block = kFlatColdThreads / 32;
   pl.hot_ctas = std::min<uint32_t>(sms, (hot_steps + kFlatHotWarps - 1) / kFlatHotWarps);
   pl.run_ctas = pl.run_warps = pl.cold_blocks = 0;
+  pl.run_cluster = false;
   if (run) {
-    if (cold_steps <= 64) {
+    if (cold_steps <= 4) {
       pl.run_ctas = 1;
-      pl.run_warps = std::min<uint32_t>(32, std::max<uint32_t>(cold_steps, 4));
+      pl.run_warps = 4;
+    } else if (cold_steps <= kFlatClusterSteps) {
+      pl.run_cluster = true;
+      pl.run_ctas = kFlatCluster;
+      pl.run_warps = std::min<uint32_t>(32, std::max<uint32_t>(4, (cold_steps + kFlatCluster - 1) / kFlatCluster));
     } else {
       pl.run_ctas = std::min<uint32_t>(sms, (cold_steps + 7) / 8);
       pl.run_warps = std::min<uint32_t>(32, (cold_steps + pl.run_ctas - 1) / pl.run_ctas);
@@ -408,7 +422,8 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   const size_t o_hid = lay.add(hot_edges * 2ull), o_cid = lay.add(cold_edges * 4ull);
   const size_t o_hw = lay.add(weighted ? hot_edges * 4ull : 0), o_cw = lay.add(weighted ? cold_edges * 4ull : 0);
   const size_t o_hmark = lay.add(hot_steps * 128ull), o_cmark = lay.add(cold_steps * 64ull);
-  const size_t o_seg = lay.add((static_cast<uint64_t>(hot_steps) + cold_steps) * 4), o_meta = lay.add(nmeta * sizeof(uint4));
+  const size_t o_seg = lay.add((static_cast<uint64_t>(hot_steps) + cold_steps) * 4);
+  const size_t o_meta = lay.add(nmeta * sizeof(uint4));
   const size_t o_spans = lay.add(max_pieces * sizeof(uint2)), o_pieces = lay.add(max_pieces * sizeof(uint2));
   const size_t o_subs = lay.add(max_subs * sizeof(flat_sub)), o_cta = lay.add((pl.hot_ctas + 1) * 4ull);
   const size_t o_part = lay.add(segments * sizeof(S)), o_head = lay.add(max_pieces * sizeof(S));
@@ -510,7 +525,8 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   uint32_t a = 0;
   for (uint32_t c = 0; c < pl.hot_ctas; ++c) {
     cta_sub.push_back(static_cast<uint32_t>(subs.size()));
-    const uint32_t b = c + 1 == pl.hot_ctas ? hot_steps : at_cost(a, hot_steps, static_cast<double>(cost[hot_steps]) * (c + 1) / pl.hot_ctas);
+    const double end = static_cast<double>(cost[hot_steps]) * (c + 1) / pl.hot_ctas;
+    const uint32_t b = c + 1 == pl.hot_ctas ? hot_steps : at_cost(a, hot_steps, end);
     for (uint32_t k = 0; k < nb; ++k) {
       const uint32_t k0 = static_cast<uint32_t>(fs.edge[k] / kHotStep);
       const uint32_t k1 = static_cast<uint32_t>(fs.edge[k + 1] / kHotStep);
@@ -519,7 +535,8 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
       subs.push_back(flat_sub{k, static_cast<uint32_t>(pieces.size())});
       uint32_t p0 = lo;
       for (uint32_t w = 0; w < kFlatHotWarps; ++w) {
-        const uint32_t p1 = w + 1 == kFlatHotWarps ? hi : at_cost(p0, hi, cost[lo] + (static_cast<double>(cost[hi]) - cost[lo]) * (w + 1) / kFlatHotWarps);
+        const double c1 = cost[lo] + (static_cast<double>(cost[hi]) - cost[lo]) * (w + 1) / kFlatHotWarps;
+        const uint32_t p1 = w + 1 == kFlatHotWarps ? hi : at_cost(p0, hi, c1);
         add(k0, p0, p1);
         p0 = p1;
       }

@@ -52,6 +52,10 @@ constexpr uint32_t kFlatBlockBytes = 229376;
 constexpr int kFlatColdLane = 8;          // edges of a lane in a cold step
 constexpr uint32_t kFlatColdStep = 32 * kFlatColdLane;
 constexpr uint32_t kFlatMaxBlocks = 24;
+// Up to this many steps (64K edges) k_flat_run's CTAs are one cluster of 8 (epoch
+// over a cooperative grid / over the cluster, one B200: RMAT s10 5.5 / 4.4 us,
+// s11 6.3 / 4.9, s12 6.5 / 6.3, s13 6.3 / 7.6).
+constexpr uint32_t kFlatCluster = 8, kFlatClusterSteps = 256;
 constexpr uint32_t kFlatHotWarps = 32;
 constexpr uint32_t kFlatColdThreads = 256;
 constexpr uint32_t kPieceFirst = 0x80000000u;  // a piece at the start of its stream
@@ -99,6 +103,7 @@ struct flat_plan {
   bool valid = false;
   uint32_t hot_ctas = 0, cold_blocks = 0, update_blocks = 0;
   uint32_t run_ctas = 0, run_warps = 0;  // not 0: k_flat_run's grid, the plan's only kernel
+  bool run_cluster = false;              // its CTAs are one cluster
   flat_view<S> v{};
   dbuf<unsigned char> mem;  // every array of v
 };
@@ -489,12 +494,18 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view<typename Updat
   }
 }
 
-// Barrier over the CTAs of a cooperative launch: sync[0] counts arrivals over
-// the whole launch (`target` of them release this barrier), sync[1] is set
-// when a CTA gives up waiting, and then every CTA returns.
+// Barrier over the CTAs of k_flat_run.  One cluster: the hardware's barrier,
+// which orders global memory over the cluster.  A cooperative launch: sync[0]
+// counts arrivals over the whole launch (`target` of them release this
+// barrier), sync[1] is set when a CTA gives up waiting, and then every CTA
+// returns.
 constexpr uint32_t kFlatSpins = 1u << 24;
-__device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target) {
+__device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target, bool cluster) {
   __shared__ int s_ok;
+  if (cluster) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  }
   __syncthreads();
   if (gridDim.x == 1) return true;
   if (threadIdx.x == 0) {
@@ -518,24 +529,27 @@ __device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target) {
 }
 
 template <class Update>
-__device__ __noinline__ void flat_poison(const flat_view<typename Update::value>& f, const Update& upd, uint32_t w0, uint32_t nwarps) {
+__device__ __noinline__ void flat_poison(const flat_view<typename Update::value>& f, const Update& upd, uint32_t w0,
+                                         uint32_t nwarps) {
   for (uint32_t w = w0; w < f.words; w += nwarps) {
     const uint32_t v = w * 32 + (threadIdx.x & 31);
     if (v < f.V) upd.poison(v);
   }
 }
 
-// Every epoch of a small graph in one cooperative launch of gridDim.x <= SMs
-// CTAs: gather, barrier, update, barrier.  The epoch kinds and the eps exit
-// follow epoch_decide; ctrl[1] = epochs run, counted from `start`.  Launches
-// bound these graphs: one epoch with a launch per degree bin / here, RMAT s10
-// 52 / 5.3 us, s12 54 / 6.4, s16 70 / 9.4, 48K uniform edges 28 / 6.5.  A CTA
-// that gives up waiting leaves NaN in its rows.
+// Every epoch of a small graph in one launch, cooperative over gridDim.x <= SMs
+// CTAs or, up to 256 steps, one cluster of 8 (one CTA alone is bound by issue,
+// and a barrier through L2 costs more than 64K edges' gathers): gather, barrier,
+// update, barrier.  The epoch kinds and the eps exit follow epoch_decide;
+// ctrl[1] = epochs run, counted from `start`.  Launches bound these graphs: one
+// epoch with a launch per degree bin / here, RMAT s10 52 / 4.4 us, s12 54 / 6.3, s16
+// 70 / 9.4, 48K uniform edges 28 / 5.8.  A CTA that gives up waiting leaves NaN
+// in its rows.
 template <class Update, bool kW>
 __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view<typename Update::value> f,
                                                                    Update upd, uint32_t start, uint32_t iteration, double scale, double eps,
                                                                    int* ctrl, double* delta, double* partials,
-                                                                   uint32_t* sync) {
+                                                                   uint32_t* sync, bool cluster) {
   using S = typename Update::value;
   __shared__ double s_red[32];
   __shared__ double s_delta;
@@ -547,7 +561,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view<ty
   for (;;) {
     upd.final_epoch = last ? 1 : 0;
     flat_piece(f, w0, flat_cold_gather<S, kW, true>{f.cid, f.cw, f.cmark, f.cseg, upd.gathered()});
-    if (!flat_barrier(sync, ++barriers * gridDim.x)) return flat_poison(f, upd, w0, nwarps);
+    if (!flat_barrier(sync, ++barriers * gridDim.x, cluster)) return flat_poison(f, upd, w0, nwarps);
     double dl = 0.0;
     for (uint32_t w = w0; w < f.words; w += nwarps) {
       const uint32_t v = w * 32 + lane;
@@ -566,7 +580,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view<ty
       dl = warp_sum(lane < cta_warps ? s_red[lane] : 0.0);
       if (threadIdx.x == 0) __stcg(sums + blockIdx.x, dl);
     }
-    if (!flat_barrier(sync, ++barriers * gridDim.x)) return flat_poison(f, upd, w0, nwarps);
+    if (!flat_barrier(sync, ++barriers * gridDim.x, cluster)) return flat_poison(f, upd, w0, nwarps);
     last = ran + 1 >= iteration;
     if (eps > 0.0) {  // every CTA sums the partials in the same order
       if (warp == 0) {
@@ -615,13 +629,24 @@ int launch_flat_run(const flat_plan<typename Upd::value>& p, const Upd& upd, uin
                     const flat_control& c, cudaStream_t st) {
   PLATO_CUDA_TRY(cudaMemsetAsync(c.ctrl, 0, 4 * sizeof(int), st));
   prof_scope ps("k_flat_run", st);
-  Upd u = upd;
-  flat_control k = c;
-  flat_view<typename Upd::value> f = p.v;
   uint32_t* sync = reinterpret_cast<uint32_t*>(c.ctrl + 2);
-  void* args[] = {&f, &u, &start, &k.iteration, &k.scale, &k.eps, &k.ctrl, &k.delta, &partials, &sync};
-  PLATO_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_flat_run<Upd, kW>), dim3(p.run_ctas),
-                                             dim3(p.run_warps * 32), args, 0, st));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(p.run_ctas);
+  cfg.blockDim = dim3(p.run_warps * 32);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  if (p.run_cluster) {
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = p.run_ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  } else {
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+  }
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  PLATO_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_flat_run<Upd, kW>, p.v, upd, start, c.iteration, c.scale, c.eps, c.ctrl,
+                                    c.delta, partials, sync, p.run_cluster));
   PLATO_LAUNCHED("k_flat_run");
   return PLATO_OK;
 }
