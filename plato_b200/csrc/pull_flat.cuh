@@ -32,6 +32,8 @@
 // 98 -> 49, 16M uniform edges over 1M vertices 107 -> 82, 64M over 1M 303 -> 144.
 #pragma once
 
+#include <utility>
+
 #include "common.cuh"
 #include "profile.cuh"
 #include "pull_merge.cuh"
@@ -333,6 +335,17 @@ __device__ __forceinline__ void flat_piece(const flat_view<typename Gather::valu
   if (lane == 0) f.carry[p] = carry + acc;
 }
 
+// The kernels of an epoch are launched behind one another with programmatic
+// serialisation: the next one's CTAs take the SMs that the last CTAs of the one
+// before leave idle, and wait here until it has ended.  (Nothing before this
+// reads what an earlier kernel wrote.)  Not so k_flat_cold behind k_flat_hot: a
+// CTA that comes to an SM before it is idle finds it with 224 KB of shared memory
+// and the rest as its L1 (RMAT s22 146 -> 197 us).  Epochs without / with it:
+// RMAT s18 19.4 / 16.6 us, s19 31.8 / 26.6, 16M uniform edges 85 / 81.
+__device__ __forceinline__ void flat_after() {
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+
 // Hot streams (bound by issue: about 300 instructions a step of 512 edges, and
 // 3.4-way bank conflicts): CTA c walks its parts [cta_sub[c], cta_sub[c+1]), each within
 // one block whose ranks it first copies to shared memory.
@@ -341,6 +354,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_hot(flat_view<S>
                                                                    const int* mode) {
   constexpr uint32_t kPer = 16 / sizeof(S);
   extern __shared__ float4 s_x4[];
+  flat_after();
   if (mode && *mode == 2) return;
   const uint32_t sub1 = f.cta_sub[blockIdx.x + 1];
   for (uint32_t sub = f.cta_sub[blockIdx.x]; sub < sub1; ++sub) {
@@ -364,6 +378,7 @@ template <class S, bool kW>
 __global__ void __launch_bounds__(kFlatColdThreads, sizeof(S) == 4 ? 5 : 4) k_flat_cold(flat_view<S> f,
                                                                                        const S* __restrict__ x,
                                                                                        const int* mode) {
+  flat_after();
   if (mode && *mode == 2) return;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= f.cold_pieces) return;
@@ -430,6 +445,7 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view<typename Updat
   constexpr int R = 2;
   __shared__ double s_red[32];
   __shared__ bool s_last;
+  flat_after();
   if (upd.skip()) return;
   const unsigned lane = threadIdx.x & 31;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -547,9 +563,9 @@ __device__ __noinline__ void flat_poison(const flat_view<typename Update::value>
 // in its rows.
 template <class Update, bool kW>
 __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view<typename Update::value> f,
-                                                                   Update upd, uint32_t start, uint32_t iteration, double scale, double eps,
-                                                                   int* ctrl, double* delta, double* partials,
-                                                                   uint32_t* sync, bool cluster) {
+                                                                   Update upd, uint32_t start, uint32_t iteration,
+                                                                   double scale, double eps, int* ctrl, double* delta,
+                                                                   double* partials, uint32_t* sync, bool cluster) {
   using S = typename Update::value;
   __shared__ double s_red[32];
   __shared__ double s_delta;
@@ -601,6 +617,22 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view<ty
   }
 }
 
+template <class... P, class... A>
+cudaError_t flat_launch(bool behind, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
+                        A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = behind ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 // The kernels of one epoch of a plan without run_ctas: sums of x into upd.
 template <class Upd, bool kW>
 int launch_flat_epoch(const flat_plan<typename Upd::value>& p, const typename Upd::value* x, const Upd& upd,
@@ -608,16 +640,18 @@ int launch_flat_epoch(const flat_plan<typename Upd::value>& p, const typename Up
   using S = typename Upd::value;
   if (p.hot_ctas) {
     prof_scope ps("k_flat_hot", st);
-    k_flat_hot<S, kW><<<p.hot_ctas, kFlatHotWarps * 32, kFlatBlockBytes, st>>>(p.v, x, c.ctrl);
+    PLATO_CUDA_TRY(flat_launch(true, k_flat_hot<S, kW>, p.hot_ctas, kFlatHotWarps * 32, kFlatBlockBytes, st, p.v,
+                               x, c.ctrl));
     PLATO_LAUNCHED("k_flat_hot");
   }
   if (p.cold_blocks) {
     prof_scope ps("k_flat_cold", st);
-    k_flat_cold<S, kW><<<p.cold_blocks, kFlatColdThreads, 0, st>>>(p.v, x, c.ctrl);
+    PLATO_CUDA_TRY(flat_launch(p.hot_ctas == 0, k_flat_cold<S, kW>, p.cold_blocks, kFlatColdThreads, 0, st, p.v, x,
+                               c.ctrl));
     PLATO_LAUNCHED("k_flat_cold");
   }
   prof_scope ps("k_flat_update", st);
-  k_flat_update<Upd><<<p.update_blocks, 256, 0, st>>>(p.v, upd, partials, c);
+  PLATO_CUDA_TRY(flat_launch(true, k_flat_update<Upd>, p.update_blocks, 256, 0, st, p.v, upd, partials, c));
   PLATO_LAUNCHED("k_flat_update");
   return PLATO_OK;
 }
