@@ -140,10 +140,18 @@ __device__ __forceinline__ uint32_t bmax(uint32_t a, uint32_t b) {
 __device__ __forceinline__ uint4 vmax4(uint4 a, uint4 b) {
   return make_uint4(bmax(a.x, b.x), bmax(a.y, b.y), bmax(a.z, b.z), bmax(a.w, b.w));
 }
-// Even and odd bytes of a word widened to 16-bit lanes, and back.
-__device__ __forceinline__ uint32_t even_bytes(uint32_t w) { return __byte_perm(w, 0u, 0x4240); }
-__device__ __forceinline__ uint32_t odd_bytes(uint32_t w) { return __byte_perm(w, 0u, 0x4341); }
-__device__ __forceinline__ uint32_t join_bytes(uint32_t e, uint32_t o) { return __byte_perm(e, o, 0x6240); }
+// The merge of narrow slices keeps even and odd bytes in the high bytes of
+// 16-bit lanes, whose order a maximum of 16-bit lanes follows whatever the low
+// bytes hold: the odd bytes lie there already, the even ones after a shift by
+// 8.  Two rows join the accumulators with one three-way maximum a word and half
+// (four instructions for two words, where taking the bytes apart cost eight).
+__device__ __forceinline__ uint32_t max_even(uint32_t acc, uint32_t a, uint32_t b) {
+  return __vimax3_u16x2(acc, a << 8, b << 8);
+}
+__device__ __forceinline__ uint32_t max_odd(uint32_t acc, uint32_t a, uint32_t b) { return __vimax3_u16x2(acc, a, b); }
+__device__ __forceinline__ uint32_t join_bytes(uint32_t e, uint32_t o) {
+  return ((e >> 8) & 0x00FF00FFu) | (o & 0xFF00FF00u);
+}
 
 __device__ __forceinline__ bool differs(uint4 a, uint4 b) {
   return ((a.x ^ b.x) | (a.y ^ b.y) | (a.z ^ b.z) | (a.w ^ b.w)) != 0u;
@@ -219,9 +227,9 @@ __device__ __forceinline__ bool team_merge(const gather_args& a, uint64_t c0, ui
                                            unsigned tmask, uint32_t* s_ids, uint4 (&agg)[VEC]) {
   constexpr int K = kChunk / T;
   constexpr int UNR = unroll_for(VEC);
-  // Up to 2 words per lane, the merge keeps even and odd bytes apart as 16-bit
-  // lanes (__vmaxu2, two per word) and joins them once at the end; wider
-  // slices keep the byte max (the split doubles the accumulator registers).
+  // Up to 2 words per lane, the merge keeps even and odd bytes apart (max_even,
+  // max_odd) and joins them once at the end; wider slices keep the byte max (the
+  // split doubles the accumulator registers).
   constexpr bool kSplit = VEC <= 2;
   bool any = false;
   uint4 ev[VEC], od[VEC];
@@ -263,18 +271,19 @@ __device__ __forceinline__ bool team_merge(const gather_args& a, uint64_t c0, ui
                         : make_uint4(0u, 0u, 0u, 0u);
       }
       if constexpr (kSplit) {
+        static_assert(!kSplit || UNR % 2 == 0, "rows join in pairs");
 #pragma unroll
-        for (int j = 0; j < UNR; ++j)
+        for (int j = 0; j < UNR; j += 2)
 #pragma unroll
           for (int q = 0; q < VEC; ++q) {
-            ev[q].x = __vmaxu2(ev[q].x, even_bytes(r[j][q].x));
-            ev[q].y = __vmaxu2(ev[q].y, even_bytes(r[j][q].y));
-            ev[q].z = __vmaxu2(ev[q].z, even_bytes(r[j][q].z));
-            ev[q].w = __vmaxu2(ev[q].w, even_bytes(r[j][q].w));
-            od[q].x = __vmaxu2(od[q].x, odd_bytes(r[j][q].x));
-            od[q].y = __vmaxu2(od[q].y, odd_bytes(r[j][q].y));
-            od[q].z = __vmaxu2(od[q].z, odd_bytes(r[j][q].z));
-            od[q].w = __vmaxu2(od[q].w, odd_bytes(r[j][q].w));
+            ev[q].x = max_even(ev[q].x, r[j][q].x, r[j + 1][q].x);
+            ev[q].y = max_even(ev[q].y, r[j][q].y, r[j + 1][q].y);
+            ev[q].z = max_even(ev[q].z, r[j][q].z, r[j + 1][q].z);
+            ev[q].w = max_even(ev[q].w, r[j][q].w, r[j + 1][q].w);
+            od[q].x = max_odd(od[q].x, r[j][q].x, r[j + 1][q].x);
+            od[q].y = max_odd(od[q].y, r[j][q].y, r[j + 1][q].y);
+            od[q].z = max_odd(od[q].z, r[j][q].z, r[j + 1][q].z);
+            od[q].w = max_odd(od[q].w, r[j][q].w, r[j + 1][q].w);
           }
       } else {
 #pragma unroll
