@@ -449,7 +449,6 @@ plato_graph::~plato_graph() {
   plato_b200::destroy_bfs_workspace(bfs_ws);
   plato_b200::destroy_hll_workspace(hll_ws);
   plato_b200::destroy_cc_workspace(cc_ws);
-  plato_b200::destroy_trust_workspace(trust_ws);
   if (stream) cudaStreamDestroy(stream);
 }
 

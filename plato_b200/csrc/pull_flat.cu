@@ -36,7 +36,7 @@ constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 600000;
 // out[0]: one past the last row above kFlatRowDeg1 edges, out[1]: how many there
 // are, out[2 + k]: gathers of the sources of block k (`uses` by source).
 __global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict__ off,
-                                                     const uint32_t* __restrict__ uses, uint32_t V, uint32_t block,
+                                                     const uint32_t* __restrict__ uses, uint32_t V,
                                                      uint32_t nblocks, unsigned long long* out) {
   __shared__ unsigned long long s_red[32];
   unsigned long long last = 0, n = 0;
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict_
   // 8 CTAs a block of sources
   const uint32_t k = blockIdx.x / 8, q = blockIdx.x % 8;
   if (k >= nblocks) return;
-  const uint32_t b = k * block, e = min(V, b + block);
+  const uint32_t b = k * kFlatBlock, e = min(V, b + kFlatBlock);
   n = 0;
   for (uint32_t v = b + q * 256 + threadIdx.x; v < e; v += 8 * 256) n += uses[v];
   n = block_sum_u64<256>(n, s_red);
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict_
 struct flat_rows {
   const uint64_t* off;
   const uint32_t* adj;
-  uint32_t V, nb, block, rows1;  // rows1: the rows of the middle streams, in whole 32-row words
+  uint32_t V, nb, rows1;  // rows1: the rows of the middle streams, in whole 32-row words
   uint32_t deg0, deg1;           // kFlatRowDeg0, kFlatRowDeg1, or 0 where no source is cold
   // hot streams that row v takes part in
   __device__ __forceinline__ uint32_t streams(uint32_t v) const {
@@ -85,7 +85,7 @@ __global__ void k_flat_split(flat_rows f, uint32_t* cnt) {
       if (k > 0 && v >= f.rows1) break;
       uint64_t lo = pos;
       if (k < ns) {
-        const uint32_t bound = (k + 1) * f.block;
+        const uint32_t bound = (k + 1) * kFlatBlock;
         uint64_t hi = end;
         while (lo < hi) {
           const uint64_t mid = (lo + hi) >> 1;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256) k_flat_fill(flat_rows f, const uint32_t* 
       const uint32_t v = lo;
       const uint32_t id = f.adj[e];
       const uint32_t ns = f.streams(v);
-      uint32_t k = id / f.block;
+      uint32_t k = id / kFlatBlock;
       if (k >= ns) k = f.nb;
       uint32_t before = 0;
       for (uint32_t j = 0; j < min(k, ns); ++j) before += cnt[f.cell(j, v)];
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) k_flat_fill(flat_rows f, const uint32_t* 
       uint64_t to = st.edge[k] + (pos[at] - st.sum[k]) + i;
       uint32_t* flags = hflags;
       if (k < f.nb) {
-        hid[to] = static_cast<uint16_t>(id - k * f.block);
+        hid[to] = static_cast<uint16_t>(id - k * kFlatBlock);
         if (w) hw[to] = w[e];
       } else {
         to -= cold0;
@@ -199,13 +199,12 @@ struct flat_crossing {
 };
 
 // Piece p continues a segment of an earlier piece; *j is its ordinal.
-template <class S>
-__device__ __forceinline__ bool flat_continues(const flat_view<S>& f, uint32_t p, uint32_t* j) {
+__device__ __forceinline__ bool flat_continues(const flat_view& f, uint32_t p, uint32_t* j) {
   const uint2 pc = f.pieces[p];
   if ((pc.x & kPieceFirst) || pc.x >= pc.y) return false;
   const size_t before = static_cast<size_t>(pc.x) * 32 - 1;
   if (p < f.cold_piece0) {
-    if (f.hmark[before] >> (flat_hot_lane<S> - 1) & 1u) return false;
+    if (f.hmark[before] >> (kFlatHotLane - 1) & 1u) return false;
     *j = f.hseg[pc.x];
   } else {
     if (f.cmark[before] >> (kFlatColdLane - 1) & 1u) return false;
@@ -217,8 +216,8 @@ __device__ __forceinline__ bool flat_continues(const flat_view<S>& f, uint32_t p
 // Segments cut by piece boundaries, one thread per piece; the first piece
 // that continues a segment records it.  fill = false marks the rows in
 // meta.z, fill = true writes the spans (meta.w scanned in between).
-template <bool kFill, class S>
-__global__ void k_flat_spans(flat_view<S> f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans) {
+template <bool kFill>
+__global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t j = 0;
   if (p >= npieces || !flat_continues(f, p, &j) || j >= segments) return;
@@ -314,18 +313,14 @@ int put(T* d, const std::vector<T>& h, cudaStream_t st) {
 
 }  // namespace
 
-template <class S>
-int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st) {
-  constexpr uint32_t kBlock = flat_block<S>, kHotStep = flat_hot_step<S>;
-  constexpr int kHotLane = flat_hot_lane<S>;
+int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   const uint32_t V = g->info.vertices;
   const uint64_t E = g->stored_edges;
   pl.valid = false;
-  if (!g->own_sources || E == 0) return PLATO_OK;
-  const uint64_t* off = out ? g->out_off.p : g->in_off.p;
-  const uint32_t* adj = out ? g->out_adj.p : g->in_adj.p;
-  const bool weighted = g->weighted && !out && sizeof(S) == 4;
-  const uint32_t nblocks = std::min<uint32_t>((V + kBlock - 1) / kBlock, kFlatMaxBlocks);
+  if (!g->relabeled || !g->own_sources || E == 0) return PLATO_OK;
+  const uint64_t* off = g->in_off.p;
+  const bool weighted = g->weighted;
+  const uint32_t nblocks = std::min<uint32_t>((V + kFlatBlock - 1) / kFlatBlock, kFlatMaxBlocks);
   cudaMemPool_t pool{};
   try {
     pool = engine_pool();
@@ -336,12 +331,12 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   PLATO_TRY(d_survey.alloc(pool, 2 + kFlatMaxBlocks));
   PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, (2 + kFlatMaxBlocks) * sizeof(unsigned long long), st));
   k_flat_survey<<<std::max(nblocks * 8, grid_for(V, 256, 148 * 4)), 256, 0, st>>>(
-      off, out ? g->in_deg.p : g->out_deg.p, V, kBlock, nblocks, d_survey.p);
+      off, g->out_deg.p, V, nblocks, d_survey.p);
   PLATO_LAUNCHED("k_flat_survey");
   unsigned long long h[2 + kFlatMaxBlocks];
   PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  flat_rows rows{off, adj, V, 0, kBlock, 0, kFlatRowDeg0, kFlatRowDeg1};
+  flat_rows rows{off, g->in_adj.p, V, 0, 0, kFlatRowDeg0, kFlatRowDeg1};
   uint32_t nb = 0;
   const bool run = E <= kFlatRunEdges;
   if (!run) {
@@ -352,7 +347,7 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   rows.nb = nb;
   // whole words; the last may be short
   rows.rows1 = nb > 1 ? std::min((static_cast<uint32_t>(h[0]) + 31) / 32 * 32, V) : 0;
-  if (nb > 0 && static_cast<uint64_t>(nb) * kBlock >= V) {  // every source is hot: no cold pass
+  if (nb > 0 && static_cast<uint64_t>(nb) * kFlatBlock >= V) {  // every source is hot: no cold pass
     rows.deg0 = rows.deg1 = 0;
     rows.rows1 = nb > 1 ? V : 0;
   }
@@ -381,13 +376,13 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   flat_starts fs{};
   uint64_t edges = 0;
   for (uint32_t k = 0; k < streams; ++k) {
-    const uint32_t step = k < nb ? kHotStep : kFlatColdStep;
+    const uint32_t step = k < nb ? kFlatHotStep : kFlatColdStep;
     fs.edge[k] = edges;
     fs.sum[k] = sum[k];
     edges += (sum[k + 1] - sum[k] + step - 1) / step * step;
   }
   const uint64_t hot_edges = fs.edge[nb], cold_edges = edges - hot_edges;
-  const uint32_t hot_steps = static_cast<uint32_t>(hot_edges / kHotStep);
+  const uint32_t hot_steps = static_cast<uint32_t>(hot_edges / kFlatHotStep);
   const uint32_t cold_steps = static_cast<uint32_t>(cold_edges / kFlatColdStep);
   // grids, and bounds on the pieces
   int sms = 0;
@@ -426,8 +421,8 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   const size_t o_meta = lay.add(nmeta * sizeof(uint4));
   const size_t o_spans = lay.add(max_pieces * sizeof(uint2)), o_pieces = lay.add(max_pieces * sizeof(uint2));
   const size_t o_subs = lay.add(max_subs * sizeof(flat_sub)), o_cta = lay.add((pl.hot_ctas + 1) * 4ull);
-  const size_t o_part = lay.add(segments * sizeof(S)), o_head = lay.add(max_pieces * sizeof(S));
-  const size_t o_carry = lay.add(max_pieces * sizeof(S));
+  const size_t o_part = lay.add(segments * sizeof(float)), o_head = lay.add(max_pieces * sizeof(float));
+  const size_t o_carry = lay.add(max_pieces * sizeof(float));
   PLATO_TRY(pl.mem.alloc(lay.bytes));
   unsigned char* mem = pl.mem.p;
   uint16_t* hid = reinterpret_cast<uint16_t*>(mem + o_hid);
@@ -452,8 +447,8 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
     const uint64_t end = k + 1 < streams ? fs.edge[k + 1] : edges;
     if (end == fs.edge[k]) continue;
     if (k < nb) {
-      PLATO_CUDA_TRY(cudaMemsetAsync(hid + (end - kHotStep), 0, kHotStep * 2, st));
-      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(hw + (end - kHotStep), 0, kHotStep * 4, st));
+      PLATO_CUDA_TRY(cudaMemsetAsync(hid + (end - kFlatHotStep), 0, kFlatHotStep * 2, st));
+      if (weighted) PLATO_CUDA_TRY(cudaMemsetAsync(hw + (end - kFlatHotStep), 0, kFlatHotStep * 4, st));
     } else {
       const uint64_t b = cold_edges - kFlatColdStep;
       PLATO_CUDA_TRY(cudaMemsetAsync(cid + b, 0, kFlatColdStep * 4, st));
@@ -475,7 +470,7 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   scratch<uint32_t> ends(st);
   PLATO_TRY(ends.alloc(pool, hot_steps + cold_steps));
   if (hot_steps) {
-    k_flat_marks<kHotLane, uint32_t><<<grid_for(hot_steps * 32ull, 256), 256, 0, st>>>(hflags.p, hot_steps,
+    k_flat_marks<kFlatHotLane, uint32_t><<<grid_for(hot_steps * 32ull, 256), 256, 0, st>>>(hflags.p, hot_steps,
                                                                                            hmark, ends.p);
     PLATO_LAUNCHED("k_flat_marks");
   }
@@ -528,8 +523,8 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
     const double end = static_cast<double>(cost[hot_steps]) * (c + 1) / pl.hot_ctas;
     const uint32_t b = c + 1 == pl.hot_ctas ? hot_steps : at_cost(a, hot_steps, end);
     for (uint32_t k = 0; k < nb; ++k) {
-      const uint32_t k0 = static_cast<uint32_t>(fs.edge[k] / kHotStep);
-      const uint32_t k1 = static_cast<uint32_t>(fs.edge[k + 1] / kHotStep);
+      const uint32_t k0 = static_cast<uint32_t>(fs.edge[k] / kFlatHotStep);
+      const uint32_t k1 = static_cast<uint32_t>(fs.edge[k + 1] / kFlatHotStep);
       const uint32_t lo = std::max(a, k0), hi = std::min(b, k1);
       if (lo >= hi) continue;
       subs.push_back(flat_sub{k, static_cast<uint32_t>(pieces.size())});
@@ -552,8 +547,8 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   PLATO_TRY(put(d_pieces, pieces, st));
   PLATO_TRY(put(d_subs, subs, st));
   PLATO_TRY(put(d_cta, cta_sub, st));
-  flat_view<S>& f = pl.v;
-  f = flat_view<S>{};
+  flat_view& f = pl.v;
+  f = flat_view{};
   f.V = f.nsrc = V;
   f.nb = nb;
   f.words = words;
@@ -573,11 +568,11 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
   f.subs = d_subs;
   f.meta = meta;
   f.spans = spans;
-  f.part = reinterpret_cast<S*>(mem + o_part);
-  f.head = reinterpret_cast<S*>(mem + o_head);
-  f.carry = reinterpret_cast<S*>(mem + o_carry);
+  f.part = reinterpret_cast<float*>(mem + o_part);
+  f.head = reinterpret_cast<float*>(mem + o_head);
+  f.carry = reinterpret_cast<float*>(mem + o_carry);
   const unsigned span_grid = (npieces + 127) / 128;
-  k_flat_spans<false, S><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr);
+  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr);
   PLATO_LAUNCHED("k_flat_spans");
   scratch<uint32_t> base(st);
   PLATO_TRY(base.alloc(pool, nmeta));
@@ -585,22 +580,18 @@ int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& pl, cudaStream_t st)
                      base.p, nmeta, pool, st));
   k_flat_span_base<<<grid_for(nmeta, 256), 256, 0, st>>>(base.p, nmeta, meta);
   PLATO_LAUNCHED("k_flat_span_base");
-  k_flat_spans<true, S><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans);
+  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans);
   PLATO_LAUNCHED("k_flat_spans");
   pl.update_blocks = std::min<uint32_t>(sms * 4, (words + 15) / 16);
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));  // the temporaries and the host vectors go
   if (pl.hot_ctas) {
-    PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         kFlatBlockBytes));
-    if constexpr (sizeof(S) == 4)
-      PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kFlatBlockBytes));
+    PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        kFlatBlockBytes));
   }
   pl.valid = true;
   return PLATO_OK;
 }
-
-template int build_flat_plan<float>(plato_graph*, bool, flat_plan<float>&, cudaStream_t);
-template int build_flat_plan<double>(plato_graph*, bool, flat_plan<double>&, cudaStream_t);
 
 }  // namespace plato_b200

@@ -42,17 +42,12 @@ struct plato_graph;
 
 namespace plato_b200 {
 
-// By the type of the gathered state: edges of a lane in a hot step (64-bit sums
-// take twice the registers) and sources of a hot block (224 KB of state).
-template <class S>
-constexpr int flat_hot_lane = sizeof(S) == 4 ? 16 : 8;
-template <class S>
-constexpr uint32_t flat_hot_step = 32u * flat_hot_lane<S>;
-template <class S>
-constexpr uint32_t flat_block = 229376u / sizeof(S);
-constexpr uint32_t kFlatBlockBytes = 229376;
-constexpr int kFlatColdLane = 8;          // edges of a lane in a cold step
+constexpr int kFlatHotLane = 16;          // edges of a lane in a hot step
+constexpr int kFlatColdLane = 8;          // and in a cold step
+constexpr uint32_t kFlatHotStep = 32 * kFlatHotLane;
 constexpr uint32_t kFlatColdStep = 32 * kFlatColdLane;
+constexpr uint32_t kFlatBlock = 57344;    // sources of a hot block
+constexpr uint32_t kFlatBlockBytes = kFlatBlock * sizeof(float);
 constexpr uint32_t kFlatMaxBlocks = 24;
 // Up to this many steps (64K edges) k_flat_run's CTAs are one cluster of 8 (epoch
 // over a cooperative grid / over the cluster, one B200: RMAT s10 5.5 / 4.4 us,
@@ -67,7 +62,6 @@ struct flat_sub {
   uint32_t block, piece0;
 };
 
-template <class S>
 struct flat_view {
   uint32_t V, nsrc, nb, words;      // words = ceil(V / 32)
   uint32_t words1;                  // 32-row words that take part in the hot streams after the first
@@ -78,7 +72,7 @@ struct flat_view {
   const float* cw;
   // a mark per lane and step: a bit per edge, set on the last of a segment,
   // and above it the number of such bits in the step's lanes before
-  const uint32_t* hmark;            // flat_hot_lane bits, 16 or 24 bits
+  const uint32_t* hmark;            // 16 + 16 bits
   const uint16_t* cmark;            // 8 + 8 bits
   const uint32_t* hseg;             // segments that end before each step
   const uint32_t* cseg;
@@ -89,9 +83,9 @@ struct flat_view {
   // first, rows whose segment crosses pieces, index of the first of those in spans
   const uint4* meta;
   const uint2* spans;               // first and last piece of a crossing segment
-  S* part;                          // [segments]
-  S* head;                          // [pieces]
-  S* carry;                         // [pieces]
+  float* part;                          // [segments]
+  float* head;                          // [pieces]
+  float* carry;                         // [pieces]
 };
 
 // Place of stream k in arrays by stream and row (or 32-row word): every row
@@ -100,21 +94,20 @@ __host__ __device__ inline uint64_t flat_place(uint32_t k, uint64_t rows, uint64
   return k == 0 ? 0 : rows + (k - 1) * rows1;
 }
 
-template <class S>
 struct flat_plan {
   bool valid = false;
   uint32_t hot_ctas = 0, cold_blocks = 0, update_blocks = 0;
   uint32_t run_ctas = 0, run_warps = 0;  // not 0: k_flat_run's grid, the plan's only kernel
   bool run_cluster = false;              // its CTAs are one cluster
-  flat_view<S> v{};
+  flat_view v{};
   dbuf<unsigned char> mem;  // every array of v
 };
 
 // Builds the plan of g's pull on `st` (pull_flat.cu): rows gather their
-// in-neighbours, or with `out` their out-neighbours.  plan.valid stays false
-// where there is nothing to gather or the sources are not g's vertices.
-template <class S>
-int build_flat_plan(plato_graph* g, bool out, flat_plan<S>& plan, cudaStream_t st);
+// in-neighbours.  plan.valid stays false where there is nothing to gather, the
+// sources are not g's vertices (a partition), or the graph keeps its caller's
+// order (its pull sums in the merge path's order, as plato_pagerank_csc_noalloc).
+int build_flat_plan(plato_graph* g, flat_plan& plan, cudaStream_t st);
 
 __device__ __forceinline__ void flat_prefetch(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
@@ -152,20 +145,17 @@ __device__ __forceinline__ void flat_weigh(const float* w, float (&v)[N]) {
 }
 
 // The edges of a lane in one step, hot: 16-bit ids into shared memory.
-template <class S, bool kW>
+template <bool kW>
 struct flat_hot_gather {
-  using value = S;
-  static constexpr int kLane = flat_hot_lane<S>;
-  static constexpr uint32_t kStep = flat_hot_step<S>;
+  static constexpr int kLane = kFlatHotLane;
+  static constexpr uint32_t kStep = kFlatHotStep;
   static constexpr uint32_t kAhead = 6;  // steps whose ids are on their way to L2
   const uint16_t* ids;
   const float* w;
   const uint32_t* marks;
   const uint32_t* seg;
-  const S* xs;
-  struct regs {
-    uint32_t w[kLane / 2];
-  };
+  const float* xs;
+  using regs = flat_words;
   __device__ __forceinline__ void ahead(uint32_t step, unsigned lane) const {
     const size_t e = static_cast<size_t>(step) * kStep;
     if (lane < kStep / 64) flat_prefetch(ids + e + lane * 64);
@@ -173,24 +163,12 @@ struct flat_hot_gather {
     if (kW && lane >= 16) flat_prefetch(w + e + (lane - 16) * 32);
   }
   __device__ __forceinline__ void load(uint32_t step, unsigned lane, regs& r) const {
-    const uint16_t* p = ids + static_cast<size_t>(step) * kStep + lane * kLane;
-    if constexpr (kLane == 16) {
-      flat_words t;
-      flat_load<true>(p, t);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) r.w[i] = t.w[i];
-    } else {
-      const uint4 t = __ldcs(reinterpret_cast<const uint4*>(p));
-      r.w[0] = t.x;
-      r.w[1] = t.y;
-      r.w[2] = t.z;
-      r.w[3] = t.w;
-    }
+    flat_load<true>(ids + static_cast<size_t>(step) * kStep + lane * kLane, r);
   }
   __device__ __forceinline__ uint32_t mark(uint32_t step, unsigned lane) const {
     return __ldcs(marks + static_cast<size_t>(step) * 32 + lane);
   }
-  __device__ __forceinline__ void values(uint32_t step, unsigned lane, const regs& r, S (&v)[kLane]) const {
+  __device__ __forceinline__ void values(uint32_t step, unsigned lane, const regs& r, float (&v)[kLane]) const {
 #pragma unroll
     for (int i = 0; i < kLane / 2; ++i) {
       v[2 * i] = xs[r.w[i] & 0xFFFFu];
@@ -203,16 +181,15 @@ struct flat_hot_gather {
 // Cold: 32-bit ids into global memory.  kRun: in a kernel that runs many
 // epochs the state is written by other SMs between epochs: plain loads, which
 // the barrier's acquire orders.
-template <class S, bool kW, bool kRun>
+template <bool kW, bool kRun>
 struct flat_cold_gather {
-  using value = S;
   static constexpr int kLane = kFlatColdLane;
   static constexpr uint32_t kAhead = kRun ? 0 : 4;
   const uint32_t* ids;
   const float* w;
   const uint16_t* marks;
   const uint32_t* seg;
-  const S* x;
+  const float* x;
   using regs = flat_words;
   __device__ __forceinline__ void ahead(uint32_t step, unsigned lane) const {
     const size_t e = static_cast<size_t>(step) * kFlatColdStep;
@@ -227,7 +204,7 @@ struct flat_cold_gather {
     const uint16_t* p = marks + static_cast<size_t>(step) * 32 + lane;
     return kRun ? __ldg(p) : __ldcs(p);
   }
-  __device__ __forceinline__ void values(uint32_t step, unsigned lane, const regs& r, S (&v)[kLane]) const {
+  __device__ __forceinline__ void values(uint32_t step, unsigned lane, const regs& r, float (&v)[kLane]) const {
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = kRun ? x[r.w[i]] : __ldg(x + r.w[i]);
     if constexpr (kW) flat_weigh<!kRun>(w + static_cast<size_t>(step) * kFlatColdStep + lane * kLane, v);
@@ -239,15 +216,9 @@ __device__ __forceinline__ void flat_store_if(uint32_t on, float* p, float v) {
   asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.global.f32 [%1], %2; }" ::"r"(on), "l"(p), "f"(v)
                : "memory");
 }
-__device__ __forceinline__ void flat_store_if(uint32_t on, double* p, double v) {
-  asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.global.f64 [%1], %2; }" ::"r"(on), "l"(p), "d"(v)
-               : "memory");
-}
-
 // One warp's walk over the steps of piece p.
 template <class Gather>
-__device__ __forceinline__ void flat_piece(const flat_view<typename Gather::value>& f, uint32_t p, const Gather& g) {
-  using S = typename Gather::value;
+__device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const Gather& g) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int N = Gather::kLane;
   constexpr uint32_t kEnds = (1u << N) - 1u;
@@ -256,7 +227,7 @@ __device__ __forceinline__ void flat_piece(const flat_view<typename Gather::valu
   const uint2 pc = f.pieces[p];
   const uint32_t s0 = pc.x & ~kPieceFirst, s1 = pc.y;
   if (s0 >= s1) {
-    if (lane == 0) f.carry[p] = S(0);
+    if (lane == 0) f.carry[p] = 0.f;
     return;
   }
   typename Gather::regs cur;
@@ -268,10 +239,10 @@ __device__ __forceinline__ void flat_piece(const flat_view<typename Gather::valu
   const bool open =
       !(pc.x & kPieceFirst) && !(__ldg(g.marks + static_cast<size_t>(s0) * 32 - 1) & (1u << (N - 1)));
   const uint32_t j0 = open ? base : 0xffffffffu;  // the segment that began in an earlier piece
-  S acc = S(0);       // this lane's part of the open segment, from steps without an end
-  S carry = S(0);     // the open segment's sum before those, the same in every lane
+  float acc = 0.f;       // this lane's part of the open segment, from steps without an end
+  float carry = 0.f;     // the open segment's sum before those, the same in every lane
   for (uint32_t s = s0; s < s1; ++s) {
-    S v[N];
+    float v[N];
     g.values(s, lane, cur, v);
     uint32_t mark_n = 0, base_n = 0;
     if (s + 1 < s1) {
@@ -289,34 +260,34 @@ __device__ __forceinline__ void flat_piece(const flat_view<typename Gather::valu
         acc += ((v[i] + v[i + 1]) + (v[i + 2] + v[i + 3])) + ((v[i + 4] + v[i + 5]) + (v[i + 6] + v[i + 7]));
     } else {
       // this lane's sum after its last segment end, joined over the lanes
-      S t = S(0);
+      float t = 0.f;
 #pragma unroll
       for (int i = 0; i < N; ++i) {
         t += v[i];
-        t = (fl >> i) & 1u ? S(0) : t;
+        t = (fl >> i) & 1u ? 0.f : t;
       }
       const unsigned le = ends & (kAll >> (31 - lane));
       const int lo = le ? 31 - __clz(le) : 0;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
-        const S o = __shfl_up_sync(kAll, t, d);
+        const float o = __shfl_up_sync(kAll, t, d);
         if (static_cast<int>(lane) - d >= lo) t += o;
       }
       carry += warp_sum(acc);
-      acc = S(0);
-      S run = __shfl_up_sync(kAll, t, 1);
-      if (lane == 0) run = S(0);
+      acc = 0.f;
+      float run = __shfl_up_sync(kAll, t, 1);
+      if (lane == 0) run = 0.f;
       if (!(ends & below)) run += carry;
       carry = __shfl_sync(kAll, t, 31);
       // the segments that end here; a step of several pieces' segment goes to head
       const uint32_t ord = base + (mark >> N);
-      S* to = f.part + ord;
+      float* to = f.part + ord;
       if (ord == j0 && fl) {
         // its first end closes a segment of an earlier piece
         const int e = __ffs(fl) - 1;
-        S h = run;
+        float h = run;
 #pragma unroll
-        for (int i = 0; i < N; ++i) h += i <= e ? v[i] : S(0);
+        for (int i = 0; i < N; ++i) h += i <= e ? v[i] : 0.f;
         f.head[p] = h;
       }
 #pragma unroll
@@ -325,7 +296,7 @@ __device__ __forceinline__ void flat_piece(const flat_view<typename Gather::valu
         const uint32_t on = fl & (1u << i);
         flat_store_if(on, to, run);
         to += on ? 1 : 0;
-        run = on ? S(0) : run;
+        run = on ? 0.f : run;
       }
     }
     mark = mark_n;
@@ -349,56 +320,54 @@ __device__ __forceinline__ void flat_after() {
 // Hot streams (bound by issue: about 300 instructions a step of 512 edges, and
 // 3.4-way bank conflicts): CTA c walks its parts [cta_sub[c], cta_sub[c+1]), each within
 // one block whose ranks it first copies to shared memory.
-template <class S, bool kW>
-__global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_hot(flat_view<S> f, const S* __restrict__ x,
+template <bool kW>
+__global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_hot(flat_view f, const float* __restrict__ x,
                                                                    const int* mode) {
-  constexpr uint32_t kPer = 16 / sizeof(S);
   extern __shared__ float4 s_x4[];
   flat_after();
   if (mode && *mode == 2) return;
   const uint32_t sub1 = f.cta_sub[blockIdx.x + 1];
   for (uint32_t sub = f.cta_sub[blockIdx.x]; sub < sub1; ++sub) {
     const flat_sub sb = f.subs[sub];
-    const uint32_t src0 = sb.block * flat_block<S>;
-    const uint32_t n = min(flat_block<S>, f.nsrc - src0), n4 = n / kPer;
+    const uint32_t src0 = sb.block * kFlatBlock;
+    const uint32_t n = min(kFlatBlock, f.nsrc - src0), n4 = n / 4;
     __syncthreads();
     const float4* x4 = reinterpret_cast<const float4*>(x + src0);
 #pragma unroll 4
     for (uint32_t i = threadIdx.x; i < n4; i += kFlatHotWarps * 32) s_x4[i] = __ldg(x4 + i);
-    if (threadIdx.x < n % kPer)
-      reinterpret_cast<S*>(s_x4)[n4 * kPer + threadIdx.x] = __ldg(x + src0 + n4 * kPer + threadIdx.x);
+    if (threadIdx.x < n % 4)
+      reinterpret_cast<float*>(s_x4)[n4 * 4 + threadIdx.x] = __ldg(x + src0 + n4 * 4 + threadIdx.x);
     __syncthreads();
-    const flat_hot_gather<S, kW> g{f.hid, f.hw, f.hmark, f.hseg, reinterpret_cast<const S*>(s_x4)};
+    const flat_hot_gather<kW> g{f.hid, f.hw, f.hmark, f.hseg, reinterpret_cast<const float*>(s_x4)};
     flat_piece(f, sb.piece0 + (threadIdx.x >> 5), g);
   }
 }
 
 // The cold stream, bound by L2 requests.
-template <class S, bool kW>
-__global__ void __launch_bounds__(kFlatColdThreads, sizeof(S) == 4 ? 5 : 4) k_flat_cold(flat_view<S> f,
-                                                                                       const S* __restrict__ x,
+template <bool kW>
+__global__ void __launch_bounds__(kFlatColdThreads, 5) k_flat_cold(flat_view f,
+                                                                                       const float* __restrict__ x,
                                                                                        const int* mode) {
   flat_after();
   if (mode && *mode == 2) return;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= f.cold_pieces) return;
-  const flat_cold_gather<S, kW, false> g{f.cid, f.cw, f.cmark, f.cseg, x};
+  const flat_cold_gather<kW, false> g{f.cid, f.cw, f.cmark, f.cseg, x};
   flat_piece(f, f.cold_piece0 + w, g);
 }
 
 // The sums of one 32-row word's segments of a stream: lane l gets row l's.
 // They were written by other SMs, in the same kernel when it runs many epochs.
-template <class S>
-__device__ __forceinline__ S flat_segment(const flat_view<S>& f, const uint4& m, unsigned lane) {
+__device__ __forceinline__ float flat_segment(const flat_view& f, const uint4& m, unsigned lane) {
   const unsigned below = (1u << lane) - 1u;
-  if (!((m.x >> lane) & 1u)) return S(0);
+  if (!((m.x >> lane) & 1u)) return 0.f;
   if (!((m.z >> lane) & 1u)) return __ldcg(f.part + m.y + __popc(m.x & below));
   const uint2 sp = __ldg(f.spans + m.w + __popc(m.z & below));
-  S y = S(0);
+  float y = 0.f;
   for (uint32_t p = sp.x; p < sp.y; p += 4) {  // 4 loads in flight
-    S t[4];
+    float t[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t[i] = p + i < sp.y ? __ldcg(f.carry + p + i) : S(0);
+    for (int i = 0; i < 4; ++i) t[i] = p + i < sp.y ? __ldcg(f.carry + p + i) : 0.f;
     y += (t[0] + t[1]) + (t[2] + t[3]);
   }
   return y + __ldcg(f.head + sp.y);
@@ -411,13 +380,12 @@ __device__ __forceinline__ uint4 flat_shfl(const uint4& m, int l) {
 
 // The sums of the hot streams between the first and the cold one, for the 32
 // rows of word w.
-template <class S>
-__device__ __forceinline__ S flat_middle(const flat_view<S>& f, uint32_t w, unsigned lane) {
-  S y = S(0);
+__device__ __forceinline__ float flat_middle(const flat_view& f, uint32_t w, unsigned lane) {
+  float y = 0.f;
   uint4 mk = make_uint4(0, 0, 0, 0);  // lane k holds the meta of stream k + 1
   if (lane + 1 < f.nb) mk = __ldg(f.meta + f.words + static_cast<size_t>(lane) * f.words1 + w);
   for (uint32_t k = 0; k + 1 < f.nb; k += 4) {
-    S t[4];
+    float t[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) t[i] = flat_segment(f, flat_shfl(mk, k + i), lane);  // streams past nb: empty
     y += (t[0] + t[1]) + (t[2] + t[3]);
@@ -439,9 +407,8 @@ struct flat_control {
 };
 
 template <class Update>
-__global__ void __launch_bounds__(256, 4) k_flat_update(flat_view<typename Update::value> f, Update upd,
+__global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
                                                         double* partials, flat_control c) {
-  using S = typename Update::value;
   constexpr int R = 2;
   __shared__ double s_red[32];
   __shared__ bool s_last;
@@ -461,7 +428,7 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view<typename Updat
   }
   for (; w < f.words; w += R * nwarps) {
     typename Update::operands ops[R];
-    S y[R], z[R];
+    float y[R], z[R];
     uint4 n0[R], n1[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -545,7 +512,7 @@ __device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target, bo
 }
 
 template <class Update>
-__device__ __noinline__ void flat_poison(const flat_view<typename Update::value>& f, const Update& upd, uint32_t w0,
+__device__ __noinline__ void flat_poison(const flat_view& f, const Update& upd, uint32_t w0,
                                          uint32_t nwarps) {
   for (uint32_t w = w0; w < f.words; w += nwarps) {
     const uint32_t v = w * 32 + (threadIdx.x & 31);
@@ -562,11 +529,10 @@ __device__ __noinline__ void flat_poison(const flat_view<typename Update::value>
 // 70 / 9.4, 48K uniform edges 28 / 5.8.  A CTA that gives up waiting leaves NaN
 // in its rows.
 template <class Update, bool kW>
-__global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view<typename Update::value> f,
+__global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
                                                                    Update upd, uint32_t start, uint32_t iteration,
                                                                    double scale, double eps, int* ctrl, double* delta,
                                                                    double* partials, uint32_t* sync, bool cluster) {
-  using S = typename Update::value;
   __shared__ double s_red[32];
   __shared__ double s_delta;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -576,14 +542,14 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view<ty
   bool last = start + 1 >= iteration;
   for (;;) {
     upd.final_epoch = last ? 1 : 0;
-    flat_piece(f, w0, flat_cold_gather<S, kW, true>{f.cid, f.cw, f.cmark, f.cseg, upd.gathered()});
+    flat_piece(f, w0, flat_cold_gather<kW, true>{f.cid, f.cw, f.cmark, f.cseg, upd.gathered()});
     if (!flat_barrier(sync, ++barriers * gridDim.x, cluster)) return flat_poison(f, upd, w0, nwarps);
     double dl = 0.0;
     for (uint32_t w = w0; w < f.words; w += nwarps) {
       const uint32_t v = w * 32 + lane;
       const bool mine = v < f.V;
       const typename Update::operands ops = upd.load_l2(mine ? v : w * 32);
-      const S y = flat_segment(f, __ldg(f.meta + w), lane);
+      const float y = flat_segment(f, __ldg(f.meta + w), lane);
       if (mine) dl += upd.apply(v, y, ops);
     }
     ++ran;
@@ -635,18 +601,17 @@ cudaError_t flat_launch(bool behind, void (*kernel)(P...), uint32_t grid, uint32
 
 // The kernels of one epoch of a plan without run_ctas: sums of x into upd.
 template <class Upd, bool kW>
-int launch_flat_epoch(const flat_plan<typename Upd::value>& p, const typename Upd::value* x, const Upd& upd,
-                      double* partials, const flat_control& c, cudaStream_t st) {
-  using S = typename Upd::value;
+int launch_flat_epoch(const flat_plan& p, const float* x, const Upd& upd, double* partials, const flat_control& c,
+                      cudaStream_t st) {
   if (p.hot_ctas) {
     prof_scope ps("k_flat_hot", st);
-    PLATO_CUDA_TRY(flat_launch(true, k_flat_hot<S, kW>, p.hot_ctas, kFlatHotWarps * 32, kFlatBlockBytes, st, p.v,
+    PLATO_CUDA_TRY(flat_launch(true, k_flat_hot<kW>, p.hot_ctas, kFlatHotWarps * 32, kFlatBlockBytes, st, p.v,
                                x, c.ctrl));
     PLATO_LAUNCHED("k_flat_hot");
   }
   if (p.cold_blocks) {
     prof_scope ps("k_flat_cold", st);
-    PLATO_CUDA_TRY(flat_launch(p.hot_ctas == 0, k_flat_cold<S, kW>, p.cold_blocks, kFlatColdThreads, 0, st, p.v, x,
+    PLATO_CUDA_TRY(flat_launch(p.hot_ctas == 0, k_flat_cold<kW>, p.cold_blocks, kFlatColdThreads, 0, st, p.v, x,
                                c.ctrl));
     PLATO_LAUNCHED("k_flat_cold");
   }
@@ -659,7 +624,7 @@ int launch_flat_epoch(const flat_plan<typename Upd::value>& p, const typename Up
 // All epochs of a plan with run_ctas.  c.ctrl [4]: [1] becomes the epochs run,
 // [2] and [3] are the barrier's; cleared here.
 template <class Upd, bool kW>
-int launch_flat_run(const flat_plan<typename Upd::value>& p, const Upd& upd, uint32_t start, double* partials,
+int launch_flat_run(const flat_plan& p, const Upd& upd, uint32_t start, double* partials,
                     const flat_control& c, cudaStream_t st) {
   PLATO_CUDA_TRY(cudaMemsetAsync(c.ctrl, 0, 4 * sizeof(int), st));
   prof_scope ps("k_flat_run", st);

@@ -57,7 +57,6 @@ __device__ __forceinline__ void epoch_decide(int* ctrl, double* last_delta, doub
 
 template <class Teleport>
 struct rank_update {
-  using value = float;
   const float* x;                 // current state
   float* xn;                      // next state
   const uint32_t* __restrict__ deg;

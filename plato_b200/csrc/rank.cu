@@ -48,7 +48,7 @@ struct rank_workspace {
   uint32_t hub_cap = 0;       // ranks the pull kernel can stage in shared memory
   bool plan_built = false;
   pull_plan plan;
-  flat_plan<float> flat;
+  flat_plan flat;
   dbuf<uint32_t> seed_bits, seed_list;  // seed-set PPR
   dbuf<float> out_stage;                // caller-id ranks before the copy to the host
   dbuf<int> ctrl;                       // device epoch control (k_epoch_control); [2], [3] k_flat_run's barrier
@@ -80,7 +80,6 @@ using cfg = pull_warp_cfg<kIPT>;
 // A vertex whose out-weights sum to 0 gets x' = inf, so its edges give
 // inf * 0 = NaN, as the reference's 0 / 0 does.
 struct wrank_update {
-  using value = float;
   const float* r;                  // current ranks
   float* rn;                       // next ranks
   float* xn;                       // next gathered state
@@ -137,7 +136,6 @@ struct wrank_update {
 // epoch itself carries the exchange that an all-gather would do after it.
 constexpr uint32_t kMaxPartitionPeers = 7;  // 8 partitions (one node) at most
 struct bcast_rank_update {
-  using value = float;
   rank_update<teleport_uniform> u;  // local replica: u.xn
   float* peers[kMaxPartitionPeers];  // this partition's slice of the next state in the other replicas
   uint32_t npeers;
@@ -272,7 +270,7 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
   rank_workspace* ws = g->rank_ws;
   const uint32_t V = g->info.vertices;
   if (!ws->plan_built) {
-    PLATO_TRY(build_flat_plan(g, false, ws->flat, st));
+    PLATO_TRY(build_flat_plan(g, ws->flat, st));
     if (!ws->flat.valid) PLATO_TRY(build_plan(g, ws->plan, st));
     ws->plan_built = true;
   }

@@ -17,9 +17,11 @@
 //                         epoch -- plato_seedset_ppr on the binned pull.
 // The selection PageRank is the reference's default run (pagerank_opts_t:
 // 100 epochs, damping 0.85, eps 0.001; pagerank.hpp:39-46, 81-146) in double
-// precision on the flat pull (pull_flat.cuh; over the out-edges for the
-// transposed graph), so the order of the ranks is the reference's up to FP64
-// rounding, and the same from run to run.
+// precision, written with the reference's functor bodies for
+// include/plato_b200/dualmode.cuh (engine.reverse() for the transposed
+// graph), so the order of the ranks is the reference's up to FP64 rounding.
+// Its pulls run on the engine's combined path: the sums of a vertex's
+// 4-edge pieces in one warp are added in lane order before one write_add.
 #include <algorithm>
 #include <exception>
 #include <mutex>
@@ -31,7 +33,6 @@
 
 #include "graph.cuh"
 #include "plato_b200/dualmode.cuh"
-#include "pull_flat.cuh"
 
 namespace plato_b200 {
 namespace {
@@ -42,56 +43,67 @@ __global__ void k_tr_init(double* x, const uint32_t* __restrict__ deg, uint32_t 
     x[v] = deg[v] > 0 ? 1.0 / deg[v] : 1.0;  // pagerank.hpp:90-98
 }
 
-__global__ void k_tr_fill(double* x, uint32_t V, double value) {
-  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V;
-       v += (uint64_t)gridDim.x * blockDim.x)
-    x[v] = value;
-}
-
 // pagerank.hpp:118-135: r = (1-d) + d*y; non-final epochs divide by the degree
-// and sum |x' - x| * deg.
-struct selection_update {
-  using value = double;
-  const double* x;  // current state
-  double* xn;       // next state
-  const uint32_t* __restrict__ deg;
-  double d;
-  int final_epoch;
-  const int* mode = nullptr;  // epoch kind on the device, as in rank_update
-
-  __device__ __forceinline__ bool skip() const { return mode && *mode == 2; }
-  __device__ __forceinline__ bool storing_rank() const { return mode ? (*mode == 1) : (final_epoch != 0); }
-
-  struct operands {
-    uint32_t dg;
-    double xo;
-  };
-  __device__ __forceinline__ operands load(uint32_t v) const { return {__ldcs(deg + v), __ldcs(x + v)}; }
-  // load() inside a kernel that runs many epochs (the state is other SMs' work)
-  __device__ __forceinline__ operands load_l2(uint32_t v) const { return {__ldg(deg + v), __ldcg(x + v)}; }
-  __device__ __forceinline__ const double* gathered() const { return x; }
-  __device__ __forceinline__ void flip() {
-    const double* t = x;
-    x = xn;
-    xn = const_cast<double*>(t);
-  }
-  __device__ __forceinline__ void poison(uint32_t v) const {
-    xn[v] = const_cast<double*>(x)[v] = __longlong_as_double(0x7fffffffffffffffll);
-  }
-  __device__ __forceinline__ double apply(uint32_t v, double y, operands o) const {
-    double r = (1.0 - d) + d * y, dl = 0.0;
-    if (!storing_rank()) {
-      if (o.dg > 0) {
-        r /= o.dg;
-        dl = fabs(r - o.xo) * o.dg;
+// and sum |x' - x| * deg, one partial per block (summed in a fixed order by
+// k_tr_control, so the exit epoch does not depend on atomic order).  The
+// epoch is final when it is the last one or when ctrl[1] says so; nothing
+// runs once ctrl[0] is set.
+__global__ void __launch_bounds__(256) k_tr_update(double* n, const double* __restrict__ c,
+                                                   const uint32_t* __restrict__ deg, uint32_t V, double d,
+                                                   int last_epoch, double* partials, const uint32_t* ctrl) {
+  __shared__ double s_red[32];
+  if (ctrl[0]) return;
+  const bool last = last_epoch || ctrl[1];
+  double dl = 0.0;
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V;
+       v += (uint64_t)gridDim.x * blockDim.x) {
+    double r = (1.0 - d) + d * n[v];
+    if (!last) {
+      if (deg[v] > 0) {
+        r /= deg[v];
+        dl += fabs(r - c[v]) * deg[v];
       } else {
-        dl = fabs(r - o.xo);
+        dl += fabs(r - c[v]);
       }
     }
-    xn[v] = r;
-    return dl;
+    n[v] = r;
   }
-};
+  dl = block_sum<256>(dl, s_red);
+  if (threadIdx.x == 0) partials[blockIdx.x] = dl;
+}
+
+// next.fill(0) of the epoch, skipped like the rest once the final epoch has
+// run (the buffer it would clear may hold the result).
+__global__ void k_tr_zero(double* n, uint32_t V, const uint32_t* ctrl) {
+  if (ctrl[0]) return;
+  for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V;
+       v += (uint64_t)gridDim.x * blockDim.x)
+    n[v] = 0.0;
+}
+
+// The eps early exit of pagerank.hpp:137-139 decided on the device, so the
+// host enqueues every epoch without waiting: the epoch's delta is the sum of
+// the update's n block partials in a fixed order; after a non-final epoch
+// with delta < eps the next epoch is the final one (ctrl[1]); after the
+// final epoch ctrl[0] stops the rest and ctrl[2] records which epoch it was.
+__global__ void __launch_bounds__(1024) k_tr_control(const double* __restrict__ partials, uint32_t n,
+                                                     double eps, uint32_t epoch, int last_epoch,
+                                                     uint32_t* ctrl) {
+  __shared__ double s_red[32];
+  if (ctrl[0]) return;  // grid-uniform
+  const uint32_t per = (n + 1023) / 1024;
+  const uint32_t b = threadIdx.x * per, e = min(n, b + per);
+  double s = 0.0;
+  for (uint32_t i = b; i < e; ++i) s += partials[i];
+  s = block_sum<1024>(s, s_red);
+  if (threadIdx.x != 0) return;
+  if (last_epoch || ctrl[1]) {
+    ctrl[0] = 1;
+    ctrl[2] = epoch;
+  } else if (s < eps) {
+    ctrl[1] = 1;
+  }
+}
 
 // Selection ranks laid out by caller id, with the caller ids beside them.
 __global__ void k_tr_keys(const double* __restrict__ r, const uint32_t* __restrict__ to_ext, uint32_t V,
@@ -145,91 +157,68 @@ std::vector<uint32_t> top_ids(const double* r, const uint32_t* to_ext, uint32_t 
   return out;
 }
 
-}  // namespace
-
-// The selection's plans (pulls over the in-edges and, transposed, over the
-// out-edges), kept with the graph, and its epoch control.
-struct trust_workspace {
-  flat_plan<double> plan[2];
-  bool built[2] = {false, false};
-  dbuf<double> x[2], partials, delta;
-  dbuf<int> ctrl;
-  int* h_ctrl = nullptr;  // pinned [8]: two control words
-  cudaEvent_t polled[2] = {nullptr, nullptr};
-  ~trust_workspace() {
-    if (h_ctrl) cudaFreeHost(h_ctrl);
-    for (cudaEvent_t e : polled)
-      if (e) cudaEventDestroy(e);
-  }
-};
-
-void destroy_trust_workspace(trust_workspace* w) { delete w; }
-
-namespace {
-
-constexpr uint32_t kSelectIterations = 100;
-constexpr double kSelectDamping = 0.85, kSelectEps = 0.001;
-
-// The selection PageRank on the flat pull (pull_flat.cuh) in 64 bits, its exit
-// decided on the device; *ranks = the state that holds them.
-int selection_ranks(plato_graph* g, bool inverse, cudaStream_t st, const double** ranks) {
-  if (!g->trust_ws) {
-    g->trust_ws = new (std::nothrow) trust_workspace();
-    if (!g->trust_ws) return set_error(PLATO_ENOMEM, "trustrank: host allocation failed");
-  }
-  trust_workspace* ws = g->trust_ws;
-  const int side = inverse ? 1 : 0;
-  const uint32_t V = g->info.vertices;
-  flat_plan<double>& pl = ws->plan[side];
-  if (!ws->built[side]) {
-    PLATO_TRY(build_flat_plan<double>(g, inverse, pl, st));
-    ws->built[side] = true;
-  }
-  *ranks = nullptr;
-  if (!pl.valid) return PLATO_OK;
-  for (auto& x : ws->x) PLATO_TRY(x.alloc(V));
-  PLATO_TRY(ws->partials.alloc(std::max<size_t>(pl.update_blocks, 2ull * pl.run_ctas)));
-  PLATO_TRY(ws->delta.alloc(1));
-  PLATO_TRY(ws->ctrl.alloc(4));
-  if (!ws->h_ctrl) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_ctrl), 8 * sizeof(int)));
-  for (cudaEvent_t& e : ws->polled)
-    if (!e) PLATO_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+// The k caller ids of highest rank under the reference's default PageRank on
+// the graph (transposed when `inverse`).
+std::vector<uint32_t> selection_top(plato_graph* g, bool inverse, uint32_t k) {
+  constexpr uint32_t kIterations = 100;
+  constexpr double kDamping = 0.85, kEps = 0.001;
+  dualmode_engine_t engine(g);
+  plato_graph_device_view view{};
+  if (plato_graph_get_device_view(g, &view) != PLATO_OK) throw std::runtime_error(plato_last_error());
+  if (inverse) engine.reverse();
   // out-degrees of the structure the pull walks: in-degrees when transposed
-  const uint32_t* deg = inverse ? g->in_deg.p : g->out_deg.p;
-  k_tr_init<<<grid_for(V, 256), 256, 0, st>>>(ws->x[0].p, deg, V);
-  PLATO_LAUNCHED("k_tr_init");
-  const flat_control c{ws->ctrl.p, ws->delta.p, 1.0, kSelectEps, kSelectIterations};
-  const auto update = [&](uint32_t epoch, const int* mode) {
-    return selection_update{ws->x[epoch & 1].p, ws->x[(epoch & 1) ^ 1].p, deg, kSelectDamping, 0, mode};
-  };
-  int ran = 0;
-  if (pl.run_ctas) {
-    PLATO_TRY((launch_flat_run<selection_update, false>(pl, update(0, nullptr), 0, ws->partials.p, c, st)));
-    PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl, ws->ctrl.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-    if (ws->h_ctrl[3]) return set_error(PLATO_ETIMEDOUT, "k_flat_run: a grid barrier ran out");
-    ran = ws->h_ctrl[1];
-  } else {
-    PLATO_CUDA_TRY(cudaMemsetAsync(ws->ctrl.p, 0, 4 * sizeof(int), st));
-    // a few epochs at a time, one batch ahead of the control word read
-    constexpr uint32_t kBatch = 6;
-    uint32_t epoch = 0, batches = 0;
-    while (epoch < kSelectIterations) {
-      for (uint32_t k = 0; k < kBatch && epoch < kSelectIterations; ++k, ++epoch)
-        PLATO_TRY((launch_flat_epoch<selection_update, false>(pl, ws->x[epoch & 1].p, update(epoch, ws->ctrl.p),
-                                                              ws->partials.p, c, st)));
-      const uint32_t slot = batches++ & 1u;
-      PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl + 4 * slot, ws->ctrl.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-      PLATO_CUDA_TRY(cudaEventRecord(ws->polled[slot], st));
-      if (batches == 1) continue;
-      PLATO_CUDA_TRY(cudaEventSynchronize(ws->polled[slot ^ 1]));
-      if (ws->h_ctrl[4 * (slot ^ 1)] == 2) break;
+  const uint32_t* deg = inverse ? view.in_degree : view.out_degree;
+  const uint32_t V = engine.vertices();
+  dense_state_t<double> x[2] = {engine.alloc_v_state<double>(), engine.alloc_v_state<double>()};
+  double* delta = nullptr;  // the update's block partials
+  uint32_t* ctrl = nullptr;
+  int* unused = nullptr;
+  const unsigned upd_blocks = grid_for(V, 256);
+  dev_alloc(&delta, upd_blocks * sizeof(double), "trustrank delta");
+  uint32_t final_epoch = 0;
+  try {
+    dev_alloc(&ctrl, 3 * sizeof(uint32_t), "trustrank control");
+    dev_alloc(&unused, sizeof(int), "trustrank slot sum");
+    check_cuda(cudaMemset(ctrl, 0, 3 * sizeof(uint32_t)), "trustrank control");
+    k_tr_init<<<grid_for(V, 256), 256>>>(x[0].data(), deg, V);
+    check_cuda(cudaGetLastError(), "k_tr_init");
+    count_launch();
+    for (uint32_t epoch = 0; epoch < kIterations; ++epoch) {
+      const double* c = x[epoch & 1].data();
+      double* n = x[(epoch & 1) ^ 1].data();
+      k_tr_zero<<<grid_for(V, 256), 256>>>(n, V, ctrl);
+      check_cuda(cudaGetLastError(), "k_tr_zero");
+      const uint32_t* done = ctrl;
+      engine.foreach_edges_device<double, int>(
+          [c, done] __device__(const auto& context, vid_t v_i, const adj_unit_list_t& adjs) {
+            if (*done) return;
+            double rank_sum = 0.0;
+            for (auto it = adjs.begin_; adjs.end_ != it; ++it) rank_sum += c[it->neighbour_];
+            context.send(mepa_ag_message_t<double>{v_i, rank_sum});
+          },
+          [n] __device__(int, mepa_ag_message_t<double>& msg) -> int {
+            atomicAdd(n + msg.v_i_, msg.message_);  // write_add (atomic.hpp:97-104)
+            return 0;
+          },
+          make_combiner([] __device__(double& into, const double& from) { into += from; }), unused);
+      const int last = epoch + 1 == kIterations ? 1 : 0;
+      k_tr_update<<<upd_blocks, 256>>>(n, c, deg, V, kDamping, last, delta, ctrl);
+      check_cuda(cudaGetLastError(), "k_tr_update");
+      k_tr_control<<<1, 1024>>>(delta, upd_blocks, kEps, epoch, last, ctrl);
+      check_cuda(cudaGetLastError(), "k_tr_control");
+      count_launch(5);
     }
-    PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-    ran = ws->h_ctrl[4 * ((batches - 1) & 1u) + 1];
+    check_cuda(cudaMemcpy(&final_epoch, ctrl + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost), "trustrank control");
+  } catch (...) {
+    dev_free(delta);
+    dev_free(ctrl);
+    dev_free(unused);
+    throw;
   }
-  *ranks = ws->x[ran & 1].p;
-  return PLATO_OK;
+  dev_free(delta);
+  dev_free(ctrl);
+  dev_free(unused);
+  return top_ids(x[(final_epoch & 1) ^ 1].data(), view.to_external, V, k);
 }
 
 int select_seeds(plato_graph* g, const plato_trustrank_opts* o, const uint8_t* good,
@@ -254,16 +243,7 @@ int select_seeds(plato_graph* g, const plato_trustrank_opts* o, const uint8_t* g
     return PLATO_OK;
   }
   const uint32_t k = std::min<uint32_t>(o->seed_num, V);
-  const double* ranks = nullptr;
-  PLATO_TRY(selection_ranks(g, o->select_method == 0, 0, &ranks));
-  dbuf<double> flat_ranks;
-  if (!ranks) {  // no edge: every vertex keeps the teleport
-    PLATO_TRY(flat_ranks.alloc(V));
-    k_tr_fill<<<grid_for(V, 256), 256>>>(flat_ranks.p, V, 1.0 - kSelectDamping);
-    PLATO_LAUNCHED("k_tr_fill");
-    ranks = flat_ranks.p;
-  }
-  const std::vector<uint32_t> order = top_ids(ranks, g->relabeled ? g->to_ext.p : nullptr, V, k);
+  const std::vector<uint32_t> order = selection_top(g, o->select_method == 0, k);
   for (uint32_t i = 0; i < k; ++i)
     if (is_good(order[i])) seeds->push_back(order[i]);
   std::sort(seeds->begin(), seeds->end());
