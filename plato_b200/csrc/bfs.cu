@@ -118,7 +118,8 @@ constexpr uint32_t kPushLaneEdges = 8;  // chunks this short are walked by one l
 // flight), and the warp walks the longer chunks together.  Large push
 // frontiers are mostly low-degree vertices with one short chunk each.
 __device__ __forceinline__ void bfs_push_step(const bfs_level_args& a) {
-  const unsigned long long nchunks = a.cur.counters[1];
+  const unsigned long long nchunks = frontier_chunks(a.cur.counters[0]);
+  unsigned long long dsum = 0;
   const unsigned lane = threadIdx.x & 31;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -137,9 +138,10 @@ __device__ __forceinline__ void bfs_push_step(const bfs_level_args& a) {
           dst = a.out_adj[e];
           fresh = bfs_claim(a, ch.x, dst, a.visited[dst >> 5]);
         }
-        frontier_append_warp(a.next, fresh, dst, a.out_deg);
+        frontier_append_warp(a.next, fresh, dst, a.out_deg, dsum);
       }
     }
+    frontier_flush(a.next, dsum);
     return;
   }
   const uint64_t ntasks = (nchunks + 31) / 32;
@@ -173,10 +175,10 @@ __device__ __forceinline__ void bfs_push_step(const bfs_level_args& a) {
         f2 = e + 2 < e_end && bfs_claim(a, u, d2, w2);
         f3 = e + 3 < e_end && bfs_claim(a, u, d3, w3);
       }
-      frontier_append_warp(a.next, f0, d0, a.out_deg);
-      frontier_append_warp(a.next, f1, d1, a.out_deg);
-      frontier_append_warp(a.next, f2, d2, a.out_deg);
-      frontier_append_warp(a.next, f3, d3, a.out_deg);
+      frontier_append_warp(a.next, f0, d0, a.out_deg, dsum);
+      frontier_append_warp(a.next, f1, d1, a.out_deg, dsum);
+      frontier_append_warp(a.next, f2, d2, a.out_deg, dsum);
+      frontier_append_warp(a.next, f3, d3, a.out_deg, dsum);
     }
     unsigned big = __ballot_sync(0xffffffffu, !own);
     while (big) {  // warp-uniform
@@ -193,10 +195,11 @@ __device__ __forceinline__ void bfs_push_step(const bfs_level_args& a) {
           dst = a.out_adj[e];
           fresh = bfs_claim(a, uu, dst, a.visited[dst >> 5]);
         }
-        frontier_append_warp(a.next, fresh, dst, a.out_deg);
+        frontier_append_warp(a.next, fresh, dst, a.out_deg, dsum);
       }
     }
   }
+  frontier_flush(a.next, dsum);
 }
 
 // Pull step: every unvisited vertex takes the first in-neighbour (CSC order)
@@ -210,6 +213,7 @@ __device__ __forceinline__ void bfs_pull_step(const bfs_level_args& a, append_sm
   const uint32_t* cur = a.cur.bits;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t rounds = (a.V + stride - 1) / stride;
+  unsigned long long dsum = 0;
   // the next row's visited bit and offsets are loaded one round ahead (only
   // this thread can mark its own rows visited during a pull step)
   uint64_t v_next = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -281,8 +285,9 @@ __device__ __forceinline__ void bfs_pull_step(const bfs_level_args& a, append_sm
       a.visited[v >> 5] |= fm;
       a.next.bits[v >> 5] |= fm;
     }
-    frontier_append_block(a.next, found, v, a.out_deg, app);  // block-uniform: same rounds everywhere
+    frontier_append_block(a.next, found, v, a.out_deg, app, dsum);  // block-uniform: same rounds everywhere
   }
+  frontier_flush(a.next, dsum);
 }
 
 __global__ void __launch_bounds__(256, 8) k_bfs_level(bfs_level_args a) {
@@ -295,7 +300,7 @@ __global__ void __launch_bounds__(256, 8) k_bfs_level(bfs_level_args a) {
   const uint32_t words = (a.V + 31) / 32;
   for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += gridDim.x * blockDim.x)
     a.spare.bits[w] = 0;
-  if (blockIdx.x == 0 && threadIdx.x < 3) a.spare.counters[threadIdx.x] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < 2) a.spare.counters[threadIdx.x] = 0;
 
   if (mode == 1)
     bfs_push_step(a);
@@ -313,8 +318,8 @@ __global__ void __launch_bounds__(256, 8) k_bfs_level(bfs_level_args a) {
   if (!s_last || threadIdx.x != 0) return;
   __threadfence();
   c->arrived = 0;
-  const unsigned long long actives = atomicAdd(&a.next.counters[0], 0ull);
-  const unsigned long long active_edges = atomicAdd(&a.next.counters[2], 0ull);
+  const uint32_t actives = frontier_members(atomicAdd(&a.next.counters[0], 0ull));
+  const unsigned long long active_edges = atomicAdd(&a.next.counters[1], 0ull);
   if (mode == 1) c->pushes += 1;
   c->level += 1;
   c->visited += actives;
@@ -363,7 +368,7 @@ __global__ void k_parents_to_external(const uint32_t* __restrict__ parent_int,
 // decided on the device from the seeded frontier's degree sum.
 __global__ void k_bfs_start(bfs_control* c, const unsigned long long* counters, double edges,
                             double threshold) {
-  const bool push = (static_cast<double>(counters[2]) / edges) < threshold;
+  const bool push = (static_cast<double>(counters[1]) / edges) < threshold;
   *c = bfs_control{push ? 1 : 0, 0, 0, 0, 1ull, push ? 1ull : 0ull, 0u};
 }
 
@@ -377,7 +382,9 @@ __global__ void k_frontier_seed_at(frontier_view f, const uint32_t* __restrict__
   const uint32_t v = *vp;
   const bool take = (threadIdx.x == 0);
   if (take) atomicOr(&f.bits[v >> 5], 1u << (v & 31));
-  frontier_append_warp(f, take, v, deg);
+  unsigned long long dsum = 0;
+  frontier_append_warp(f, take, v, deg, dsum);
+  frontier_flush(f, dsum);
 }
 
 // A launch inside a capture: its error is checked, and it is counted once

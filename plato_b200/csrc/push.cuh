@@ -8,10 +8,12 @@
 //   chunks   work items (vertex, k): edges [out_off[v] + k*C, min(+C, out_off[v+1]))
 //            of a member, C = kPushChunk, so a hub's out-edges spread over
 //            many warps and no warp walks more than C edges,
-//   counters [0] members, [1] chunks, [2] sum of member out-degrees
-//            (= active_edges of dualmode.hpp:264-277).
-// Members are appended with warp-aggregated atomics: one atomic per warp for
-// the queue slot, one for the chunk range, one for the degree sum.
+//   counters [0] members (low 32 bits) and chunks (high 32 bits), [1] sum of
+//            member out-degrees (= active_edges of dualmode.hpp:264-277).
+// Members are appended with warp-aggregated atomics: one atomic per warp takes
+// the queue slots and the chunk range together; the degrees add up in the lanes
+// and reach the counter once per warp (frontier_flush).  With an atomic for each
+// of the three per 32 edges, a push level waited on the counters' line.
 #pragma once
 
 #include "common.cuh"
@@ -34,7 +36,7 @@ struct push_frontier {
   dbuf<uint32_t> queue;
   dbuf<uint2> chunks;
   dbuf<unsigned long long> counters;
-  unsigned long long* h_counters = nullptr;  // pinned [3]
+  unsigned long long* h_counters = nullptr;  // pinned [2]
   push_frontier() = default;
   push_frontier(const push_frontier&) = delete;
   push_frontier& operator=(const push_frontier&) = delete;
@@ -48,83 +50,90 @@ __device__ __forceinline__ bool test_bit(const uint32_t* bits, uint32_t v) {
   return (bits[v >> 5] >> (v & 31)) & 1u;
 }
 
+__device__ __forceinline__ uint32_t frontier_members(unsigned long long c) { return static_cast<uint32_t>(c); }
+__host__ __device__ __forceinline__ uint32_t frontier_chunks(unsigned long long c) {
+  return static_cast<uint32_t>(c >> 32);
+}
+
+// Exclusive scan over the lanes of the chunk counts; *total = their sum.
+__device__ __forceinline__ uint32_t frontier_scan(uint32_t n, uint32_t* total) {
+  const unsigned lane = threadIdx.x & 31;
+  uint32_t inc = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= static_cast<unsigned>(o)) inc += t;
+  }
+  *total = __shfl_sync(0xffffffffu, inc, 31);
+  return inc - n;
+}
+
 // Warp-collective append of the lanes with `take` set (all 32 lanes call).
+// Each lane adds its member's degree to dsum (frontier_flush).
 __device__ __forceinline__ void frontier_append_warp(frontier_view f, bool take, uint32_t v,
-                                                     const uint32_t* __restrict__ deg) {
+                                                     const uint32_t* __restrict__ deg, unsigned long long& dsum) {
   const unsigned lane = threadIdx.x & 31;
   const unsigned m = __ballot_sync(0xffffffffu, take);
   if (m == 0) return;
-  const unsigned leader = __ffs(m) - 1;
-  unsigned long long base = 0;
-  if (lane == leader) base = atomicAdd(&f.counters[0], static_cast<unsigned long long>(__popc(m)));
-  base = __shfl_sync(0xffffffffu, base, leader);
   const uint32_t dg = take ? deg[v] : 0u;
-  if (take) f.queue[base + __popc(m & ((1u << lane) - 1u))] = v;
-  // chunk range: warp inclusive scan of the chunk counts
+  dsum += dg;
   const uint32_t nch = (dg + kPushChunk - 1) / kPushChunk;
-  uint32_t inc = nch;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= static_cast<unsigned>(o)) inc += t;
+  uint32_t tot = 0, before = 0;
+  if (__any_sync(0xffffffffu, nch > 1)) {
+    before = frontier_scan(nch, &tot);
+  } else {  // no member spans chunks: positions by ballot
+    const unsigned has = __ballot_sync(0xffffffffu, nch != 0);
+    tot = __popc(has);
+    before = __popc(has & ((1u << lane) - 1u));
   }
-  const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
-  unsigned long long cbase = 0;
-  if (lane == leader && tot) cbase = atomicAdd(&f.counters[1], static_cast<unsigned long long>(tot));
-  cbase = __shfl_sync(0xffffffffu, cbase, leader);
-  for (uint32_t k = 0; k < nch; ++k) f.chunks[cbase + (inc - nch) + k] = make_uint2(v, k);
-  const unsigned long long dsum = warp_sum(static_cast<unsigned long long>(dg));
-  if (lane == leader && dsum) atomicAdd(&f.counters[2], dsum);
+  unsigned long long base = 0;
+  if (lane == 0)
+    base = atomicAdd(&f.counters[0],
+                     static_cast<unsigned long long>(tot) << 32 | static_cast<unsigned long long>(__popc(m)));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (take) {
+    f.queue[frontier_members(base) + __popc(m & ((1u << lane) - 1u))] = v;
+    for (uint32_t k = 0; k < nch; ++k) f.chunks[frontier_chunks(base) + before + k] = make_uint2(v, k);
+  }
+}
+
+// Adds the lanes' degree sums to the frontier (all 32 lanes call, once).
+__device__ __forceinline__ void frontier_flush(frontier_view f, unsigned long long dsum) {
+  dsum = warp_sum(dsum);
+  if ((threadIdx.x & 31) == 0 && dsum) atomicAdd(&f.counters[1], dsum);
 }
 
 // Block-collective append (every thread of the block calls, the same number
-// of times): warps reserve their slots with shared-memory atomics and one
-// thread per block takes the block's ranges from the global counters, so the
-// counters see one atomic per block and call instead of one per warp.
+// of times): warps reserve their slots with one shared-memory atomic and one
+// thread per block takes the block's ranges from the global counter, so the
+// counter sees one atomic per block and call instead of one per warp.
 struct append_smem {
-  unsigned long long base_q, base_c, dsum;
-  uint32_t cnt_q, cnt_c;
+  unsigned long long base, cnt;  // chunks << 32 | members
 };
 
 __device__ __forceinline__ void frontier_append_block(frontier_view f, bool take, uint32_t v,
-                                                      const uint32_t* __restrict__ deg,
-                                                      append_smem& sm) {
+                                                      const uint32_t* __restrict__ deg, append_smem& sm,
+                                                      unsigned long long& dsum) {
   const unsigned lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    sm.cnt_q = 0;
-    sm.cnt_c = 0;
-    sm.dsum = 0;
-  }
-  __syncthreads();
+  if (threadIdx.x == 0) sm.cnt = 0;
+  if (__syncthreads_or(take) == 0) return;  // block-uniform
   const unsigned m = __ballot_sync(0xffffffffu, take);
   const uint32_t dg = take ? deg[v] : 0u;
+  dsum += dg;
   const uint32_t nch = (dg + kPushChunk - 1) / kPushChunk;
-  uint32_t inc = nch;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= static_cast<unsigned>(o)) inc += t;
-  }
-  const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
-  const unsigned long long dsum = warp_sum(static_cast<unsigned long long>(dg));
-  uint32_t wq = 0, wc = 0;
-  if (lane == 0 && m) {
-    wq = atomicAdd(&sm.cnt_q, static_cast<uint32_t>(__popc(m)));
-    if (tot) wc = atomicAdd(&sm.cnt_c, tot);
-    if (dsum) atomicAdd(&sm.dsum, dsum);
-  }
-  wq = __shfl_sync(0xffffffffu, wq, 0);
-  wc = __shfl_sync(0xffffffffu, wc, 0);
+  uint32_t tot = 0;
+  const uint32_t before = frontier_scan(nch, &tot);
+  unsigned long long w = 0;
+  if (lane == 0 && m)
+    w = atomicAdd(&sm.cnt, static_cast<unsigned long long>(tot) << 32 | static_cast<unsigned long long>(__popc(m)));
+  w = __shfl_sync(0xffffffffu, w, 0);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (sm.cnt_q) sm.base_q = atomicAdd(&f.counters[0], static_cast<unsigned long long>(sm.cnt_q));
-    if (sm.cnt_c) sm.base_c = atomicAdd(&f.counters[1], static_cast<unsigned long long>(sm.cnt_c));
-    if (sm.dsum) atomicAdd(&f.counters[2], sm.dsum);
-  }
+  if (threadIdx.x == 0) sm.base = atomicAdd(&f.counters[0], sm.cnt);
   __syncthreads();
   if (take) {
-    f.queue[sm.base_q + wq + __popc(m & ((1u << lane) - 1u))] = v;
-    for (uint32_t k = 0; k < nch; ++k) f.chunks[sm.base_c + wc + (inc - nch) + k] = make_uint2(v, k);
+    const unsigned long long at = sm.base + w;  // both halves: neither sum reaches 2^32
+    f.queue[frontier_members(at) + __popc(m & ((1u << lane) - 1u))] = v;
+    for (uint32_t k = 0; k < nch; ++k) f.chunks[frontier_chunks(at) + before + k] = make_uint2(v, k);
   }
 }
 
@@ -132,7 +141,9 @@ static __global__ void k_frontier_seed(frontier_view f, uint32_t v, const uint32
   // one warp
   const bool take = (threadIdx.x == 0);
   if (take) atomicOr(&f.bits[v >> 5], 1u << (v & 31));
-  frontier_append_warp(f, take, v, deg);
+  unsigned long long dsum = 0;
+  frontier_append_warp(f, take, v, deg, dsum);
+  frontier_flush(f, dsum);
 }
 
 inline int frontier_alloc(push_frontier& f, const plato_graph* g) {
@@ -141,15 +152,15 @@ inline int frontier_alloc(push_frontier& f, const plato_graph* g) {
   PLATO_TRY(f.bits.alloc((V + 31) / 32));
   PLATO_TRY(f.queue.alloc(V));
   PLATO_TRY(f.chunks.alloc(static_cast<size_t>(V) + g->stored_edges / kPushChunk + 1));
-  PLATO_TRY(f.counters.alloc(3));
+  PLATO_TRY(f.counters.alloc(2));
   if (!f.h_counters)
-    PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&f.h_counters), 3 * sizeof(unsigned long long)));
+    PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&f.h_counters), 2 * sizeof(unsigned long long)));
   return PLATO_OK;
 }
 
 inline int frontier_reset(push_frontier& f, uint32_t V, cudaStream_t st) {
   PLATO_CUDA_TRY(cudaMemsetAsync(f.bits.p, 0, ((V + 31) / 32) * sizeof(uint32_t), st));
-  PLATO_CUDA_TRY(cudaMemsetAsync(f.counters.p, 0, 3 * sizeof(unsigned long long), st));
+  PLATO_CUDA_TRY(cudaMemsetAsync(f.counters.p, 0, 2 * sizeof(unsigned long long), st));
   return PLATO_OK;
 }
 
@@ -161,7 +172,7 @@ inline int frontier_seed(push_frontier& f, const plato_graph* g, uint32_t v, cud
 
 // Copies the counters to the host (synchronises `st`).
 inline int frontier_read(push_frontier& f, cudaStream_t st) {
-  PLATO_CUDA_TRY(cudaMemcpyAsync(f.h_counters, f.counters.p, 3 * sizeof(unsigned long long),
+  PLATO_CUDA_TRY(cudaMemcpyAsync(f.h_counters, f.counters.p, 2 * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
   return PLATO_OK;
@@ -169,7 +180,7 @@ inline int frontier_read(push_frontier& f, cudaStream_t st) {
 
 inline int frontier_active_edges(push_frontier& f, cudaStream_t st, uint64_t* active_edges) {
   PLATO_TRY(frontier_read(f, st));
-  *active_edges = f.h_counters[2];
+  *active_edges = f.h_counters[1];
   return PLATO_OK;
 }
 
@@ -189,6 +200,7 @@ static __global__ void __launch_bounds__(256) k_ppr_push(frontier_view f, unsign
   const unsigned lane = threadIdx.x & 31;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  unsigned long long dsum = 0;
   for (uint64_t c = warp; c < nchunks; c += nwarps) {
     const uint2 ch = f.chunks[c];
     const uint32_t u = ch.x;
@@ -206,15 +218,16 @@ static __global__ void __launch_bounds__(256) k_ppr_push(frontier_view f, unsign
         const uint32_t bit = 1u << (dst & 31);
         if (!(f.bits[dst >> 5] & bit)) fresh = !(atomicOr(&f.bits[dst >> 5], bit) & bit);
       }
-      frontier_append_warp(f, fresh, dst, deg);
+      frontier_append_warp(f, fresh, dst, deg, dsum);
     }
   }
+  frontier_flush(f, dsum);
 }
 
 inline int frontier_push_scatter(push_frontier& f, const plato_graph* g, const float* x, float* y,
                                  cudaStream_t st) {
   // the chunk count was read by the preceding frontier_active_edges()
-  const unsigned long long nchunks = f.h_counters[1];
+  const unsigned long long nchunks = frontier_chunks(f.h_counters[0]);
   if (nchunks == 0) return PLATO_OK;
   const unsigned blocks = grid_for(nchunks * 32, 256, 148 * 16);
   k_ppr_push<<<blocks, 256, 0, st>>>(f.view(), nchunks, g->out_off.p, g->out_adj.p, g->out_deg.p,
