@@ -103,3 +103,26 @@ def test_seed_sets_and_single_queries(scale):
             assert abs(st.iterations - epochs) <= 1
             # the bar, and one epoch that moves less than eps where one side ends earlier
             assert np.abs(got.astype(np.float64) - want).sum() <= 1e-6 + 1e-6
+
+
+def test_no_room_for_the_plan():
+    """With less memory left than the plan takes (RMAT s20: 50 MB and its
+    scratch) the merge path answers; a later graph gets its plan again."""
+    import torch
+
+    V, s, d = pb.rmat(20, 16, 9)
+    want, epochs, _ = RefGraph(V, s, d, True).pagerank(10, 0.85, 0.0)
+    with pb.Graph(1000, s[:100] % 1000, d[:100] % 1000, True, relabel=False) as small:
+        small.pagerank(2, 0.85, 0.0)  # the merge path's kernels are loaded
+    with pb.Graph(V, s, d, True) as g:
+        free, _ = torch.cuda.mem_get_info()
+        hog = torch.empty(max(free - (32 << 20), 0), dtype=torch.uint8, device="cuda")
+        try:
+            got, st = g.pagerank(10, 0.85, 0.0)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        again, _ = g.pagerank(10, 0.85, 0.0)
+    assert st.iterations == epochs
+    assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
+    np.testing.assert_array_equal(got, again)  # the graph stays on its path
