@@ -27,9 +27,9 @@
 // flight a lane); L1 hits go at 560-790 G/s, shared memory at 1700 G/s.  RMAT
 // s24's 263M gathers are 0.95 ms of L2 requests; its hottest 57344 sources are
 // 46% of them, 24 blocks 90%.  RMAT s24, one PageRank epoch on one B200: 826 us
-// with the degree bins (pull_binned.cuh), 532 us here: k_flat_hot 210 us (210M
-// edges), k_flat_cold 229 (53M), k_flat_update 96.  RMAT s22 220 -> 138 us, s20
-// 98 -> 49, 16M uniform edges over 1M vertices 107 -> 82, 64M over 1M 303 -> 144.
+// with degree bins (pull_binned.cuh), 503 us here: k_flat_hot 211 us (210M
+// edges), k_flat_cold 231 (53M), k_flat_update 82.  RMAT s22 220 -> 139 us, s20
+// 98 -> 47, 16M uniform edges over 1M vertices 107 -> 81, 64M over 1M 303 -> 135.
 #pragma once
 
 #include <utility>
@@ -378,25 +378,32 @@ __device__ __forceinline__ uint4 flat_shfl(const uint4& m, int l) {
                     __shfl_sync(0xffffffffu, m.z, l), __shfl_sync(0xffffffffu, m.w, l));
 }
 
-// The sums of the hot streams between the first and the cold one, for the 32
-// rows of word w.
-__device__ __forceinline__ float flat_middle(const flat_view& f, uint32_t w, unsigned lane) {
+// The metas of word w in the hot streams between the first and the cold one:
+// lane k holds stream k + 1's.
+__device__ __forceinline__ uint4 flat_middle_meta(const flat_view& f, uint32_t w, unsigned lane) {
+  if (w >= f.words1 || lane + 1 >= f.nb) return make_uint4(0, 0, 0, 0);
+  return __ldg(f.meta + f.words + static_cast<size_t>(lane) * f.words1 + w);
+}
+
+// The sums of those streams for the word's 32 rows, 8 streams' loads in flight
+// (a chain of 23 streams at RMAT s24; epoch with 4 / 8: s24 518 / 503 us, s22
+// 140.5 / 139.5, 64M uniform edges over 1M vertices 137.5 / 135).
+__device__ __forceinline__ float flat_middle(const flat_view& f, const uint4& mk, unsigned lane) {
   float y = 0.f;
-  uint4 mk = make_uint4(0, 0, 0, 0);  // lane k holds the meta of stream k + 1
-  if (lane + 1 < f.nb) mk = __ldg(f.meta + f.words + static_cast<size_t>(lane) * f.words1 + w);
-  for (uint32_t k = 0; k + 1 < f.nb; k += 4) {
-    float t[4];
+  for (uint32_t k = 0; k + 1 < f.nb; k += 8) {
+    float t[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t[i] = flat_segment(f, flat_shfl(mk, k + i), lane);  // streams past nb: empty
-    y += (t[0] + t[1]) + (t[2] + t[3]);
+    for (int i = 0; i < 8; ++i) t[i] = flat_segment(f, flat_shfl(mk, k + i), lane);  // streams past nb: empty
+    y += ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
   }
   return y;
 }
 
 // Adds each row's segment sums, in stream order, and applies the update.  A
 // warp takes two words of 32 rows at a time, nwarps apart, and loads the metas
-// of its next two one round ahead: the sums' loads wait for the metas, and
-// what bounds the kernel is how many of them are in flight.
+// of its next two one round ahead, as the sums' loads wait for the metas.  RMAT
+// s24: 82 us (about 170 instructions a word, issue 42% busy, the rest latency);
+// 1 / 3 / 4 words at a time with 6 / 3 / 2 CTAs per SM 113 / 94 / 118.
 // With c.ctrl the last CTA to finish sums the partials in a fixed order and
 // takes the epoch decision (epoch_decide).
 struct flat_control {
@@ -429,7 +436,9 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
   for (; w < f.words; w += R * nwarps) {
     typename Update::operands ops[R];
     float y[R], z[R];
-    uint4 n0[R], n1[R];
+    uint4 n0[R], n1[R], mk[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) mk[r] = flat_middle_meta(f, w + r * nwarps, lane);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const uint32_t v = (w + r * nwarps) * 32 + lane;
@@ -449,7 +458,7 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const uint32_t wr = w + r * nwarps, v = wr * 32 + lane;
-      if (wr < f.words1) y[r] += flat_middle(f, wr, lane);
+      if (wr < f.words1) y[r] += flat_middle(f, mk[r], lane);
       y[r] += z[r];
       if (wr < f.words && v < f.V) dl += upd.apply(v, y[r], ops[r]);
       m0[r] = n0[r];
