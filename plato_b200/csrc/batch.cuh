@@ -219,6 +219,37 @@ __device__ __forceinline__ void merge_search(const uint32_t* s_rowend, int nrows
   edge = diag - lo;
 }
 
+// Adds to y what the groups before `end` hold of row `row` (their open row,
+// s_ckey, does not decrease with the group), last group first.  At kt 8 a CTA
+// has 128 groups and a hub row lies in all of them: their number is searched
+// first, so the loads overlap instead of each waiting for the key before it
+// (8 slots, RMAT s19: 13.1 -> 12.4 ms; at wider tiles the walk is the faster).
+template <int KT, int VEC>
+__device__ __forceinline__ void batch_add_groups(const uint32_t* s_ckey, const float* s_cval, int end, int row,
+                                                 int lane_g, float (&y)[VEC]) {
+  const float* v = s_cval + lane_g * VEC;
+  if constexpr (KT > 8) {
+    for (int g2 = end - 1; g2 >= 0 && s_ckey[g2] == static_cast<uint32_t>(row); --g2) {
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) y[c] += v[g2 * KT + c];
+    }
+  } else {
+    int lo = 0, hi = end;
+    while (lo < hi) {
+      const int m = (lo + hi) >> 1;
+      if (s_ckey[m] < static_cast<uint32_t>(row))
+        lo = m + 1;
+      else
+        hi = m;
+    }
+#pragma unroll 4
+    for (int g2 = end - 1; g2 >= lo; --g2) {
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) y[c] += v[g2 * KT + c];
+    }
+  }
+}
+
 template <int GL, int VEC>
 __global__ void __launch_bounds__(256, kBatchMinBlocks) k_batch_pull(batch_pass p0) {
   constexpr int KT = GL * VEC, NG = 256 / GL, TILE = batch_tile_items(KT), IPG = TILE / NG;
@@ -261,7 +292,15 @@ __global__ void __launch_bounds__(256, kBatchMinBlocks) k_batch_pull(batch_pass 
   if (!__syncthreads_or(mine)) return;  // every column of this tile is idle
   const uint32_t lflags = lane_flags_of<VEC>(st);
 
-  const uint32_t t = blockIdx.x;
+  // Tiles from both ends in turn: on a relabelled graph the first ones are long
+  // rows, bound by the gathers, and the last ones short rows, bound by the
+  // latency of an update after every few gathers.  In tile order the short rows
+  // run alone at the end; side by side they hide behind the gathers.  One B200,
+  // in order / from the end / from both: 64 queries at kt 64 on RMAT s21 48.1 /
+  // 41.7 / 41.5 ms, 256 at kt 128 on s19 59.0 / 48.9 / 48.9, 16 at kt 8 on s20
+  // 17.2 / 16.9 / 16.0, 8 slots on s19 14.4 / 12.5 / 12.5 (the last two with the
+  // search of batch_add_groups).
+  const uint32_t t = (blockIdx.x & 1) ? blockIdx.x >> 1 : gridDim.x - 1 - (blockIdx.x >> 1);
   const uint32_t i0 = p.trow[t], i1 = p.trow[t + 1];
   const uint64_t j0 = p.tedge[t], j1 = p.tedge[t + 1];
   const int nrows = static_cast<int>(i1 - i0), nnz = static_cast<int>(j1 - j0);
@@ -341,10 +380,7 @@ __global__ void __launch_bounds__(256, kBatchMinBlocks) k_batch_pull(batch_pass 
     float y[VEC];
 #pragma unroll
     for (int c = 0; c < VEC; ++c) y[c] = s_hacc[g * KT + lane_g * VEC + c];
-    for (int g2 = g - 1; g2 >= 0 && s_ckey[g2] == static_cast<uint32_t>(head); --g2) {
-#pragma unroll
-      for (int c = 0; c < VEC; ++c) y[c] += s_cval[g2 * KT + lane_g * VEC + c];
-    }
+    batch_add_groups<KT, VEC>(s_ckey, s_cval, g, head, lane_g, y);
     if (head == 0 && spans) {
 #pragma unroll
       for (int c = 0; c < VEC; ++c) p.thead[static_cast<size_t>(t) * KT + lane_g * VEC + c] = y[c];
@@ -356,10 +392,7 @@ __global__ void __launch_bounds__(256, kBatchMinBlocks) k_batch_pull(batch_pass 
     float y[VEC];
 #pragma unroll
     for (int c = 0; c < VEC; ++c) y[c] = 0.f;
-    for (int g2 = NG - 1; g2 >= 0 && s_ckey[g2] == static_cast<uint32_t>(nrows); --g2) {
-#pragma unroll
-      for (int c = 0; c < VEC; ++c) y[c] += s_cval[g2 * KT + lane_g * VEC + c];
-    }
+    batch_add_groups<KT, VEC>(s_ckey, s_cval, NG, nrows, lane_g, y);
 #pragma unroll
     for (int c = 0; c < VEC; ++c) p.tcarry[static_cast<size_t>(t) * KT + lane_g * VEC + c] = y[c];
   }
