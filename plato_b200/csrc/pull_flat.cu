@@ -406,7 +406,7 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   } else if (cold_steps) {
     // a wave of resident CTAs, and more (up to about five waves, so that the
     // last one is short) while a warp keeps 8 steps
-    const uint32_t wave = sms * 5u, fill = cold_steps / (8 * per_block);
+    const uint32_t wave = sms * kFlatColdCtas, fill = cold_steps / (8 * per_block);
     pl.cold_blocks = std::min<uint32_t>((cold_steps + per_block - 1) / per_block,
                                         std::min<uint32_t>(sms * 24u, std::max(wave, fill)));
   }
@@ -555,6 +555,7 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   f.words1 = words1;
   f.cold_piece0 = cold_piece0;
   f.cold_pieces = npieces - cold_piece0;
+  f.cold_back = pl.cold_blocks > sms * kFlatColdCtas;
   f.hid = hid;
   f.cid = cid;
   f.hw = hw;

@@ -27,8 +27,8 @@
 // flight a lane); L1 hits go at 560-790 G/s, shared memory at 1700 G/s.  RMAT
 // s24's 263M gathers are 0.95 ms of L2 requests; its hottest 57344 sources are
 // 46% of them, 24 blocks 90%.  RMAT s24, one PageRank epoch on one B200: 826 us
-// with degree bins (pull_binned.cuh), 503 us here: k_flat_hot 211 us (210M
-// edges), k_flat_cold 231 (53M), k_flat_update 82.  RMAT s22 220 -> 139 us, s20
+// with degree bins (pull_binned.cuh), 497 us here: k_flat_hot 211 us (210M
+// edges), k_flat_cold 226 (53M), k_flat_update 82.  RMAT s22 220 -> 132 us, s20
 // 98 -> 47, 16M uniform edges over 1M vertices 107 -> 81, 64M over 1M 303 -> 135.
 #pragma once
 
@@ -55,6 +55,7 @@ constexpr uint32_t kFlatMaxBlocks = 24;
 constexpr uint32_t kFlatCluster = 8, kFlatClusterSteps = 256;
 constexpr uint32_t kFlatHotWarps = 32;
 constexpr uint32_t kFlatColdThreads = 256;
+constexpr uint32_t kFlatColdCtas = 5;      // resident per SM
 constexpr uint32_t kPieceFirst = 0x80000000u;  // a piece at the start of its stream
 
 // A part of one hot block that a CTA walks, its steps shared by its 32 warps.
@@ -66,6 +67,7 @@ struct flat_view {
   uint32_t V, nsrc, nb, words;      // words = ceil(V / 32)
   uint32_t words1;                  // 32-row words that take part in the hot streams after the first
   uint32_t cold_piece0, cold_pieces;
+  uint32_t cold_back;               // k_flat_cold's CTAs take the pieces from the end
   const uint16_t* hid;              // hot ids, relative to their block
   const uint32_t* cid;              // cold ids
   const float* hw;                  // weights of the same edges, or null
@@ -343,14 +345,18 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_hot(flat_view f,
   }
 }
 
-// The cold stream, bound by L2 requests.
+// The cold stream, bound by L2 requests.  Its last pieces hold the short rows, a
+// segment every few edges, and take longest.  A grid of more than one wave
+// starts with them (epoch in order / from the end: RMAT s22 140 / 132 us, s23 257
+// / 250, s24 503 / 497); within a wave all run at once, and the update's CTAs
+// follow better in order (s18 16.7 / 18.0, s19 27.3 / 32.2, s21 72.4 / 73.0).
 template <bool kW>
-__global__ void __launch_bounds__(kFlatColdThreads, 5) k_flat_cold(flat_view f,
-                                                                                       const float* __restrict__ x,
-                                                                                       const int* mode) {
+__global__ void __launch_bounds__(kFlatColdThreads, kFlatColdCtas)
+    k_flat_cold(flat_view f, const float* __restrict__ x, const int* mode) {
   flat_after();
   if (mode && *mode == 2) return;
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t cta = f.cold_back ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const uint32_t w = (cta * blockDim.x + threadIdx.x) >> 5;
   if (w >= f.cold_pieces) return;
   const flat_cold_gather<kW, false> g{f.cid, f.cw, f.cmark, f.cseg, x};
   flat_piece(f, f.cold_piece0 + w, g);

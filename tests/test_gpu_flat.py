@@ -105,6 +105,18 @@ def test_seed_sets_and_single_queries(scale):
             assert np.abs(got.astype(np.float64) - want).sum() <= 1e-6 + 1e-6
 
 
+@pytest.mark.parametrize("E", [11 << 20, 16 << 20])
+def test_cold_stream_waves(E):
+    """One wave of cold pieces, taken in order, and more, taken from the end."""
+    V, s, d = _random(1000003, E, 11, 0.01)
+    want, _, _ = RefGraph(V, s, d, True).pagerank(5, 0.85, 0.0)
+    with pb.Graph(V, s, d, True) as g:
+        got, _ = g.pagerank(5, 0.85, 0.0)
+        again, _ = g.pagerank(5, 0.85, 0.0)
+    assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
+    np.testing.assert_array_equal(got, again)
+
+
 def test_no_room_for_the_plan():
     """With less memory left than the plan takes (RMAT s20: 50 MB and its
     scratch) the merge path answers; a later graph gets its plan again."""
