@@ -364,7 +364,8 @@ __device__ __forceinline__ void row_done(const gather_args& a, uint32_t v, int t
 // one lane; with rows handed to fixed teams and hubs in a kernel of their own it
 // was a 2048-source row.  Hyperanf, one B200, before / now: P = 4 / 6 / 8 / 12 on
 // RMAT s16 symmetrised 14.3 / 2.6 / 0.91 / 8.6 -> 1.1 / 0.73 / 0.77 / 6.3 ms, on
-// s20 15.1 / 4.4 / 7.1 / 102 -> 4.7 / 3.0 / 5.9 / 76, P = 6 on s22 10.0 -> 9.8.
+// s20 15.1 / 4.4 / 7.1 / 102 -> 4.7 / 3.0 / 5.9 / 76, P = 6 on s22 10.0 -> 9.8
+// (and with three-way maxima, max_odd, P = 6 on s20 2.65, on s22 9.5).
 template <int T, int VEC>
 __global__ void __launch_bounds__(kHllThreads, VEC <= 2 ? 4 : 3) k_hll_rows(gather_args a) {
   constexpr int SLICE = T * VEC * 16;
