@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctrl[0] = 2;
     ctrl[1] = static_cast<int>(ran);
-    if (eps > 0.0) *delta = ran > start + 1 ? s_delta : 0.0;
+    if (eps > 0.0 && ran > start + 1) *delta = s_delta;
   }
 }
 

@@ -417,7 +417,7 @@ int run_flat_epochs(plato_graph* g, const Upd& upd, uint32_t iteration, uint32_t
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
   if (ws->h_ctrl[3]) return set_error(PLATO_ETIMEDOUT, "k_flat_run: a grid barrier ran out");
   *ran = static_cast<uint32_t>(ws->h_ctrl[1]) - start;
-  *delta = *ws->h_delta;
+  if (*ran > 1) *delta = *ws->h_delta;
   return PLATO_OK;
 }
 
@@ -427,7 +427,8 @@ int run_flat_epochs(plato_graph* g, const Upd& upd, uint32_t iteration, uint32_t
 // epoch ends in its decision on the device (pagerank.hpp:137-139) and the host
 // enqueues a few epochs at a time, one batch ahead of the control word it
 // reads, so the device does not wait for the host; the epochs past the final
-// one return at once.  `scale` converts the delta to the reference's units.
+// one return at once.  `scale` converts the delta to the reference's units;
+// *delta keeps its value where no epoch but the final one runs, which has none.
 template <bool kW, class Make>
 int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteration, uint32_t start, double eps,
                     double scale, cudaStream_t st, int* cur, uint32_t* ran, double* delta) {
@@ -474,7 +475,7 @@ int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteratio
   seen = ws->h_ctrl + 4 * ((batches - 1) & 1u);
   *ran = static_cast<uint32_t>(seen[1]) - start;
   *cur = (cur0 + static_cast<int>(*ran)) & 1;
-  *delta = *ws->h_delta;
+  if (*ran > 1) *delta = *ws->h_delta;
   return PLATO_OK;
 }
 
