@@ -553,6 +553,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t cta_warps = blockDim.x >> 5;
   const uint32_t w0 = blockIdx.x * cta_warps + warp, nwarps = gridDim.x * cta_warps;
+  const bool deltas = !(eps <= 0.0);  // as run_pull_epochs: an eps that is no number never ends the epochs
   uint32_t barriers = 0, ran = start;
   bool last = start + 1 >= iteration;
   for (;;) {
@@ -570,7 +571,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
     ++ran;
     if (last) break;
     double* sums = partials + (ran & 1u) * gridDim.x;
-    if (eps > 0.0) {
+    if (deltas) {
       dl = warp_sum(dl);
       if (lane == 0) s_red[warp] = dl;
       __syncthreads();
@@ -579,7 +580,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
     }
     if (!flat_barrier(sync, ++barriers * gridDim.x, cluster)) return flat_poison(f, upd, w0, nwarps);
     last = ran + 1 >= iteration;
-    if (eps > 0.0) {  // every CTA sums the partials in the same order
+    if (deltas) {  // every CTA sums the partials in the same order
       if (warp == 0) {
         double t = 0.0;
         for (uint32_t i = lane; i < gridDim.x; i += 32) t += __ldcg(sums + i);
@@ -594,7 +595,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctrl[0] = 2;
     ctrl[1] = static_cast<int>(ran);
-    if (eps > 0.0 && ran > start + 1) *delta = s_delta;
+    if (deltas && ran > start + 1) *delta = s_delta;
   }
 }
 

@@ -26,3 +26,16 @@ def test_delta_of_the_push_epochs_outlives_a_final_pull(scale, ef):
     assert (st.iterations, st.push_iterations) == (epochs, pushes) == (2, 1)
     assert delta > 1.0 and st.delta == pytest.approx(delta, rel=1e-5)  # 32-bit terms, 2^-24 each
     assert one.delta == 0.0  # no epoch with a delta ran
+
+
+@pytest.mark.parametrize("scale", [10, 18])
+def test_delta_with_an_eps_that_is_no_number(scale):
+    """NaN ends no epoch early and asks for the deltas, as an eps that no delta
+    reaches does: the same ranks and the same delta, also after other calls."""
+    V, s, d = pb.rmat(scale, 20, 5)
+    with pb.Graph(V, s, d, True) as g:
+        want, ws = g.pagerank(6, 0.85, 1e-300)
+        g.pagerank(20, 0.85, 1e-300)  # leaves a smaller delta
+        got, st = g.pagerank(6, 0.85, float("nan"))
+    np.testing.assert_array_equal(got, want)
+    assert (st.iterations, st.delta) == (ws.iterations, ws.delta)
