@@ -39,8 +39,10 @@ extern "C" {
 #define PLATO_EINVAL      1  /* bad argument (null pointer, id out of range, ...) */
 #define PLATO_ENOMEM      2  /* device or host allocation failed / over budget     */
 #define PLATO_ECUDA       3  /* a CUDA runtime call failed                          */
-#define PLATO_ETIMEDOUT   4  /* a bounded device wait for another partition ran out
-                                (plato_partition_p2p_state)                          */
+#define PLATO_ETIMEDOUT   4  /* a bounded device wait ran out: for another partition
+                                (plato_partition_p2p_state), or of the blocks of a
+                                kernel for one another (plato_pagerank and the other
+                                rank calls: the ranks are then NaN)                   */
 #define PLATO_EBUSY       5  /* server full: no slot or HBM budget for the request  */
 #define PLATO_ENOTFOUND   6  /* nothing ready / unknown request id                  */
 
@@ -271,7 +273,9 @@ int plato_nstep_degrees(plato_graph* g, const plato_nstep_opts* opts, const plat
 /* ---- algorithms (device output buffers, caller's CUDA stream) ------------- */
 /* Same as plato_pagerank but writes the ranks to device memory d_ranks [V]
  * (caller ids) on `stream` (a cudaStream_t; NULL = legacy default stream).
- * With opts->eps == 0 nothing is read back and the call does not synchronise. */
+ * With opts->eps == 0 nothing is read back and the call does not synchronise;
+ * a device wait that runs out (PLATO_ETIMEDOUT elsewhere) then shows as NaN
+ * ranks. */
 int plato_pagerank_device(plato_graph* g, const plato_pagerank_opts* opts, float* d_ranks,
                           void* stream, plato_run_stats* stats);
 
@@ -407,6 +411,11 @@ int plato_diag_pull_ceiling(plato_graph* g, uint32_t mode, uint32_t reps, double
  * vertex order. */
 int plato_diag_batch_ceiling(plato_graph* g, uint32_t kt, uint32_t mode, uint32_t reps, double* ms_per_launch,
                              uint64_t* edges, double* checksum);
+/* No counterpart in the reference.  How often a block of this graph's
+ * one-launch epochs reads a barrier before it gives up (2^24 at first, many
+ * seconds).  With 0 the next such call gives up at its first barrier and
+ * returns PLATO_ETIMEDOUT: the way to see that failure without a fault. */
+int plato_diag_barrier_polls(plato_graph* g, uint32_t polls);
 
 /* ---- batched multi-source personalized pagerank --------------------------
  * K queries, query q's seed set is seeds[seed_offsets[q] .. seed_offsets[q+1]).

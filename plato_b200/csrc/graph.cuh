@@ -22,6 +22,8 @@ struct merge_tiles {
   dbuf<uint64_t> edge;  // [count + 1]
 };
 
+constexpr uint32_t kBarrierPolls = 1u << 24;  // of a device-wide barrier, before a kernel gives up
+
 struct rank_workspace;   // rank.cu
 struct bfs_workspace;    // bfs.cu
 class batch_engine;      // ppr_batch.cu
@@ -53,6 +55,7 @@ struct plato_graph {
   cudaStream_t stream = nullptr;  // stream of the host-buffer entry points
   std::mutex mu;                  // one algorithm call at a time per graph
   plato_b200::host_copy_user host_copies;
+  uint32_t barrier_polls = plato_b200::kBarrierPolls;  // plato_diag_barrier_polls
 
   std::map<uint32_t, plato_b200::merge_tiles> tiles;  // merge-path tiles by items per tile
   plato_b200::rank_workspace* rank_ws = nullptr;

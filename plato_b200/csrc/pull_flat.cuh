@@ -417,6 +417,7 @@ struct flat_control {
   double* delta;
   double scale, eps;
   uint32_t iteration;
+  uint32_t polls;  // of a grid barrier of k_flat_run, before it gives up
 };
 
 template <class Update>
@@ -495,10 +496,9 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
 // Barrier over the CTAs of k_flat_run.  One cluster: the hardware's barrier,
 // which orders global memory over the cluster.  A cooperative launch: sync[0]
 // counts arrivals over the whole launch (`target` of them release this
-// barrier), sync[1] is set when a CTA gives up waiting, and then every CTA
-// returns.
-constexpr uint32_t kFlatSpins = 1u << 24;
-__device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target, bool cluster) {
+// barrier), sync[1] is set when a CTA gives up waiting after `polls` reads
+// (kBarrierPolls: many seconds), and then every CTA returns.
+__device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target, bool cluster, uint32_t polls) {
   __shared__ int s_ok;
   if (cluster) {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -509,7 +509,7 @@ __device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target, bo
   if (threadIdx.x == 0) {
     int ok = 0;
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(sync) : "memory");
-    for (uint32_t n = 0; n < kFlatSpins; ++n) {
+    for (uint32_t n = 0; n < polls; ++n) {
       uint32_t seen, failed;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync) : "memory");
       if (seen >= target) {
@@ -542,12 +542,13 @@ __device__ __noinline__ void flat_poison(const flat_view& f, const Update& upd, 
 // ctrl[1] = epochs run, counted from `start`.  Launches bound these graphs: one
 // epoch with a launch per degree bin / here, RMAT s10 52 / 4.4 us, s12 54 / 6.3, s16
 // 70 / 9.4, 48K uniform edges 28 / 5.8.  A CTA that gives up waiting leaves NaN
-// in its rows.
+// in its rows; the host finds the give-up word with the results.
 template <class Update, bool kW>
 __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
                                                                    Update upd, uint32_t start, uint32_t iteration,
                                                                    double scale, double eps, int* ctrl, double* delta,
-                                                                   double* partials, uint32_t* sync, bool cluster) {
+                                                                   double* partials, uint32_t* sync, bool cluster,
+                                                                   uint32_t polls) {
   __shared__ double s_red[32];
   __shared__ double s_delta;
   const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -559,7 +560,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
   for (;;) {
     upd.final_epoch = last ? 1 : 0;
     flat_piece(f, w0, flat_cold_gather<kW, true>{f.cid, f.cw, f.cmark, f.cseg, upd.gathered()});
-    if (!flat_barrier(sync, ++barriers * gridDim.x, cluster)) return flat_poison(f, upd, w0, nwarps);
+    if (!flat_barrier(sync, ++barriers * gridDim.x, cluster, polls)) return flat_poison(f, upd, w0, nwarps);
     double dl = 0.0;
     for (uint32_t w = w0; w < f.words; w += nwarps) {
       const uint32_t v = w * 32 + lane;
@@ -578,7 +579,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
       dl = warp_sum(lane < cta_warps ? s_red[lane] : 0.0);
       if (threadIdx.x == 0) __stcg(sums + blockIdx.x, dl);
     }
-    if (!flat_barrier(sync, ++barriers * gridDim.x, cluster)) return flat_poison(f, upd, w0, nwarps);
+    if (!flat_barrier(sync, ++barriers * gridDim.x, cluster, polls)) return flat_poison(f, upd, w0, nwarps);
     last = ran + 1 >= iteration;
     if (deltas) {  // every CTA sums the partials in the same order
       if (warp == 0) {
@@ -661,7 +662,7 @@ int launch_flat_run(const flat_plan& p, const Upd& upd, uint32_t start, double* 
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   PLATO_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_flat_run<Upd, kW>, p.v, upd, start, c.iteration, c.scale, c.eps, c.ctrl,
-                                    c.delta, partials, sync, p.run_cluster));
+                                    c.delta, partials, sync, p.run_cluster, c.polls));
   PLATO_LAUNCHED("k_flat_run");
   return PLATO_OK;
 }

@@ -55,6 +55,7 @@ struct rank_workspace {
   double* h_delta = nullptr;  // pinned
   int* h_ctrl = nullptr;      // pinned [8]: two control words
   cudaEvent_t polled[2] = {nullptr, nullptr};  // control words copied to h_ctrl
+  bool unread_barrier = false;  // this call's k_flat_run may have given up, and the host has not looked
   push_frontier frontier;
   ~rank_workspace() {
     if (h_delta) cudaFreeHost(h_delta);
@@ -402,20 +403,26 @@ int check_rank_opts(uint32_t iteration, double damping) {
   return PLATO_OK;
 }
 
+int barrier_ran_out() { return set_error(PLATO_ETIMEDOUT, "k_flat_run: a grid barrier ran out"); }
+
 // Every pull epoch of a small graph in one launch (k_flat_run); `upd` starts
-// at the current state.  With eps > 0 the host waits for the epoch count.
+// at the current state.  With eps > 0 the host waits for the epoch count and
+// the barriers' give-up word; without, with_host_output reads the word.
 template <class Upd, bool kW>
 int run_flat_epochs(plato_graph* g, const Upd& upd, uint32_t iteration, uint32_t start, double eps, double scale,
                     cudaStream_t st, uint32_t* ran, double* delta) {
   rank_workspace* ws = g->rank_ws;
-  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration};
+  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration, g->barrier_polls};
   PLATO_TRY((launch_flat_run<Upd, kW>(ws->flat, upd, start, ws->partials.p, c, st)));
   *ran = iteration - start;
-  if (eps <= 0.0) return PLATO_OK;
+  if (eps <= 0.0) {
+    ws->unread_barrier = ws->flat.run_ctas > 1 && !ws->flat.run_cluster;
+    return PLATO_OK;
+  }
   PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl, ws->ctrl.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_delta, ws->delta.p, sizeof(double), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  if (ws->h_ctrl[3]) return set_error(PLATO_ETIMEDOUT, "k_flat_run: a grid barrier ran out");
+  if (ws->h_ctrl[3]) return barrier_ran_out();
   *ran = static_cast<uint32_t>(ws->h_ctrl[1]) - start;
   if (*ran > 1) *delta = *ws->h_delta;
   return PLATO_OK;
@@ -451,7 +458,7 @@ int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteratio
   }
   const int init[4] = {start == iteration - 1 ? 1 : 0, static_cast<int>(start), 0, 0};
   PLATO_CUDA_TRY(cudaMemcpyAsync(ws->ctrl.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration};
+  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration, g->barrier_polls};
   const int cur0 = *cur;
   constexpr uint32_t kBatch = 6;
   uint32_t launched = 0, batches = 0;
@@ -721,10 +728,15 @@ template <class F>
 int with_host_output(plato_graph* g, float* host, F&& run) {
   cudaStream_t st = g->stream;
   PLATO_TRY(ensure_ws(g, st));
-  dbuf<float>& out = g->rank_ws->out_stage;  // kept on the graph: no allocation per call
+  rank_workspace* ws = g->rank_ws;
+  dbuf<float>& out = ws->out_stage;  // kept on the graph: no allocation per call
   PLATO_TRY(out.alloc(g->info.vertices));
+  ws->unread_barrier = false;
   PLATO_TRY(run(out.p, st));
-  return copy_to_host(host, out.p, g->info.vertices * sizeof(float), st);
+  if (ws->unread_barrier)
+    PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl, ws->ctrl.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  PLATO_TRY(copy_to_host(host, out.p, g->info.vertices * sizeof(float), st));
+  return ws->unread_barrier && ws->h_ctrl[3] ? barrier_ran_out() : PLATO_OK;
 }
 
 // One pull epoch of a partition by the degree bins of ws->plan.
@@ -882,4 +894,11 @@ extern "C" int plato_weighted_pagerank(plato_graph* g, const plato_pagerank_opts
   return with_host_output(g, ranks, [&](float* d_out, cudaStream_t st) {
     return wpagerank_impl(g, opts, d_out, st, stats);
   });
+}
+
+extern "C" int plato_diag_barrier_polls(plato_graph* g, uint32_t polls) {
+  if (!g) return set_error(PLATO_EINVAL, "plato_diag_barrier_polls: null graph");
+  std::lock_guard<std::mutex> lock(g->mu);
+  g->barrier_polls = polls;
+  return PLATO_OK;
 }

@@ -6,6 +6,7 @@ import pytest
 
 import plato_b200 as pb
 from oracle import RefGraph
+from plato_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +40,34 @@ def test_delta_with_an_eps_that_is_no_number(scale):
         got, st = g.pagerank(6, 0.85, float("nan"))
     np.testing.assert_array_equal(got, want)
     assert (st.iterations, st.delta) == (ws.iterations, ws.delta)
+
+
+def test_a_barrier_that_runs_out_is_an_error():
+    """With no polls allowed the blocks of the one-launch epochs give up at
+    their first barrier: every rank call that hands out host ranks says so,
+    with and without an early exit, and the graph answers again afterwards."""
+    V, s, d = pb.rmat(15, 16, 6)
+    w = np.random.default_rng(2).uniform(0.1, 10, s.size)
+    lib = _lib.load()
+    src = int(s[0])
+
+    def calls(g, eps):
+        return [lambda: g.pagerank(10, 0.85, eps)[0],
+                lambda: g.weighted_pagerank(10, 0.85, eps)[0],
+                lambda: g.personalized_pagerank(src, 10, 0.85, eps, pb.PLATO_PPR_PULL)[0],
+                lambda: g.personalized_pagerank(src, 10, 0.85, eps, pb.PLATO_PPR_PUSHPULL)[0],
+                lambda: g.seedset_ppr([src, 1], 10, 0.85, eps)[0]]
+
+    with pb.Graph(V, s, d, True, weights=w) as g:
+        for eps in (0.0, 1e-9):
+            want = [call() for call in calls(g, eps)]
+            _lib.check(lib.plato_diag_barrier_polls(g.handle, 0), "polls")
+            for call in calls(g, eps):
+                with pytest.raises(_lib.PlatoError) as e:
+                    call()
+                assert e.value.code == _lib.PLATO_ETIMEDOUT
+            _lib.check(lib.plato_diag_barrier_polls(g.handle, 1 << 24), "polls")
+            for call, ranks in zip(calls(g, eps), want):
+                # the push epochs add in any order
+                np.testing.assert_allclose(call(), ranks, rtol=0, atol=1e-6 * ranks.max())
+    assert lib.plato_diag_barrier_polls(None, 0) == _lib.PLATO_EINVAL
