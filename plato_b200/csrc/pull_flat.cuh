@@ -493,6 +493,14 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
   }
 }
 
+// All arrivals of a barrier are in.  The count goes round after 2^32 arrivals
+// (14.5M epochs on 148 CTAs); no two CTAs are more than a barrier apart.
+constexpr __host__ __device__ bool flat_arrived(uint32_t seen, uint32_t target) {
+  return static_cast<int32_t>(seen - target) >= 0;
+}
+static_assert(flat_arrived(148, 148) && !flat_arrived(147, 148) && flat_arrived(4, 0xFFFFFFF0u) &&
+              !flat_arrived(0xFFFFFFF0u, 4), "also where the count has gone round");
+
 // Barrier over the CTAs of k_flat_run.  One cluster: the hardware's barrier,
 // which orders global memory over the cluster.  A cooperative launch: sync[0]
 // counts arrivals over the whole launch (`target` of them release this
@@ -512,7 +520,7 @@ __device__ __forceinline__ bool flat_barrier(uint32_t* sync, uint32_t target, bo
     for (uint32_t n = 0; n < polls; ++n) {
       uint32_t seen, failed;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(sync) : "memory");
-      if (seen >= target) {
+      if (flat_arrived(seen, target)) {
         ok = 1;
         break;
       }
