@@ -23,7 +23,7 @@
 
 namespace plato_b200 {
 
-// Degree-bin plan of a partition (see pull_binned.cuh).
+// Degree-bin plan (see pull_binned.cuh).
 struct pull_plan {
   bool valid = false;
   uint32_t n_long = 0, n_items = 0, n_hubs = 0;
@@ -186,9 +186,9 @@ int set_pull_smem_attr(int device, uint32_t* hub_cap) {
   return PLATO_OK;
 }
 
-// Builds a partition's degree-bin plan when its columns are sorted by
-// descending in-degree; otherwise plan.valid stays false and the merge-path
-// kernel handles the pull.
+// Builds the degree-bin plan when the columns are sorted by descending
+// in-degree (relabelled graphs, partitions); otherwise plan.valid stays false
+// and the merge-path kernel handles the pull.
 int build_plan(plato_graph* g, pull_plan& pl, cudaStream_t st) {
   const uint32_t V = g->info.vertices;
   if (!g->relabeled) return PLATO_OK;
@@ -263,6 +263,19 @@ int build_plan(plato_graph* g, pull_plan& pl, cudaStream_t st) {
   return PLATO_OK;
 }
 
+// Builds a plan that its graph can do without: no memory for it is no error.
+template <class Plan, class Build>
+int plan_or_none(Plan& plan, Build&& build) {
+  int rc = PLATO_OK;
+  try {
+    rc = build();
+  } catch (const std::bad_alloc&) {
+    rc = PLATO_ENOMEM;
+  }
+  if (rc != PLATO_OK) plan = Plan{};
+  return rc == PLATO_ENOMEM ? PLATO_OK : rc;
+}
+
 int ensure_ws(plato_graph* g, cudaStream_t st) {
   if (!g->rank_ws) {
     g->rank_ws = new (std::nothrow) rank_workspace();
@@ -272,12 +285,13 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
   const uint32_t V = g->info.vertices;
   if (!ws->plan_built) {
     // The flat plan takes 2-4 bytes an edge beside the graph, and as much again
-    // while it is built.  A graph that leaves no room for it pulls by the merge
-    // path, which needs no plan (RMAT s24: 2.6 ms an epoch instead of 0.53).
-    const int rc = build_flat_plan(g, ws->flat, st);
-    if (rc != PLATO_OK) ws->flat = flat_plan{};
-    if (rc != PLATO_OK && rc != PLATO_ENOMEM) return rc;
-    if (!g->own_sources) PLATO_TRY(build_plan(g, ws->plan, st));
+    // while it is built.  A graph that leaves no room for it pulls by the degree
+    // bins, which need a few bytes per long row (RMAT s24: 0.83 ms an epoch
+    // instead of 0.50), and without room for those by the merge path (2.6 ms).
+    // It keeps its path when memory comes free: the paths sum in different
+    // orders, and a graph's ranks are the same from call to call.
+    PLATO_TRY(plan_or_none(ws->flat, [&] { return build_flat_plan(g, ws->flat, st); }));
+    if (!ws->flat.valid) PLATO_TRY(plan_or_none(ws->plan, [&] { return build_plan(g, ws->plan, st); }));
     ws->plan_built = true;
   }
   if (!ws->flat.valid && !ws->plan.valid) PLATO_TRY(ensure_pull_tiles(g, cfg::kItems, st));
@@ -345,12 +359,64 @@ int partial_count(const plato_graph* g) {
   return static_cast<int>(g->rank_ws->sms + (W + 255) / 256);
 }
 
-// The kernels of one pull epoch (pull_epoch_with).
+// One pull epoch by the degree bins of ws->plan.
 template <class Upd, bool kW>
-int pull_sums_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st,
-                   const flat_control& c) {
+int launch_bins(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st) {
   rank_workspace* ws = g->rank_ws;
-  if (ws->flat.valid) return launch_flat_epoch<Upd, kW>(ws->flat, x, upd, ws->partials.p, c, st);
+  const pull_plan& pl = ws->plan;
+  const pull_plan_view pv{pl.n_long, pl.rows_begin[3], g->info.vertices, pl.n_items, pl.items.p,
+                          pl.n_hubs, pl.hub_rows.p, pl.hub_item0.p, pl.hub_pieces.p,
+                          pl.piece_sum.p};
+  double* part = ws->partials.p;
+  if (pl.blocks_long) {
+    prof_scope ps("k_pull_long", st);
+    k_pull_long<Upd, kW><<<pl.blocks_long, 256, 0, st>>>(pv, g->in_off.p, g->in_adj.p, x, upd, part, w);
+    PLATO_LAUNCHED("k_pull_long");
+  }
+  part += pl.blocks_long;
+  if (pl.blocks_hubs) {
+    prof_scope ps("k_pull_hubs", st);
+    k_pull_hubs<Upd><<<pl.blocks_hubs, 256, 0, st>>>(pv, upd, part);
+    PLATO_LAUNCHED("k_pull_hubs");
+  }
+  part += pl.blocks_hubs;
+  if (pl.blocks_rows[0]) {
+    prof_scope ps("k_pull_rows16", st);
+    k_pull_rows<16, Upd, kW><<<pl.blocks_rows[0], 256, 0, st>>>(
+        pl.rows_begin[0], pl.rows_begin[1], g->in_off.p, g->in_adj.p, x, upd, part, w);
+    PLATO_LAUNCHED("k_pull_rows16");
+  }
+  part += pl.blocks_rows[0];
+  if (pl.blocks_rows[1]) {
+    prof_scope ps("k_pull_rows8", st);
+    k_pull_rows<8, Upd, kW><<<pl.blocks_rows[1], 256, 0, st>>>(
+        pl.rows_begin[1], pl.rows_begin[2], g->in_off.p, g->in_adj.p, x, upd, part, w);
+    PLATO_LAUNCHED("k_pull_rows8");
+  }
+  part += pl.blocks_rows[1];
+  if (pl.blocks_rows[2]) {
+    prof_scope ps("k_pull_rows4", st);
+    k_pull_rows<4, Upd, kW><<<pl.blocks_rows[2], 256, 0, st>>>(
+        pl.rows_begin[2], pl.rows_begin[3], g->in_off.p, g->in_adj.p, x, upd, part, w);
+    PLATO_LAUNCHED("k_pull_rows4");
+  }
+  part += pl.blocks_rows[2];
+  if (pl.blocks_short) {
+    prof_scope ps("k_pull_short", st);
+    k_pull_short<Upd, kW><<<pl.blocks_short, 256, 0, st>>>(pv, g->in_off.p, g->in_adj.p, x, upd, part, w);
+    PLATO_LAUNCHED("k_pull_short");
+  }
+  return PLATO_OK;
+}
+
+// One pull epoch without a flat plan gathering x (times the edge weights w
+// when kW) with the fused update `upd`: the degree bins, or the persistent
+// warp-tile merge path + cross-range fixup.  Partial deltas go to ws->partials
+// (one per CTA of each kernel).
+template <class Upd, bool kW>
+int pull_rows_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st) {
+  rank_workspace* ws = g->rank_ws;
+  if (ws->plan.valid) return launch_bins<Upd, kW>(g, x, upd, w, st);
   const merge_tiles& mt = g->tiles.at(cfg::kItems);
   const uint32_t H = std::min<uint32_t>(g->info.vertices, ws->hub_cap);
   pull_warp_args a{mt.row.p, mt.edge.p, mt.count, g->stored_edges, g->in_off.p, g->in_adj.p,
@@ -370,22 +436,23 @@ int pull_sums_with(plato_graph* g, const float* x, const Upd& upd, const float* 
   return PLATO_OK;
 }
 
-// One pull epoch gathering x (times the edge weights w when kW) with the
-// fused update `upd`: the flat plan on a relabelled graph, else the
-// persistent warp-tile merge path + cross-range fixup.  Partial deltas go to
-// ws->partials (one per CTA of each kernel).  With c.ctrl the epoch also ends
-// in its decision (epoch_decide), which upd.mode reads.
+// One pull epoch of a whole graph: its flat plan, else pull_rows_with.  With
+// c.ctrl the epoch also ends in its decision (epoch_decide), which upd.mode
+// reads.
 template <class Upd, bool kW>
 int pull_epoch_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st,
                     const flat_control& c = flat_control{}) {
-  PLATO_TRY((pull_sums_with<Upd, kW>(g, x, upd, w, st, c)));
-  if (c.ctrl && !g->rank_ws->flat.valid) {
-    k_epoch_control<<<1, 1024, 0, st>>>(g->rank_ws->partials.p, static_cast<uint32_t>(partial_count(g)), c.ctrl,
-                                        c.delta, c.scale, c.eps, c.iteration);
+  rank_workspace* ws = g->rank_ws;
+  if (ws->flat.valid) return launch_flat_epoch<Upd, kW>(ws->flat, x, upd, ws->partials.p, c, st);
+  PLATO_TRY((pull_rows_with<Upd, kW>(g, x, upd, w, st)));
+  if (c.ctrl) {
+    k_epoch_control<<<1, 1024, 0, st>>>(ws->partials.p, static_cast<uint32_t>(partial_count(g)), c.ctrl, c.delta,
+                                        c.scale, c.eps, c.iteration);
     PLATO_LAUNCHED("k_epoch_control");
   }
   return PLATO_OK;
 }
+
 // Reads back the epoch's delta (sum of the partials).  Synchronises `st`.
 int read_delta(plato_graph* g, uint32_t nparts, cudaStream_t st, double* out) {
   rank_workspace* ws = g->rank_ws;
@@ -739,64 +806,6 @@ int with_host_output(plato_graph* g, float* host, F&& run) {
   return ws->unread_barrier && ws->h_ctrl[3] ? barrier_ran_out() : PLATO_OK;
 }
 
-// One pull epoch of a partition by the degree bins of ws->plan.
-template <class Upd>
-int launch_bins(plato_graph* g, const float* x, const Upd& upd, cudaStream_t st) {
-  rank_workspace* ws = g->rank_ws;
-  const pull_plan& pl = ws->plan;
-  const pull_plan_view pv{pl.n_long, pl.rows_begin[3], g->info.vertices, pl.n_items, pl.items.p,
-                          pl.n_hubs, pl.hub_rows.p, pl.hub_item0.p, pl.hub_pieces.p,
-                          pl.piece_sum.p};
-  double* part = ws->partials.p;
-  if (pl.blocks_long) {
-    prof_scope ps("k_pull_long", st);
-    k_pull_long<Upd><<<pl.blocks_long, 256, 0, st>>>(pv, g->in_off.p, g->in_adj.p, x, upd, part);
-    PLATO_LAUNCHED("k_pull_long");
-  }
-  part += pl.blocks_long;
-  if (pl.blocks_hubs) {
-    prof_scope ps("k_pull_hubs", st);
-    k_pull_hubs<Upd><<<pl.blocks_hubs, 256, 0, st>>>(pv, upd, part);
-    PLATO_LAUNCHED("k_pull_hubs");
-  }
-  part += pl.blocks_hubs;
-  if (pl.blocks_rows[0]) {
-    prof_scope ps("k_pull_rows16", st);
-    k_pull_rows<16, Upd><<<pl.blocks_rows[0], 256, 0, st>>>(
-        pl.rows_begin[0], pl.rows_begin[1], g->in_off.p, g->in_adj.p, x, upd, part);
-    PLATO_LAUNCHED("k_pull_rows16");
-  }
-  part += pl.blocks_rows[0];
-  if (pl.blocks_rows[1]) {
-    prof_scope ps("k_pull_rows8", st);
-    k_pull_rows<8, Upd><<<pl.blocks_rows[1], 256, 0, st>>>(
-        pl.rows_begin[1], pl.rows_begin[2], g->in_off.p, g->in_adj.p, x, upd, part);
-    PLATO_LAUNCHED("k_pull_rows8");
-  }
-  part += pl.blocks_rows[1];
-  if (pl.blocks_rows[2]) {
-    prof_scope ps("k_pull_rows4", st);
-    k_pull_rows<4, Upd><<<pl.blocks_rows[2], 256, 0, st>>>(
-        pl.rows_begin[2], pl.rows_begin[3], g->in_off.p, g->in_adj.p, x, upd, part);
-    PLATO_LAUNCHED("k_pull_rows4");
-  }
-  part += pl.blocks_rows[2];
-  if (pl.blocks_short) {
-    prof_scope ps("k_pull_short", st);
-    k_pull_short<Upd><<<pl.blocks_short, 256, 0, st>>>(pv, g->in_off.p, g->in_adj.p, x, upd, part);
-    PLATO_LAUNCHED("k_pull_short");
-  }
-  return PLATO_OK;
-}
-
-// A partition's epoch: the degree bins, or the merge path where its rows are
-// not sorted by in-degree.
-template <class Upd>
-int partition_epoch(plato_graph* g, const float* x, const Upd& upd, cudaStream_t st) {
-  if (g->rank_ws->plan.valid) return launch_bins(g, x, upd, st);
-  return pull_epoch_with<Upd, false>(g, x, upd, nullptr, st);
-}
-
 }  // namespace
 
 // 1D partitions (partition.cu): the workspace of a partition's rows, and one
@@ -810,7 +819,7 @@ int pull_epoch_partition(plato_graph* g, const float* x_gather, const float* x_o
   PLATO_TRY(ensure_ws(g, st));
   const rank_update<teleport_uniform> upd{x_old, xn, g->out_deg.p, teleport_uniform{tele}, d,
                                           final_epoch ? 1 : 0};
-  PLATO_TRY(partition_epoch(g, x_gather, upd, st));
+  PLATO_TRY((pull_rows_with<rank_update<teleport_uniform>, false>(g, x_gather, upd, nullptr, st)));
   if (d_partial_sum) {
     k_sum_partials<<<1, 1024, 0, st>>>(g->rank_ws->partials.p, static_cast<uint32_t>(partial_count(g)),
                                        d_partial_sum);
@@ -834,7 +843,7 @@ int pull_epoch_partition_bcast(plato_graph* g, const float* x_gather, const floa
                                         mode};
   for (uint32_t k = 0; k < npeers; ++k) upd.peers[k] = peers[k];
   upd.npeers = npeers;
-  PLATO_TRY(partition_epoch(g, x_gather, upd, st));
+  PLATO_TRY((pull_rows_with<bcast_rank_update, false>(g, x_gather, upd, nullptr, st)));
   if (d_partial_sum) {
     k_sum_partials<<<1, 1024, 0, st>>>(g->rank_ws->partials.p, static_cast<uint32_t>(partial_count(g)),
                                        d_partial_sum);

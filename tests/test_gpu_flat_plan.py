@@ -1,6 +1,8 @@
 """The flat pull's reports and plans at the edges of what takes it: the delta
 of a call whose only pull epoch is the final one, and graphs whose rows,
 sources or memory do not suit a flat plan."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -71,3 +73,75 @@ def test_a_barrier_that_runs_out_is_an_error():
                 # the push epochs add in any order
                 np.testing.assert_allclose(call(), ranks, rtol=0, atol=1e-6 * ranks.max())
     assert lib.plato_diag_barrier_polls(None, 0) == _lib.PLATO_EINVAL
+
+
+def _launched(call, names):
+    """The kernels among `names` that `call` launches, and its result."""
+    lib = _lib.load()
+    _lib.check(lib.plato_profile_enable(1), "profile")
+    _lib.check(lib.plato_profile_reset(), "profile")
+    try:
+        out = call()
+    finally:
+        lib.plato_profile_enable(0)
+    hit = set()
+    for n in names:
+        ms, k = C.c_double(), C.c_uint64()
+        _lib.check(lib.plato_profile_read(n.encode(), C.byref(ms), C.byref(k)), n)
+        if k.value:
+            hit.add(n)
+    return hit, out
+
+
+KERNELS = ["k_flat_hot", "k_flat_cold", "k_flat_update", "k_flat_run", "k_pull_long", "k_pull_rows16", "k_pull_rows8",
+           "k_pull_rows4", "k_pull_short", "k_pull_hubs", "k_pull_warp"]
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_bins_answer_without_room_for_the_plan(weighted):
+    """With 32 MB left the flat plan of RMAT s20 does not fit and the degree
+    bins answer, weights and early exit too; the graph stays with them when the
+    memory comes free, and the next graph gets its plan."""
+    import torch
+
+    V, s, d = pb.rmat(20, 16, 9)
+    w = np.random.default_rng(3).uniform(0.1, 10, s.size) if weighted else None
+
+    def call(g, eps=0.0):
+        return g.weighted_pagerank(12, 0.85, eps) if weighted else g.pagerank(12, 0.85, eps)
+
+    eps = 2e-2 * V
+    with pb.Graph(V, s, d, True, weights=w) as g:
+        plan, (want, _) = _launched(lambda: call(g), KERNELS)
+        want_early, early = call(g, eps)
+        assert "k_flat_cold" in plan and not any(n.startswith("k_pull") for n in plan)
+        assert early.iterations < 12
+    with pb.Graph(V, s, d, True, weights=w) as g:
+        free, _ = torch.cuda.mem_get_info()
+        hog = torch.empty(max(free - (32 << 20), 0), dtype=torch.uint8, device="cuda")
+        try:
+            bins, (got, _) = _launched(lambda: call(g), KERNELS)
+            got_early, st = call(g, eps)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        later, (again, _) = _launched(lambda: call(g), KERNELS)
+        with pb.Graph(V, s, d, True, weights=w) as g2:
+            fresh, (new, _) = _launched(lambda: call(g2), KERNELS)
+    assert {"k_pull_long", "k_pull_short"} <= bins and bins == later
+    assert not any(n.startswith("k_flat") or n == "k_pull_warp" for n in bins)
+    assert fresh == plan
+    unit = V if weighted else 1  # sums of 32-bit ranks in two orders, each within 1e-6 of the oracle's
+    assert np.abs(got.astype(np.float64) - want).sum() / unit <= 2e-6
+    assert np.abs(got_early.astype(np.float64) - want_early).sum() / unit <= 2e-6
+    assert st.iterations == early.iterations and st.delta == pytest.approx(early.delta, rel=1e-3)
+    np.testing.assert_array_equal(again, got)
+    np.testing.assert_array_equal(new, want)
+
+
+def test_a_graph_without_edges_takes_the_bins():
+    V = 70001
+    with pb.Graph(V, np.zeros(0, np.uint32), np.zeros(0, np.uint32), True) as g:
+        hit, (got, st) = _launched(lambda: g.pagerank(4, 0.85, 0.0), KERNELS)
+    assert hit == {"k_pull_short"} and st.iterations == 4
+    np.testing.assert_allclose(got, 0.15 / V, rtol=1e-6)
