@@ -168,7 +168,9 @@ int plato_graph_get_device_view(const plato_graph* g, plato_graph_device_view* v
 /* Out-degrees computed from the in-edge structure, in caller ids
  * (generate_dense_out_degrees_fg, plato/graph/structure.hpp:291-346). */
 int plato_graph_out_degrees(plato_graph* g, uint32_t* degrees_out /* host [V] */);
-/* Bytes of HBM held by the graph. */
+/* Bytes of HBM held by the graph: its arrays, the plan of its pull epochs (from
+ * its first rank call) and the index that plato_connected_components keeps.
+ * The vertex-sized workspaces of the calls come on top. */
 int plato_graph_device_bytes(const plato_graph* g, uint64_t* bytes);
 
 /* ---- algorithms (host output buffers) ------------------------------------ */

@@ -524,6 +524,13 @@ class dualmode_engine_t {
 
   const plato_graph_info& graph_info() const { return info_; }
   uint32_t vertices() const { return view_.vertices; }
+  // Device memory that the engine keeps between calls: chunk and piece indexes, queue.
+  uint64_t index_bytes() const {
+    uint64_t n = (chunks_ ? sizeof(uint2) * nchunks_ : 0) + (queue_ ? 4ull * view_.vertices : 0);
+    for (const piece_index& pi : pieces_)
+      if (pi.built) n += 4ull * pi.ncols + 8ull * (pi.ncols + 1ull) + 4ull * ((pi.npieces + 31) / 32);
+    return n;
+  }
 
   template <typename T>
   dense_state_t<T> alloc_v_state() const { return dense_state_t<T>(view_.vertices); }

@@ -170,6 +170,7 @@ int cc_impl(plato_graph* g, const plato_dualmode_opts* eo, plato_vid_t* labels_o
     }
     std::swap(active_current, active_next);
   }
+  g->cc_index_bytes = engine.index_bytes();
   if (stats) {
     *stats = plato_run_stats{};
     stats->iterations = epochs;
@@ -231,6 +232,7 @@ extern "C" int plato_connected_components(plato_graph* g, const plato_dualmode_o
   } catch (const std::exception& e) {
     destroy_cc_workspace(g->cc_ws);  // its index may be half built
     g->cc_ws = nullptr;
+    g->cc_index_bytes = 0;
     return set_error(PLATO_ECUDA, std::string("plato_connected_components: ") + e.what());
   }
 }

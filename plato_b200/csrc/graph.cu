@@ -537,7 +537,7 @@ extern "C" int plato_graph_out_degrees(plato_graph* g, uint32_t* degrees_out) {
 
 extern "C" int plato_graph_device_bytes(const plato_graph* g, uint64_t* bytes) {
   if (!g || !bytes) return set_error(PLATO_EINVAL, "plato_graph_device_bytes: null argument");
-  *bytes = g->in_off.bytes() + g->out_off.bytes() + g->in_adj.bytes() + g->out_adj.bytes() +
+  *bytes = g->plan_bytes + g->cc_index_bytes + g->in_off.bytes() + g->out_off.bytes() + g->in_adj.bytes() + g->out_adj.bytes() +
            g->out_deg.bytes() + g->in_deg.bytes() + g->to_int.bytes() + g->to_ext.bytes() +
            g->in_w.bytes() + g->out_wsum.bytes();
   return PLATO_OK;

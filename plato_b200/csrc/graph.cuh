@@ -2,6 +2,7 @@
 // vertex order, plus lazily built per-algorithm metadata and workspaces.
 #pragma once
 
+#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -55,6 +56,8 @@ struct plato_graph {
   cudaStream_t stream = nullptr;  // stream of the host-buffer entry points
   std::mutex mu;                  // one algorithm call at a time per graph
   plato_b200::host_copy_user host_copies;
+  // what the calls keep of the graph's size, for plato_graph_device_bytes (which takes no lock)
+  std::atomic<uint64_t> plan_bytes{0}, cc_index_bytes{0};
   uint32_t barrier_polls = plato_b200::kBarrierPolls;  // plato_diag_barrier_polls
 
   std::map<uint32_t, plato_b200::merge_tiles> tiles;  // merge-path tiles by items per tile

@@ -32,6 +32,9 @@ struct pull_plan {
   dbuf<uint2> items;
   dbuf<uint32_t> hub_rows, hub_item0, hub_pieces;
   dbuf<float> piece_sum;
+  uint64_t bytes() const {
+    return items.bytes() + hub_rows.bytes() + hub_item0.bytes() + hub_pieces.bytes() + piece_sum.bytes();
+  }
   uint32_t partials() const {
     return blocks_long + blocks_hubs + blocks_rows[0] + blocks_rows[1] + blocks_rows[2] + blocks_short;
   }
@@ -292,6 +295,7 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
     // orders, and a graph's ranks are the same from call to call.
     PLATO_TRY(plan_or_none(ws->flat, [&] { return build_flat_plan(g, ws->flat, st); }));
     if (!ws->flat.valid) PLATO_TRY(plan_or_none(ws->plan, [&] { return build_plan(g, ws->plan, st); }));
+    g->plan_bytes = ws->flat.mem.bytes() + ws->plan.bytes();
     ws->plan_built = true;
   }
   if (!ws->flat.valid && !ws->plan.valid) PLATO_TRY(ensure_pull_tiles(g, cfg::kItems, st));

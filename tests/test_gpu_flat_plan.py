@@ -145,3 +145,20 @@ def test_a_graph_without_edges_takes_the_bins():
         hit, (got, st) = _launched(lambda: g.pagerank(4, 0.85, 0.0), KERNELS)
     assert hit == {"k_pull_short"} and st.iterations == 4
     np.testing.assert_allclose(got, 0.15 / V, rtol=1e-6)
+
+
+def test_device_bytes_count_the_plan_and_the_index():
+    """The flat plan holds every edge once more, 2 bytes (hot) or 4 (cold), and
+    the components' index the non-empty columns' starts."""
+    V, s, d = pb.rmat(18, 16, 4)
+    with pb.Graph(V, s, d, True) as g:
+        E = g.device_view().stored_edges
+        plain = g.device_bytes()
+        g.pagerank(2, 0.85, 0.0)
+        ranked = g.device_bytes()
+        assert 2 * E <= ranked - plain <= 6 * E
+        g.pagerank(2, 0.85, 0.0)
+        assert g.device_bytes() == ranked  # kept, not built again
+        g.connected_components()
+        columns = np.unique(d).size
+        assert g.device_bytes() - ranked >= 12 * columns
