@@ -149,6 +149,12 @@ __global__ void __launch_bounds__(256) k_flat_fill(flat_rows f, const uint32_t* 
   }
 }
 
+// The stream of place i in arrays by stream and 32-row word.
+__device__ __forceinline__ uint32_t flat_stream_of(uint64_t i, uint32_t nb, uint32_t words, uint32_t words1) {
+  if (i < words) return 0;
+  return words1 ? static_cast<uint32_t>(min(static_cast<uint64_t>(nb), 1 + (i - words) / words1)) : nb;
+}
+
 // Rows with a segment, 32 at a time, and the ordinal of the first.
 __global__ void k_flat_meta(flat_rows f, const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ ord,
                             uint32_t words, uint64_t total, uint4* meta) {
@@ -156,11 +162,8 @@ __global__ void k_flat_meta(flat_rows f, const uint32_t* __restrict__ cnt, const
   const uint32_t words1 = (f.rows1 + 31) / 32;
   const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < total; i += nwarps) {
-    uint32_t k = 0, w = static_cast<uint32_t>(i);
-    if (i >= words) {
-      k = words1 ? static_cast<uint32_t>(min(static_cast<uint64_t>(f.nb), 1 + (i - words) / words1)) : f.nb;
-      w = static_cast<uint32_t>(i - flat_place(k, words, words1));
-    }
+    const uint32_t k = flat_stream_of(i, f.nb, words, words1);
+    const uint32_t w = static_cast<uint32_t>(i - flat_place(k, words, words1));
     const uint32_t v = w * 32 + lane;
     const bool has = v < f.V && cnt[f.cell(k, v)] != 0;
     const unsigned m = __ballot_sync(0xffffffffu, has);
@@ -215,9 +218,11 @@ __device__ __forceinline__ bool flat_continues(const flat_view& f, uint32_t p, u
 
 // Segments cut by piece boundaries, one thread per piece; the first piece
 // that continues a segment records it.  fill = false marks the rows in
-// meta.z, fill = true writes the spans (meta.w scanned in between).
+// meta.z and finds the last word with a wide span, fill = true writes the spans
+// (meta.w scanned in between).
 template <bool kFill>
-__global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans) {
+__global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans,
+                             uint32_t* wide_words) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t j = 0;
   if (p >= npieces || !flat_continues(f, p, &j) || j >= segments) return;
@@ -245,10 +250,15 @@ __global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, u
   uint32_t bits = f.meta[lo].x;
   for (uint32_t n = j - f.meta[lo].y; n > 0; --n) bits &= bits - 1;
   const uint32_t bit = bits & (0u - bits);
-  if (!kFill)
+  if (!kFill) {
     atomicOr(&meta[lo].z, bit);
-  else
+    if (last - q > kFlatWideSpan) {
+      const uint64_t word = lo - flat_place(flat_stream_of(lo, f.nb, f.words, f.words1), f.words, f.words1);
+      atomicMax(wide_words, static_cast<uint32_t>(word) + 1u);
+    }
+  } else {
     spans[meta[lo].w + __popc(meta[lo].z & (bit - 1u))] = make_uint2(q, last);
+  }
 }
 
 __global__ void k_flat_span_base(const uint32_t* __restrict__ scan, uint64_t n, uint4* meta) {
@@ -573,7 +583,10 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   f.head = reinterpret_cast<float*>(mem + o_head);
   f.carry = reinterpret_cast<float*>(mem + o_carry);
   const unsigned span_grid = (npieces + 127) / 128;
-  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr);
+  scratch<uint32_t> wide(st);
+  PLATO_TRY(wide.alloc(pool, 1));
+  PLATO_CUDA_TRY(cudaMemsetAsync(wide.p, 0, 4, st));
+  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr, wide.p);
   PLATO_LAUNCHED("k_flat_spans");
   scratch<uint32_t> base(st);
   PLATO_TRY(base.alloc(pool, nmeta));
@@ -581,10 +594,11 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
                      base.p, nmeta, pool, st));
   k_flat_span_base<<<grid_for(nmeta, 256), 256, 0, st>>>(base.p, nmeta, meta);
   PLATO_LAUNCHED("k_flat_span_base");
-  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans);
+  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans, nullptr);
   PLATO_LAUNCHED("k_flat_spans");
-  pl.update_blocks = std::min<uint32_t>(sms * 4, (words + 15) / 16);
+  PLATO_CUDA_TRY(cudaMemcpyAsync(&f.wide_words, wide.p, 4, cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));  // the temporaries and the host vectors go
+  pl.update_blocks = f.wide_words + std::min<uint32_t>(sms * 4, (words - f.wide_words + 15) / 16);
   if (pl.hot_ctas) {
     PLATO_CUDA_TRY(cudaFuncSetAttribute(k_flat_hot<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         kFlatBlockBytes));

@@ -66,6 +66,7 @@ struct flat_sub {
 struct flat_view {
   uint32_t V, nsrc, nb, words;      // words = ceil(V / 32)
   uint32_t words1;                  // 32-row words that take part in the hot streams after the first
+  uint32_t wide_words;              // the first words, which hold every segment across more than kFlatWideSpan pieces
   uint32_t cold_piece0, cold_pieces;
   uint32_t cold_back;               // k_flat_cold's CTAs take the pieces from the end
   const uint16_t* hid;              // hot ids, relative to their block
@@ -364,6 +365,7 @@ __global__ void __launch_bounds__(kFlatColdThreads, kFlatColdCtas)
 
 // The sums of one 32-row word's segments of a stream: lane l gets row l's.
 // They were written by other SMs, in the same kernel when it runs many epochs.
+// A lane adds the pieces of its row's segment four at a time.
 __device__ __forceinline__ float flat_segment(const flat_view& f, const uint4& m, unsigned lane) {
   const unsigned below = (1u << lane) - 1u;
   if (!((m.x >> lane) & 1u)) return 0.f;
@@ -377,6 +379,47 @@ __device__ __forceinline__ float flat_segment(const flat_view& f, const uint4& m
     y += (t[0] + t[1]) + (t[2] + t[3]);
   }
   return y + __ldcg(f.head + sp.y);
+}
+
+// The same where a segment may cross many pieces (a hub row crosses all pieces
+// of a stream): the warp adds those longer than kFlatWideSpan one after another,
+// 256 pieces in flight each.  Lanes alone wait for L2 every four pieces, but all
+// rows of the word at once.  One epoch with all segments added by their lanes /
+// the warp from 32, 16, 8 pieces up, one B200: 1M edges into one vertex 77 /
+// 13.8, 13.8, 13.9 us; RMAT s16 8.8 / 8.9, 9.0, 14.2; s14 6.3 / 6.3, 6.3, 6.6.
+constexpr uint32_t kFlatWideSpan = 32;
+__device__ __forceinline__ float flat_wide_segment(const flat_view& f, const uint4& m, unsigned lane) {
+  const unsigned below = (1u << lane) - 1u;
+  float y = 0.f, h = 0.f;
+  if (((m.x & ~m.z) >> lane) & 1u) y = __ldcg(f.part + m.y + __popc(m.x & below));
+  if (m.z == 0) return y;  // the same in every lane
+  uint2 sp = make_uint2(0u, 0u);
+  if ((m.z >> lane) & 1u) {
+    sp = __ldg(f.spans + m.w + __popc(m.z & below));
+    h = __ldcg(f.head + sp.y);
+  }
+  const bool wide = sp.y - sp.x > kFlatWideSpan;
+  if (!wide)
+    for (uint32_t p = sp.x; p < sp.y; p += 4) {
+      float t[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) t[i] = p + i < sp.y ? __ldcg(f.carry + p + i) : 0.f;
+      y += (t[0] + t[1]) + (t[2] + t[3]);
+    }
+  for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+    const int l = __ffs(todo) - 1;
+    const uint32_t p0 = __shfl_sync(0xffffffffu, sp.x, l), p1 = __shfl_sync(0xffffffffu, sp.y, l);
+    float a = 0.f;
+    for (uint32_t p = p0 + lane; p < p1; p += 256) {
+      float t[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t[i] = p + 32 * i < p1 ? __ldcg(f.carry + p + 32 * i) : 0.f;
+      a += ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+    }
+    a = warp_sum(a);
+    if (lane == static_cast<unsigned>(l)) y = a;
+  }
+  return y + h;
 }
 
 __device__ __forceinline__ uint4 flat_shfl(const uint4& m, int l) {
@@ -410,6 +453,10 @@ __device__ __forceinline__ float flat_middle(const flat_view& f, const uint4& mk
 // of its next two one round ahead, as the sums' loads wait for the metas.  RMAT
 // s24: 82 us (about 170 instructions a word, issue 42% busy, the rest latency);
 // 1 / 3 / 4 words at a time with 6 / 3 / 2 CTAs per SM 113 / 94 / 118.
+// The first wide_words words have a CTA each, whose warps share the streams
+// (epoch with the lanes' sums only / so: 5M edges into one vertex of 1M 220 /
+// 15.4 us, 16M 303 / 27.4, 64M 275 / 55; flat_wide_segment in the main loop
+// spills).
 // With c.ctrl the last CTA to finish sums the partials in a fixed order and
 // takes the epoch decision (epoch_decide).
 struct flat_control {
@@ -426,13 +473,32 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
   constexpr int R = 2;
   __shared__ double s_red[32];
   __shared__ bool s_last;
+  __shared__ float s_wide[8][32];
   flat_after();
   if (upd.skip()) return;
   const unsigned lane = threadIdx.x & 31;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t nwarps = ((gridDim.x - f.wide_words) * blockDim.x) >> 5;
   const uint4* cold = f.meta + flat_place(f.nb, f.words, f.words1);
   double dl = 0.0;
-  uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  uint32_t w = f.words;
+  if (blockIdx.x < f.wide_words) {
+    const uint32_t warp = threadIdx.x >> 5;
+    float y = 0.f;
+    for (uint32_t k = warp; k <= f.nb; k += 8)
+      if (k == 0 || k == f.nb || blockIdx.x < f.words1)
+        y += flat_wide_segment(f, __ldg(f.meta + flat_place(k, f.words, f.words1) + blockIdx.x), lane);
+    s_wide[warp][lane] = y;
+    __syncthreads();
+    if (warp == 0) {
+      y = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) y += s_wide[i][lane];
+      const uint32_t v = blockIdx.x * 32 + lane;
+      if (v < f.V) dl = upd.apply(v, y, upd.load(v));
+    }
+  } else {
+    w = f.wide_words + (((blockIdx.x - f.wide_words) * blockDim.x + threadIdx.x) >> 5);
+  }
   uint4 m0[R], m1[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -574,7 +640,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_run(flat_view f,
       const uint32_t v = w * 32 + lane;
       const bool mine = v < f.V;
       const typename Update::operands ops = upd.load_l2(mine ? v : w * 32);
-      const float y = flat_segment(f, __ldg(f.meta + w), lane);
+      const float y = flat_wide_segment(f, __ldg(f.meta + w), lane);
       if (mine) dl += upd.apply(v, y, ops);
     }
     ++ran;

@@ -162,3 +162,22 @@ def test_device_bytes_count_the_plan_and_the_index():
         g.connected_components()
         columns = np.unique(d).size
         assert g.device_bytes() - ranked >= 12 * columns
+
+
+@pytest.mark.parametrize("V,E,share", [(40, 20000, 1.0), (1000, 300000, 0.5), (100003, 3000000, 1.0),
+                                       (100003, 4000000, 1.0), (1000003, 5000000, 0.9), (200003, 12000000, 0.7),
+                                       (1500007, 20000000, 0.5)])
+def test_rows_across_many_pieces(V, E, share):
+    """A vertex with most of the in-edges crosses every piece of its streams:
+    on the one-launch path, in the cold stream, where all sources are hot, and
+    in both kinds of stream.  L1 <= 1e-6, and the same from run to run."""
+    rng = np.random.default_rng(E)
+    s = rng.integers(0, V, E, dtype=np.uint32)
+    d = rng.integers(0, V, E, dtype=np.uint32)
+    d[rng.random(E) < share] = 1
+    want, _, _ = RefGraph(V, s, d, True).pagerank(6, 0.85, 0.0)
+    with pb.Graph(V, s, d, True) as g:
+        got, _ = g.pagerank(6, 0.85, 0.0)
+        again, _ = g.pagerank(6, 0.85, 0.0)
+    assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
+    np.testing.assert_array_equal(got, again)
