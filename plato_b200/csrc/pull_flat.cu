@@ -221,8 +221,8 @@ __device__ __forceinline__ bool flat_continues(const flat_view& f, uint32_t p, u
 // meta.z and finds the last word with a wide span, fill = true writes the spans
 // (meta.w scanned in between).
 template <bool kFill>
-__global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, uint4* meta, uint2* spans,
-                             uint32_t* wide_words) {
+__global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t hot_steps, uint32_t cold_steps,
+                             uint32_t segments, uint4* meta, uint2* spans, uint32_t* wide_words) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t j = 0;
   if (p >= npieces || !flat_continues(f, p, &j) || j >= segments) return;
@@ -230,14 +230,20 @@ __global__ void k_flat_spans(flat_view f, uint32_t npieces, uint32_t segments, u
   while (f.pieces[q].x >= f.pieces[q].y && !(f.pieces[q].x & kPieceFirst)) --q;
   uint32_t jq = 0;
   if (flat_continues(f, q, &jq) && jq == j) return;
-  uint32_t last = p;
-  for (uint32_t r = p + 1; r < npieces; ++r) {
-    const uint2 pc = f.pieces[r];
-    if (pc.x & kPieceFirst) break;
-    if (pc.x >= pc.y) continue;
-    uint32_t jr = 0;
-    if (!flat_continues(f, r, &jr) || jr != j) break;
-    last = r;
+  // j ends in the last step before which at most j segments have ended, and in
+  // the last piece that starts no later: an empty piece starts no later than the
+  // next one.  (A hub row crosses thousands of pieces: both by search.)
+  const bool hot = p < f.cold_piece0;
+  const uint32_t* ended = hot ? f.hseg : f.cseg;
+  uint32_t s_end = f.pieces[p].x, s_hi = (hot ? hot_steps : cold_steps) - 1;
+  while (s_end < s_hi) {
+    const uint32_t mid = s_end + (s_hi - s_end + 1) / 2;
+    if (ended[mid] <= j) s_end = mid; else s_hi = mid - 1;
+  }
+  uint32_t last = p, p_hi = (hot ? f.cold_piece0 : npieces) - 1;
+  while (last < p_hi) {
+    const uint32_t mid = last + (p_hi - last + 1) / 2;
+    if ((f.pieces[mid].x & ~kPieceFirst) <= s_end) last = mid; else p_hi = mid - 1;
   }
   // the row: the last word whose first ordinal is at most j
   const uint64_t total = flat_place(f.nb, f.words, f.words1) + f.words;
@@ -586,7 +592,8 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   scratch<uint32_t> wide(st);
   PLATO_TRY(wide.alloc(pool, 1));
   PLATO_CUDA_TRY(cudaMemsetAsync(wide.p, 0, 4, st));
-  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, nullptr, wide.p);
+  k_flat_spans<false><<<span_grid, 128, 0, st>>>(pl.v, npieces, hot_steps, cold_steps, segments, meta, nullptr,
+                                                wide.p);
   PLATO_LAUNCHED("k_flat_spans");
   scratch<uint32_t> base(st);
   PLATO_TRY(base.alloc(pool, nmeta));
@@ -594,7 +601,8 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
                      base.p, nmeta, pool, st));
   k_flat_span_base<<<grid_for(nmeta, 256), 256, 0, st>>>(base.p, nmeta, meta);
   PLATO_LAUNCHED("k_flat_span_base");
-  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, segments, meta, spans, nullptr);
+  k_flat_spans<true><<<span_grid, 128, 0, st>>>(pl.v, npieces, hot_steps, cold_steps, segments, meta, spans,
+                                               nullptr);
   PLATO_LAUNCHED("k_flat_spans");
   PLATO_CUDA_TRY(cudaMemcpyAsync(&f.wide_words, wide.p, 4, cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));  // the temporaries and the host vectors go
