@@ -31,6 +31,9 @@ constexpr uint32_t kFlatRowDeg1 = 64;
 // one / three launches: RMAT s16 9.3 / 14.2 us, s17 12.8 / 15.6, s18 21.1 /
 // 19.4; 3.2M uniform edges 19.2 / 25.6).
 constexpr uint64_t kFlatRunEdges = 3500000;
+// ... and rows: its warps also update every 32-row word (uniform edges, 0.1 a row:
+// 4M rows 21.5 / 30.1, 8M 56.8 / 51.7, 16M 118 / 98).
+constexpr uint32_t kFlatRunRows = 6000000;
 constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 600000;
 
 // out[0]: one past the last row above kFlatRowDeg1 edges, out[1]: how many there
@@ -354,7 +357,7 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
   flat_rows rows{off, g->in_adj.p, V, 0, 0, kFlatRowDeg0, kFlatRowDeg1};
   uint32_t nb = 0;
-  const bool run = E <= kFlatRunEdges;
+  const bool run = E <= kFlatRunEdges && V <= kFlatRunRows;
   if (!run) {
     unsigned long long hot = h[2];
     for (nb = 1; nb < nblocks && h[2 + nb] >= std::max(kFlatMore, h[1]) && h[1] > 0; ++nb) hot += h[2 + nb];
@@ -408,16 +411,17 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   pl.run_ctas = pl.run_warps = pl.cold_blocks = 0;
   pl.run_cluster = false;
   if (run) {
-    if (cold_steps <= 4) {
+    const uint32_t work = std::max(cold_steps, words);  // a warp each, as far as they go
+    if (work <= 4) {
       pl.run_ctas = 1;
       pl.run_warps = 4;
-    } else if (cold_steps <= kFlatClusterSteps) {
+    } else if (work <= kFlatClusterSteps) {
       pl.run_cluster = true;
       pl.run_ctas = kFlatCluster;
-      pl.run_warps = std::min<uint32_t>(32, std::max<uint32_t>(4, (cold_steps + kFlatCluster - 1) / kFlatCluster));
+      pl.run_warps = std::min<uint32_t>(32, std::max<uint32_t>(4, (work + kFlatCluster - 1) / kFlatCluster));
     } else {
-      pl.run_ctas = std::min<uint32_t>(sms, (cold_steps + 7) / 8);
-      pl.run_warps = std::min<uint32_t>(32, (cold_steps + pl.run_ctas - 1) / pl.run_ctas);
+      pl.run_ctas = std::min<uint32_t>(sms, (work + 7) / 8);
+      pl.run_warps = std::min<uint32_t>(32, (work + pl.run_ctas - 1) / pl.run_ctas);
     }
   } else if (cold_steps) {
     // a wave of resident CTAs, and more (up to about five waves, so that the

@@ -49,7 +49,7 @@ constexpr uint32_t kFlatColdStep = 32 * kFlatColdLane;
 constexpr uint32_t kFlatBlock = 57344;    // sources of a hot block
 constexpr uint32_t kFlatBlockBytes = kFlatBlock * sizeof(float);
 constexpr uint32_t kFlatMaxBlocks = 24;
-// Up to this many steps (64K edges) k_flat_run's CTAs are one cluster of 8 (epoch
+// Up to this many steps (64K edges) and words k_flat_run's CTAs are one cluster of 8 (epoch
 // over a cooperative grid / over the cluster, one B200: RMAT s10 5.5 / 4.4 us,
 // s11 6.3 / 4.9, s12 6.5 / 6.3, s13 6.3 / 7.6).
 constexpr uint32_t kFlatCluster = 8, kFlatClusterSteps = 256;
@@ -612,7 +612,9 @@ __device__ __noinline__ void flat_poison(const flat_view& f, const Update& upd, 
 // Every epoch of a small graph in one launch, cooperative over gridDim.x <= SMs
 // CTAs or, up to 256 steps, one cluster of 8 (one CTA alone is bound by issue,
 // and a barrier through L2 costs more than 64K edges' gathers): gather, barrier,
-// update, barrier.  The epoch kinds and the eps exit follow epoch_decide;
+// update, barrier.  The grid has a warp for every step and every 32-row word, as
+// far as they go (by the steps alone, 1000 edges over 1M vertices 3.0 ms an epoch).
+// The epoch kinds and the eps exit follow epoch_decide;
 // ctrl[1] = epochs run, counted from `start`.  Launches bound these graphs: one
 // epoch with a launch per degree bin / here, RMAT s10 52 / 4.4 us, s12 54 / 6.3, s16
 // 70 / 9.4, 48K uniform edges 28 / 5.8.  A CTA that gives up waiting leaves NaN

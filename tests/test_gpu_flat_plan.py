@@ -181,3 +181,27 @@ def test_rows_across_many_pieces(V, E, share):
         again, _ = g.pagerank(6, 0.85, 0.0)
     assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
     np.testing.assert_array_equal(got, again)
+
+
+def _uniform(V, E):
+    rng = np.random.default_rng(V + E)
+    return V, rng.integers(0, V, E, dtype=np.uint32), rng.integers(0, V, E, dtype=np.uint32)
+
+
+@pytest.mark.parametrize("V,E", [(8192, 8), (8193, 8), (300007, 8), (1000003, 500000), (6000000, 900000),
+                                 (6000001, 900000)])
+def test_few_edges_over_many_rows(V, E):
+    """The warps of the one-launch epochs follow the rows too, up to 6M of
+    them; with a first row that is long, so that no shorter way answers."""
+    _, s, d = _uniform(V, E)
+    s, d = np.append(s, np.arange(600, dtype=np.uint32)), np.append(d, np.full(600, 5, np.uint32))
+    want, _, _ = RefGraph(V, s, d, True).pagerank(5, 0.85, 0.0)
+    with pb.Graph(V, s, d, True) as g:
+        hit, (got, _) = _launched(lambda: g.pagerank(5, 0.85, 0.0), KERNELS)
+        ms, n = C.c_double(), C.c_uint64()
+        if V <= 1000003:  # by the edges alone 300007 rows took 0.9 ms an epoch
+            lib = _lib.load()
+            assert hit == {"k_flat_run"}
+            _lib.check(lib.plato_profile_read(b"k_flat_run", C.byref(ms), C.byref(n)), "read")
+            assert n.value == 1 and ms.value < 1.0
+    assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
