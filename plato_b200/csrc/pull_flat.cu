@@ -36,23 +36,64 @@ constexpr uint64_t kFlatRunEdges = 3500000;
 constexpr uint32_t kFlatRunRows = 6000000;
 constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 600000;
 
+// Which graphs pull by the degree bins instead (pull_binned.cuh).  A row costs
+// a flat plan a segment's store, load and meta, the bins only its offsets; what
+// it saves is gathers, and the launch of a kernel a bin (about 6 us each).  One
+// epoch, flat / bins, one B200:
+//   no row above kShortMax (4) edges, one bin: rings of 10K / 100K / 1M / 4M
+//   vertices 4.7 / 4.4, 5.3 / 4.4, 12.0 / 10.1, 35.9 / 29.2 us, grids 5.1 / 4.4,
+//   5.7 / 4.9, 14.6 / 10.6, 46 / 32, 4 random in-edges a row 5.3 / 4.4, 6.7 / 6.5,
+//   25.5 / 22.6, 95 / 76; up to kFlatClusterSteps words one cluster runs all
+//   epochs (5K vertices 3.7-4.4 / 4.4);
+//   rows up to 16 (two bins), uniform: 600K rows with 3.5 edges 19.9 / 20.9, 1M
+//   with 1.5 / 2.5 / 3.5 19.3 / 21.0, 26.1 / 23.0, 31.5 / 29.1, 4M with 0.5 / 1 /
+//   2.5 35.0 / 37.4, 51.0 / 42.2, 82.0 / 63.9, 8M with 0.1 / 1 51.7 / 45.0, 99 /
+//   73, 16M with 2.5 / 3.5 302 / 300, 365 / 491;
+//   longer ones too: 2M with 5 66.1 / 69.4, 4M with 5 / 6 121 / 118, 133 / 136, 8M
+//   with 5 234 / 221; RMAT s22 with 4.4 29.9 / 92.5 (half of the edges in them).
+struct flat_census {
+  uint64_t rows, few, some;      // all rows, rows of 1..4 and of 5..16 edges
+  uint64_t edges, long_edges;    // all edges, those in rows above 16
+};
+bool flat_bins_suit(const flat_census& c) {
+  if (c.some == 0 && c.long_edges == 0) return c.rows > 32ull * kFlatClusterSteps;
+  if (c.rows > 10000000 && 2 * c.edges > 5 * c.rows) return false;
+  if (c.long_edges == 0) return (c.few + c.some >= 900000 && c.edges >= 2500000) || c.rows >= 6000000;
+  return 20 * c.long_edges <= c.edges && c.edges <= 6 * c.rows && c.few + c.some >= 2500000;
+}
+
 // out[0]: one past the last row above kFlatRowDeg1 edges, out[1]: how many there
-// are, out[2 + k]: gathers of the sources of block k (`uses` by source).
+// are, out[2..4]: few, some and long_edges of the census, out[kFlatSurvey + k]:
+// gathers of the sources of block k (`uses` by source).
+constexpr uint32_t kFlatSurvey = 5;
 __global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict__ off,
                                                      const uint32_t* __restrict__ uses, uint32_t V,
                                                      uint32_t nblocks, unsigned long long* out) {
   __shared__ unsigned long long s_red[32];
-  unsigned long long last = 0, n = 0;
-  for (uint64_t v = blockIdx.x * 256ull + threadIdx.x; v < V; v += gridDim.x * 256ull)
-    if (off[v + 1] - off[v] > kFlatRowDeg1) {
+  unsigned long long last = 0, n = 0, few = 0, some = 0, longs = 0;
+  for (uint64_t v = blockIdx.x * 256ull + threadIdx.x; v < V; v += gridDim.x * 256ull) {
+    const uint64_t d = off[v + 1] - off[v];
+    if (d > kFlatRowDeg1) {
       last = v + 1;
       ++n;
     }
+    few += d > 0 && d <= 4;
+    some += d > 4 && d <= 16;
+    longs += d > 16 ? d : 0;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
   if ((threadIdx.x & 31) == 0 && last) atomicMax(out, last);
   n = block_sum_u64<256>(n, s_red);
   if (threadIdx.x == 0 && n) atomicAdd(out + 1, n);
+  few = block_sum_u64<256>(few, s_red);
+  some = block_sum_u64<256>(some, s_red);
+  longs = block_sum_u64<256>(longs, s_red);
+  if (threadIdx.x == 0) {
+    if (few) atomicAdd(out + 2, few);
+    if (some) atomicAdd(out + 3, some);
+    if (longs) atomicAdd(out + 4, longs);
+  }
   // 8 CTAs a block of sources
   const uint32_t k = blockIdx.x / 8, q = blockIdx.x % 8;
   if (k >= nblocks) return;
@@ -60,7 +101,7 @@ __global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict_
   n = 0;
   for (uint32_t v = b + q * 256 + threadIdx.x; v < e; v += 8 * 256) n += uses[v];
   n = block_sum_u64<256>(n, s_red);
-  if (threadIdx.x == 0) atomicAdd(out + 2 + k, n);
+  if (threadIdx.x == 0) atomicAdd(out + kFlatSurvey + k, n);
 }
 
 struct flat_rows {
@@ -347,20 +388,22 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
     return set_error(PLATO_ECUDA, e.what());
   }
   scratch<unsigned long long> d_survey(st);
-  PLATO_TRY(d_survey.alloc(pool, 2 + kFlatMaxBlocks));
-  PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, (2 + kFlatMaxBlocks) * sizeof(unsigned long long), st));
+  PLATO_TRY(d_survey.alloc(pool, kFlatSurvey + kFlatMaxBlocks));
+  PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, (kFlatSurvey + kFlatMaxBlocks) * sizeof(unsigned long long), st));
   k_flat_survey<<<std::max(nblocks * 8, grid_for(V, 256, 148 * 4)), 256, 0, st>>>(
       off, g->out_deg.p, V, nblocks, d_survey.p);
   PLATO_LAUNCHED("k_flat_survey");
-  unsigned long long h[2 + kFlatMaxBlocks];
+  unsigned long long h[kFlatSurvey + kFlatMaxBlocks];
   PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
+  if (flat_bins_suit(flat_census{V, h[2], h[3], E, h[4]})) return PLATO_OK;
   flat_rows rows{off, g->in_adj.p, V, 0, 0, kFlatRowDeg0, kFlatRowDeg1};
   uint32_t nb = 0;
   const bool run = E <= kFlatRunEdges && V <= kFlatRunRows;
   if (!run) {
-    unsigned long long hot = h[2];
-    for (nb = 1; nb < nblocks && h[2 + nb] >= std::max(kFlatMore, h[1]) && h[1] > 0; ++nb) hot += h[2 + nb];
+    const unsigned long long* uses = h + kFlatSurvey;
+    unsigned long long hot = uses[0];
+    for (nb = 1; nb < nblocks && uses[nb] >= std::max(kFlatMore, h[1]) && h[1] > 0; ++nb) hot += uses[nb];
     if (hot < kFlatFirst) nb = 0;
   }
   rows.nb = nb;

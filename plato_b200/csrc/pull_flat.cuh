@@ -108,8 +108,9 @@ struct flat_plan {
 
 // Builds the plan of g's pull on `st` (pull_flat.cu): rows gather their
 // in-neighbours.  plan.valid stays false where there is nothing to gather, the
-// sources are not g's vertices (a partition), or the graph keeps its caller's
-// order (its pull sums in the merge path's order, as plato_pagerank_csc_noalloc).
+// sources are not g's vertices (a partition), the rows are short (the degree
+// bins are the faster), or the graph keeps its caller's order (its pull sums in
+// the merge path's order, as plato_pagerank_csc_noalloc).
 int build_flat_plan(plato_graph* g, flat_plan& plan, cudaStream_t st);
 
 __device__ __forceinline__ void flat_prefetch(const void* p) {

@@ -205,3 +205,47 @@ def test_few_edges_over_many_rows(V, E):
             _lib.check(lib.plato_profile_read(b"k_flat_run", C.byref(ms), C.byref(n)), "read")
             assert n.value == 1 and ms.value < 1.0
     assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
+
+
+def _ring(V):
+    i = np.arange(V, dtype=np.uint32)
+    return V, i, (i + 1) % np.uint32(V)
+
+
+def _capped(V, k):
+    """k in-edges for every vertex but one, which has none."""
+    rng = np.random.default_rng(V + k)
+    d = np.repeat(np.arange(V, dtype=np.uint32), k)
+    s = rng.integers(0, V, d.size, dtype=np.uint32)
+    return V, s[d != 0], d[d != 0]
+
+
+ONE, TWO = {"k_pull_short"}, {"k_pull_short", "k_pull_rows4"}
+RUN, COLD = {"k_flat_run"}, {"k_flat_cold", "k_flat_update"}
+
+
+@pytest.mark.parametrize("graph,kernels", [
+    (_ring(8192), RUN), (_ring(8193), ONE), (_ring(100003), ONE), (_capped(8193, 4), ONE), (_capped(8193, 5), RUN),
+    (_uniform(1000003, 1000), ONE), (_uniform(1000003, 500000), RUN), (_uniform(1000003, 1500000), RUN),
+    (_uniform(1000003, 2600000), TWO), (_capped(500001, 8), COLD), (_capped(900002, 5), {"k_pull_rows4"} | ONE),
+    (_uniform(1000003, 6000000), COLD), (_uniform(6000001, 600000), None), (_uniform(4000037, 20000000), None),
+    (pb.rmat(16, 1, 3), RUN), (pb.rmat(22, 1, 3), COLD)])
+def test_short_rows_take_the_bins(graph, kernels):
+    """Which kernels answer, on both sides of each limit of the rule; the ranks
+    against the oracle (L1 <= 1e-6) and against the merge path, which takes any
+    graph (each within 1e-6 of the oracle's)."""
+    V, s, d = graph
+    want, _, _ = RefGraph(V, s, d, True).pagerank(5, 0.85, 0.0)
+    with pb.Graph(V, s, d, True) as g:
+        hit, (got, st) = _launched(lambda: g.pagerank(5, 0.85, 0.0), KERNELS)
+        again, early = g.pagerank(50, 0.85, 1e-2 * V)
+    with pb.Graph(V, s, d, True, relabel=False) as g:
+        plain, (general, _) = _launched(lambda: g.pagerank(5, 0.85, 0.0), KERNELS)
+        late, same = g.pagerank(50, 0.85, 1e-2 * V)
+    assert plain == {"k_pull_warp"}
+    assert kernels is None or hit == kernels
+    assert st.iterations == 5 and early.iterations == same.iterations
+    assert early.delta == pytest.approx(same.delta, rel=1e-4)
+    assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
+    assert np.abs(got.astype(np.float64) - general).sum() <= 2e-6
+    assert np.abs(again.astype(np.float64) - late).sum() <= 2e-6
