@@ -17,14 +17,21 @@ namespace {
 // rows above kFlatRowDeg1 in the further blocks: a segment costs a store and a
 // load of its sum, so it has to hold a few edges (RMAT s24, epoch: further
 // blocks above 32 / 48 / 64 / 96 / 128 in-edges 562 / 539 / 532 / 537 / 577 us;
-// block 0 above 4 / 8 / 16 / 32: 580 / 577 / 583 / 589).  There are hot streams
-// where they hold kFlatFirst edges: below, one more launch and the copies of the
-// blocks cost what the gathers save (epoch without / with them: RMAT s18 20.6 /
-// 24.4 us, s19 32.4 / 33.4, s20 55.8 / 48.5; 64M uniform edges over 1M vertices
-// 262 / 144).  A further block is used where it
-// holds kFlatMore edges, and one per row that takes part (RMAT s22 with 4 / 6 /
-// 10 / 16 blocks 153 / 144 / 138 / 144 us; s24 with 1 / 3 / 6 / 10 / 16 / 24:
-// 743 / 674 / 633 / 595 / 577 / 568).
+// block 0 above 4 / 8 / 16 / 32: 580 / 577 / 583 / 589).  What a block holds is
+// counted over the rows that take part.  A further block is used where that is
+// kFlatMore edges and one more for each such row: its copies and segments cost
+// something too (us an epoch with 1 / 4 / 10 / 16 / 24 blocks, and how many are
+// chosen: RMAT s21 84.9 / 72.8 / 74.8 / 76.8 / 83.4, 4; s22 168 / 142 / 134 / 133
+// / 138, 10; s23 342 / 290 / 260 / 251 / 251, 15; s24 with 10 / 16 / 20 / 22 / 24
+// 537 / 521 / 503 / 497 / 507, 22; s22 with 6 edges a vertex 85.7 / 76.9 / 80.8 /
+// 81.1 / 87.3, 5).  There are hot streams where all of them together hold
+// kFlatFirst: below, one more launch costs what the gathers save (edges that
+// would be hot, epoch without / with them: RMAT s19 6.5M 26.4 / 27.5, s20 with 10
+// a vertex 8.0M 38.2 / 38.0, s19 with 20 8.6M 31.6 / 33.1, s21 with 6 8.9M 57.5 /
+// 48.1, s20 13.6M 51.0 / 45.6).  A count that took
+// in the rows below the limits gave uniform edges with one long row streams that
+// were all but empty: 16M over 1M vertices 162 us instead of 80, 64M over 4M 378
+// instead of 288.
 constexpr uint32_t kFlatRowDeg0 = 8;
 constexpr uint32_t kFlatRowDeg1 = 64;
 // Up to this many edges all epochs run in one launch (k_flat_run; epoch with
@@ -34,7 +41,16 @@ constexpr uint64_t kFlatRunEdges = 3500000;
 // ... and rows: its warps also update every 32-row word (uniform edges, 0.1 a row:
 // 4M rows 21.5 / 30.1, 8M 56.8 / 51.7, 16M 118 / 98).
 constexpr uint32_t kFlatRunRows = 6000000;
-constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 600000;
+constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 400000;
+// Where the blocks cover all sources, every row can take part in every stream
+// and no cold pass is left.  That pays from 1.5 edges a segment, unless block 0
+// has most of the gathers, which then come from L1 anyway (without / with it:
+// uniform edges over 1M vertices, 16M 80 / 91.5, 24M 108 / 105, 32M 143 / 116, 64M
+// 256 / 135; 8M over 300K 38 / 28; RMAT s19 26.2 / 28.1, s20 43.9 / 47.4).
+bool flat_all_hot(uint64_t rows, uint64_t edges, uint64_t first_block, uint32_t blocks) {
+  return static_cast<uint64_t>(blocks) * kFlatBlock >= rows && 2 * edges >= 3 * rows * blocks &&
+         2 * first_block < edges;
+}
 
 // Which graphs pull by the degree bins instead (pull_binned.cuh).  A row costs
 // a flat plan a segment's store, load and meta, the bins only its offsets; what
@@ -63,12 +79,12 @@ bool flat_bins_suit(const flat_census& c) {
 }
 
 // out[0]: one past the last row above kFlatRowDeg1 edges, out[1]: how many there
-// are, out[2..4]: few, some and long_edges of the census, out[kFlatSurvey + k]:
-// gathers of the sources of block k (`uses` by source).
-constexpr uint32_t kFlatSurvey = 5;
+// are, out[2..4]: few, some and long_edges of the census, out[5]: gathers of the
+// sources of block 0 (`uses` by source), out[kFlatSurvey + k]: k_flat_uses.
+constexpr uint32_t kFlatSurvey = 6;
 __global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict__ off,
                                                      const uint32_t* __restrict__ uses, uint32_t V,
-                                                     uint32_t nblocks, unsigned long long* out) {
+                                                     unsigned long long* out) {
   __shared__ unsigned long long s_red[32];
   unsigned long long last = 0, n = 0, few = 0, some = 0, longs = 0;
   for (uint64_t v = blockIdx.x * 256ull + threadIdx.x; v < V; v += gridDim.x * 256ull) {
@@ -94,14 +110,46 @@ __global__ void __launch_bounds__(256) k_flat_survey(const uint64_t* __restrict_
     if (some) atomicAdd(out + 3, some);
     if (longs) atomicAdd(out + 4, longs);
   }
-  // 8 CTAs a block of sources
-  const uint32_t k = blockIdx.x / 8, q = blockIdx.x % 8;
-  if (k >= nblocks) return;
-  const uint32_t b = k * kFlatBlock, e = min(V, b + kFlatBlock);
   n = 0;
-  for (uint32_t v = b + q * 256 + threadIdx.x; v < e; v += 8 * 256) n += uses[v];
+  for (uint64_t v = blockIdx.x * 256ull + threadIdx.x; v < min(V, kFlatBlock); v += gridDim.x * 256ull) n += uses[v];
   n = block_sum_u64<256>(n, s_red);
-  if (threadIdx.x == 0) atomicAdd(out + kFlatSurvey + k, n);
+  if (threadIdx.x == 0 && n) atomicAdd(out + 5, n);
+}
+
+__device__ __forceinline__ uint64_t flat_lower_bound(const uint32_t* __restrict__ adj, uint64_t lo, uint64_t hi,
+                                                     uint32_t bound) {
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (adj[mid] < bound) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// out[k]: edges of block k in the rows that take part in its stream.  A warp
+// takes 32 rows; the rows of block 0 alone a lane each, the others one after
+// another with a block a lane.
+__global__ void __launch_bounds__(256) k_flat_uses(const uint64_t* __restrict__ off, const uint32_t* __restrict__ adj,
+                                                   uint32_t V, uint32_t nblocks, unsigned long long* out) {
+  static_assert(kFlatMaxBlocks <= 32, "a block a lane");
+  const unsigned lane = threadIdx.x & 31;
+  const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  unsigned long long first = 0, mine = 0;
+  for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w < (V + 31ull) / 32; w += nwarps) {
+    const uint64_t v = w * 32 + lane;
+    const uint64_t b = v < V ? off[v] : 0, e = v < V ? off[v + 1] : 0;
+    const bool all = e - b > kFlatRowDeg1;
+    if (!all && e - b > kFlatRowDeg0) first += flat_lower_bound(adj, b, e, kFlatBlock) - b;
+    for (unsigned todo = __ballot_sync(0xffffffffu, all); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const uint64_t rb = __shfl_sync(0xffffffffu, b, l), re = __shfl_sync(0xffffffffu, e, l);
+      const uint64_t end = lane < nblocks ? flat_lower_bound(adj, rb, re, (lane + 1) * kFlatBlock) : re;
+      const uint64_t begin = __shfl_up_sync(0xffffffffu, end, 1);
+      if (lane < nblocks) mine += end - (lane ? begin : rb);
+    }
+  }
+  first = warp_sum(first);
+  if (lane == 0) mine += first;
+  if (lane < nblocks && mine) atomicAdd(out + lane, mine);
 }
 
 struct flat_rows {
@@ -128,14 +176,7 @@ __global__ void k_flat_split(flat_rows f, uint32_t* cnt) {
     for (uint32_t k = 0; k < f.nb; ++k) {
       if (k > 0 && v >= f.rows1) break;
       uint64_t lo = pos;
-      if (k < ns) {
-        const uint32_t bound = (k + 1) * kFlatBlock;
-        uint64_t hi = end;
-        while (lo < hi) {
-          const uint64_t mid = (lo + hi) >> 1;
-          if (f.adj[mid] < bound) lo = mid + 1; else hi = mid;
-        }
-      }
+      if (k < ns) lo = flat_lower_bound(f.adj, pos, end, (k + 1) * kFlatBlock);
       cnt[f.cell(k, v)] = static_cast<uint32_t>(lo - pos);
       pos = lo;
     }
@@ -390,29 +431,32 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   scratch<unsigned long long> d_survey(st);
   PLATO_TRY(d_survey.alloc(pool, kFlatSurvey + kFlatMaxBlocks));
   PLATO_CUDA_TRY(cudaMemsetAsync(d_survey.p, 0, (kFlatSurvey + kFlatMaxBlocks) * sizeof(unsigned long long), st));
-  k_flat_survey<<<std::max(nblocks * 8, grid_for(V, 256, 148 * 4)), 256, 0, st>>>(
-      off, g->out_deg.p, V, nblocks, d_survey.p);
+  k_flat_survey<<<grid_for(V, 256, 148 * 4), 256, 0, st>>>(off, g->out_deg.p, V, d_survey.p);
   PLATO_LAUNCHED("k_flat_survey");
+  const bool run = E <= kFlatRunEdges && V <= kFlatRunRows;
+  if (!run) {
+    k_flat_uses<<<grid_for(V, 256, 148 * 8), 256, 0, st>>>(off, g->in_adj.p, V, nblocks, d_survey.p + kFlatSurvey);
+    PLATO_LAUNCHED("k_flat_uses");
+  }
   unsigned long long h[kFlatSurvey + kFlatMaxBlocks];
   PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
   if (flat_bins_suit(flat_census{V, h[2], h[3], E, h[4]})) return PLATO_OK;
   flat_rows rows{off, g->in_adj.p, V, 0, 0, kFlatRowDeg0, kFlatRowDeg1};
   uint32_t nb = 0;
-  const bool run = E <= kFlatRunEdges && V <= kFlatRunRows;
-  if (!run) {
+  const bool all_hot = !run && flat_all_hot(V, E, h[5], nblocks);
+  if (all_hot) {
+    nb = nblocks;
+    rows.deg0 = rows.deg1 = 0;
+  } else if (!run) {
     const unsigned long long* uses = h + kFlatSurvey;
     unsigned long long hot = uses[0];
-    for (nb = 1; nb < nblocks && uses[nb] >= std::max(kFlatMore, h[1]) && h[1] > 0; ++nb) hot += uses[nb];
+    for (nb = 1; nb < nblocks && uses[nb] >= kFlatMore + h[1]; ++nb) hot += uses[nb];
     if (hot < kFlatFirst) nb = 0;
   }
   rows.nb = nb;
   // whole words; the last may be short
-  rows.rows1 = nb > 1 ? std::min((static_cast<uint32_t>(h[0]) + 31) / 32 * 32, V) : 0;
-  if (nb > 0 && static_cast<uint64_t>(nb) * kFlatBlock >= V) {  // every source is hot: no cold pass
-    rows.deg0 = rows.deg1 = 0;
-    rows.rows1 = nb > 1 ? V : 0;
-  }
+  rows.rows1 = nb <= 1 ? 0 : all_hot ? V : std::min((static_cast<uint32_t>(h[0]) + 31) / 32 * 32, V);
   const uint32_t streams = nb + 1, words = (V + 31) / 32, words1 = (rows.rows1 + 31) / 32;
   const uint64_t cells = flat_place(nb, V, rows.rows1) + V;
 

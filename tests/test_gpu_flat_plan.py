@@ -249,3 +249,27 @@ def test_short_rows_take_the_bins(graph, kernels):
     assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
     assert np.abs(got.astype(np.float64) - general).sum() <= 2e-6
     assert np.abs(again.astype(np.float64) - late).sum() <= 2e-6
+
+
+HOT = {"k_flat_hot", "k_flat_cold", "k_flat_update"}
+ALL_HOT = {"k_flat_hot", "k_flat_update"}
+
+
+@pytest.mark.parametrize("V,E,long_row,kernels", [
+    (300001, 3600000, 0, ALL_HOT), (300001, 3600000, 65, ALL_HOT), (1000003, 16000000, 65, COLD),
+    (1000003, 16000000, 400000, COLD), (1376256, 49545216, 0, ALL_HOT), (1376256, 49545215, 65, COLD),
+    (1376257, 50000000, 65, COLD), (57344, 4000000, 0, COLD), (57345, 5000000, 100, COLD),
+    (300001, 12000000, 9000000, ALL_HOT), (1100003, 15000000, 14000000, HOT), (172032, 774144, 0, RUN)])
+def test_streams_follow_the_rows_that_take_part(V, E, long_row, kernels):
+    """Hot streams where the rows that take part fill them: not for one long
+    row beside short ones, for all rows where the blocks cover the sources and
+    a segment has 1.5 edges.  L1 <= 1e-6 of the oracle's ranks."""
+    _, s, d = _uniform(V, E)
+    d[:long_row] = 7
+    want, _, _ = RefGraph(V, s, d, True).pagerank(3, 0.85, 0.0)
+    with pb.Graph(V, s, d, True) as g:
+        hit, (got, _) = _launched(lambda: g.pagerank(3, 0.85, 0.0), KERNELS)
+        again, _ = g.pagerank(3, 0.85, 0.0)
+    assert hit == kernels
+    assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
+    np.testing.assert_array_equal(got, again)
