@@ -6,14 +6,17 @@
 // algorithms.  copy_to_host stages it itself: the device writes pinned chunks
 // at the link's rate, and several host threads move finished chunks to the
 // caller while later ones arrive.  The staging memory is one block per process
-// (kHalves * kHalfBytes), used by one call at a time; a call that finds it
-// busy, a small result and a caller's pinned buffer take the plain copy.  The
-// block is freed with the last graph.
+// (kHalves * kHalfBytes, portable: every device's copies use it), used by one
+// call at a time; a call that finds it busy, a small result and a caller's
+// pinned buffer take the plain copy.  It is
+// freed with the last graph.
+
 #include <omp.h>
 
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <new>
 
 #include "common.cuh"
 #include "host_copy.hpp"
@@ -25,34 +28,47 @@ constexpr size_t kChunk = 256u << 10, kHalfBytes = 4u << 20, kHalves = 2;
 constexpr size_t kChunks = kHalfBytes / kChunk;
 constexpr size_t kSmall = 1u << 20;  // below, waking the threads costs more than they save
 constexpr int kThreads = 8;
+constexpr int kDevices = 64;
 
 struct staging {
   std::mutex mu;  // held by the copy that uses the block
   unsigned char* p = nullptr;
-  int device = -1;  // of the events
-  cudaEvent_t done[kHalves * kChunks] = {};
+  cudaEvent_t* done[kDevices] = {};  // [kHalves * kChunks] of a device
   void release() {
-    for (cudaEvent_t& e : done) {
-      if (e) cudaEventDestroy(e);
-      e = nullptr;
+    for (cudaEvent_t*& d : done) {
+      for (size_t i = 0; d && i < kHalves * kChunks; ++i)
+        if (d[i]) cudaEventDestroy(d[i]);
+      delete[] d;
+      d = nullptr;
     }
     if (p) cudaFreeHost(p);
     p = nullptr;
-    device = -1;
   }
-  bool ready(int dev) {
-    if (p && device == dev) return true;
-    release();
-    if (cudaHostAlloc(reinterpret_cast<void**>(&p), kHalves * kHalfBytes, cudaHostAllocPortable) != cudaSuccess)
-      p = nullptr;
-    for (cudaEvent_t& e : done)
-      if (p && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-        e = nullptr;
-        release();
+  // The events of device `dev`, or null: no block, take the plain copy.
+  cudaEvent_t* ready(int dev) {
+    if (dev < 0 || dev >= kDevices) return nullptr;
+    if (!p) {
+      if (cudaHostAlloc(reinterpret_cast<void**>(&p), kHalves * kHalfBytes, cudaHostAllocPortable) != cudaSuccess) {
+        p = nullptr;
+        cudaGetLastError();
+        return nullptr;
       }
-    if (!p) cudaGetLastError();
-    device = p ? dev : -1;
-    return p != nullptr;
+    }
+    if (!done[dev]) {
+      cudaEvent_t* d = new (std::nothrow) cudaEvent_t[kHalves * kChunks]();
+      bool ok = d != nullptr;
+      for (size_t i = 0; ok && i < kHalves * kChunks; ++i)
+        ok = cudaEventCreateWithFlags(&d[i], cudaEventDisableTiming) == cudaSuccess;
+      if (!ok) {
+        cudaGetLastError();
+        for (size_t i = 0; d && i < kHalves * kChunks; ++i)
+          if (d[i]) cudaEventDestroy(d[i]);
+        delete[] d;
+        return nullptr;
+      }
+      done[dev] = d;
+    }
+    return done[dev];
   }
 };
 
@@ -99,7 +115,11 @@ int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   std::unique_lock<std::mutex> lock(g_stage.mu, std::try_to_lock);
   int dev = 0;
   PLATO_CUDA_TRY(cudaGetDevice(&dev));
-  if (!lock.owns_lock() || !g_stage.ready(dev)) return plain_copy(dst, src, bytes, st);
+  cudaEvent_t* const done = lock.owns_lock() ? g_stage.ready(dev) : nullptr;
+  if (!done) {
+    if (lock.owns_lock()) lock.unlock();
+    return plain_copy(dst, src, bytes, st);
+  }
   unsigned char* out = static_cast<unsigned char*>(dst);
   const unsigned char* in = static_cast<const unsigned char*>(src);
   // part `k` of the result goes through half k % 2, a chunk at a time
@@ -109,7 +129,7 @@ int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     for (size_t c = lo, i = (k % kHalves) * kChunks; c < hi; c += kChunk, ++i) {
       cudaError_t e = cudaMemcpyAsync(g_stage.p + (k % kHalves) * kHalfBytes + (c - lo), in + c,
                                       std::min(kChunk, hi - c), cudaMemcpyDeviceToHost, st);
-      if (e == cudaSuccess) e = cudaEventRecord(g_stage.done[i], st);
+      if (e == cudaSuccess) e = cudaEventRecord(done[i], st);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -123,7 +143,7 @@ int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     int failed = 0;
 #pragma omp parallel for schedule(dynamic, 1) num_threads(threads) reduction(| : failed)
     for (int i = 0; i < n; ++i) {
-      if (cudaEventSynchronize(g_stage.done[(k % kHalves) * kChunks + i]) != cudaSuccess) {
+      if (cudaEventSynchronize(done[(k % kHalves) * kChunks + i]) != cudaSuccess) {
         failed = 1;
         continue;
       }
