@@ -10,13 +10,18 @@
 // call at a time; a call that finds it busy, a small result and a caller's
 // pinned buffer take the plain copy.  It is
 // freed with the last graph.
-
+//
+// The other host threads only move bytes.  Whatever they call of the CUDA
+// runtime would use their own current device, and set it up if it is not the
+// caller's.
 #include <omp.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <thread>
 
 #include "common.cuh"
 #include "host_copy.hpp"
@@ -140,17 +145,33 @@ int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   for (size_t k = 0; k < parts && err == cudaSuccess; ++k) {
     const size_t lo = k * kHalfBytes, hi = std::min(bytes, lo + kHalfBytes);
     const int n = static_cast<int>((hi - lo + kChunk - 1) / kChunk);
-    int failed = 0;
-#pragma omp parallel for schedule(dynamic, 1) num_threads(threads) reduction(| : failed)
-    for (int i = 0; i < n; ++i) {
-      if (cudaEventSynchronize(done[(k % kHalves) * kChunks + i]) != cudaSuccess) {
-        failed = 1;
-        continue;
+    const cudaEvent_t* arrived = done + (k % kHalves) * kChunks;
+    const unsigned char* half = g_stage.p + (k % kHalves) * kHalfBytes;
+    auto move = [&](int i) {
+      const size_t at = static_cast<size_t>(i) * kChunk;
+      std::memcpy(out + lo + at, half + at, std::min(kChunk, hi - lo - at));
+    };
+    // This thread waits for the chunks one after another, the others take what has
+    // arrived; the wait for the work before the first chunk is this thread's alone.
+    err = cudaEventSynchronize(arrived[0]);
+    if (err != cudaSuccess) break;
+    std::atomic<int> next{0}, in_memory{1};  // chunks taken, chunks there (n + 1: give up)
+#pragma omp parallel num_threads(threads)
+    {
+      if (omp_get_thread_num() == 0)
+        for (int i = 1; i < n; ++i) {
+          if (omp_get_num_threads() == 1) move(next.fetch_add(1));
+          err = cudaEventSynchronize(arrived[i]);
+          in_memory.store(err == cudaSuccess ? i + 1 : n + 1, std::memory_order_release);
+          if (err != cudaSuccess) break;
+        }
+      for (int i = next.fetch_add(1); i < n; i = next.fetch_add(1)) {
+        int there;
+        while ((there = in_memory.load(std::memory_order_acquire)) <= i) std::this_thread::yield();
+        if (there > n) break;
+        move(i);
       }
-      const size_t at = lo + static_cast<size_t>(i) * kChunk;
-      std::memcpy(out + at, g_stage.p + (k % kHalves) * kHalfBytes + (at - lo), std::min(kChunk, hi - at));
     }
-    if (failed) err = cudaErrorUnknown;
     if (err == cudaSuccess && k + kHalves < parts) err = enqueue(k + kHalves);
   }
   const cudaError_t sync = cudaStreamSynchronize(st);  // also before the block is given back after an error

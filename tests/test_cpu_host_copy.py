@@ -54,6 +54,14 @@ def test_two_devices_share_the_block(lib):
     assert _counts(lib)["events"] == 0
 
 
+def test_only_the_caller_calls_cuda(lib):
+    user = lib.test_user()
+    for _ in range(10):
+        _copy(lib, 9 * MB, dev=1)
+    assert _counts(lib)["foreign"] == 0
+    lib.test_user_gone(user)
+
+
 @pytest.mark.parametrize("fail", [0, 1, 7, 15, 16, 20, 40])
 def test_a_failed_wait_is_an_error(lib, fail):
     user = lib.test_user()
