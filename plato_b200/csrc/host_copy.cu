@@ -8,7 +8,9 @@
 // caller while later ones arrive.  The staging memory is one block per process
 // (kHalves * kHalfBytes, portable: every device's copies use it), used by one
 // call at a time; a call that finds it busy, a small result and a caller's
-// pinned buffer take the plain copy.  It is
+// pinned buffer take the plain copy.  Pinning the block costs 2-8 ms, as much as
+// staging saves on some 50 MB, so the first kBefore bytes go the plain way: a
+// program that takes one result from a graph does not pay for the block.  It is
 // freed with the last graph.
 //
 // The other host threads only move bytes.  Whatever they call of the CUDA
@@ -32,12 +34,14 @@ namespace {
 constexpr size_t kChunk = 256u << 10, kHalfBytes = 4u << 20, kHalves = 2;
 constexpr size_t kChunks = kHalfBytes / kChunk;
 constexpr size_t kSmall = 1u << 20;  // below, waking the threads costs more than they save
+constexpr size_t kBefore = 16u << 20;
 constexpr int kThreads = 8;
 constexpr int kDevices = 64;
 
 struct staging {
   std::mutex mu;  // held by the copy that uses the block
   unsigned char* p = nullptr;
+  size_t before = 0;  // bytes that went the plain way
   cudaEvent_t* done[kDevices] = {};  // [kHalves * kChunks] of a device
   void release() {
     for (cudaEvent_t*& d : done) {
@@ -48,11 +52,16 @@ struct staging {
     }
     if (p) cudaFreeHost(p);
     p = nullptr;
+    before = 0;
   }
-  // The events of device `dev`, or null: no block, take the plain copy.
-  cudaEvent_t* ready(int dev) {
+  // The events of device `dev`, or null: no block (yet), take the plain copy.
+  cudaEvent_t* ready(int dev, size_t bytes) {
     if (dev < 0 || dev >= kDevices) return nullptr;
     if (!p) {
+      if (before < kBefore) {
+        before += bytes;
+        return nullptr;
+      }
       if (cudaHostAlloc(reinterpret_cast<void**>(&p), kHalves * kHalfBytes, cudaHostAllocPortable) != cudaSuccess) {
         p = nullptr;
         cudaGetLastError();
@@ -120,7 +129,7 @@ int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   std::unique_lock<std::mutex> lock(g_stage.mu, std::try_to_lock);
   int dev = 0;
   PLATO_CUDA_TRY(cudaGetDevice(&dev));
-  cudaEvent_t* const done = lock.owns_lock() ? g_stage.ready(dev) : nullptr;
+  cudaEvent_t* const done = lock.owns_lock() ? g_stage.ready(dev, bytes) : nullptr;
   if (!done) {
     if (lock.owns_lock()) lock.unlock();
     return plain_copy(dst, src, bytes, st);

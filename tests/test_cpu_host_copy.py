@@ -43,6 +43,26 @@ def _copy(lib, n, dev=0, fail=-1):
     return rc
 
 
+def test_the_blocks_life(lib):
+    user = lib.test_user()
+    before = _counts(lib)
+    for _ in range(4):  # 16 MB go the plain way: one result of a graph does not pay for the block
+        _copy(lib, 4 * MB)
+    assert _counts(lib) == before
+    _copy(lib, MB - 1)  # small: always plain
+    assert _counts(lib) == before
+    for n in (MB, 4 * MB, 4 * MB + 1, 8 * MB, 9 * MB + 12345, 21 * MB + 4):
+        _copy(lib, n)
+    c = _counts(lib)
+    assert c["allocs"] == before["allocs"] + 1 and c["staged"] > 0
+    other = lib.test_user()
+    lib.test_user_gone(user)
+    assert _counts(lib)["frees"] == before["frees"]
+    lib.test_user_gone(other)
+    c = _counts(lib)
+    assert c["frees"] == c["allocs"] and c["events"] == 0
+
+
 def test_two_devices_share_the_block(lib):
     user = lib.test_user()
     start = _counts(lib)["allocs"]
