@@ -146,8 +146,19 @@ static __global__ void k_frontier_seed(frontier_view f, uint32_t v, const uint32
   frontier_flush(f, dsum);
 }
 
+// Members and chunks count in 32 bits each (counters[0]).  The chunk list alone
+// of a graph past that is 34 GB beside its 100 GB of offsets, degrees and ids.
+constexpr bool frontier_fits(uint64_t vertices, uint64_t edges) {
+  return vertices + edges / kPushChunk + 1 <= 0xFFFFFFFFull;
+}
+static_assert(frontier_fits(0xFFFFFFFEull, kPushChunk - 1) && !frontier_fits(0xFFFFFFFEull, kPushChunk) &&
+              frontier_fits(1, 0xFFFFFFFDull * kPushChunk) && !frontier_fits(1, 0xFFFFFFFEull * kPushChunk),
+              "up to 2^32 - 1 of each");
+
 inline int frontier_alloc(push_frontier& f, const plato_graph* g) {
   const uint32_t V = g->info.vertices;
+  if (!frontier_fits(V, g->stored_edges))
+    return set_error(PLATO_ENOMEM, "push frontier: more than 2^32 - 1 chunks of out-edges");
   f.V = V;
   PLATO_TRY(f.bits.alloc((V + 31) / 32));
   PLATO_TRY(f.queue.alloc(V));
