@@ -220,7 +220,25 @@ __device__ __forceinline__ void flat_store_if(uint32_t on, float* p, float v) {
   asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.global.f32 [%1], %2; }" ::"r"(on), "l"(p), "f"(v)
                : "memory");
 }
+
+// An addition of its own, not one that the compiler keeps from an earlier use.
+__device__ __forceinline__ float flat_add(float a, float b) {
+  float c;
+  asm("add.f32 %0, %1, %2;" : "=f"(c) : "f"(a), "f"(b));
+  return c;
+}
+
 // One warp's walk over the steps of piece p.
+//
+// Rounding.  A lane adds its edges in pairs, so a row of n edges meets about
+// n / 2 running sums; and the steps without an end, of which a hub row has
+// thousands, keep what each addition rounds away (a few large terms are common
+// there: a hub's own edge beside its leaves').  Largest relative error of a
+// rank, edges one by one / so / by the degree bins: RMAT s18 5.2 / 4.2 / 3.6e-7,
+// s24 4.9 / 4.2 / 3.8e-7, 18M uniform edges 4.4 / 3.9 / 3.3e-7; 64M edges into
+// one vertex with its own 64 among them 1.7e-6 / 6e-8 / 3.6e-7.  Both cost
+// nothing measurable: the second loop forms its pair sums again (flat_add), as
+// eight more registers across the scan spill (RMAT s22 133 -> 139 us).
 template <class Gather>
 __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const Gather& g) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -244,6 +262,7 @@ __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const
       !(pc.x & kPieceFirst) && !(__ldg(g.marks + static_cast<size_t>(s0) * 32 - 1) & (1u << (N - 1)));
   const uint32_t j0 = open ? base : 0xffffffffu;  // the segment that began in an earlier piece
   float acc = 0.f;       // this lane's part of the open segment, from steps without an end
+  float lost = 0.f;      // and what its additions have rounded away
   float carry = 0.f;     // the open segment's sum before those, the same in every lane
   for (uint32_t s = s0; s < s1; ++s) {
     float v[N];
@@ -259,16 +278,20 @@ __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const
     const uint32_t fl = mark & kEnds;
     const unsigned ends = __ballot_sync(kAll, fl != 0);
     if (ends == 0) {
+      float a = 0.f;
 #pragma unroll
       for (int i = 0; i < N; i += 8)
-        acc += ((v[i] + v[i + 1]) + (v[i + 2] + v[i + 3])) + ((v[i + 4] + v[i + 5]) + (v[i + 6] + v[i + 7]));
+        a += ((v[i] + v[i + 1]) + (v[i + 2] + v[i + 3])) + ((v[i + 4] + v[i + 5]) + (v[i + 6] + v[i + 7]));
+      const float b = acc + a, d = b - acc;  // the sum, and its exact error (Knuth's two-sum)
+      lost += (acc - (b - d)) + (a - d);
+      acc = b;
     } else {
       // this lane's sum after its last segment end, joined over the lanes
       float t = 0.f;
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        t += v[i];
-        t = (fl >> i) & 1u ? 0.f : t;
+      for (int i = 0; i < N; i += 2) {
+        t = (fl >> i) & 1u ? v[i + 1] : t + (v[i] + v[i + 1]);
+        t = (fl >> (i + 1)) & 1u ? 0.f : t;
       }
       const unsigned le = ends & (kAll >> (31 - lane));
       const int lo = le ? 31 - __clz(le) : 0;
@@ -277,8 +300,8 @@ __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const
         const float o = __shfl_up_sync(kAll, t, d);
         if (static_cast<int>(lane) - d >= lo) t += o;
       }
-      carry += warp_sum(acc);
-      acc = 0.f;
+      carry += warp_sum(acc + lost);
+      acc = lost = 0.f;
       float run = __shfl_up_sync(kAll, t, 1);
       if (lane == 0) run = 0.f;
       if (!(ends & below)) run += carry;
@@ -289,24 +312,26 @@ __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const
       if (ord == j0 && fl) {
         // its first end closes a segment of an earlier piece
         const int e = __ffs(fl) - 1;
-        float h = run;
+        float h = 0.f;
 #pragma unroll
-        for (int i = 0; i < N; ++i) h += i <= e ? v[i] : 0.f;
-        f.head[p] = h;
+        for (int i = 0; i < N; i += 2) h += (i <= e ? v[i] : 0.f) + (i < e ? v[i + 1] : 0.f);
+        f.head[p] = run + h;
       }
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        run += v[i];
-        const uint32_t on = fl & (1u << i);
-        flat_store_if(on, to, run);
-        to += on ? 1 : 0;
-        run = on ? 0.f : run;
+      for (int i = 0; i < N; i += 2) {
+        const uint32_t on0 = fl & (1u << i), on1 = fl & (2u << i);
+        flat_store_if(on0, to, run + v[i]);
+        to += on0 ? 1 : 0;
+        run = on0 ? v[i + 1] : run + flat_add(v[i], v[i + 1]);
+        flat_store_if(on1, to, run);
+        to += on1 ? 1 : 0;
+        run = on1 ? 0.f : run;
       }
     }
     mark = mark_n;
     base = base_n;
   }
-  acc = warp_sum(acc);
+  acc = warp_sum(acc + lost);
   if (lane == 0) f.carry[p] = carry + acc;
 }
 
@@ -407,18 +432,18 @@ __device__ __forceinline__ float flat_wide_segment(const flat_view& f, const uin
       for (int i = 0; i < 4; ++i) t[i] = p + i < sp.y ? __ldcg(f.carry + p + i) : 0.f;
       y += (t[0] + t[1]) + (t[2] + t[3]);
     }
-  for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+  for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {  // in 64 bits: up to 28K pieces
     const int l = __ffs(todo) - 1;
     const uint32_t p0 = __shfl_sync(0xffffffffu, sp.x, l), p1 = __shfl_sync(0xffffffffu, sp.y, l);
-    float a = 0.f;
+    double a = 0.0;
     for (uint32_t p = p0 + lane; p < p1; p += 256) {
       float t[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) t[i] = p + 32 * i < p1 ? __ldcg(f.carry + p + 32 * i) : 0.f;
-      a += ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+      a += static_cast<double>(((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7])));
     }
     a = warp_sum(a);
-    if (lane == static_cast<unsigned>(l)) y = a;
+    if (lane == static_cast<unsigned>(l)) y = static_cast<float>(a);
   }
   return y + h;
 }
@@ -474,7 +499,7 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
   constexpr int R = 2;
   __shared__ double s_red[32];
   __shared__ bool s_last;
-  __shared__ float s_wide[8][32];
+  __shared__ double s_wide[8][32];
   flat_after();
   if (upd.skip()) return;
   const unsigned lane = threadIdx.x & 31;
@@ -484,18 +509,18 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
   uint32_t w = f.words;
   if (blockIdx.x < f.wide_words) {
     const uint32_t warp = threadIdx.x >> 5;
-    float y = 0.f;
+    double y = 0.0;
     for (uint32_t k = warp; k <= f.nb; k += 8)
       if (k == 0 || k == f.nb || blockIdx.x < f.words1)
         y += flat_wide_segment(f, __ldg(f.meta + flat_place(k, f.words, f.words1) + blockIdx.x), lane);
     s_wide[warp][lane] = y;
     __syncthreads();
     if (warp == 0) {
-      y = 0.f;
+      y = 0.0;
 #pragma unroll
       for (int i = 0; i < 8; ++i) y += s_wide[i][lane];
       const uint32_t v = blockIdx.x * 32 + lane;
-      if (v < f.V) dl = upd.apply(v, y, upd.load(v));
+      if (v < f.V) dl = upd.apply(v, static_cast<float>(y), upd.load(v));
     }
   } else {
     w = f.wide_words + (((blockIdx.x - f.wide_words) * blockDim.x + threadIdx.x) >> 5);

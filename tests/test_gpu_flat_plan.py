@@ -273,3 +273,25 @@ def test_streams_follow_the_rows_that_take_part(V, E, long_row, kernels):
     assert hit == kernels
     assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
     np.testing.assert_array_equal(got, again)
+
+
+@pytest.mark.parametrize("E", [64000000, 3000000])
+def test_small_terms_beside_large_ones(E):
+    """Every edge ends in vertex 1, its own among them: a few terms near 0.008
+    among millions near 1e-9, which a running 32-bit sum would round away one
+    by one.  The oracle's bar (1e-6) on every rank, relatively."""
+    import torch
+
+    V = 1000003
+    rng = np.random.default_rng(E)
+    s, d = rng.integers(0, V, E, dtype=np.uint32), np.ones(E, np.uint32)
+    deg = np.maximum(np.bincount(s, minlength=V), 1)
+    src, out = torch.as_tensor(s.astype(np.int64)), torch.as_tensor(deg.astype(np.float64))
+    x = 1.0 / V / out
+    for _ in range(4):
+        r = torch.full((V,), 0.15 / V, dtype=torch.float64)
+        r[1] += 0.85 * x[src].sum()
+        x = r / out
+    with pb.Graph(V, s, d, True) as g:
+        got, _ = g.pagerank(4, 0.85, 0.0)
+    np.testing.assert_allclose(got, r.numpy(), rtol=1e-6, atol=0)
