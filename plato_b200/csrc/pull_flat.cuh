@@ -227,6 +227,9 @@ __device__ __forceinline__ float flat_add(float a, float b) {
   asm("add.f32 %0, %1, %2;" : "=f"(c) : "f"(a), "f"(b));
   return c;
 }
+// A sum and what its additions rounded away, which is no number once the sum
+// is infinite.
+__device__ __forceinline__ float flat_mend(float sum, float lost) { return lost == lost ? sum + lost : sum; }
 
 // One warp's walk over the steps of piece p.
 //
@@ -300,7 +303,7 @@ __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const
         const float o = __shfl_up_sync(kAll, t, d);
         if (static_cast<int>(lane) - d >= lo) t += o;
       }
-      carry += warp_sum(acc + lost);
+      carry += warp_sum(flat_mend(acc, lost));
       acc = lost = 0.f;
       float run = __shfl_up_sync(kAll, t, 1);
       if (lane == 0) run = 0.f;
@@ -331,7 +334,7 @@ __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const
     mark = mark_n;
     base = base_n;
   }
-  acc = warp_sum(acc + lost);
+  acc = warp_sum(flat_mend(acc, lost));
   if (lane == 0) f.carry[p] = carry + acc;
 }
 

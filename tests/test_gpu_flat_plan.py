@@ -295,3 +295,25 @@ def test_small_terms_beside_large_ones(E):
     with pb.Graph(V, s, d, True) as g:
         got, _ = g.pagerank(4, 0.85, 0.0)
     np.testing.assert_allclose(got, r.numpy(), rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("V,E,share", [(900, 60000, 0.9), (100003, 3000000, 0.9), (300001, 12000000, 0.8),
+                                       (100003, 12000000, 0.5)])
+def test_infinite_terms_make_infinite_rows(V, E, share):
+    """Weights so small that 1 / their sum is infinite: a target's rank is
+    infinite, not NaN, whether its row ends in a step or crosses thousands; as
+    by the merge path."""
+    rng = np.random.default_rng(E)
+    s = rng.integers(0, V, E, dtype=np.uint32)
+    d = rng.integers(0, V, E, dtype=np.uint32)
+    d[rng.random(E) < share] = 1
+    w = np.ones(E)
+    w[s == 3] = 1e-42
+    hit = np.zeros(V, bool)
+    hit[d[s == 3]] = True
+    assert hit[1]
+    for relabel in (False, True):
+        with pb.Graph(V, s, d, True, relabel=relabel, weights=w) as g:
+            got, _ = g.weighted_pagerank(1, 0.85, 0.0)
+        np.testing.assert_array_equal(np.isposinf(got), hit)
+        assert np.isfinite(got[~hit]).all()
