@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import plato_b200 as pb
-from oracle import RefGraph
+from oracle import RefGraph, fp64
 from plato_b200 import _lib
 
 pytestmark = pytest.mark.gpu
@@ -317,3 +317,59 @@ def test_infinite_terms_make_infinite_rows(V, E, share):
             got, _ = g.weighted_pagerank(1, 0.85, 0.0)
         np.testing.assert_array_equal(np.isposinf(got), hit)
         assert np.isfinite(got[~hit]).all()
+
+
+def _weighted_graph(kind):
+    if kind == "hot and cold":
+        V, s, d = pb.rmat(20, 12, 7)
+    else:
+        V, s, d = _uniform(1000003, 9000000)
+    return V, s, d, np.random.default_rng(5).uniform(0.1, 10, s.size)
+
+
+@pytest.mark.parametrize("kind,kernels", [("hot and cold", HOT), ("cold", COLD)])
+@pytest.mark.parametrize("early", [False, True])
+def test_weights_of_the_cold_stream(kind, kernels, early):
+    """Weighted epochs above one launch, with a cold stream: 32-bit ids, their
+    weights and padding."""
+    V, s, d, w = _weighted_graph(kind)
+    eps = 1e-6 * V if early else 0.0
+    want, epochs, _ = fp64.weighted_pagerank(V, s, d, w, True, 80 if early else 12, 0.85, eps)
+    with pb.Graph(V, s, d, True, weights=w) as g:
+        hit, (got, st) = _launched(lambda: g.weighted_pagerank(80 if early else 12, 0.85, eps), KERNELS)
+        again, _ = g.weighted_pagerank(80 if early else 12, 0.85, eps)
+    assert hit == kernels
+    assert abs(st.iterations - epochs) <= (1 if early else 0)
+    assert np.abs(got - want).sum() / V <= 1e-6
+    np.testing.assert_array_equal(got, again)
+
+
+@pytest.mark.parametrize("kind", ["hot and cold", "cold"])
+def test_not_a_number_beside_cold_edges(kind):
+    """A vertex whose out-weights are all 0 gathers as inf, its targets become
+    NaN in the first epoch, no other row does."""
+    V, s, d, w = _weighted_graph(kind)
+    v = int(s[s.size // 2])
+    w[s == v] = 0.0
+    hit = np.zeros(V, bool)
+    hit[d[s == v]] = True
+    with pb.Graph(V, s, d, True, weights=w) as g:
+        got, _ = g.weighted_pagerank(1, 0.85, 0.0)
+    np.testing.assert_array_equal(np.isnan(got), hit)
+
+
+@pytest.mark.parametrize("scale,ef,kernels", [(10, 24, RUN), (18, 24, COLD), (19, 24, HOT)])
+@pytest.mark.parametrize("eps", [0.0, 1e-6])
+def test_seed_sets(scale, ef, kernels, eps):
+    """Seed-set queries through each form of the flat pull."""
+    V, s, d = pb.rmat(scale, ef, 8)
+    ref = RefGraph(V, s, d, True)
+    seeds = np.random.default_rng(scale).choice(V, 17, replace=False).astype(np.uint32)
+    iteration = 100 if eps else 20
+    want, epochs, delta = ref.seedset_ppr(seeds, iteration, 0.85, eps)
+    with pb.Graph(V, s, d, True) as g:
+        hit, (got, st) = _launched(lambda: g.seedset_ppr(seeds, iteration, 0.85, eps), KERNELS)
+    assert hit == kernels
+    assert abs(st.iterations - epochs) <= (1 if eps else 0)
+    # the bar, and one epoch that moves less than eps where one side ends earlier
+    assert np.abs(got.astype(np.float64) - want).sum() <= 1e-6 + eps
