@@ -34,9 +34,12 @@ namespace {
 // instead of 288.
 constexpr uint32_t kFlatRowDeg0 = 8;
 constexpr uint32_t kFlatRowDeg1 = 64;
-// Up to this many edges all epochs run in one launch (k_flat_run; epoch with
-// one / three launches: RMAT s16 9.3 / 14.2 us, s17 12.8 / 15.6, s18 21.1 /
-// 19.4; 3.2M uniform edges 19.2 / 25.6).
+// Up to this many edges all epochs run in one launch (k_flat_run).  The line lies
+// between graphs with hubs, whose separate kernels gather from a larger L1, and
+// graphs without (epoch in one launch / in separate ones: RMAT s16 1.0M edges 9.0
+// / 10.0 us, s17 1.9M 12.2 / 12.7, s18 2.0M 13.3 / 12.8, 2.5M 16.4 / 13.3, 3.9M
+// 21.5 / 15.6; uniform over 200K rows 2M 14.3 / 15.3, 3M 17.8 / 18.8, 4M 21.0 /
+// 22.1, over 500K 3M 23.2 / 22.4).
 constexpr uint64_t kFlatRunEdges = 3500000;
 // ... and rows: its warps also update every 32-row word (uniform edges, 0.1 a row:
 // 4M rows 21.5 / 30.1, 8M 56.8 / 51.7, 16M 118 / 98).
@@ -656,7 +659,7 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   PLATO_TRY(put(d_cta, cta_sub, st));
   flat_view& f = pl.v;
   f = flat_view{};
-  f.V = f.nsrc = V;
+  f.V = V;
   f.nb = nb;
   f.words = words;
   f.words1 = words1;

@@ -64,7 +64,7 @@ struct flat_sub {
 };
 
 struct flat_view {
-  uint32_t V, nsrc, nb, words;      // words = ceil(V / 32)
+  uint32_t V, nb, words;            // words = ceil(V / 32)
   uint32_t words1;                  // 32-row words that take part in the hot streams after the first
   uint32_t wide_words;              // the first words, which hold every segment across more than kFlatWideSpan pieces
   uint32_t cold_piece0, cold_pieces;
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_hot(flat_view f,
   for (uint32_t sub = f.cta_sub[blockIdx.x]; sub < sub1; ++sub) {
     const flat_sub sb = f.subs[sub];
     const uint32_t src0 = sb.block * kFlatBlock;
-    const uint32_t n = min(kFlatBlock, f.nsrc - src0), n4 = n / 4;
+    const uint32_t n = min(kFlatBlock, f.V - src0), n4 = n / 4;
     __syncthreads();
     const float4* x4 = reinterpret_cast<const float4*>(x + src0);
 #pragma unroll 4
