@@ -239,9 +239,11 @@ __device__ __forceinline__ float flat_mend(float sum, float lost) { return lost 
 // there: a hub's own edge beside its leaves').  Largest relative error of a
 // rank, edges one by one / so / by the degree bins: RMAT s18 5.2 / 4.2 / 3.6e-7,
 // s24 4.9 / 4.2 / 3.8e-7, 18M uniform edges 4.4 / 3.9 / 3.3e-7; 64M edges into
-// one vertex with its own 64 among them 1.7e-6 / 6e-8 / 3.6e-7.  Both cost
-// nothing measurable: the second loop forms its pair sums again (flat_add), as
-// eight more registers across the scan spill (RMAT s22 133 -> 139 us).
+// one vertex with its own 64 among them 1.7e-6 / 6e-8 / 3.6e-7.  Epoch one by
+// one / so: RMAT s16 8.9 / 8.6 us, s20 44.3 / 45.1, s22 133.8 / 133.8, 64M uniform
+// edges over 1M vertices 135 / 132, RMAT s21 with weights 105 / 106.  A hot step's
+// second loop forms its pair sums again (flat_add): kept across the scan, eight
+// more registers spill (s22 139 us); a cold step's four do not.
 template <class Gather>
 __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const Gather& g) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -325,7 +327,7 @@ __device__ __forceinline__ void flat_piece(const flat_view& f, uint32_t p, const
         const uint32_t on0 = fl & (1u << i), on1 = fl & (2u << i);
         flat_store_if(on0, to, run + v[i]);
         to += on0 ? 1 : 0;
-        run = on0 ? v[i + 1] : run + flat_add(v[i], v[i + 1]);
+        run = on0 ? v[i + 1] : run + (N == 8 ? v[i] + v[i + 1] : flat_add(v[i], v[i + 1]));
         flat_store_if(on1, to, run);
         to += on1 ? 1 : 0;
         run = on1 ? 0.f : run;
