@@ -46,8 +46,7 @@ def _copy(lib, n, dev=0, fail=-1):
 def test_the_blocks_life(lib):
     user = lib.test_user()
     before = _counts(lib)
-    for _ in range(4):  # 16 MB go the plain way: one result of a graph does not pay for the block
-        _copy(lib, 4 * MB)
+    _copy(lib, 4 * MB)  # goes the plain way: one result of a graph does not pay for the block
     assert _counts(lib) == before
     _copy(lib, MB - 1)  # small: always plain
     assert _counts(lib) == before
@@ -85,8 +84,7 @@ def test_only_the_caller_calls_cuda(lib):
 @pytest.mark.parametrize("fail", [0, 1, 7, 15, 16, 20, 40])
 def test_a_failed_wait_is_an_error(lib, fail):
     user = lib.test_user()
-    for _ in range(4):
-        _copy(lib, 4 * MB)
+    _copy(lib, 4 * MB)
     assert _copy(lib, 10 * MB, fail=fail) == (3 if fail < 40 else 0)  # PLATO_ECUDA; 10 MB have 40 chunks
     _copy(lib, 10 * MB)  # the block is usable again
     lib.test_user_gone(user)
