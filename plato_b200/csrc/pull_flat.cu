@@ -21,14 +21,14 @@ namespace {
 // counted over the rows that take part.  A further block is used where that is
 // kFlatMore edges and one more for each such row: its copies and segments cost
 // something too (us an epoch with 1 / 4 / 10 / 16 / 24 blocks, and how many are
-// chosen: RMAT s21 84.9 / 72.8 / 74.8 / 76.8 / 83.4, 4; s22 168 / 142 / 134 / 133
-// / 138, 10; s23 342 / 290 / 260 / 251 / 251, 15; s24 with 10 / 16 / 20 / 22 / 24
+// chosen: RMAT s21 84.9 / 72.8 / 74.8 / 76.8 / 83.4, 7; s22 168 / 142 / 134 / 133
+// / 138, 11; s23 342 / 290 / 260 / 251 / 251, 16; s24 with 10 / 16 / 20 / 22 / 24
 // 537 / 521 / 503 / 497 / 507, 22; s22 with 6 edges a vertex 85.7 / 76.9 / 80.8 /
 // 81.1 / 87.3, 5).  There are hot streams where all of them together hold
 // kFlatFirst: below, one more launch costs what the gathers save (edges that
 // would be hot, epoch without / with them: RMAT s19 6.5M 26.4 / 27.5, s20 with 10
-// a vertex 8.0M 38.2 / 38.0, s19 with 20 8.6M 31.6 / 33.1, s21 with 6 8.9M 57.5 /
-// 48.1, s20 13.6M 51.0 / 45.6).  A count that took
+// a vertex 8.3M 36.1 / 37.7, s19 with 20 8.6M 31.6 / 33.1, s21 with 6 8.9M 57.5 /
+// 48.1, s20 13.9M 51.0 / 45.3).  A count that took
 // in the rows below the limits gave uniform edges with one long row streams that
 // were all but empty: 16M over 1M vertices 162 us instead of 80, 64M over 4M 378
 // instead of 288.
@@ -44,7 +44,7 @@ constexpr uint64_t kFlatRunEdges = 3500000;
 // ... and rows: its warps also update every 32-row word (uniform edges, 0.1 a row:
 // 4M rows 21.5 / 30.1, 8M 56.8 / 51.7, 16M 118 / 98).
 constexpr uint32_t kFlatRunRows = 6000000;
-constexpr unsigned long long kFlatFirst = 8000000, kFlatMore = 400000;
+constexpr unsigned long long kFlatFirst = 8500000, kFlatMore = 250000;
 // Where the blocks cover all sources, every row can take part in every stream
 // and no cold pass is left.  That pays from 1.5 edges a segment, unless block 0
 // has most of the gathers, which then come from L1 anyway (without / with it:
