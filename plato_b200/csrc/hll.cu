@@ -366,7 +366,16 @@ __device__ __forceinline__ void row_done(const gather_args& a, uint32_t v, int t
 // RMAT s16 symmetrised 14.3 / 2.6 / 0.91 / 8.6 -> 1.1 / 0.73 / 0.77 / 6.3 ms, on
 // s20 15.1 / 4.4 / 7.1 / 102 -> 4.7 / 3.0 / 5.9 / 76, P = 6 on s22 10.0 -> 9.8
 // (and with three-way maxima, max_odd, P = 6 on s20 2.65, on s22 9.5).
-template <int T, int VEC>
+//
+// kLong = false (rows up to 512 bytes): no row has more than team_deg sources.
+// The rows alone, and each warp's first chunks by its number: three cursors that
+// every warp asks in vain cost such an epoch more than they balance (hyperanf of
+// 8 epochs, with them / without: a ring of 20K vertices at P = 4 / 6 / 9 0.95 / 0.76,
+// 0.56 / 0.47, 0.66 / 0.56 ms, 300K uniform edges over 30K at P = 4 0.99 / 0.77, a
+// grid of 250K at P = 6 0.97 / 0.89).  By number go at most 8 chunks a warp of
+// wide teams and 1 or 2 of narrow ones, the rest dynamically: 1M sparse rows at
+// P = 4 all by number take 1.5 ms instead of 0.93.
+template <int T, int VEC, bool kLong>
 __global__ void __launch_bounds__(kHllThreads, VEC <= 2 ? 4 : 3) k_hll_rows(gather_args a) {
   constexpr int SLICE = T * VEC * 16;
   constexpr int kWarps = kHllThreads / 32;
@@ -382,53 +391,55 @@ __global__ void __launch_bounds__(kHllThreads, VEC <= 2 ? 4 : 3) k_hll_rows(gath
   const int tb = lane - tl;
   const unsigned tmask = T == 32 ? kAll : (((1u << T) - 1u) << tb);
   unsigned long long n_chg = 0, deg_chg = 0;
-  for (;;) {  // hubs
-    if (threadIdx.x == 0) s_next = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 2), 1u);
-    __syncthreads();
-    const uint32_t h = s_next;
-    __syncthreads();
-    if (h >= a.n_hubs) break;
-    const uint32_t v = a.hubs[h];
-    if (a.covered && !test_bit(a.covered, v)) continue;
-    const uint64_t b = __ldg(a.off + v), e = __ldg(a.off + v + 1);
-    const bool stale = a.stale && test_bit(a.stale, v);
-    bool row_changed = false;
-    unsigned long long sfx = 0;
-    uint32_t zeros = 0;
-    for (uint32_t pass = 0; pass < a.passes; ++pass) {
-      const size_t col = static_cast<size_t>(pass) * SLICE + static_cast<size_t>(tl) * 16;
-      uint4 agg[VEC];
+  if constexpr (kLong) {
+    for (;;) {  // hubs
+      if (threadIdx.x == 0) s_next = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 2), 1u);
+      __syncthreads();
+      const uint32_t h = s_next;
+      __syncthreads();
+      if (h >= a.n_hubs) break;
+      const uint32_t v = a.hubs[h];
+      if (a.covered && !test_bit(a.covered, v)) continue;
+      const uint64_t b = __ldg(a.off + v), e = __ldg(a.off + v + 1);
+      const bool stale = a.stale && test_bit(a.stale, v);
+      bool row_changed = false;
+      unsigned long long sfx = 0;
+      uint32_t zeros = 0;
+      for (uint32_t pass = 0; pass < a.passes; ++pass) {
+        const size_t col = static_cast<size_t>(pass) * SLICE + static_cast<size_t>(tl) * 16;
+        uint4 agg[VEC];
 #pragma unroll
-      for (int q = 0; q < VEC; ++q) agg[q] = make_uint4(0u, 0u, 0u, 0u);
-      bool any = team_merge<T, VEC>(a, b + static_cast<uint64_t>(threadIdx.x / T) * kChunk, e,
-                                    static_cast<uint64_t>(kTeams) * kChunk, col, tl, tb, tmask, s_ids, agg);
+        for (int q = 0; q < VEC; ++q) agg[q] = make_uint4(0u, 0u, 0u, 0u);
+        bool any = team_merge<T, VEC>(a, b + static_cast<uint64_t>(threadIdx.x / T) * kChunk, e,
+                                      static_cast<uint64_t>(kTeams) * kChunk, col, tl, tb, tmask, s_ids, agg);
 #pragma unroll
-      for (int o = T; o < 32; o <<= 1)
+        for (int o = T; o < 32; o <<= 1)
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) agg[q] = vmax4(agg[q], shfl_xor4(kAll, agg[q], o));
-      if (lane < T) {
+          for (int q = 0; q < VEC; ++q) agg[q] = vmax4(agg[q], shfl_xor4(kAll, agg[q], o));
+        if (lane < T) {
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) part[warp][q * T + tl] = agg[q];
-      }
-      any = __syncthreads_or(any);
-      if (!any && !stale) break;  // block-uniform
-      if (warp == 0 && lane < T) {
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-          uint4 x = part[0][q * T + tl];
-#pragma unroll
-          for (int w = 1; w < kWarps; ++w) x = vmax4(x, part[w][q * T + tl]);
-          agg[q] = x;
+          for (int q = 0; q < VEC; ++q) part[warp][q * T + tl] = agg[q];
         }
-        uint4 own[VEC];
-        load_own<T, VEC>(a, v, col, own);
-        row_changed |= team_apply<T, VEC>(a, v, col, stale, tmask, own, agg, sfx, zeros);
+        any = __syncthreads_or(any);
+        if (!any && !stale) break;  // block-uniform
+        if (warp == 0 && lane < T) {
+#pragma unroll
+          for (int q = 0; q < VEC; ++q) {
+            uint4 x = part[0][q * T + tl];
+#pragma unroll
+            for (int w = 1; w < kWarps; ++w) x = vmax4(x, part[w][q * T + tl]);
+            agg[q] = x;
+          }
+          uint4 own[VEC];
+          load_own<T, VEC>(a, v, col, own);
+          row_changed |= team_apply<T, VEC>(a, v, col, stale, tmask, own, agg, sfx, zeros);
+        }
+        __syncthreads();  // part is rewritten by the next pass or row
       }
-      __syncthreads();  // part is rewritten by the next pass or row
+      if (warp == 0 && lane < T && row_changed) row_done<T>(a, v, tl, tmask, sfx, zeros, n_chg, deg_chg);
     }
-    if (warp == 0 && lane < T && row_changed) row_done<T>(a, v, tl, tmask, sfx, zeros, n_chg, deg_chg);
   }
-  if constexpr (T < 32) {
+  if constexpr (kLong && T < 32) {
     for (;;) {  // rows split over a warp's teams
       uint32_t i = 0;
       if (lane == 0) i = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 3), 1u);
@@ -465,10 +476,19 @@ __global__ void __launch_bounds__(kHllThreads, VEC <= 2 ? 4 : 3) k_hll_rows(gath
     }
   }
   const uint32_t nchunks = (a.V + kTPW - 1) / kTPW;
+  uint32_t mine = (blockIdx.x * kWarps + warp) * a.grab;  // first chunk (kLong = false)
   for (;;) {
     uint32_t c0 = 0;
-    if (lane == 0) c0 = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 4), a.grab);
-    c0 = __shfl_sync(kAll, c0, 0);
+    if constexpr (kLong) {
+      if (lane == 0) c0 = atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 4), a.grab);
+      c0 = __shfl_sync(kAll, c0, 0);
+    } else {
+      const uint32_t given = gridDim.x * kWarps * a.grab;
+      c0 = mine;
+      if (c0 == kNoVertex && lane == 0) c0 = given + atomicAdd(reinterpret_cast<unsigned int*>(a.counters + 4), a.grab);
+      c0 = __shfl_sync(kAll, c0, 0);
+      mine = given < nchunks ? kNoVertex : nchunks;
+    }
     if (c0 >= nchunks) break;
     const uint32_t c1 = min(nchunks, c0 + a.grab);
     uint64_t nb = 0, ne = 0;
@@ -1100,13 +1120,24 @@ class hll_engine {
     static int per_sm = 0;  // resident CTAs: the rows are taken dynamically
     if (per_sm == 0) {
       int n = 0;
-      PLATO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_hll_rows<T, VEC>, kHllThreads, 0));
+      PLATO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_hll_rows<T, VEC, true>, kHllThreads, 0));
       per_sm = std::max(n, 1);
     }
-    const uint32_t warps = 148u * per_sm * (kHllThreads / 32);
-    a.grab = std::min(8u, std::max(1u, V_ / (32 / T) / (8 * warps)));
+    constexpr uint32_t kWarps = kHllThreads / 32;
+    const uint32_t ctas = 148u * per_sm;
+    a.grab = std::min(8u, std::max(1u, V_ / (32 / T) / (8 * ctas * kWarps)));
     prof_scope ps("k_hll_rows", st_);
-    k_hll_rows<T, VEC><<<148u * per_sm, kHllThreads, 0, st_>>>(a);
+    const uint64_t chunks = (static_cast<uint64_t>(V_) + 32 / T - 1) / (32 / T);
+    if constexpr (VEC == 1) {
+      if (a.n_hubs + a.n_mids == 0 && (T < 32 || chunks <= 8ull * ctas * kWarps)) {
+        const uint64_t share = (chunks + ctas * kWarps - 1) / (ctas * kWarps);
+        a.grab = std::max(a.grab, static_cast<uint32_t>(std::min<uint64_t>(share, std::clamp(T / 2, 1, 8))));
+        k_hll_rows<T, VEC, false><<<grid_for(chunks, kWarps * a.grab, ctas), kHllThreads, 0, st_>>>(a);
+        PLATO_LAUNCHED("k_hll_rows");
+        return PLATO_OK;
+      }
+    }
+    k_hll_rows<T, VEC, true><<<ctas, kHllThreads, 0, st_>>>(a);
     PLATO_LAUNCHED("k_hll_rows");
     return PLATO_OK;
   }
