@@ -63,7 +63,10 @@ bool flat_all_hot(uint64_t rows, uint64_t edges, uint64_t first_block, uint32_t 
 //   vertices 4.7 / 4.4, 5.3 / 4.4, 12.0 / 10.1, 35.9 / 29.2 us, grids 5.1 / 4.4,
 //   5.7 / 4.9, 14.6 / 10.6, 46 / 32, 4 random in-edges a row 5.3 / 4.4, 6.7 / 6.5,
 //   25.5 / 22.6, 95 / 76; up to kFlatClusterSteps words one cluster runs all
-//   epochs (5K vertices 3.7-4.4 / 4.4);
+//   epochs (5K vertices 3.7-4.4 / 4.4).  With an early exit each of their epochs
+//   has its decision in a kernel of its own, and the one-launch epochs are the
+//   faster (30 epochs: grids of 90K / 250K / 1M vertices 220 / 318, 263 / 380, 443 /
+//   502 us): where there are such, the graph has both plans;
 //   rows up to 16 (two bins), uniform: 600K rows with 3.5 edges 19.9 / 20.9, 1M
 //   with 1.5 / 2.5 / 3.5 19.3 / 21.0, 26.1 / 23.0, 31.5 / 29.1, 4M with 0.5 / 1 /
 //   2.5 35.0 / 37.4, 51.0 / 42.2, 82.0 / 63.9, 8M with 0.1 / 1 51.7 / 45.0, 99 /
@@ -74,11 +77,18 @@ struct flat_census {
   uint64_t rows, few, some;      // all rows, rows of 1..4 and of 5..16 edges
   uint64_t edges, long_edges;    // all edges, those in rows above 16
 };
-bool flat_bins_suit(const flat_census& c) {
-  if (c.some == 0 && c.long_edges == 0) return c.rows > 32ull * kFlatClusterSteps;
-  if (c.rows > 10000000 && 2 * c.edges > 5 * c.rows) return false;
-  if (c.long_edges == 0) return (c.few + c.some >= 900000 && c.edges >= 2500000) || c.rows >= 6000000;
-  return 20 * c.long_edges <= c.edges && c.edges <= 6 * c.rows && c.few + c.some >= 2500000;
+enum class flat_use { always, early_exit, never };
+flat_use flat_suits(const flat_census& c, bool run) {
+  if (c.some == 0 && c.long_edges == 0)
+    return c.rows <= 32ull * kFlatClusterSteps ? flat_use::always : run ? flat_use::early_exit : flat_use::never;
+  bool bins;
+  if (c.rows > 10000000 && 2 * c.edges > 5 * c.rows)
+    bins = false;
+  else if (c.long_edges == 0)
+    bins = (c.few + c.some >= 900000 && c.edges >= 2500000) || c.rows >= 6000000;
+  else
+    bins = 20 * c.long_edges <= c.edges && c.edges <= 6 * c.rows && c.few + c.some >= 2500000;
+  return bins ? flat_use::never : flat_use::always;
 }
 
 // out[0]: one past the last row above kFlatRowDeg1 edges, out[1]: how many there
@@ -444,7 +454,9 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   unsigned long long h[kFlatSurvey + kFlatMaxBlocks];
   PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  if (flat_bins_suit(flat_census{V, h[2], h[3], E, h[4]})) return PLATO_OK;
+  const flat_use use = flat_suits(flat_census{V, h[2], h[3], E, h[4]}, run);
+  if (use == flat_use::never) return PLATO_OK;
+  pl.early_only = use == flat_use::early_exit;
   flat_rows rows{off, g->in_adj.p, V, 0, 0, kFlatRowDeg0, kFlatRowDeg1};
   uint32_t nb = 0;
   const bool all_hot = !run && flat_all_hot(V, E, h[5], nblocks);

@@ -99,6 +99,7 @@ __host__ __device__ inline uint64_t flat_place(uint32_t k, uint64_t rows, uint64
 
 struct flat_plan {
   bool valid = false;
+  bool early_only = false;               // epochs without an early exit are the bins'
   uint32_t hot_ctas = 0, cold_blocks = 0, update_blocks = 0;
   uint32_t run_ctas = 0, run_warps = 0;  // not 0: k_flat_run's grid, the plan's only kernel
   bool run_cluster = false;              // its CTAs are one cluster

@@ -294,7 +294,7 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
     // It keeps its path when memory comes free: the paths sum in different
     // orders, and a graph's ranks are the same from call to call.
     PLATO_TRY(plan_or_none(ws->flat, [&] { return build_flat_plan(g, ws->flat, st); }));
-    if (!ws->flat.valid) PLATO_TRY(plan_or_none(ws->plan, [&] { return build_plan(g, ws->plan, st); }));
+    if (!ws->flat.valid || ws->flat.early_only) PLATO_TRY(plan_or_none(ws->plan, [&] { return build_plan(g, ws->plan, st); }));
     g->plan_bytes = ws->flat.mem.bytes() + ws->plan.bytes();
     ws->plan_built = true;
   }
@@ -440,6 +440,11 @@ int pull_rows_with(plato_graph* g, const float* x, const Upd& upd, const float* 
   return PLATO_OK;
 }
 
+// The plan of a call's pull epochs: with `early` they end in decisions.
+bool flat_pulls(const rank_workspace* ws, bool early) {
+  return ws->flat.valid && (early || !ws->flat.early_only || !ws->plan.valid);
+}
+
 // One pull epoch of a whole graph: its flat plan, else pull_rows_with.  With
 // c.ctrl the epoch also ends in its decision (epoch_decide), which upd.mode
 // reads.
@@ -447,7 +452,8 @@ template <class Upd, bool kW>
 int pull_epoch_with(plato_graph* g, const float* x, const Upd& upd, const float* w, cudaStream_t st,
                     const flat_control& c = flat_control{}) {
   rank_workspace* ws = g->rank_ws;
-  if (ws->flat.valid) return launch_flat_epoch<Upd, kW>(ws->flat, x, upd, ws->partials.p, c, st);
+  if (flat_pulls(ws, c.ctrl != nullptr))
+    return launch_flat_epoch<Upd, kW>(ws->flat, x, upd, ws->partials.p, c, st);
   PLATO_TRY((pull_rows_with<Upd, kW>(g, x, upd, w, st)));
   if (c.ctrl) {
     k_epoch_control<<<1, 1024, 0, st>>>(ws->partials.p, static_cast<uint32_t>(partial_count(g)), c.ctrl, c.delta,
@@ -514,7 +520,7 @@ int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteratio
   using Upd = decltype(make(0, false, nullptr));
   *ran = 0;
   if (start >= iteration) return PLATO_OK;
-  if (ws->flat.run_ctas) {
+  if (ws->flat.run_ctas && flat_pulls(ws, !(eps <= 0.0))) {
     PLATO_TRY((run_flat_epochs<Upd, kW>(g, make(*cur, false, nullptr), iteration, start, eps, scale, st, ran, delta)));
     *cur = (*cur + static_cast<int>(*ran)) & 1;
     return PLATO_OK;

@@ -225,7 +225,7 @@ RUN, COLD = {"k_flat_run"}, {"k_flat_cold", "k_flat_update"}
 
 
 @pytest.mark.parametrize("graph,kernels", [
-    (_ring(8192), RUN), (_ring(8193), ONE), (_ring(100003), ONE), (_capped(8193, 4), ONE), (_capped(8193, 5), RUN),
+    (_ring(8192), RUN), (_ring(8193), ONE), (_ring(100003), ONE), (_capped(8193, 4), ONE), (_capped(8193, 5), RUN), (_capped(900001, 4), ONE),
     (_uniform(1000003, 1000), ONE), (_uniform(1000003, 500000), RUN), (_uniform(1000003, 1500000), RUN),
     (_uniform(1000003, 2600000), TWO), (_capped(500001, 8), COLD), (_capped(900002, 5), {"k_pull_rows4"} | ONE),
     (_uniform(1000003, 6000000), COLD), (_uniform(6000001, 600000), None), (_uniform(4000037, 20000000), None),
@@ -238,7 +238,9 @@ def test_short_rows_take_the_bins(graph, kernels):
     want, _, _ = RefGraph(V, s, d, True).pagerank(5, 0.85, 0.0)
     with pb.Graph(V, s, d, True) as g:
         hit, (got, st) = _launched(lambda: g.pagerank(5, 0.85, 0.0), KERNELS)
-        again, early = g.pagerank(50, 0.85, 1e-2 * V)
+        exits, (again, early) = _launched(lambda: g.pagerank(50, 0.85, 1e-2 * V), KERNELS)
+    if kernels == ONE:  # decisions in one launch beat a kernel for each
+        assert exits == (RUN if s.size <= 3500000 and V <= 6000000 else ONE)
     with pb.Graph(V, s, d, True, relabel=False) as g:
         plain, (general, _) = _launched(lambda: g.pagerank(5, 0.85, 0.0), KERNELS)
         late, same = g.pagerank(50, 0.85, 1e-2 * V)
