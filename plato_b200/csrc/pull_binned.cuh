@@ -368,8 +368,8 @@ __global__ void __launch_bounds__(256) k_pull_short(pull_plan_view pv, const uin
 // brings the delta to the reference's units.
 static __global__ void __launch_bounds__(1024) k_epoch_control(const double* __restrict__ partials,
                                                                uint32_t n, int* ctrl, double* delta,
-                                                               double scale, double eps,
-                                                               uint32_t iteration) {
+                                                               double scale, double eps, uint32_t iteration,
+                                                               unsigned long long* seen = nullptr) {
   __shared__ double s_red[32];
   if (ctrl[0] == 2) return;  // block-uniform
   const uint32_t per = (n + 1023) / 1024;
@@ -377,7 +377,7 @@ static __global__ void __launch_bounds__(1024) k_epoch_control(const double* __r
   double s = 0.0;
   for (uint32_t i = b; i < e; ++i) s += partials[i];
   s = block_sum<1024>(s, s_red);
-  if (threadIdx.x == 0) epoch_decide(ctrl, delta, s * scale, eps, iteration);
+  if (threadIdx.x == 0) epoch_decide(ctrl, delta, s * scale, eps, iteration, seen);
 }
 
 }  // namespace plato_b200

@@ -497,6 +497,7 @@ struct flat_control {
   double scale, eps;
   uint32_t iteration;
   uint32_t polls;  // of a grid barrier of k_flat_run, before it gives up
+  unsigned long long* seen = nullptr;  // the decision on the host, as it falls (epoch_decide)
 };
 
 template <class Update>
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(256, 4) k_flat_update(flat_view f, Update upd,
   t = block_sum<256>(t, s_red);
   if (threadIdx.x == 0) {
     c.ctrl[2] = 0;
-    epoch_decide(c.ctrl, c.delta, t * c.scale, c.eps, c.iteration);
+    epoch_decide(c.ctrl, c.delta, t * c.scale, c.eps, c.iteration, c.seen);
   }
 }
 

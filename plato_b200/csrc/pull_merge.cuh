@@ -42,17 +42,21 @@ struct teleport_seeds {  // trustrank.hpp:226-245: (seed ? (1-d)/|S| : 0)
 
 // The eps early exit of pagerank.hpp:137-139 after an epoch whose delta is
 // `delta`: ctrl[0] = mode of the next epoch (0 normal, 1 final, 2 done),
-// ctrl[1] = epochs run, *last_delta = delta of the last non-final epoch.
+// ctrl[1] = epochs run, *last_delta = delta of the last non-final epoch.  `seen`
+// (or null): host memory that gets both, epochs << 32 | mode, in one store.
 __device__ __forceinline__ void epoch_decide(int* ctrl, double* last_delta, double delta, double eps,
-                                             uint32_t iteration) {
+                                             uint32_t iteration, unsigned long long* seen = nullptr) {
   const int mode = ctrl[0], ran = ctrl[1] + 1;
-  ctrl[1] = ran;
-  if (mode == 1) {
-    ctrl[0] = 2;
-    return;
+  int next = mode == 1 ? 2 : 0;
+  if (mode != 1) {
+    *last_delta = delta;
+    if ((eps > 0.0 && delta < eps) || static_cast<uint32_t>(ran) >= iteration - 1) next = 1;
   }
-  *last_delta = delta;
-  if ((eps > 0.0 && delta < eps) || static_cast<uint32_t>(ran) >= iteration - 1) ctrl[0] = 1;
+  ctrl[1] = ran;
+  ctrl[0] = next;
+  if (seen)  // there at the latest when the kernel ends
+    *static_cast<volatile unsigned long long*>(seen) =
+        static_cast<unsigned long long>(static_cast<uint32_t>(ran)) << 32 | static_cast<uint32_t>(next);
 }
 
 template <class Teleport>

@@ -56,15 +56,14 @@ struct rank_workspace {
   dbuf<float> out_stage;                // caller-id ranks before the copy to the host
   dbuf<int> ctrl;                       // device epoch control (k_epoch_control); [2], [3] k_flat_run's barrier
   double* h_delta = nullptr;  // pinned
-  int* h_ctrl = nullptr;      // pinned [8]: two control words
-  cudaEvent_t polled[2] = {nullptr, nullptr};  // control words copied to h_ctrl
+  int* h_ctrl = nullptr;      // pinned [4]
+  unsigned long long* h_seen = nullptr;  // pinned: the last epoch's decision (epoch_decide)
   bool unread_barrier = false;  // this call's k_flat_run may have given up, and the host has not looked
   push_frontier frontier;
   ~rank_workspace() {
     if (h_delta) cudaFreeHost(h_delta);
     if (h_ctrl) cudaFreeHost(h_ctrl);
-    for (cudaEvent_t e : polled)
-      if (e) cudaEventDestroy(e);
+    if (h_seen) cudaFreeHost(h_seen);
   }
 };
 
@@ -317,9 +316,8 @@ int ensure_ws(plato_graph* g, cudaStream_t st) {
   PLATO_TRY(ws->delta.alloc(1));
   PLATO_TRY(ws->ctrl.alloc(4));
   if (!ws->h_delta) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_delta), sizeof(double)));
-  if (!ws->h_ctrl) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_ctrl), 8 * sizeof(int)));
-  for (cudaEvent_t& e : ws->polled)
-    if (!e) PLATO_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  if (!ws->h_ctrl) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_ctrl), 4 * sizeof(int)));
+  if (!ws->h_seen) PLATO_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&ws->h_seen), sizeof(*ws->h_seen)));
   uint32_t cap_a = 0, cap_b = 0;
   PLATO_TRY(set_pull_smem_attr<rank_update<teleport_uniform>>(g->device, &cap_a));
   PLATO_TRY(set_pull_smem_attr<rank_update<teleport_single>>(g->device, &cap_b));
@@ -457,7 +455,7 @@ int pull_epoch_with(plato_graph* g, const float* x, const Upd& upd, const float*
   PLATO_TRY((pull_rows_with<Upd, kW>(g, x, upd, w, st)));
   if (c.ctrl) {
     k_epoch_control<<<1, 1024, 0, st>>>(ws->partials.p, static_cast<uint32_t>(partial_count(g)), c.ctrl, c.delta,
-                                        c.scale, c.eps, c.iteration);
+                                        c.scale, c.eps, c.iteration, c.seen);
     PLATO_LAUNCHED("k_epoch_control");
   }
   return PLATO_OK;
@@ -508,10 +506,14 @@ int run_flat_epochs(plato_graph* g, const Upd& upd, uint32_t iteration, uint32_t
 // Pull epochs [start, iteration); make(c, last, mode) is the update that reads
 // state c and writes state c ^ 1 (epochs alternate, *cur holds the state).  With
 // eps == 0 the schedule is known and nothing is read back.  With eps > 0 each
-// epoch ends in its decision on the device (pagerank.hpp:137-139) and the host
-// enqueues a few epochs at a time, one batch ahead of the control word it
-// reads, so the device does not wait for the host; the epochs past the final
-// one return at once.  `scale` converts the delta to the reference's units;
+// epoch ends in its decision on the device (pagerank.hpp:137-139), which the
+// device also stores in host memory, and the host keeps kAhead epochs enqueued
+// past the last decision it sees: the device does not wait for the host, and at
+// most kAhead epochs past the final one find nothing to do (2-6 us each).  Exit after
+// 2 / 7 / 13 epochs, the control word copied back every 6 epochs and read a copy
+// late / so: RMAT s14 in the caller's order 184 / 112, 344 / 245, 526 / 419 us, s18
+// with 24 edges a vertex 116 / 86, 242 / 209, 391 / 357.
+// `scale` converts the delta to the reference's units;
 // *delta keeps its value where no epoch but the final one runs, which has none.
 template <bool kW, class Make>
 int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteration, uint32_t start, double eps,
@@ -535,29 +537,29 @@ int run_pull_epochs(plato_graph* g, Make make, const float* w, uint32_t iteratio
   }
   const int init[4] = {start == iteration - 1 ? 1 : 0, static_cast<int>(start), 0, 0};
   PLATO_CUDA_TRY(cudaMemcpyAsync(ws->ctrl.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration, g->barrier_polls};
+  const flat_control c{ws->ctrl.p, ws->delta.p, scale, eps, iteration, g->barrier_polls, ws->h_seen};
   const int cur0 = *cur;
-  constexpr uint32_t kBatch = 6;
-  uint32_t launched = 0, batches = 0;
-  const int* seen = ws->h_ctrl;  // the last control word read
-  while (start + launched < iteration) {
-    const uint32_t n = std::min(kBatch, iteration - start - launched);
-    for (uint32_t k = 0; k < n; ++k, ++launched) {
-      const int p = (cur0 + static_cast<int>(launched)) & 1;
-      PLATO_TRY((pull_epoch_with<Upd, kW>(g, ws->x[p].p, make(p, false, ws->ctrl.p), w, st, c)));
+  constexpr uint32_t kAhead = 3;
+  volatile unsigned long long* seen = ws->h_seen;
+  *seen = static_cast<unsigned long long>(start) << 32 | static_cast<uint32_t>(init[0]);
+  auto decided = [&] { return static_cast<uint32_t>(*seen >> 32) - start; };
+  auto done = [&] { return static_cast<uint32_t>(*seen) == 2; };
+  for (uint32_t launched = 0; start + launched < iteration && !done();) {
+    const int p = (cur0 + static_cast<int>(launched)) & 1;
+    PLATO_TRY((pull_epoch_with<Upd, kW>(g, ws->x[p].p, make(p, false, ws->ctrl.p), w, st, c)));
+    ++launched;
+    for (uint32_t spins = 1; launched - decided() >= kAhead && !done(); ++spins) {
+      if (spins % 64) continue;
+      const cudaError_t e = cudaStreamQuery(st);  // an error ends the wait
+      if (e == cudaErrorNotReady)
+        cudaGetLastError();
+      else if (e != cudaSuccess)
+        return set_error(PLATO_ECUDA, std::string("pull epochs failed: ") + cudaGetErrorString(e));
     }
-    const uint32_t slot = batches++ & 1u;
-    PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_ctrl + 4 * slot, ws->ctrl.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    PLATO_CUDA_TRY(cudaEventRecord(ws->polled[slot], st));
-    if (batches == 1) continue;
-    PLATO_CUDA_TRY(cudaEventSynchronize(ws->polled[slot ^ 1]));
-    seen = ws->h_ctrl + 4 * (slot ^ 1);
-    if (seen[0] == 2) break;
   }
   PLATO_CUDA_TRY(cudaMemcpyAsync(ws->h_delta, ws->delta.p, sizeof(double), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  seen = ws->h_ctrl + 4 * ((batches - 1) & 1u);
-  *ran = static_cast<uint32_t>(seen[1]) - start;
+  *ran = decided();
   *cur = (cur0 + static_cast<int>(*ran)) & 1;
   if (*ran > 1) *delta = *ws->h_delta;
   return PLATO_OK;

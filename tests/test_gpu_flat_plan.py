@@ -375,3 +375,25 @@ def test_seed_sets(scale, ef, kernels, eps):
     assert abs(st.iterations - epochs) <= (1 if eps else 0)
     # the bar, and one epoch that moves less than eps where one side ends earlier
     assert np.abs(got.astype(np.float64) - want).sum() <= 1e-6 + eps
+
+
+@pytest.mark.parametrize("name", ["one launch", "separate kernels", "bins", "caller's order"])
+@pytest.mark.parametrize("iteration", [1, 2, 3, 4, 5, 9])
+def test_epochs_of_an_early_exit(name, iteration):
+    """Exits after the first epoch, in the middle and never, around the number of
+    epochs that are enqueued ahead: epochs and delta as the oracle's, ranks those
+    of as many epochs without an exit."""
+    V, s, d = {"one launch": lambda: pb.rmat(13, 16, 2), "separate kernels": lambda: pb.rmat(18, 24, 2),
+               "bins": lambda: _capped(1200001, 4), "caller's order": lambda: pb.rmat(13, 16, 2)}[name]()
+    ref = RefGraph(V, s, d, True)
+    third = ref.pagerank(4, 0.85, 1e-300)[2]
+    with pb.Graph(V, s, d, True, relabel=name != "caller's order") as g:
+        for eps in (10.0 * V, third * 1.01, 1e-300):
+            got, st = g.pagerank(iteration, 0.85, eps)
+            want, epochs, dl = ref.pagerank(iteration, 0.85, eps)
+            assert st.iterations == epochs
+            if epochs > 1:
+                assert st.delta == pytest.approx(dl, rel=1e-3)
+            assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
+            fixed, _ = g.pagerank(epochs, 0.85, 0.0)
+            assert np.abs(got.astype(np.float64) - fixed).sum() <= 2e-6
