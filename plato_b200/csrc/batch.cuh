@@ -223,7 +223,11 @@ __device__ __forceinline__ void merge_search(const uint32_t* s_rowend, int nrows
 // s_ckey, does not decrease with the group), last group first.  At kt 8 a CTA
 // has 128 groups and a hub row lies in all of them: their number is searched
 // first, so the loads overlap instead of each waiting for the key before it
-// (8 slots, RMAT s19: 13.1 -> 12.4 ms; at wider tiles the walk is the faster).
+// (8 slots, RMAT s19: 13.1 -> 12.4 ms; at wider tiles the walk is the faster), but
+// only past a few groups, where rows without hubs end (64 queries on 8M symmetrised
+// uniform edges over 1M vertices, walked / searched / searched after 4: 22.0 / 23.0 /
+// 22.1 ms).
+constexpr int kBatchWalk = 4;  // groups walked before the search
 template <int KT, int VEC>
 __device__ __forceinline__ void batch_add_groups(const uint32_t* s_ckey, const float* s_cval, int end, int row,
                                                  int lane_g, float (&y)[VEC]) {
@@ -234,7 +238,13 @@ __device__ __forceinline__ void batch_add_groups(const uint32_t* s_ckey, const f
       for (int c = 0; c < VEC; ++c) y[c] += v[g2 * KT + c];
     }
   } else {
-    int lo = 0, hi = end;
+    int g2 = end - 1;
+    for (const int walk = max(end - kBatchWalk, 0); g2 >= walk; --g2) {
+      if (s_ckey[g2] != static_cast<uint32_t>(row)) return;
+#pragma unroll
+      for (int c = 0; c < VEC; ++c) y[c] += v[g2 * KT + c];
+    }
+    int lo = 0, hi = g2 + 1;
     while (lo < hi) {
       const int m = (lo + hi) >> 1;
       if (s_ckey[m] < static_cast<uint32_t>(row))
@@ -243,7 +253,7 @@ __device__ __forceinline__ void batch_add_groups(const uint32_t* s_ckey, const f
         hi = m;
     }
 #pragma unroll 4
-    for (int g2 = end - 1; g2 >= lo; --g2) {
+    for (; g2 >= lo; --g2) {
 #pragma unroll
       for (int c = 0; c < VEC; ++c) y[c] += v[g2 * KT + c];
     }
