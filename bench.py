@@ -47,7 +47,7 @@ SCALE, EDGEFACTOR, SEED = 24, 16, 3
 ITERATIONS, DAMPING = 20, 0.85
 METRIC = "PageRank GTEPS (RMAT s24 ef16, 20 iterations, pull)"
 # kernels of one pull epoch: the flat streams (relabelled graphs), the degree bins
-# (partitions) or the merge path
+# (partitions, short rows, no room for a flat plan) or the merge path
 FLAT_KERNELS = ["k_flat_hot", "k_flat_cold", "k_flat_update", "k_flat_run"]
 PULL_KERNELS = FLAT_KERNELS + ["k_pull_long", "k_pull_rows16", "k_pull_rows8", "k_pull_rows4", "k_pull_short",
                 "k_pull_hubs", "k_pull_warp", "k_pull_warp_fixup"]

@@ -50,10 +50,10 @@ extern "C" {
 
 /* graph creation flags.  By default the engine renumbers vertices by
  * descending in-degree inside the graph (results still cross the ABI in
- * caller ids): the pull kernels then work on contiguous degree bins.
+ * caller ids): the pull kernels then work on blocks of sources or bins of rows.
  * PLATO_GRAPH_NO_RELABEL keeps the caller's order (the device view's CSC is
  * then indexed by caller ids); pull epochs on such a graph take the
- * merge-path kernel, about 2.5x slower.  PLATO_GRAPH_RELABEL asks for the
+ * merge-path kernel, 2 to 5x slower.  PLATO_GRAPH_RELABEL asks for the
  * default explicitly; both together -> PLATO_EINVAL. */
 #define PLATO_GRAPH_RELABEL    0x1u
 #define PLATO_GRAPH_NO_RELABEL 0x2u

@@ -27,9 +27,9 @@
 // flight a lane); L1 hits go at 560-790 G/s, shared memory at 1700 G/s.  RMAT
 // s24's 263M gathers are 0.95 ms of L2 requests; its hottest 57344 sources are
 // 46% of them, 24 blocks 90%.  RMAT s24, one PageRank epoch on one B200: 826 us
-// with degree bins (pull_binned.cuh), 497 us here: k_flat_hot 211 us (210M
-// edges), k_flat_cold 226 (53M), k_flat_update 82.  RMAT s22 220 -> 132 us, s20
-// 98 -> 47, 16M uniform edges over 1M vertices 107 -> 81, 64M over 1M 303 -> 135.
+// with degree bins (pull_binned.cuh), 495 us here: k_flat_hot 211 us (210M
+// edges), k_flat_cold 226 (53M), k_flat_update 82.  RMAT s22 219 -> 130 us, s20
+// 98 -> 45, 16M uniform edges over 1M vertices 107 -> 80, 64M over 1M 300 -> 132.
 #pragma once
 
 #include <utility>
@@ -352,8 +352,8 @@ __device__ __forceinline__ void flat_after() {
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
 
-// Hot streams (bound by issue: about 300 instructions a step of 512 edges, and
-// 3.4-way bank conflicts): CTA c walks its parts [cta_sub[c], cta_sub[c+1]), each within
+// Hot streams (bound by the L1/shared pipe, 78% busy at RMAT s22: 3.4-way bank
+// conflicts and the segments' stores; about 300 instructions a step of 512 edges): CTA c walks its parts [cta_sub[c], cta_sub[c+1]), each within
 // one block whose ranks it first copies to shared memory.
 template <bool kW>
 __global__ void __launch_bounds__(kFlatHotWarps * 32, 1) k_flat_hot(flat_view f, const float* __restrict__ x,

@@ -14,7 +14,7 @@
 //   trust (trustrank, :163-259)  seed-set PPR with those seeds: init 1/|S|
 //                         (divided by the out-degree) on seeds, teleport
 //                         (1-d)/|S| on seeds, eps early exit into a final
-//                         epoch -- plato_seedset_ppr on the binned pull.
+//                         epoch -- plato_seedset_ppr.
 // The selection PageRank is the reference's default run (pagerank_opts_t:
 // 100 epochs, damping 0.85, eps 0.001; pagerank.hpp:39-46, 81-146) in double
 // precision, written with the reference's functor bodies for
