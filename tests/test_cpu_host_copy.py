@@ -17,7 +17,7 @@ def lib(tmp_path_factory):
     out = tmp_path_factory.mktemp("hostcopy") / "libhostcopy.so"
     cmd = [b.nvcc()] + b.NVCC_FLAGS + ["-shared", "--cudart", "none", "-o", str(out), str(b.CSRC / "host_copy.cu"),
                                        str(b.CSRC / "errors.cpp"), str(b.ROOT / "tests/hostcopy/fake_cudart.cpp"),
-                                       "-lgomp"]
+                                       "-lgomp", "-Xlinker", "-Bsymbolic"]  # these calls, whatever else is loaded
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     lib = C.CDLL(str(out))
