@@ -28,10 +28,9 @@ namespace {
 // kFlatFirst: below, one more launch costs what the gathers save (edges that
 // would be hot, epoch without / with them: RMAT s19 6.5M 26.4 / 27.5, s20 with 10
 // a vertex 8.3M 36.1 / 37.7, s19 with 20 8.6M 31.6 / 33.1, s21 with 6 8.9M 57.5 /
-// 48.1, s20 13.9M 51.0 / 45.3).  A count that took
-// in the rows below the limits gave uniform edges with one long row streams that
-// were all but empty: 16M over 1M vertices 162 us instead of 80, 64M over 4M 378
-// instead of 288.
+// 48.1, s20 13.9M 51.0 / 45.3).  A count that took in the rows below the limits gave
+// uniform edges with one long row streams that were all but empty: 16M over 1M
+// vertices 162 us instead of 80, 64M over 4M 378 instead of 288.
 constexpr uint32_t kFlatRowDeg0 = 8;
 constexpr uint32_t kFlatRowDeg1 = 64;
 // Up to this many edges all epochs run in one launch (k_flat_run).  The line lies
@@ -73,9 +72,13 @@ bool flat_all_hot(uint64_t rows, uint64_t edges, uint64_t first_block, uint32_t 
 //   73, 16M with 2.5 / 3.5 302 / 300, 365 / 491;
 //   longer ones too: 2M with 5 66.1 / 69.4, 4M with 5 / 6 121 / 118, 133 / 136, 8M
 //   with 5 234 / 221; RMAT s22 with 4.4 29.9 / 92.5 (half of the edges in them).
+// With weights the bins' rows above 4 edges fall behind sooner (40 epochs: 1M rows
+// with 2.5 / 3.6 edges 1.32 / 1.36, 1.57 / 1.77 ms, 2M with 2.5 2.37 / 2.11, 4M with
+// 2.5 / 5 4.24 / 3.85, 5.89 / 7.31).
 struct flat_census {
   uint64_t rows, few, some;      // all rows, rows of 1..4 and of 5..16 edges
   uint64_t edges, long_edges;    // all edges, those in rows above 16
+  bool weighted;
 };
 enum class flat_use { always, early_exit, never };
 flat_use flat_suits(const flat_census& c, bool run) {
@@ -85,9 +88,9 @@ flat_use flat_suits(const flat_census& c, bool run) {
   if (c.rows > 10000000 && 2 * c.edges > 5 * c.rows)
     bins = false;
   else if (c.long_edges == 0)
-    bins = (c.few + c.some >= 900000 && c.edges >= 2500000) || c.rows >= 6000000;
+    bins = (c.few + c.some >= (c.weighted ? 1500000 : 900000) && c.edges >= 2500000) || c.rows >= 6000000;
   else
-    bins = 20 * c.long_edges <= c.edges && c.edges <= 6 * c.rows && c.few + c.some >= 2500000;
+    bins = !c.weighted && 20 * c.long_edges <= c.edges && c.edges <= 6 * c.rows && c.few + c.some >= 2500000;
   return bins ? flat_use::never : flat_use::always;
 }
 
@@ -454,7 +457,7 @@ int build_flat_plan(plato_graph* g, flat_plan& pl, cudaStream_t st) {
   unsigned long long h[kFlatSurvey + kFlatMaxBlocks];
   PLATO_CUDA_TRY(cudaMemcpyAsync(h, d_survey.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   PLATO_CUDA_TRY(cudaStreamSynchronize(st));
-  const flat_use use = flat_suits(flat_census{V, h[2], h[3], E, h[4]}, run);
+  const flat_use use = flat_suits(flat_census{V, h[2], h[3], E, h[4], weighted}, run);
   if (use == flat_use::never) return PLATO_OK;
   pl.early_only = use == flat_use::early_exit;
   flat_rows rows{off, g->in_adj.p, V, 0, 0, kFlatRowDeg0, kFlatRowDeg1};

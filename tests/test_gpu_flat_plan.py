@@ -397,3 +397,21 @@ def test_epochs_of_an_early_exit(name, iteration):
             assert np.abs(got.astype(np.float64) - want / V).sum() <= 1e-6
             fixed, _ = g.pagerank(epochs, 0.85, 0.0)
             assert np.abs(got.astype(np.float64) - fixed).sum() <= 2e-6
+
+
+@pytest.mark.parametrize("graph,kernels", [
+    (_ring(100003), ONE), (_uniform(1000003, 2600000), RUN), (_uniform(2000003, 5000000), TWO),
+    (_uniform(1000003, 3600000), COLD), (_uniform(4000037, 20000000), COLD), (_capped(1200001, 4), ONE)])
+def test_short_rows_with_weights(graph, kernels):
+    """The same rule with weights, whose limits lie higher; a fixed number of
+    epochs and an early exit, against the oracle's bar."""
+    V, s, d = graph
+    w = np.random.default_rng(V).uniform(0.1, 10, s.size)
+    want, _, _ = fp64.weighted_pagerank(V, s, d, w, True, 6, 0.85, 0.0)
+    with pb.Graph(V, s, d, True, weights=w) as g:
+        hit, (got, _) = _launched(lambda: g.weighted_pagerank(6, 0.85, 0.0), KERNELS)
+        early, st = g.weighted_pagerank(6, 0.85, 1e-300)
+    assert hit == kernels and 2 <= st.iterations <= 6  # the ring's ranks stand still, to the last bit
+    assert np.nansum(np.abs(got - want)) / V <= 1e-6
+    assert np.nansum(np.abs(early - want)) / V <= 1e-6
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
